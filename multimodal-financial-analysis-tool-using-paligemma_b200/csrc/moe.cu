@@ -35,33 +35,11 @@ __device__ __forceinline__ float dot_smem(const float* __restrict__ hs, const T*
   return warp_sum(acc);
 }
 
+// One warp: softmax over a token's logits s[0 .. n_route), the `top` largest of score + correction, weights = score * scale.
 template <typename T>
-__global__ void moe_route_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
-                                 float* __restrict__ shared_gate, const T* __restrict__ h, int ldh,
-                                 const T* __restrict__ w_router, const T* __restrict__ correction,
-                                 const T* __restrict__ w_sg, int T_, int D, int n_route, int top, float scale) {
-  extern __shared__ float smem[];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int t = blockIdx.x;
-  float* hs = smem;                               // [D]
-  float* s = smem + D;                            // scores [n_route]
-  float* c = s + n_route;                         // choice scores [n_route]
-  const T* hr = h + (size_t)t * ldh;
-  for (int k = threadIdx.x; k < D; k += blockDim.x) hs[k] = to_f<T>(hr[k]);
-  __syncthreads();
-  for (int e = warp; e < n_route + 1; e += warps) {
-    if (e < n_route) {
-      const float z = dot_smem<T>(hs, w_router + (size_t)e * D, D, lane);
-      if (lane == 0) s[e] = z;
-    } else if (w_sg && shared_gate) {
-      const float z = dot_smem<T>(hs, w_sg, D, lane);
-      if (lane == 0) shared_gate[t] = 1.f / (1.f + expf(-z));
-    }
-  }
-  __syncthreads();
-  if (warp != 0) return;
+__device__ __forceinline__ void route_softmax_pick(float* __restrict__ s, float* __restrict__ c, const T* __restrict__ correction,
+                                                   int32_t* __restrict__ topk_idx, float* __restrict__ topk_w, size_t t, int n_route,
+                                                   int top, float scale, int lane) {
   float mx = -INFINITY;
   for (int e = lane; e < n_route; e += 32) mx = fmaxf(mx, s[e]);
   mx = warp_max(mx);
@@ -96,39 +74,11 @@ __global__ void moe_route_kernel(int32_t* __restrict__ topk_idx, float* __restri
   }
 }
 
-// ------------------------------------------------------------------ router with sigmoid scores and expert groups: one CTA per token
-// z = h W_router^T in fp32, s = sigmoid(z); the choice scores are c = s + correction.  The experts form n_groups equal
-// groups of neighbours; a group's score is the sum of its two largest choice scores (of the one, for groups of one),
-// and only the experts of the `keep` best groups can be chosen (the others' choice scores count as -inf).  The `top`
-// largest choice scores are chosen (ties: lowest index); the weights are the chosen s (without the correction)
-// divided by their sum + 1e-20.
+// One warp: the choice among a token's sigmoid scores s and choice scores c (experts in groups), as described below.
 template <typename T>
-__global__ void moe_route_grouped_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
-                                         const T* __restrict__ h, int ldh, const T* __restrict__ w_router,
-                                         const T* __restrict__ correction, int T_, int D, int n_route, int top,
-                                         int n_groups, int keep) {
-  extern __shared__ float smem[];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int t = blockIdx.x;
-  float* hs = smem;                               // [D]
-  float* s = smem + D;                            // scores [n_route]
-  float* c = s + n_route;                         // choice scores [n_route]
-  float* gs = c + n_route;                        // group scores [n_groups]
-  const T* hr = h + (size_t)t * ldh;
-  for (int k = threadIdx.x; k < D; k += blockDim.x) hs[k] = to_f<T>(hr[k]);
-  __syncthreads();
-  for (int e = warp; e < n_route; e += warps) {
-    const float z = dot_smem<T>(hs, w_router + (size_t)e * D, D, lane);
-    if (lane == 0) {
-      const float sc = 1.f / (1.f + expf(-z));
-      s[e] = sc;
-      c[e] = sc + (correction ? to_f<T>(correction[e]) : 0.f);
-    }
-  }
-  __syncthreads();
-  if (warp != 0) return;
+__device__ __forceinline__ void route_grouped_pick(float* __restrict__ s, float* __restrict__ c, float* __restrict__ gs,
+                                                   int32_t* __restrict__ topk_idx, float* __restrict__ topk_w, size_t t, int n_route,
+                                                   int top, int n_groups, int keep, int lane) {
   if (n_groups > 1 && keep < n_groups) {
     const int gsz = n_route / n_groups;
     for (int g = lane; g < n_groups; g += 32) {
@@ -186,6 +136,170 @@ __global__ void moe_route_grouped_kernel(int32_t* __restrict__ topk_idx, float* 
   }
   const float inv = 1.f / (wsum + 1e-20f);
   for (int k = lane; k < top; k += 32) topk_w[(size_t)t * top + k] *= inv;
+}
+
+template <typename T>
+__global__ void moe_route_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
+                                 float* __restrict__ shared_gate, const T* __restrict__ h, int ldh,
+                                 const T* __restrict__ w_router, const T* __restrict__ correction,
+                                 const T* __restrict__ w_sg, int T_, int D, int n_route, int top, float scale) {
+  extern __shared__ float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int t = blockIdx.x;
+  float* hs = smem;                               // [D]
+  float* s = smem + D;                            // scores [n_route]
+  float* c = s + n_route;                         // choice scores [n_route]
+  const T* hr = h + (size_t)t * ldh;
+  for (int k = threadIdx.x; k < D; k += blockDim.x) hs[k] = to_f<T>(hr[k]);
+  __syncthreads();
+  for (int e = warp; e < n_route + 1; e += warps) {
+    if (e < n_route) {
+      const float z = dot_smem<T>(hs, w_router + (size_t)e * D, D, lane);
+      if (lane == 0) s[e] = z;
+    } else if (w_sg && shared_gate) {
+      const float z = dot_smem<T>(hs, w_sg, D, lane);
+      if (lane == 0) shared_gate[t] = 1.f / (1.f + expf(-z));
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  route_softmax_pick<T>(s, c, correction, topk_idx, topk_w, (size_t)t, n_route, top, scale, lane);
+}
+
+// ------------------------------------------------------------------ router with sigmoid scores and expert groups: one CTA per token
+// z = h W_router^T in fp32, s = sigmoid(z); the choice scores are c = s + correction.  The experts form n_groups equal
+// groups of neighbours; a group's score is the sum of its two largest choice scores (of the one, for groups of one),
+// and only the experts of the `keep` best groups can be chosen (the others' choice scores count as -inf).  The `top`
+// largest choice scores are chosen (ties: lowest index); the weights are the chosen s (without the correction)
+// divided by their sum + 1e-20.
+template <typename T>
+__global__ void moe_route_grouped_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
+                                         const T* __restrict__ h, int ldh, const T* __restrict__ w_router,
+                                         const T* __restrict__ correction, int T_, int D, int n_route, int top,
+                                         int n_groups, int keep) {
+  extern __shared__ float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int t = blockIdx.x;
+  float* hs = smem;                               // [D]
+  float* s = smem + D;                            // scores [n_route]
+  float* c = s + n_route;                         // choice scores [n_route]
+  float* gs = c + n_route;                        // group scores [n_groups]
+  const T* hr = h + (size_t)t * ldh;
+  for (int k = threadIdx.x; k < D; k += blockDim.x) hs[k] = to_f<T>(hr[k]);
+  __syncthreads();
+  for (int e = warp; e < n_route; e += warps) {
+    const float z = dot_smem<T>(hs, w_router + (size_t)e * D, D, lane);
+    if (lane == 0) {
+      const float sc = 1.f / (1.f + expf(-z));
+      s[e] = sc;
+      c[e] = sc + (correction ? to_f<T>(correction[e]) : 0.f);
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  route_grouped_pick<T>(s, c, gs, topk_idx, topk_w, (size_t)t, n_route, top, n_groups, keep, lane);
+}
+
+// ------------------------------------------------------------------ both routers over many tokens
+// A CTA per token reads the whole router matrix for one row (8192 tokens x 16 experts x 2048 columns: 133 us, the router rows
+// out of L1 / L2 once per token).  Here a warp takes RT_TOK tokens and RT_E router rows at a time: a 16-byte load of a router
+// row feeds RT_TOK * 8 FMAs out of registers, the RT_TOK * RT_E = 32 lane partials meet in a transposed butterfly (31 shuffles
+// leave lane L with the sum of pair L).  All loads of a step go out together (with a branch per router row in front of its
+// load the same size took 82 us): that size runs in 36 us.  Products and sums stay fp32.
+constexpr int RT_TOK = 4, RT_E = 8, RT_WARPS = 4;
+
+template <typename T, bool GROUPED>
+__global__ void __launch_bounds__(RT_WARPS * 32)
+moe_route_tile_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w, float* __restrict__ shared_gate,
+                      const T* __restrict__ h, int ldh, const T* __restrict__ w_router, const T* __restrict__ correction,
+                      const T* __restrict__ w_sg, int n_tokens, int D, int n_route, int top, float scale, int n_groups, int keep) {
+  extern __shared__ float smem[];
+  constexpr int V = Vec<T>::N;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = (blockIdx.x * RT_WARPS + warp) * RT_TOK;
+  if (t0 >= n_tokens) return;                     // nothing below waits for another warp
+  const int nt = min(RT_TOK, n_tokens - t0);
+  const int per_tok = 2 * n_route + (GROUPED ? n_groups : 0);
+  float* st = smem + (size_t)warp * RT_TOK * per_tok;      // per token: scores, choice scores (, group scores)
+  const T* hr[RT_TOK];
+#pragma unroll
+  for (int i = 0; i < RT_TOK; ++i) hr[i] = h + (size_t)(t0 + min(i, nt - 1)) * ldh;
+  const int rows = n_route + (!GROUPED && w_sg && shared_gate ? 1 : 0);
+  for (int e0 = 0; e0 < rows; e0 += RT_E) {
+    float acc[RT_TOK * RT_E];
+#pragma unroll
+    for (int i = 0; i < RT_TOK * RT_E; ++i) acc[i] = 0.f;
+    const T* wr[RT_E];                            // rows behind the last one repeat it; nobody reads their sums
+#pragma unroll
+    for (int e = 0; e < RT_E; ++e) {
+      const int r = min(e0 + e, rows - 1);
+      wr[e] = r < n_route ? w_router + (size_t)r * D : w_sg;
+    }
+    for (int k = lane * V; k < D; k += 32 * V) {
+      uint4 xv[RT_TOK], wv[RT_E];                 // all loads of the step in flight together
+#pragma unroll
+      for (int i = 0; i < RT_TOK; ++i) xv[i] = ldg_cached(hr[i] + k);
+#pragma unroll
+      for (int e = 0; e < RT_E; ++e) wv[e] = ldg_cached(wr[e] + k);
+      float x[RT_TOK][V];
+#pragma unroll
+      for (int i = 0; i < RT_TOK; ++i) unpack<T>(xv[i], x[i]);
+#pragma unroll
+      for (int e = 0; e < RT_E; ++e) {
+        float f[V];
+        unpack<T>(wv[e], f);
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+          for (int i = 0; i < RT_TOK; ++i) acc[i * RT_E + e] = fmaf(x[i][v], f[v], acc[i * RT_E + e]);
+      }
+    }
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+      const bool up = (lane & w) != 0;
+#pragma unroll
+      for (int i = 0; i < w; ++i) {
+        const float keep_v = up ? acc[i + w] : acc[i];
+        const float send = up ? acc[i] : acc[i + w];
+        acc[i] = keep_v + __shfl_xor_sync(0xffffffffu, send, w);
+      }
+    }
+    const int i = lane / RT_E, e = e0 + lane % RT_E;
+    const float z = acc[0];
+    if (i < nt && e < n_route) {
+      float* s = st + i * per_tok;
+      if (GROUPED) {
+        const float sc = 1.f / (1.f + expf(-z));
+        s[e] = sc;
+        s[n_route + e] = sc + (correction ? to_f<T>(correction[e]) : 0.f);
+      } else {
+        s[e] = z;
+      }
+    } else if (i < nt && e == n_route && e < rows) {
+      shared_gate[t0 + i] = 1.f / (1.f + expf(-z));
+    }
+  }
+  __syncwarp();
+  for (int i = 0; i < nt; ++i) {
+    float* s = st + i * per_tok;
+    if (GROUPED) route_grouped_pick<T>(s, s + n_route, s + 2 * n_route, topk_idx, topk_w, (size_t)(t0 + i), n_route, top, n_groups, keep, lane);
+    else route_softmax_pick<T>(s, s + n_route, correction, topk_idx, topk_w, (size_t)(t0 + i), n_route, top, scale, lane);
+  }
+}
+
+// The tile kernel takes 16-byte loads of both operands and pays from the token count on at which its warps fill the chip;
+// below that a CTA per token, a warp per routed output, has the shorter chain (8 tokens in one go there).
+template <typename T>
+static bool route_tile_wanted(const void* h, int ldh, const void* w_router, const void* w_sg, int n_tokens, int D, size_t smem) {
+  constexpr int V = Vec<T>::N;
+  return n_tokens >= 512 && D % V == 0 && ldh % V == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(w_router) & 15) == 0 && (reinterpret_cast<uintptr_t>(w_sg) & 15) == 0 && smem <= 96 * 1024;
 }
 
 // ------------------------------------------------------------------ router whose weights are a softmax over the chosen logits
@@ -521,6 +635,67 @@ __global__ void moe_combine_kernel(float* __restrict__ x, T* __restrict__ out, i
   }
 }
 
+// 16 bytes of a row per thread, the rows of a token's experts requested COMBINE_K at a time: 8192 tokens x 2 rows x 2048
+// columns in 23 us, near the copy rate (an element per thread and load: 55 us).  Sums run in the order of k.
+constexpr int COMBINE_K = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(float* __restrict__ x, T* __restrict__ out, int ldo, const T* __restrict__ y, int ldy,
+                       const int32_t* __restrict__ pair_pos, const float* __restrict__ topk_w, const T* __restrict__ h, int ldh,
+                       const T* __restrict__ shared_out, int lds, const float* __restrict__ shared_gate, int D, int top) {
+  constexpr int V = Vec<T>::N;
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t t = blockIdx.x;
+  const float sg = shared_out && shared_gate ? shared_gate[t] : 1.f;
+  for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
+    float acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = 0.f;
+    uint4 so = make_uint4(0, 0, 0, 0);
+    if (shared_out) so = ldg_cached(shared_out + t * lds + c);
+    for (int k0 = 0; k0 < top; k0 += COMBINE_K) {
+      uint4 r[COMBINE_K];
+      float w[COMBINE_K];
+#pragma unroll
+      for (int k = 0; k < COMBINE_K; ++k) {
+        if (k0 + k < top) {
+          const int pos = pair_pos[t * top + k0 + k];
+          w[k] = topk_w[t * top + k0 + k];
+          r[k] = ldg_cached(pos >= 0 ? y + (size_t)pos * ldy + c : h + t * ldh + c);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < COMBINE_K; ++k) {
+        if (k0 + k < top) {
+          float f[V];
+          unpack<T>(r[k], f);
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[i] = fmaf(w[k], f[i], acc[i]);
+        }
+      }
+    }
+    if (shared_out) {
+      float f[V];
+      unpack<T>(so, f);
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = fmaf(sg, f[i], acc[i]);
+    }
+    if (out) {
+      *reinterpret_cast<uint4*>(out + t * ldo + c) = pack<T>(acc);
+    } else {
+      float4* xr = reinterpret_cast<float4*>(x + t * D + c);
+#pragma unroll
+      for (int i = 0; i < V; i += 4) {
+        float4 v = xr[i / 4];
+        v.x += acc[i]; v.y += acc[i + 1]; v.z += acc[i + 2]; v.w += acc[i + 3];
+        xr[i / 4] = v;
+      }
+    }
+  }
+}
+
 // rows of the grouped order: out[pos] = a[row_map[pos]] (16-byte copies when the rows allow, else elements)
 template <typename T>
 __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ a, int lda,
@@ -554,10 +729,15 @@ extern "C" int pg_moe_route(int32_t* topk_idx, float* topk_w, float* shared_gate
                             int D, int n_route, int top, float scale, int dtype, void* stream) {
   if (n_tokens <= 0) return PG_OK;
   PG_REQUIRE(top >= 1 && top <= n_route && n_route <= 4096, "moe_route: top %d of %d routed outputs", top, n_route);
-  const int warps = n_route + 1 < 8 ? 4 : 8;
+  const int warps = n_route + 1 < 4 ? 4 : (n_route + 1 < 32 ? n_route + 1 : 32);   // a warp per routed output: one short chain
   const size_t smem = sizeof(float) * ((size_t)D + 2 * (size_t)n_route);
   PG_REQUIRE(smem <= 200 * 1024, "moe_route: D=%d with %d routed outputs does not fit shared memory", D, n_route);
   PG_DISPATCH_DTYPE(dtype, T, {
+    const size_t tile_smem = sizeof(float) * (size_t)RT_WARPS * RT_TOK * 2 * n_route;
+    if (route_tile_wanted<T>(h, ldh, w_router, w_shared_gate, n_tokens, D, tile_smem))
+      return launch_pdl("moe_route", moe_route_tile_kernel<T, false>, dim3(cdiv(n_tokens, RT_WARPS * RT_TOK)), dim3(RT_WARPS * 32),
+                        tile_smem, (cudaStream_t)stream, topk_idx, topk_w, shared_gate, (const T*)h, ldh, (const T*)w_router,
+                        (const T*)correction, (const T*)w_shared_gate, n_tokens, D, n_route, top, scale, 1, 1);
     auto kern = moe_route_kernel<T>;
     return launch_pdl("moe_route", kern, dim3(n_tokens), dim3(warps * 32), smem, (cudaStream_t)stream, topk_idx, topk_w,
                       shared_gate, (const T*)h, ldh, (const T*)w_router, (const T*)correction, (const T*)w_shared_gate,
@@ -620,10 +800,15 @@ extern "C" int pg_moe_route_grouped(int32_t* topk_idx, float* topk_w, const void
   PG_REQUIRE(n_groups >= 1 && n_route % n_groups == 0 && keep >= 1 && keep <= n_groups &&
                  (long long)keep * (n_route / n_groups) >= top,
              "moe_route: %d groups over %d experts, %d kept, top %d", n_groups, n_route, keep, top);
-  const int warps = n_route < 8 ? 4 : 8;
+  const int warps = n_route < 4 ? 4 : (n_route < 32 ? n_route : 32);   // a warp per routed output: one short chain
   const size_t smem = sizeof(float) * ((size_t)D + 2 * (size_t)n_route + n_groups);
   PG_REQUIRE(smem <= 200 * 1024, "moe_route: D=%d with %d routed outputs does not fit shared memory", D, n_route);
   PG_DISPATCH_DTYPE(dtype, T, {
+    const size_t tile_smem = sizeof(float) * (size_t)RT_WARPS * RT_TOK * (2 * n_route + n_groups);
+    if (route_tile_wanted<T>(h, ldh, w_router, nullptr, n_tokens, D, tile_smem))
+      return launch_pdl("moe_route_grouped", moe_route_tile_kernel<T, true>, dim3(cdiv(n_tokens, RT_WARPS * RT_TOK)),
+                        dim3(RT_WARPS * 32), tile_smem, (cudaStream_t)stream, topk_idx, topk_w, (float*)nullptr, (const T*)h, ldh,
+                        (const T*)w_router, (const T*)correction, (const T*)nullptr, n_tokens, D, n_route, top, 1.f, n_groups, keep);
     auto kern = moe_route_grouped_kernel<T>;
     return launch_pdl("moe_route_grouped", kern, dim3(n_tokens), dim3(warps * 32), smem, (cudaStream_t)stream, topk_idx,
                       topk_w, (const T*)h, ldh, (const T*)w_router, (const T*)correction, n_tokens, D, n_route, top,
@@ -654,7 +839,15 @@ static int moe_combine_any(float* x, void* out, int ldo, const void* y, int ldy,
                            const float* topk_w, const void* h, int ldh, const void* shared_out, int lds,
                            const float* shared_gate, int n_tokens, int D, int top, int dtype, void* stream) {
   if (n_tokens <= 0) return PG_OK;
+  auto fits = [](const void* p, long long ld, int vec) { return !p || (((uintptr_t)p & 15) == 0 && ld % vec == 0); };
   PG_DISPATCH_DTYPE(dtype, T, {
+    constexpr int V = Vec<T>::N;
+    if (D % V == 0 && fits(x, D, 4) && fits(out, ldo, V) && fits(y, ldy, V) && fits(h, ldh, V) && fits(shared_out, lds, V)) {
+      const int vecs = D / V, threads = vecs >= 256 ? 256 : (vecs + 31) / 32 * 32;
+      return launch_pdl("moe_combine", moe_combine_vec_kernel<T>, dim3(n_tokens), dim3(threads), 0, (cudaStream_t)stream, x,
+                        (T*)out, ldo, (const T*)y, ldy, pair_pos, topk_w, (const T*)h, ldh, (const T*)shared_out, lds,
+                        shared_gate, D, top);
+    }
     const int threads = n_tokens <= 64 ? (D >= 2048 ? 512 : 256) : 128;
     return launch_pdl("moe_combine", moe_combine_kernel<T>, dim3(n_tokens), dim3(threads), 0, (cudaStream_t)stream, x,
                       (T*)out, ldo, (const T*)y, ldy, pair_pos, topk_w, (const T*)h, ldh, (const T*)shared_out, lds,
