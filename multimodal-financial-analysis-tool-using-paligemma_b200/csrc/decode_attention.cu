@@ -9,10 +9,13 @@
 // registers, the warps of a CTA merge through shared memory and the CTAs of the cluster merge
 // through distributed shared memory — no global workspace, no atomics, one launch.
 // Work is tiny (T*1 KB per layer); the design goal is latency, not bandwidth.
+//
+// 16-bit models with head_dim 256 and up to 8 query heads per KV head take decode_attention_mma_kernel instead (below).
 #include <cmath>
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "mma_frag.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -291,6 +294,12 @@ decode_attention_cluster_kernel(T* __restrict__ out, const T* __restrict__ q, co
   cluster.sync();  // nobody leaves while a peer may still read its shared memory
 }
 
+// x / 2^k == x * 2^-k exactly (no underflow at these magnitudes): skip the IEEE division routine
+static float exact_reciprocal(float scale_div) {
+  int ex = 0;
+  return (frexpf(scale_div, &ex) == 0.5f) ? 1.0f / scale_div : 0.f;
+}
+
 template <typename T, int G, int NCH, int DC_NS>
 static int launch_da_ns(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table,
                      int pt_stride, int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv,
@@ -298,9 +307,7 @@ static int launch_da_ns(void* out, const void* q, const void* k_pool, const void
   constexpr int TB = NCH == 1 ? 4 : 2;
   auto kern = decode_attention_cluster_kernel<T, G, NCH, TB, DC_NS>;
   if (DC_NS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  // x / 2^k == x * 2^-k exactly (no underflow at these magnitudes): skip the IEEE division routine
-  int ex = 0;
-  const float scale_mul = (frexpf(scale_div, &ex) == 0.5f) ? 1.0f / scale_div : 0.f;
+  const float scale_mul = exact_reciprocal(scale_div);
   const size_t smem = ((size_t)DC_WARPS * G * hd + 2 * DC_WARPS * G + (size_t)G * hd + 2 * G) * sizeof(float);
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -358,6 +365,246 @@ static int launch_da(void* out, const void* q, const void* k_pool, const void* v
 #undef PG_DA_NS
 }
 
+// ------------------------------------------------------------------------------------------------ head_dim 256 on mma.sync
+// The kernel above is bound by its chain, not by bytes: 255 registers x 256 threads fill an SM, so a cluster of 16 CTAs needs 16
+// free SMs of one GPC (8 sequences do not fit at once: 1345 cached tokens took 39.7 us for 11 MB), and every token costs a
+// warp 8 x 16 FMAs plus a 31-shuffle butterfly.  Here the 8 query heads are the N dimension of mma.m16n8k16:
+//   S^T [16 tokens x 8 heads] = K Q^T     A = 16 key rows,   B = the query rows
+//   O^T [256 dims x 8 heads] += V^T P^T   A = V transposed,  B = the weights
+// A warp takes 16 tokens at a time and all operands go from global memory straight into fragments with 16-byte loads: the
+// contraction index of S^T is permuted (lane j of a quad owns 8 consecutive columns of every 32) and so are the rows of O^T
+// (lane group r owns 8 consecutive columns of every 64), which neither product notices.  The weights stay fp32: they enter
+// as three 16-bit terms (8 + 8 + 8 mantissa bits in bf16), so that P V is the fp32 product; only QK^T's operands are 16-bit,
+// as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
+// Measured (launch alone, cold cache): 1 sequence x 262 tokens 13.5 -> 9.5 us, 8 x 1345 39.7 -> 14.2 us, 32 x 389 23.6 -> 12.1 us;
+// inside the captured step 4.0, 23 and 5.1 us per layer less.
+constexpr int DM_WARPS = 4, DM_HD = 256, DM_G = 8;
+
+template <typename T, int NS>
+__global__ void __launch_bounds__(DM_WARPS * 32, 2)
+decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_pool,
+                            const T* __restrict__ v_pool, const int32_t* __restrict__ page_table, int pt_stride, int page_size,
+                            const int32_t* __restrict__ kv_len, int kv_len_add, int nq, int nkv, float scale_div,
+                            float scale_mul, Prefetch pf) {
+  constexpr int KB = DM_HD / 32, VB = DM_HD / 64;
+  cg::cluster_group cluster = cg::this_cluster();
+  pdl_launch_dependents();
+  l2_prefetch_slice(pf);
+  const int rank = (int)cluster.block_rank(), b = blockIdx.y, kvh = blockIdx.z, G = nq / nkv;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, r = lane >> 2, j = lane & 3;
+  __shared__ __align__(16) float s_acc[DM_WARPS][DM_G][DM_HD];
+  __shared__ __align__(16) float c_acc[DM_G][DM_HD];      // CTA-level partial (read by peers)
+  __shared__ float s_m[DM_WARPS][DM_G], s_l[DM_WARPS][DM_G], c_m[DM_G], c_l[DM_G];
+  __shared__ int s_pt[DC_MAX_PT];
+  pdl_wait();  // q and this step's K/V row come from the preceding qkv kernel
+
+  // the length, the page-table row and the query rows are requested together
+  const int T_len = kv_len[b] + kv_len_add;
+  const int32_t* pt = page_table + (size_t)b * pt_stride;
+  const int pt_n = min(pt_stride, DC_MAX_PT);
+  for (int i = threadIdx.x; i < pt_n; i += DM_WARPS * 32) s_pt[i] = pt[i];
+  uint4 qf[KB];
+  {
+    const T* qr = q + ((size_t)b * nq + (size_t)kvh * G + r) * DM_HD + j * 8;
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) qf[kb] = r < G ? ldg_cached(qr + kb * 32) : make_uint4(0, 0, 0, 0);
+  }
+  float acc[VB][4][4];
+#pragma unroll
+  for (int vb = 0; vb < VB; ++vb)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // heads 2j and 2j + 1, the same in every lane group
+  __syncthreads();
+
+  const int chunks = (T_len + 15) / 16;
+  const size_t row_elems = (size_t)nkv * DM_HD;
+  // chunk c: CTA c % NS first, so that a short context spreads over the SMs before it stacks up in one
+  for (int c = rank + NS * wid; c < chunks; c += NS * DM_WARPS) {
+    const int t0 = c * 16, pi = t0 / page_size;               // page_size is a multiple of 16: one page per chunk
+    const int page = pi < pt_n ? s_pt[pi] : pt[pi];
+    const size_t base = ((size_t)page * page_size + t0 % page_size) * row_elems + (size_t)kvh * DM_HD;
+    const int last = T_len - 1 - t0;                          // rows behind the last token repeat it with weight 0
+    const T* kp = k_pool + base + j * 8;
+    const T* vp = v_pool + base + r * 8;
+    const size_t k0 = (size_t)min(r, last) * row_elems, k1 = (size_t)min(r + 8, last) * row_elems;
+    const size_t v0 = (size_t)min(2 * j, last) * row_elems, v1 = (size_t)min(2 * j + 1, last) * row_elems;
+    const size_t v2 = (size_t)min(2 * j + 8, last) * row_elems, v3 = (size_t)min(2 * j + 9, last) * row_elems;
+    uint4 ka[KB], kc[KB], va[VB][4];
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) { ka[kb] = ldg_cached(kp + k0 + kb * 32); kc[kb] = ldg_cached(kp + k1 + kb * 32); }
+#pragma unroll
+    for (int vb = 0; vb < VB; ++vb) {
+      va[vb][0] = ldg_cached(vp + v0 + vb * 64); va[vb][1] = ldg_cached(vp + v1 + vb * 64);
+      va[vb][2] = ldg_cached(vp + v2 + vb * 64); va[vb][3] = ldg_cached(vp + v3 + vb * 64);
+    }
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) {
+      mma_16816<T>(s0, ka[kb].x, kc[kb].x, ka[kb].y, kc[kb].y, qf[kb].x, qf[kb].y);
+      mma_16816<T>(s1, ka[kb].z, kc[kb].z, ka[kb].w, kc[kb].w, qf[kb].z, qf[kb].w);
+    }
+    // s[0], s[1]: token r, heads 2j, 2j + 1;  s[2], s[3]: token r + 8
+    float p[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      // matmul output rounded to the model dtype, then "/ sqrt(head_dim)" (modeling_gemma.py:266); a power-of-two divisor is
+      // applied as an exact multiply
+      const float sr = rnd<T>(s0[e] + s1[e]);
+      const float sc = (scale_mul != 0.f) ? sr * scale_mul : rnd<T>(sr / scale_div);
+      p[e] = (e < 2 ? r : r + 8) <= last ? sc : -INFINITY;
+    }
+    float corr[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mx = fmaxf(p[h], p[h + 2]);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float mn = fmaxf(m[h], mx);
+      corr[h] = __expf(m[h] - mn);
+      m[h] = mn;
+      p[h] = __expf(p[h] - mn);
+      p[h + 2] = __expf(p[h + 2] - mn);
+      l[h] = l[h] * corr[h] + (p[h] + p[h + 2]);              // this lane's tokens; the lanes meet at the end
+    }
+    uint32_t pb[3][2];                                        // three 16-bit terms of the weights, as B fragments
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      pb[n][0] = transpose_8x8(split_pair<T>(p[0], p[1]));
+      pb[n][1] = transpose_8x8(split_pair<T>(p[2], p[3]));
+    }
+#pragma unroll
+    for (int vb = 0; vb < VB; ++vb) {
+      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&va[vb][0]);
+      const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&va[vb][1]);
+      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&va[vb][2]);
+      const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&va[vb][3]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // rows r and r + 8 of this product: columns 64 vb + 8 r + 2 i and + 1
+        const uint32_t a0 = __byte_perm(w0[i], w1[i], 0x5410), a1 = __byte_perm(w0[i], w1[i], 0x7632);
+        const uint32_t a2 = __byte_perm(w2[i], w3[i], 0x5410), a3 = __byte_perm(w2[i], w3[i], 0x7632);
+        float (&o)[4] = acc[vb][i];
+        o[0] *= corr[0]; o[1] *= corr[1]; o[2] *= corr[0]; o[3] *= corr[1];
+#pragma unroll
+        for (int n = 0; n < 3; ++n) mma_16816<T>(o, a0, a1, a2, a3, pb[n][0], pb[n][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], o);
+
+  // ---- merge the warps of this CTA (those that met a chunk)
+  const int busy = min(DM_WARPS, (max(0, chunks - rank) + NS - 1) / NS);
+  if (wid < busy) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (r == 0) { s_m[wid][2 * j + h] = m[h]; s_l[wid][2 * j + h] = l[h]; }
+#pragma unroll
+      for (int vb = 0; vb < VB; ++vb) {
+        float4* dst = reinterpret_cast<float4*>(&s_acc[wid][2 * j + h][vb * 64 + r * 8]);
+        dst[0] = make_float4(acc[vb][0][h], acc[vb][0][h + 2], acc[vb][1][h], acc[vb][1][h + 2]);
+        dst[1] = make_float4(acc[vb][2][h], acc[vb][2][h + 2], acc[vb][3][h], acc[vb][3][h + 2]);
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x * 4; e < G * DM_HD; e += DM_WARPS * 32 * 4) {
+    const int g = e / DM_HD, d = e % DM_HD;
+    float M = -INFINITY;
+    for (int w = 0; w < busy; ++w) M = fmaxf(M, s_m[w][g]);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float L = 0.f;
+    for (int w = 0; w < busy; ++w) {
+      const float f = __expf(s_m[w][g] - M);
+      const float4 v = *reinterpret_cast<const float4*>(&s_acc[w][g][d]);
+      a.x = fmaf(f, v.x, a.x); a.y = fmaf(f, v.y, a.y); a.z = fmaf(f, v.z, a.z); a.w = fmaf(f, v.w, a.w);
+      L = fmaf(f, s_l[w][g], L);
+    }
+    *reinterpret_cast<float4*>(&c_acc[g][d]) = a;
+    if (d == 0) { c_m[g] = M; c_l[g] = L; }
+  }
+  cluster.sync();  // every CTA's partial is visible cluster-wide
+
+  // ---- merge the CTAs that met a chunk: CTA `rank` finalises its slice of the G * 256 outputs through DSMEM
+  const int n_cta = min(NS, chunks);
+  const int per = (G * DM_HD + NS - 1) / NS, e_end = min(G * DM_HD, (rank + 1) * per);
+  for (int e = rank * per + threadIdx.x; e < e_end; e += DM_WARPS * 32) {
+    const int g = e / DM_HD, d = e % DM_HD;
+    float pm[NS], pl[NS], pa[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      const bool have = i < n_cta;
+      pm[i] = have ? *cluster.map_shared_rank(&c_m[g], i) : -INFINITY;
+      pl[i] = have ? *cluster.map_shared_rank(&c_l[g], i) : 0.f;
+      pa[i] = have ? *cluster.map_shared_rank(&c_acc[g][d], i) : 0.f;
+    }
+    float M = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) M = fmaxf(M, pm[i]);
+    float a = 0.f, L = 0.f;
+#pragma unroll
+    for (int i = 0; i < NS; ++i)
+      if (i < n_cta) {
+        const float w = __expf(pm[i] - M);
+        a = fmaf(w, pa[i], a);
+        L = fmaf(w, pl[i], L);
+      }
+    out[((size_t)b * nq + (size_t)kvh * G + g) * DM_HD + d] = from_f<T>(a / L);
+  }
+  cluster.sync();  // nobody leaves while a peer may still read its shared memory
+}
+
+template <typename T, int NS>
+static int launch_dm(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
+                     int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
+                     cudaStream_t st) {
+  auto kern = decode_attention_mma_kernel<T, NS>;
+  if (NS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(NS, B, nkv);
+  cfg.blockDim = dim3(DM_WARPS * 32);
+  cfg.stream = st;
+  static const int pdl = env_int("PG_PDL", 1);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = NS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (T*)out, (const T*)q, (const T*)k_pool, (const T*)v_pool, page_table, pt_stride,
+                                     page_size, kv_len, kv_len_add, nq, nkv, scale_div, exact_reciprocal(scale_div), pf);
+  if (e != cudaSuccess) {
+    set_error("decode_attention launch: %s", cudaGetErrorString(e));
+    cudaGetLastError();
+    return PG_ERR_CUDA;
+  }
+  return check_launch("decode_attention");
+}
+
+template <typename T>
+static int launch_dm_ns(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
+                        int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
+                        cudaStream_t st) {
+  // as many CTAs per (sequence, kv head) as keep the launch within one wave of two per SM (16 is a non-portable size)
+  const int seqs = B * nkv;
+#define PG_DM(N_) \
+  return launch_dm<T, N_>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st)
+  if (seqs <= 18) PG_DM(16);
+  if (seqs <= 37) PG_DM(8);
+  if (seqs <= 74) PG_DM(4);
+  if (seqs <= 148) PG_DM(2);
+  PG_DM(1);
+#undef PG_DM
+}
+
 }  // namespace pg
 
 using namespace pg;
@@ -374,6 +621,15 @@ int pg_decode_attention(void* out, const void* q, const void* k_pool, const void
   PG_REQUIRE(B > 0 && B <= 65535 && nq % nkv == 0, "decode_attention: bad shape");
   const int G = nq / nkv;
   cudaStream_t st = (cudaStream_t)stream;
+  // the mma kernel: 16-bit pools of 256-wide heads in 16-byte aligned rows, whole 16-token chunks inside a page, and query
+  // heads that fit its 8 columns; everything else (fp32, other head sizes) stays on the general kernel
+  const bool aligned = (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+  if (hd == DM_HD && (G == 1 || G == 2 || G == 4 || G == DM_G) && page_size > 0 && page_size % 16 == 0 && aligned) {
+#define PG_DM_ARGS out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st
+    if (dtype == PG_BF16) return launch_dm_ns<bf16>(PG_DM_ARGS);
+    if (dtype == PG_F16) return launch_dm_ns<f16>(PG_DM_ARGS);
+#undef PG_DM_ARGS
+  }
 #define PG_DA(GG, NCH) \
   return launch_da<T, GG, NCH>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, hd, scale_div, pf, st)
   PG_DISPATCH_DTYPE(dtype, T, {

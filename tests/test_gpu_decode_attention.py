@@ -1,0 +1,39 @@
+"""Decode attention of 256-wide heads in 16-bit types at the edges of its 16-token chunks, pages, warps and cluster sizes,
+against float64 with the scores rounded to the model type as the reference materialises them."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+@pytest.mark.parametrize("dtype,rel", [(torch.bfloat16, 4e-3), (torch.float16, 6e-4)])
+@pytest.mark.parametrize("B,T,G,nkv,page", [(1, 1, 8, 1, 64), (1, 16, 8, 1, 16), (2, 17, 8, 1, 64), (3, 65, 4, 2, 64), (1, 262, 8, 1, 64),
+                                            (1, 1025, 2, 1, 32), (19, 130, 8, 1, 64), (40, 31, 1, 3, 64), (80, 257, 8, 1, 64),
+                                            (150, 48, 8, 1, 64), (2, 2100, 8, 1, 64)])
+def test_chunks_pages_and_clusters(dtype, rel, B, T, G, nkv, page):
+    from pg_b200 import _cabi as cabi
+    hd, nq = 256, G * nkv
+    g = torch.Generator(device="cuda").manual_seed(B * 1000 + T)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    lens = torch.randint(max(1, T - 40), T + 1, (B,), device="cuda", generator=g)
+    lens[0] = T
+    cols = -(-T // page)
+    pages = B * cols + 2
+    kp, vp, q = new(pages, page, nkv * hd), new(pages, page, nkv * hd), new(B, nq * hd)
+    pt = torch.randperm(pages, device="cuda", generator=g)[:B * cols].to(torch.int32).view(B, cols)
+    out = torch.zeros(B, nq * hd, dtype=dtype, device="cuda")
+    kvl = (lens - 1).to(torch.int32)
+    cabi.check(cabi.lib().pg_decode_attention(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page,
+                                              kvl.data_ptr(), 1, B, nq, nkv, hd, math.sqrt(hd), None, None, 0, cabi.DTYPE_CODE[dtype],
+                                              cabi.stream()))
+    for b in sorted({0, B // 2, B - 1}):
+        n = int(lens[b])
+        k, v = (p[pt[b].long()].reshape(-1, nkv, hd)[:n].to(F64).repeat_interleave(G, 1) for p in (kp, vp))
+        s = torch.einsum("hd,nhd->hn", q[b].view(nq, hd).to(F64), k).to(dtype).to(F64) / math.sqrt(hd)
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1), v).reshape(-1)
+        got = out[b].to(F64)
+        # one rounding of the result (2^-9 and 2^-12 relative at most) and the odd score that rounds the other way
+        assert float((got - want).norm() / want.norm()) < rel
