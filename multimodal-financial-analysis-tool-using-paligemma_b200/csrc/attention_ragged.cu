@@ -19,6 +19,9 @@
 // denominator once (after all partial sums are merged), and explicit row strides of the key and the value pool, so
 // that the value rows may be a prefix of the key rows of ONE pool (latent attention: key [c | k_rot], value c).
 //
+// 16-bit steps with key and value widths of 64, 128 or 256 (or 256 and 192) run attention_ragged_mma_kernel
+// (attention_ragged_mma.cu); fp32 and other widths the two kernels below.
+//
 // attention_ragged_kernel: one warp per (token, head).  32 keys per iteration, one key per lane for the dot
 // product (the query row lives in shared memory as fp32), running (max, sum) rescaling, then the lanes switch to the
 // value columns and walk the 32 keys with the weights broadcast by shuffles.  Warps of a CTA are the heads of the
@@ -30,7 +33,7 @@
 // slices (CTAs) and over the warps of a CTA; the partial (max, sum, acc) triples are merged through shared memory
 // and, across slices, through a caller-owned fp32 workspace by attention_ragged_merge_kernel, always in a fixed
 // order.  A lane owns ceil(vdim / 32) contiguous value columns, fetched with one vector load per key.
-#include "common.cuh"
+#include "attention_ragged.cuh"
 
 namespace pg {
 
@@ -87,50 +90,6 @@ __device__ __forceinline__ void load_cols(const T* __restrict__ src, float* f) {
     for (int i = 0; i < DPL; ++i) f[i] = to_f<T>(src[i]);
   }
 }
-
-struct RagAttnParams {
-  void* out; int ld_out;
-  const void* q; int ld_q;
-  const void* gate; int ld_gate;
-  const void* k_pool; const void* v_pool;
-  const int32_t* page_table; int pt_stride; int page_size;
-  const int32_t* tok_slot; const int32_t* tok_pos;
-  int n_tokens, H, G, dim, vdim;
-  float scale; int window;
-  const float* slopes;
-  int keep_first;                // positions < keep_first stay visible behind the window
-  int sigmoid_weights;           // 0: softmax over the visible keys; 1: weight = sigmoid(score + head_bias[h])
-  const float* head_bias;        // per query head, added to the score (NULL: none)
-  int gate_per_head;             // 0: gate[t][h * vdim + c]; 1: gate[t][h]
-  float out_scale;
-  int ld_k, ld_v;                // elements between the rows of the key / value pool (>= G * dim, G * vdim)
-  const float* sink;             // per query head: exp(sink[h]) joins the softmax denominator (no key, no value)
-  int chunk;                     // > 0: a key is visible only inside the query's block of `chunk` positions
-  const float* out_rot;          // [vdim / 2]: the result is turned back by -position * out_rot[m] (rotated values)
-  int out_rot_interleaved;       // pairs (2m, 2m + 1) instead of (m, m + vdim / 2)
-  float softcap;                 // > 0: score <- softcap * tanh(score / softcap)
-  float temp_coef; int temp_every;   // query temperature 1 + temp_coef * ln(floor((pos + 1) / temp_every) + 1)
-};
-
-// The factor of q . k for a query at position pos.
-__device__ __forceinline__ float query_scale(const RagAttnParams& p, int pos) {
-  return p.temp_every > 0 ? p.scale * (1.f + p.temp_coef * logf((float)((pos + 1) / p.temp_every + 1))) : p.scale;
-}
-__device__ __forceinline__ float capped(const RagAttnParams& p, float s) {
-  return p.softcap > 0.f ? p.softcap * tanhf(s / p.softcap) : s;
-}
-
-// The visible keys of a token at position pos as one list: n_keep kept first positions, then [lo, pos].
-struct KeyRange {
-  int lo, n_keep, count;
-  __device__ __forceinline__ KeyRange(int pos, int window, int keep_first, int chunk = 0) {
-    lo = window > 0 ? max(0, pos - window + 1) : 0;
-    if (chunk > 0) lo = max(lo, pos / chunk * chunk);   // blocks are counted from position 0 of the sequence
-    n_keep = min(max(keep_first, 0), lo);
-    count = n_keep + pos - lo + 1;
-  }
-  __device__ __forceinline__ int key(int v) const { return v < n_keep ? v : lo + (v - n_keep); }
-};
 
 // Process keys [lo, hi] (inclusive) of one (token, head) for the calling warp; (m, l, acc) are the running state.
 template <typename T, int DPL>
@@ -537,6 +496,7 @@ extern "C" int pg_attention_ragged_capped(void* out, int ld_out, const void* q, 
                      sigmoid_weights ? 1 : 0, head_bias, gate_per_head ? 1 : 0, out_scale, ld_k, ld_v, sink, chunk, out_rot,
                      out_rot_interleaved ? 1 : 0, softcap, temp_coef, temp_every};
   cudaStream_t st = (cudaStream_t)stream;
+  if (attention_ragged_mma_wanted(p, dtype)) return attention_ragged_mma(p, dtype, st);
   const int dpl = (vdim + 31) / 32;
   PG_DISPATCH_DTYPE(dtype, T, {
     if (dpl <= 1) return launch_ragged<T, 1>(p, ws, ws_floats, st);
