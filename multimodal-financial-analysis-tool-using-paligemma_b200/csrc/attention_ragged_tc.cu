@@ -4,20 +4,24 @@
 // positions (tile = {first token row, rows, page-table row, first position}).  One CTA = one (tile, head).  The keys a
 // tile can see are the positions [max(0, pos0 - window + 1), pos0 + rows - 1] of its sequence, walked page by page
 // (key tile = page = 64 keys, fetched by TMA from the paged pools; the append kernel has written the step's own keys
-// before this launch).  Two passes over the key tiles, both on the tensor cores, as in attention_tc.cu:
-//   pass 0: S = Q K^T (tcgen05.mma, fp32 in TMEM) -> thread r owns query row r: s = S * scale - slope_h * (i - j),
-//           masked outside 0 <= i - j < window, running row maximum (no shuffles);
-//   pass 1: S again (K double-buffered, V in one buffer), p = exp(s - max) in fp32, row sum from the fp32 values, P rounded to the model dtype into a
-//           K-major SWIZZLE_128B tile, O += P V with V as an MN-major operand straight from its [key, vdim] page.
+// before this launch).  ONE pass over the key tiles:
+//   S(t) = Q K^T (tcgen05.mma, fp32) into one of two TMEM buffers, issued one tile ahead of the softmax;
+//   thread r owns query row r: z = log2(e) (S * scale - slope_h * (i - j)), masked outside 0 <= i - j < window, in fp32; the row's
+//   reference maximum is raised (and O, sum rescaled, after the products that still add to it) only when a tile exceeds it
+//   by more than 2^8; p = exp2(z - m), row sum from the fp32 values, P rounded to the model dtype and stored over the S
+//   columns it came from: O += P V takes P as the TMEM operand and V as an MN-major operand straight from its page.
+// What bounds it: the softmax's instructions (about 8 per score) and the exponentials; the tiles' products and copies
+// run beside them, and the two CTAs of an SM fill each other's waits.  Most tiles lie wholly inside the causal window of
+// all 128 rows and take a loop without masks.  The two-pass form before it (row maximum first, S computed twice, P through
+// shared memory, masks on every score) took 557 us for 4 prompts of 2048 tokens, 16 heads of 128, window 1024; this takes 248 us.
 // Epilogue: O / sum, times sigmoid(gate), rounded once.  Key width and value width are independent multiples of 64.
 // Extensions (pg_attention_ragged_tc_ex): keep_first > 0 keeps the first keep_first positions visible behind the
 // window: the key tiles are then the pages that hold them (as far as they lie before the window's first page)
-// followed by the window's pages.  sigmoid_weights: ONE pass, p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
+// followed by the window's pages.  sigmoid_weights: p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
 // gate may be one value per (token, head); the result is multiplied by out_scale before it is rounded.
 // pg_attention_ragged_tc_capped adds a query temperature and a softcap (both fp32, as in attention_ragged.cu; the kernel is
 // instantiated with and without the cap).  A capped score is bounded, so its softmax needs no maximum: with a cap of at
-// most 40 and bf16 weights (fp32's exponent range) the kernel runs ONE pass with p = exp(s - max(0, sink)), half the
-// MMAs of the two-pass form.  Head sizes are multiples of 8: the operand maps are {column, head, row} tensors, so the
+// most 40 and bf16 weights (fp32's exponent range) p = exp(s - max(0, sink)).  Head sizes are multiples of 8: the operand maps are {column, head, row} tensors, so the
 // 64-column tiles of a narrower head are filled up with zeros by the TMA unit.  When the value rows are the key rows (or a
 // prefix of them) of ONE pool, P V reads V from the K tile that S = Q K^T has just used and nothing is loaded twice.
 // Every mbarrier wait is bounded: a wait that gives up sets the error flag, the roles leave their loops, the CTA lets
@@ -49,6 +53,52 @@ __device__ __forceinline__ bool wait_lim(uint32_t bar, uint32_t parity, volatile
   return false;
 }
 
+// A (the weights) from TMEM: 128 lanes, two 16-bit values of a row per column
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+        "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack_pair<bf16>(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack_pair<f16>(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+constexpr float W_LOG2E = 1.4426950408889634f;
+constexpr float W_RAISE = 8.f;    // a row's reference maximum follows when a score exceeds it by more than 2^8: weights of at
+                                  // most 256 keep their relative precision in 16 bits
+
 struct WinParams {
   void* out; int ld_out;
   const void* gate; int ld_gate;
@@ -73,28 +123,28 @@ struct WinParams {
 };
 
 template <typename T, bool CAP>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, 2)
 attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, WinParams p) {
   constexpr int FMT = std::is_same<T, bf16>::value ? 1 : 0;
   const int KB = (p.dim + 63) / 64, VB = (p.vdim + 63) / 64;          // 64-column tiles of a head, zero-filled behind it
-  const int Q_BYTES = WQ * KB * 128, K_BYTES = WK * KB * 128, V_BYTES = p.tied ? 0 : WK * VB * 128, P_BYTES = WQ * WK * 2;
-  const int S_COL = 0, O_COL = WK;
-  const int tmem_cols = (WK + VB * 64 <= 256) ? 256 : 512;
+  const int Q_BYTES = WQ * KB * 128, K_BYTES = WK * KB * 128, V_BYTES = p.tied ? 0 : WK * VB * 128;
+  const int O_COL = 2 * WK;                                           // S (and P over it) of even / odd tiles, then O
+  const int tmem_cols = (O_COL + VB * 64 <= 256) ? 256 : 512;         // 256 (heads of up to 128): two CTAs share an SM
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  // K tiles are double-buffered (tile it+1 is requested as soon as S(it) has been issued); V has ONE buffer, requested
-  // when the previous P V has finished and hidden behind S and the softmax of its own tile: 99 KB at 128-wide heads,
-  // so that two CTAs share an SM and overlap each other's load -> MMA -> softmax -> MMA chains
-  const uint32_t s_q = base, s_k0 = s_q + Q_BYTES, s_vb = s_k0 + 2 * K_BYTES, s_p = s_vb + V_BYTES;
+  const uint32_t s_q = base, s_k0 = s_q + Q_BYTES, s_v0 = s_k0 + 2 * K_BYTES, bars = s_v0 + 2 * V_BYTES;
   auto s_k = [&](int bf) { return s_k0 + bf * K_BYTES; };
-  const uint32_t bars = s_p + P_BYTES;
-  const uint32_t bar_q = bars, bar_kv0 = bars + 8, bar_s = bars + 16, bar_sfree = bars + 24, bar_p = bars + 32,
-                 bar_o = bars + 40, bar_kv1 = bars + 48, bar_v = bars + 56, tmem_slot = bars + 64;
-  auto bar_kv = [&](int bf) { return bf ? bar_kv1 : bar_kv0; };
+  auto s_v = [&](int bf) { return p.tied ? s_k(bf) : s_v0 + bf * V_BYTES; };
+  // one barrier per buffer: tile t completes phase t >> 1 of barrier t & 1
+  const uint32_t bar_q = bars, tmem_slot = bars + 88;
+  auto bar_k = [&](int t) { return bars + 8 + 8 * (t & 1); };         // K(t) has landed
+  auto bar_v = [&](int t) { return bars + 24 + 8 * (t & 1); };        // V(t) has landed
+  auto bar_s = [&](int t) { return bars + 40 + 8 * (t & 1); };        // S(t) is computed
+  auto bar_p = [&](int t) { return bars + 56 + 8 * (t & 1); };        // P(t) is stored (and O rescaled)
+  auto bar_o = [&](int t) { return bars + 72 + 8 * (t & 1); };        // P(t) V(t) has been added to O
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-  uint8_t* p_ptr = smem_raw + (s_p - smem_u32(smem_raw));
   __shared__ int s_fail;
   volatile int* fail = &s_fail;
   if (threadIdx.x == 0) s_fail = 0;
@@ -104,8 +154,10 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   const int h = blockIdx.y, kvh = h / p.kv_group;
 
   if (warp == 1 && lane == 0) {
-    mbar_init(bar_q, 1); mbar_init(bar_kv0, 1); mbar_init(bar_kv1, 1); mbar_init(bar_s, 1); mbar_init(bar_sfree, 128);
-    mbar_init(bar_p, 128); mbar_init(bar_o, 1); mbar_init(bar_v, 1);
+    mbar_init(bar_q, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_k(i), 1); mbar_init(bar_v(i), 1); mbar_init(bar_s(i), 1); mbar_init(bar_p(i), 128); mbar_init(bar_o(i), 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -116,6 +168,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  auto wait = [&](uint32_t bar, int t) { return wait_lim(bar, (t >> 1) & 1, fail); };
   pdl_wait();  // q, the pools, the tile list and the page table come from the preceding kernels / copies
   const int32_t* tile = p.tiles + 4 * (size_t)blockIdx.x;
   const int row0 = tile[0], rows = tile[1], slot = tile[2], pos0 = tile[3];
@@ -128,120 +181,148 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   const int n_tiles = n_keep + hi / WK - t_lo + 1;
   auto page_of = [&](int t) { return t < n_keep ? t : t_lo + (t - n_keep); };   // key tile -> page of the sequence
   const int32_t* pt_row = p.page_table + (size_t)slot * p.pt_stride;
-  const bool sig = p.sigmoid_weights != 0, one_pass = sig || (CAP && p.bounded);
+  const bool sig = p.sigmoid_weights != 0, fixed_max = sig || (CAP && p.bounded);
 
   if (warp == 0 && lane == 0) {
-    // ===================== TMA + MMA issuer (one thread) =====================
-    const uint32_t idesc_s = umma_idesc(FMT, WQ, WK);
-    const uint32_t idesc_o = umma_idesc(FMT, WQ, VB * 64) | (1u << 16);            // B (= V) is MN-major
+    // ===================== TMA producer =====================
     mbar_expect_tx(bar_q, Q_BYTES);
     for (int kb = 0; kb < KB; ++kb)
       tma_load_3d(s_q + kb * (WQ * 128), &map_q, bar_q, kb * 64, h, row0);
-    const int total = one_pass ? n_tiles : 2 * n_tiles;
-    auto request = [&](int i) {   // K of flat step i into K buffer i & 1
-      const int t = page_of(i >= n_tiles ? i - n_tiles : i), bf = i & 1;
-      const int row = pt_row[t] * WK;
-      mbar_expect_tx(bar_kv(bf), K_BYTES);
-      for (int kb = 0; kb < KB; ++kb)
-        tma_load_3d(s_k(bf) + kb * (WK * 128), &map_k, bar_kv(bf), kb * 64, kvh, row);
-    };
-    auto request_v = [&](int t) {   // V of key tile t (pass 1) into the V buffer
+    for (int t = 0; t < n_tiles; ++t) {
+      // the buffers held tile t - 2: its K is free after S(t - 2), its V (or a tied K) after P V of t - 2
       const int row = pt_row[page_of(t)] * WK;
-      mbar_expect_tx(bar_v, V_BYTES);
+      if (t > 1 && !(p.tied ? wait(bar_o(t), t - 2) : wait(bar_s(t), t - 2))) break;
+      mbar_expect_tx(bar_k(t), K_BYTES);
+      for (int kb = 0; kb < KB; ++kb)
+        tma_load_3d(s_k(t & 1) + kb * (WK * 128), &map_k, bar_k(t), kb * 64, kvh, row);
+      if (p.tied) continue;
+      if (t > 1 && !wait(bar_o(t), t - 2)) break;
+      mbar_expect_tx(bar_v(t), V_BYTES);
       for (int vb = 0; vb < VB; ++vb)
-        tma_load_3d(s_vb + vb * (WK * 128), &map_v, bar_v, vb * 64, kvh, row);
-    };
-    request(0);
-    if (!wait_lim(bar_q, 0, fail)) goto issuer_done;
-    for (int it = 0; it < total; ++it) {
-      const int pass = (one_pass || it >= n_tiles) ? 1 : 0, t = it >= n_tiles ? it - n_tiles : it, bf = it & 1;
-      if (it > 0 && !wait_lim(bar_sfree, (it - 1) & 1, fail)) goto issuer_done;          // S of the previous tile was read
-      if (pass == 1 && t > 0 && !wait_lim(bar_o, (t - 1) & 1, fail)) goto issuer_done;   // previous PV done with V and P
-      if (pass == 1 && !p.tied) request_v(t);                      // lands behind S(it) and the softmax of this tile
-      if (!wait_lim(bar_kv(bf), (it >> 1) & 1, fail)) goto issuer_done;
-      tc_fence_after();
-      for (int ks = 0; ks < (p.dim + 15) / 16; ++ks) {             // S = Q K^T
-        const uint32_t off_q = (ks / 4) * (WQ * 128) + (ks % 4) * 32, off_k = (ks / 4) * (WK * 128) + (ks % 4) * 32;
-        umma(tmem_base + S_COL, umma_desc(s_q + off_q), umma_desc(s_k(bf) + off_k), idesc_s, ks > 0 ? 1u : 0u);
-      }
-      umma_commit(bar_s);
-      if (it + 1 < total) request(it + 1);                         // the other K buffer is free (bar_sfree above)
-      if (pass == 1) {
-        if (!wait_lim(bar_p, t & 1, fail)) goto issuer_done;       // P tile is in shared memory
-        if (!p.tied && !wait_lim(bar_v, t & 1, fail)) goto issuer_done;   // and so is V
-        const uint32_t s_val = p.tied ? s_k(bf) : s_vb;            // a tied tile stays until the next tile's P V is over
-        tc_fence_after();
-        for (int ks = 0; ks < WK / 16; ++ks) {                     // O += P V
-          umma(tmem_base + O_COL, umma_desc(s_p + ks * 32), umma_desc_mn_w(s_val + ks * 2048, WK * 128), idesc_o,
-               (t > 0 || ks > 0) ? 1u : 0u);
-        }
-        umma_commit(bar_o);
-      }
+        tma_load_3d(s_v(t & 1) + vb * (WK * 128), &map_v, bar_v(t), vb * 64, kvh, row);
     }
-  issuer_done:;
+  } else if (warp == 1 && lane == 0) {
+    // ===================== MMA issuer =====================
+    const uint32_t idesc_s = umma_idesc(FMT, WQ, WK);
+    const uint32_t idesc_o = umma_idesc(FMT, WQ, VB * 64) | (1u << 16);            // B (= V) is MN-major
+    auto issue_s = [&](int t) {                                      // S(t) = Q K(t)^T
+      if (!wait(bar_k(t), t)) return false;
+      tc_fence_after();
+      for (int ks = 0; ks < (p.dim + 15) / 16; ++ks) {
+        const uint32_t off_q = (ks / 4) * (WQ * 128) + (ks % 4) * 32, off_k = (ks / 4) * (WK * 128) + (ks % 4) * 32;
+        umma(tmem_base + (t & 1) * WK, umma_desc(s_q + off_q), umma_desc(s_k(t & 1) + off_k), idesc_s, ks > 0 ? 1u : 0u);
+      }
+      umma_commit(bar_s(t));
+      return true;
+    };
+    bool ok = wait_lim(bar_q, 0, fail) && issue_s(0);
+    for (int t = 0; ok && t < n_tiles; ++t) {
+      if (t + 1 < n_tiles) {                                         // P(t - 1) lies where S(t + 1) goes
+        if (t > 0 && !wait(bar_o(t - 1), t - 1)) break;
+        if (!issue_s(t + 1)) break;
+      }
+      if (!wait(bar_p(t), t)) break;
+      if (!p.tied && !wait(bar_v(t), t)) break;
+      tc_fence_after();
+      for (int ks = 0; ks < WK / 16; ++ks)                           // O += P(t) V(t)
+        umma_ts(tmem_base + O_COL, tmem_base + (t & 1) * WK + ks * 8, umma_desc_mn_w(s_v(t & 1) + ks * 2048, WK * 128), idesc_o,
+                (t > 0 || ks > 0) ? 1u : 0u);
+      umma_commit(bar_o(t));
+    }
   } else if (warp >= 4) {
     // ===================== softmax + epilogue: thread <-> query row =====================
     const int qw = warp & 3, r = qw * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
     const int i = pos0 + r;                                        // this row's position
-    const float slope = p.slopes ? p.slopes[h] : 0.f, hbias = p.head_bias ? p.head_bias[h] : 0.f;
+    const float slope = (p.slopes ? p.slopes[h] : 0.f) * W_LOG2E, hbias = (p.head_bias ? p.head_bias[h] : 0.f) * W_LOG2E;
     const int blk0 = p.chunk > 0 ? i / p.chunk * p.chunk : 0;      // first position of this row's block
-    float m = -INFINITY, l = 0.f;
-    if (CAP && p.bounded) m = p.sink ? fmaxf(p.sink[h], 0.f) : 0.f;  // any value near the scores does: they are bounded
+    const int blk_last = p.chunk > 0 ? (pos0 + WQ - 1) / p.chunk * p.chunk : 0;
+    float m = -INFINITY, l = 0.f;                                  // m in units of log2
+    if (CAP && p.bounded) m = (p.sink ? fmaxf(p.sink[h], 0.f) : 0.f) * W_LOG2E;  // any value near the scores does: they are bounded
+    if (sig) m = 0.f;
     float qscale = p.scale;
     if (CAP && p.temp_every > 0) qscale *= 1.f + p.temp_coef * logf((float)((i + 1) / p.temp_every + 1));
     const float cap_in = CAP ? 2.f * qscale / p.softcap : 0.f, cap_out = 2.f * p.softcap;
-    int it = 0;
+    const float qs2 = qscale * W_LOG2E;
     bool ok = true;
-    for (int pass = one_pass ? 1 : 0; pass < 2 && ok; ++pass) {
-      for (int t = 0; t < n_tiles; ++t, ++it) {
-        if (!wait_lim(bar_s, it & 1, fail)) { ok = false; break; }
-        tc_fence_after();
-        if (pass == 1 && t > 0 && !wait_lim(bar_o, (t - 1) & 1, fail)) { ok = false; break; }   // P buffer is free again
-        const int j0 = page_of(t) * WK;
-#pragma unroll 1
-        for (int c = 0; c < WK / 32; ++c) {
-          float s[32];
-          tmem_ld32(t_row + S_COL + c * 32, s);
-          tmem_ld_wait();
-#pragma unroll
-          for (int jj = 0; jj < 32; ++jj) {
-            const int j = j0 + c * 32 + jj, back = i - j;
-            const bool vis = back >= 0 && j >= blk0 && (p.window <= 0 || back < p.window || j < p.keep_first);
-            float sc = s[jj] * qscale;
-            if (CAP)           // cap * tanh(z / cap) = cap - 2 cap / (exp(2 z / cap) + 1): absolute error a few 1e-7 of the cap
-              sc = p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f);
-            s[jj] = vis ? sc - slope * (float)back + hbias : -INFINITY;
-          }
-          if (pass == 0) {
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj) m = fmaxf(m, s[jj]);
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
-              s[jj] = sig ? 1.f / (1.f + __expf(-s[jj])) : __expf(s[jj] - m);   // exp(+inf) -> weight 0 when masked
-              l += s[jj];
-            }
-            // P[r][c*32 .. +31] into the K-major SWIZZLE_128B tile (128 rows x 128 B)
-            uint8_t* blk = p_ptr + r * 128;
-#pragma unroll
-            for (int q0 = 0; q0 < 32; q0 += 8) {
-              const int chunk = (c * 4 + q0 / 8) ^ (r & 7);
-              *reinterpret_cast<uint4*>(blk + chunk * 16) = pack<T>(s + q0);
-            }
-          }
-        }
-        tc_fence_before();
-        if (pass == 1) {
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy smem writes -> UMMA
-          mbar_arrive(bar_p);
-        }
-        mbar_arrive(bar_sfree);
-      }
-    }
-    if (ok && wait_lim(bar_o, (n_tiles - 1) & 1, fail)) {
+    for (int t = 0; t < n_tiles; ++t) {
+      if (!wait(bar_s(t), t)) { ok = false; break; }
       tc_fence_after();
-      if (p.sink && !sig) l += __expf(p.sink[h] - m);              // a logit without key or value, counted once
+      const int j0 = page_of(t) * WK;
+      float s[WK];
+      tmem_ld32(t_row + (t & 1) * WK, s);
+      tmem_ld32(t_row + (t & 1) * WK + 32, s + 32);
+      tmem_ld_wait();
+      if (CAP) {       // cap * tanh(z / cap) = cap - 2 cap / (exp(2 z / cap) + 1): absolute error a few 1e-7 of the cap
+#pragma unroll
+        for (int jj = 0; jj < WK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * W_LOG2E;
+      }
+      const float d0 = (float)(j0 - i);                            // exact, and so is d0 + jj = j - i
+#pragma unroll
+      for (int jj = 0; jj < WK; ++jj) {
+        const float z = fmaf(slope, d0 + (float)jj, hbias);
+        s[jj] = CAP ? s[jj] + z : fmaf(s[jj], qs2, z);
+      }
+      // whole tiles that every row sees need no masks
+      const bool full = j0 + WK - 1 <= pos0 && j0 >= blk_last &&
+                        (p.window <= 0 || pos0 + WQ - 1 - j0 < p.window || j0 + WK <= p.keep_first);
+      if (!full) {
+#pragma unroll
+        for (int jj = 0; jj < WK; ++jj) {
+          const int j = j0 + jj, back = i - j;
+          const bool vis = back >= 0 && j >= blk0 && (p.window <= 0 || back < p.window || j < p.keep_first);
+          s[jj] = vis ? s[jj] : -INFINITY;
+        }
+      }
+      if (!fixed_max) {
+        float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+        for (int jj = 4; jj < WK; ++jj) mx[jj & 3] = fmaxf(mx[jj & 3], s[jj]);
+        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        if (__any_sync(0xffffffffu, top > m + W_RAISE)) {          // m == -inf: any visible key raises it
+          const float m_new = fmaxf(m, top);
+          if (t > 0) {
+            const float corr = m_new == m ? 1.f : exp2_approx(m - m_new);
+            l *= corr;
+            if (!wait(bar_o(t - 1), t - 1)) { ok = false; break; }   // nothing adds to O until this tile's P is handed over
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < VB * 4; ++c) {
+              float o[16];
+              tmem_ld16(t_row + O_COL + c * 16, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj) o[jj] *= corr;
+              tmem_st16(t_row + O_COL + c * 16, reinterpret_cast<const uint32_t*>(o));
+            }
+          }
+          m = m_new;
+        }
+      }
+      if (sig) {
+#pragma unroll
+        for (int jj = 0; jj < WK; ++jj) s[jj] = __fdividef(1.f, 1.f + exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
+      } else {
+        const float ref = m == -INFINITY ? 0.f : m;                // a row that has seen no key yet
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int jj = 0; jj < WK; ++jj) {
+          s[jj] = exp2_approx(s[jj] - ref);
+          sum[jj & 3] += s[jj];
+        }
+        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      }
+      uint32_t pk[WK / 2];
+#pragma unroll
+      for (int jj = 0; jj < WK / 2; ++jj) pk[jj] = pack_pair<T>(s[2 * jj], s[2 * jj + 1]);
+      tmem_st32(t_row + (t & 1) * WK, pk);                         // over the first 32 of this row's S columns
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(bar_p(t));
+    }
+    if (ok && wait(bar_o(n_tiles - 1), n_tiles - 1)) {
+      tc_fence_after();
+      if (p.sink && !sig) l += exp2_approx(p.sink[h] * W_LOG2E - m);   // a logit without key or value, counted once
       float inv = (sig ? 1.f : 1.f / l) * p.out_scale;
       const size_t trow = (size_t)row0 + r;
       T* orow = reinterpret_cast<T*>(p.out) + trow * p.ld_out + (size_t)h * p.vdim;
@@ -258,7 +339,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
             float v = o[q0 + jj];
-            if (grow) v *= 1.f / (1.f + __expf(-gt[jj]));
+            if (grow) v *= __fdividef(1.f, 1.f + __expf(-gt[jj]));
             w[jj] = v;
           }
           *reinterpret_cast<uint4*>(orow + c * 32 + q0) = pack<T>(w);
@@ -410,8 +491,8 @@ extern "C" int pg_attention_ragged_tc_capped(void* out, int ld_out, const void* 
                      gate_per_head ? 1 : 0, out_scale, sink, chunk, out_rot, out_rot_interleaved ? 1 : 0, softcap, temp_coef,
                      temp_every, tied, bounded};
   const int kb = cdiv(dim, 64), vb = cdiv(vdim, 64);
-  const size_t smem = 1024 + (size_t)tc::WQ * kb * 128 + 2 * (size_t)tc::WK * kb * 128 + (tied ? 0 : (size_t)tc::WK * vb * 128) +
-                      (size_t)tc::WQ * tc::WK * 2 + 72 + 16;
+  const size_t smem = 1024 + (size_t)tc::WQ * kb * 128 + 2 * (size_t)tc::WK * kb * 128 +
+                      (tied ? 0 : 2 * (size_t)tc::WK * vb * 128) + 88 + 8;
   cudaStream_t st = (cudaStream_t)stream;
   dim3 grid(n_tiles, n_heads);
   auto run = [&](auto kern) -> int {
