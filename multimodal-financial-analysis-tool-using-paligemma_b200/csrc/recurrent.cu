@@ -269,11 +269,14 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //     S <- decay_h S + k v^T,        o = S^T q
 // lightning_prep_kernel  (elementwise)  the activations in fp32, one packed record [q | k | v] per (token, head) with
 //                                       q, k padded to dp = dim rounded up to 4 floats and v to vp likewise (zeros).
-// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): a thread owns a quarter of
-//                                       the rows of one value column (the layout of the delta-rule kernel above: rows
-//                                       4 (m RG + rg) + e), so a token costs one fused multiply-add per state element
-//                                       for the update, one for the output, and two shuffle steps.  The records of
-//                                       the next CH tokens arrive by cp.async into the other half of a double buffer.
+// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): RG lanes share two value columns,
+//                                       a thread owns rows 4 (m RG + rg) + e of both.  What bounds it is issue slots: a
+//                                       token costs a multiply and two fused multiply-adds per state element, so they run
+//                                       on pairs of rows (fma.rn.f32x2: the same roundings, half the instructions), the
+//                                       q and k a thread reads serve two columns, and the two column sums meet in
+//                                       log2(RG) shuffles together.  The records of the next CH tokens arrive by cp.async
+//                                       into the other half of a double buffer.  4 x 2048 tokens, 16 heads of 128: one
+//                                       column per thread and scalar arithmetic 842 us, this 787 us.
 //                                       The state is read from and written back to the slot once per launch, which
 //                                       makes a prompt portion and a single decoded token the same case and the
 //                                       result independent of where the sequence was cut.
@@ -299,6 +302,31 @@ __global__ void lightning_prep_kernel(float* __restrict__ rec, const T* __restri
       a = a * sigmoid_f(a);
     }
     out[i] = a;
+  }
+}
+
+// The same with 16-byte loads, for head sizes and rows that are whole vectors: 8 records' columns per thread and step
+// (8192 tokens of 16 heads of 128: an element per thread 156 us, this 56 us; 302 MB move).
+template <typename T>
+__global__ void __launch_bounds__(256)
+lightning_prep_vec_kernel(float* __restrict__ rec, const T* __restrict__ proj, int ld, int q_col0, int k_col0, int v_col0,
+                          int heads, int dim, int vdim) {
+  constexpr int V = Vec<T>::N;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int rs = 2 * dim + vdim, per_head = rs / V;
+  const T* row = proj + (size_t)blockIdx.x * ld;
+  float* out = rec + (size_t)blockIdx.x * heads * rs;
+  for (int i = threadIdx.x; i < heads * per_head; i += blockDim.x) {
+    const int h = i / per_head, c = (i - h * per_head) * V;
+    const int col = c < dim ? q_col0 + h * dim + c : (c < 2 * dim ? k_col0 + h * dim + c - dim : v_col0 + h * vdim + c - 2 * dim);
+    float f[V];
+    unpack<T>(ldg_cached(row + col), f);
+#pragma unroll
+    for (int k = 0; k < V; ++k) f[k] = f[k] * sigmoid_f(f[k]);
+    float4* dst = reinterpret_cast<float4*>(out + (size_t)h * rs + c);
+#pragma unroll
+    for (int k = 0; k < V; k += 4) dst[k / 4] = make_float4(f[k], f[k + 1], f[k + 2], f[k + 3]);
   }
 }
 
@@ -463,12 +491,35 @@ __global__ void retention_prep_kernel(float* __restrict__ rec, const T* __restri
 //                                       mixer's direct term, with v its unscaled input).
 enum { DECAY_HEAD = 0, DECAY_TOKEN = 1, DECAY_CHANNEL = 2 };
 
+// pairs of fp32 values (two state rows) in one 64-bit register pair
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 halves_of(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 template <int DMAX, int RG, int CH, int DK>
 __global__ void __launch_bounds__(256)
 lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ rec,
                  const float* __restrict__ decay, const float* __restrict__ skip, const int32_t* __restrict__ segs,
                  int heads, int dim, int vdim, int dp, int vp) {
-  constexpr int NG = DMAX / (4 * RG);               // groups of four rows per thread (RG lanes share a value column)
+  constexpr int NG = DMAX / (4 * RG);               // groups of four rows per thread (RG lanes share two value columns)
   extern __shared__ __align__(16) float sh[];       // [2][CH][q DMAX | k DMAX | (decays DMAX) | v VT | (decay)]
   pdl_launch_dependents();
   pdl_wait();
@@ -477,20 +528,22 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   if (n <= 0) return;
   constexpr bool TD = DK == DECAY_TOKEN, CD = DK == DECAY_CHANNEL;
   constexpr int XP = TD ? 4 : 0, NV = CD ? 3 : 2;   // NV: vectors of key width in a record
-  const int VT = blockDim.x / RG, RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP;
-  const int h = blockIdx.y, j0 = blockIdx.z * VT, jl = threadIdx.x / RG, j = j0 + jl, rg = threadIdx.x % RG;
-  const bool live = j < vdim;
+  const int VT = 2 * (blockDim.x / RG), RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP;
+  const int h = blockIdx.y, j0 = blockIdx.z * VT, jl = 2 * (threadIdx.x / RG), j = j0 + jl, rg = threadIdx.x % RG;
   const float lam_h = DK == DECAY_HEAD ? decay[h] : 0.f, skip_h = skip ? skip[h] : 0.f;
   for (int idx = threadIdx.x; idx < 2 * CH * RSZ; idx += blockDim.x) sh[idx] = 0.f;   // padding the copies never write
-  float S[NG * 4];
+  f32x2 S[2][NG * 2];                               // [column][pair of rows]
   float* st = state + ((size_t)slot * heads + h) * dim * vdim;
 #pragma unroll
-  for (int m = 0; m < NG; ++m)
+  for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 4 * (m * RG + rg) + e;
-      S[m * 4 + e] = (live && i < dim) ? st[(size_t)i * vdim + j] : 0.f;
-    }
+    for (int m = 0; m < NG; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const int i = 4 * (m * RG + rg) + e;
+        S[c][m * 2 + e / 2] = pair_of((j + c < vdim && i < dim) ? st[(size_t)i * vdim + j + c] : 0.f,
+                                      (j + c < vdim && i + 1 < dim) ? st[(size_t)(i + 1) * vdim + j + c] : 0.f);
+      }
   __syncthreads();
   const int qk_pieces = dp / 4, v_pieces = min(VT, vp - j0) / 4, pieces = NV * qk_pieces + v_pieces + (TD ? 1 : 0);
   auto fetch = [&](int t0, int buf) {               // records of tokens [t0, t0 + CH) of this head -> buffer buf
@@ -509,46 +562,58 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   };
   fetch(0, 0);
   int buf = 0;
+  const bool second = (rg & 1) != 0;                // the column whose sum this lane ends up with
+  const bool writes = rg < 2 && j + rg < vdim;
+  float* orow = out + (size_t)row0 * heads * vdim + (size_t)h * vdim + j + (second ? 1 : 0);
+  const size_t ostep = (size_t)heads * vdim;
   for (int t0 = 0; t0 < n; t0 += CH, buf ^= 1) {
     const int nt = min(CH, n - t0);
     if (t0 + CH < n) { fetch(t0 + CH, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
     __syncthreads();
-#pragma unroll 2
+#pragma unroll 4
     for (int tt = 0; tt < nt; ++tt) {
       const float* r = sh + ((size_t)buf * CH + tt) * RSZ;
-      const float vj = r[NV * DMAX + jl];
+      const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
+      const f32x2 v0 = pair_of(vj.x, vj.x), v1 = pair_of(vj.y, vj.y);
       const float lam = TD ? r[NV * DMAX + VT] : lam_h;
-      const float* qr = r + 4 * rg;
-      const float* kr = r + DMAX + 4 * rg;
-      const float* ar = r + 2 * DMAX + 4 * rg;       // decays per key channel (CD)
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+      const f32x2 lam2 = pair_of(lam, lam);
+      f32x2 o0[2] = {0ull, 0ull}, o1[2] = {0ull, 0ull};
 #pragma unroll
       for (int m = 0; m < NG; ++m) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + 4 * RG * m);
-        const float4 q4 = *reinterpret_cast<const float4*>(qr + 4 * RG * m);
-        float4 a4 = make_float4(lam, lam, lam, lam);
-        if (CD) a4 = *reinterpret_cast<const float4*>(ar + 4 * RG * m);
-        S[4 * m] = fmaf(k4.x, vj, a4.x * S[4 * m]);
-        S[4 * m + 1] = fmaf(k4.y, vj, a4.y * S[4 * m + 1]);
-        S[4 * m + 2] = fmaf(k4.z, vj, a4.z * S[4 * m + 2]);
-        S[4 * m + 3] = fmaf(k4.w, vj, a4.w * S[4 * m + 3]);
-        o0 = fmaf(q4.x, S[4 * m], o0); o1 = fmaf(q4.y, S[4 * m + 1], o1);
-        o2 = fmaf(q4.z, S[4 * m + 2], o2); o3 = fmaf(q4.w, S[4 * m + 3], o3);
+        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(r + 4 * rg + 4 * RG * m);
+        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(r + DMAX + 4 * rg + 4 * RG * m);
+        ulonglong2 a4 = make_ulonglong2(lam2, lam2);
+        if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r + 2 * DMAX + 4 * rg + 4 * RG * m);   // decays per key channel
+        S[0][2 * m] = fma2(k4.x, v0, mul2(a4.x, S[0][2 * m]));
+        S[0][2 * m + 1] = fma2(k4.y, v0, mul2(a4.y, S[0][2 * m + 1]));
+        S[1][2 * m] = fma2(k4.x, v1, mul2(a4.x, S[1][2 * m]));
+        S[1][2 * m + 1] = fma2(k4.y, v1, mul2(a4.y, S[1][2 * m + 1]));
+        o0[0] = fma2(q4.x, S[0][2 * m], o0[0]);
+        o0[1] = fma2(q4.y, S[0][2 * m + 1], o0[1]);
+        o1[0] = fma2(q4.x, S[1][2 * m], o1[0]);
+        o1[1] = fma2(q4.y, S[1][2 * m + 1], o1[1]);
       }
-      float o = (o0 + o1) + (o2 + o3);
+      const float2 a0 = halves_of(o0[0]), a1 = halves_of(o0[1]), b0 = halves_of(o1[0]), b1 = halves_of(o1[1]);
+      const float c0 = (a0.x + a0.y) + (a1.x + a1.y), c1 = (b0.x + b0.y) + (b1.x + b1.y);
+      // lanes with an even rg collect column j, the others column j + 1
+      float o = (second ? c1 : c0) + __shfl_xor_sync(0xffffffffu, second ? c0 : c1, 1);
 #pragma unroll
-      for (int sh_ = 1; sh_ < RG; sh_ <<= 1) o += __shfl_xor_sync(0xffffffffu, o, sh_);
-      if (live && rg == 0) out[((size_t)row0 + t0 + tt) * heads * vdim + h * vdim + j] = fmaf(skip_h, vj, o);
+      for (int sh_ = 2; sh_ < RG; sh_ <<= 1) o += __shfl_xor_sync(0xffffffffu, o, sh_);
+      if (writes) orow[(size_t)(t0 + tt) * ostep] = fmaf(skip_h, second ? vj.y : vj.x, o);
     }
     __syncthreads();                                // every thread is done with this buffer before it is refilled
   }
-  if (live) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (j + c >= vdim) continue;
 #pragma unroll
     for (int m = 0; m < NG; ++m)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 4; e += 2) {
         const int i = 4 * (m * RG + rg) + e;
-        if (i < dim) st[(size_t)i * vdim + j] = S[m * 4 + e];
+        const float2 v = halves_of(S[c][m * 2 + e / 2]);
+        if (i < dim) st[(size_t)i * vdim + j + c] = v.x;
+        if (i + 1 < dim) st[(size_t)(i + 1) * vdim + j + c] = v.y;
       }
   }
 }
@@ -557,12 +622,12 @@ template <int DMAX, int RG, int CH>
 static int launch_lightning(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
                             const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
   const int dp = (dim + 3) / 4 * 4, vp = (vdim + 3) / 4 * 4;
-  // value columns per CTA: as many as 256 threads hold for prompt-sized work (few fat CTAs, about one per SM, beat
-  // many thin ones: 0.75 against 0.87 ms at 4 x 2048 tokens, 8 heads of 128), fewer while the CTAs do not fill the SMs
-  int vt = 256 / RG;
-  while (vt > 8 && (vt / 2 >= vdim || (long long)n_segs * heads * cdiv(vdim, vt) < 100)) vt /= 2;
+  // value columns per CTA: as many as 256 threads hold (every CTA of a head fetches all of q and k), fewer while the CTAs do
+  // not fill the SMs; a CTA keeps a whole warp
+  int vt = 512 / RG;
+  while (vt > 64 / RG && vt > 8 && (vt / 2 >= vdim || (long long)n_segs * heads * cdiv(vdim, vt) < 148)) vt /= 2;
   static const int vt_env = env_int("PG_LIGHTNING_VT", 0);
-  if (vt_env >= 8 && vt_env <= 256 / RG && (vt_env & (vt_env - 1)) == 0) vt = vt_env;
+  if (vt_env >= 8 && vt_env >= 64 / RG && vt_env <= 512 / RG && (vt_env & (vt_env - 1)) == 0) vt = vt_env;
   const size_t smem = sizeof(float) * 2 * CH * ((dk == DECAY_CHANNEL ? 3 : 2) * DMAX + vt + (dk == DECAY_TOKEN ? 4 : 0));
   // An ordinary launch, not a programmatic dependent one: CTAs that become resident while the preceding kernel still
   // fills the machine are placed on the few SMs with room, and a recurrence of a few hundred long-lived CTAs then runs
@@ -574,7 +639,7 @@ static int launch_lightning(float* out, float* state, const float* rec, const fl
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
-  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3(vt * RG), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim, dp, vp);
+  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3(vt / 2 * RG), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim, dp, vp);
   return check_launch("lightning");
 }
 
@@ -660,6 +725,13 @@ extern "C" int pg_lightning_prep(float* rec, const void* proj, int ld, int q_col
   PG_REQUIRE(rec && proj && heads > 0 && dim > 0 && vdim > 0, "lightning_prep: bad arguments");
   const int dp = (dim + 3) / 4 * 4, vp = (vdim + 3) / 4 * 4;
   PG_DISPATCH_DTYPE(dtype, T, {
+    constexpr int V = Vec<T>::N;
+    if (dim % V == 0 && vdim % V == 0 && ld % V == 0 && q_col0 % V == 0 && k_col0 % V == 0 && v_col0 % V == 0 &&
+        (((uintptr_t)proj | (uintptr_t)rec) & 15) == 0) {
+      const int vecs = heads * (2 * dim + vdim) / V, threads = vecs >= 256 ? 256 : (vecs + 31) / 32 * 32;
+      return launch_pdl("lightning_prep", lightning_prep_vec_kernel<T>, dim3(n_tokens), dim3(threads), 0, (cudaStream_t)stream, rec,
+                        (const T*)proj, ld, q_col0, k_col0, v_col0, heads, dim, vdim);
+    }
     return launch_pdl("lightning_prep", lightning_prep_kernel<T>, dim3(n_tokens), dim3(256), 0, (cudaStream_t)stream, rec,
                       (const T*)proj, ld, q_col0, k_col0, v_col0, (long long)n_tokens, heads, dim, vdim, dp, vp);
   });
