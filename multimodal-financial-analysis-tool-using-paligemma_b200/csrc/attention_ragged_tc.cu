@@ -36,68 +36,6 @@ namespace tc {
 constexpr int WQ = 128;   // query rows per CTA == TMEM lanes
 constexpr int WK = 64;    // keys per tile == page size
 
-__device__ __forceinline__ uint64_t umma_desc_mn_w(uint32_t smem_addr, uint32_t lbo_bytes) {
-  // MN-major, SWIZZLE_128B: 64 contiguous MN elements (128 B) per K row, 8-row groups 1024 B apart (SBO),
-  // next 64-element MN block lbo_bytes away (LBO)
-  return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16) | (64ull << 32) |
-         (1ull << 46) | (2ull << 61);
-}
-
-constexpr uint32_t W_WAIT_LIMIT = 1u << 22;
-__device__ __forceinline__ bool wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
-  for (uint32_t it = 0; it < W_WAIT_LIMIT; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 255u && *fail) return false;
-  }
-  *fail = 1;
-  return false;
-}
-
-// A (the weights) from TMEM: 128 lanes, two 16-bit values of a row per column
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
-        "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float exp2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack_pair<bf16>(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-template <> __device__ __forceinline__ uint32_t pack_pair<f16>(float lo, float hi) {
-  const __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-constexpr float W_LOG2E = 1.4426950408889634f;
-constexpr float W_RAISE = 8.f;    // a row's reference maximum follows when a score exceeds it by more than 2^8: weights of at
-                                  // most 256 keep their relative precision in 16 bits
 
 struct WinParams {
   void* out; int ld_out;
@@ -168,7 +106,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  auto wait = [&](uint32_t bar, int t) { return wait_lim(bar, (t >> 1) & 1, fail); };
+  auto wait = [&](uint32_t bar, int t) { return mbar_wait_lim(bar, (t >> 1) & 1, fail); };
   pdl_wait();  // q, the pools, the tile list and the page table come from the preceding kernels / copies
   const int32_t* tile = p.tiles + 4 * (size_t)blockIdx.x;
   const int row0 = tile[0], rows = tile[1], slot = tile[2], pos0 = tile[3];
@@ -215,7 +153,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       umma_commit(bar_s(t));
       return true;
     };
-    bool ok = wait_lim(bar_q, 0, fail) && issue_s(0);
+    bool ok = mbar_wait_lim(bar_q, 0, fail) && issue_s(0);
     for (int t = 0; ok && t < n_tiles; ++t) {
       if (t + 1 < n_tiles) {                                         // P(t - 1) lies where S(t + 1) goes
         if (t > 0 && !wait(bar_o(t - 1), t - 1)) break;
@@ -225,7 +163,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       if (!p.tied && !wait(bar_v(t), t)) break;
       tc_fence_after();
       for (int ks = 0; ks < WK / 16; ++ks)                           // O += P(t) V(t)
-        umma_ts(tmem_base + O_COL, tmem_base + (t & 1) * WK + ks * 8, umma_desc_mn_w(s_v(t & 1) + ks * 2048, WK * 128), idesc_o,
+        umma_ts(tmem_base + O_COL, tmem_base + (t & 1) * WK + ks * 8, umma_desc_mn(s_v(t & 1) + ks * 2048, WK * 128), idesc_o,
                 (t > 0 || ks > 0) ? 1u : 0u);
       umma_commit(bar_o(t));
     }
@@ -234,16 +172,16 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int qw = warp & 3, r = qw * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
     const int i = pos0 + r;                                        // this row's position
-    const float slope = (p.slopes ? p.slopes[h] : 0.f) * W_LOG2E, hbias = (p.head_bias ? p.head_bias[h] : 0.f) * W_LOG2E;
+    const float slope = (p.slopes ? p.slopes[h] : 0.f) * LOG2E_F, hbias = (p.head_bias ? p.head_bias[h] : 0.f) * LOG2E_F;
     const int blk0 = p.chunk > 0 ? i / p.chunk * p.chunk : 0;      // first position of this row's block
     const int blk_last = p.chunk > 0 ? (pos0 + WQ - 1) / p.chunk * p.chunk : 0;
     float m = -INFINITY, l = 0.f;                                  // m in units of log2
-    if (CAP && p.bounded) m = (p.sink ? fmaxf(p.sink[h], 0.f) : 0.f) * W_LOG2E;  // any value near the scores does: they are bounded
+    if (CAP && p.bounded) m = (p.sink ? fmaxf(p.sink[h], 0.f) : 0.f) * LOG2E_F;  // any value near the scores does: they are bounded
     if (sig) m = 0.f;
     float qscale = p.scale;
     if (CAP && p.temp_every > 0) qscale *= 1.f + p.temp_coef * logf((float)((i + 1) / p.temp_every + 1));
     const float cap_in = CAP ? 2.f * qscale / p.softcap : 0.f, cap_out = 2.f * p.softcap;
-    const float qs2 = qscale * W_LOG2E;
+    const float qs2 = qscale * LOG2E_F;
     bool ok = true;
     for (int t = 0; t < n_tiles; ++t) {
       if (!wait(bar_s(t), t)) { ok = false; break; }
@@ -255,7 +193,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       tmem_ld_wait();
       if (CAP) {       // cap * tanh(z / cap) = cap - 2 cap / (exp(2 z / cap) + 1): absolute error a few 1e-7 of the cap
 #pragma unroll
-        for (int jj = 0; jj < WK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * W_LOG2E;
+        for (int jj = 0; jj < WK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * LOG2E_F;
       }
       const float d0 = (float)(j0 - i);                            // exact, and so is d0 + jj = j - i
 #pragma unroll
@@ -279,7 +217,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll
         for (int jj = 4; jj < WK; ++jj) mx[jj & 3] = fmaxf(mx[jj & 3], s[jj]);
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-        if (__any_sync(0xffffffffu, top > m + W_RAISE)) {          // m == -inf: any visible key raises it
+        if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {          // m == -inf: any visible key raises it
           const float m_new = fmaxf(m, top);
           if (t > 0) {
             const float corr = m_new == m ? 1.f : exp2_approx(m - m_new);
@@ -322,7 +260,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     }
     if (ok && wait(bar_o(n_tiles - 1), n_tiles - 1)) {
       tc_fence_after();
-      if (p.sink && !sig) l += exp2_approx(p.sink[h] * W_LOG2E - m);   // a logit without key or value, counted once
+      if (p.sink && !sig) l += exp2_approx(p.sink[h] * LOG2E_F - m);   // a logit without key or value, counted once
       float inv = (sig ? 1.f : 1.f / l) * p.out_scale;
       const size_t trow = (size_t)row0 + r;
       T* orow = reinterpret_cast<T*>(p.out) + trow * p.ld_out + (size_t)h * p.vdim;

@@ -2,14 +2,14 @@
 // Reference: GemmaAttention.forward (modeling_gemma.py:262-288, additive mask all zeros) and
 // SiglipAttention.forward (modeling_siglip.py:116-131); fp32 softmax, scale applied after QK^T.
 //
-// One CTA = 128 query rows of one (batch, head).  Two passes over the keys, both on tensor cores:
-//   pass 0: S = Q K^T per key tile (tcgen05.mma, fp32 in TMEM) -> each thread owns one query row,
-//           reads its S row with tcgen05.ld and keeps the running max (no shuffles at all);
-//   pass 1: S again, p = exp(s - max) -> bf16 P tile written to shared memory in the K-major
-//           SWIZZLE_128B layout -> O += P V with V consumed as an MN-major operand straight from its
-//           natural [key, dim] layout (no transpose), O accumulating in TMEM with no rescaling.
-// Recomputing QK^T costs tensor-core time that is idle anyway and removes the online-softmax
-// correction of O.  Q, K, V tiles arrive by TMA; K/V may be contiguous or paged (page == key tile).
+// One CTA = 128 query rows of one (batch, head); ONE pass over the 64-key tiles:
+//   S(t) = Q K^T (tcgen05.mma, fp32) into one of two TMEM buffers, issued one tile ahead of the softmax; each thread owns one
+//   query row (no shuffles), raises the row's reference maximum (and rescales O and the sum) only when a tile exceeds it by
+//   more than 2^8, p = exp(s - max) in fp32, rounded to the model dtype over the S columns it came from; O += P V with P as
+//   the TMEM operand and V as an MN-major operand straight from its natural [key, dim] layout (no transpose).
+// K and V tiles are double-buffered and arrive by TMA; K/V may be contiguous or paged (page == key tile).  What bounds a prompt is
+// the chain of its key tiles (24 CTAs for 260 tokens of 8 heads): the two-pass form (row maximum first, S computed twice, P
+// through shared memory) took 41.9 us there, this takes 15.1 us; 4 x 323 tokens 51.8 -> 17.2 us.
 // Head rows may be padded (hd_stride > hd): the SigLIP path pads 72 -> 128 with zero weights.
 #include <cmath>
 
@@ -19,13 +19,6 @@ namespace pg {
 namespace tc {
 
 constexpr int AQ = 128;  // query rows per CTA == TMEM lanes
-
-__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr, uint32_t lbo_bytes) {
-  // MN-major, SWIZZLE_128B: 64 contiguous MN elements (128 B) per K row, 8-row groups 1024 B apart (SBO),
-  // next 64-element MN block lbo_bytes away (LBO)
-  return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16) | (64ull << 32) |
-         (1ull << 46) | (2ull << 61);
-}
 
 struct AttnParams {
   void* out;
@@ -41,29 +34,32 @@ struct AttnParams {
   float scale_mul;                               // != 0: the scaling is exactly s*scale_mul (power-of-two divisor)
 };
 
-template <typename T, int HDP, int KT>  // HDP: padded head dim in shared memory (128 or 256); KT: keys per tile
+template <typename T, int HDP>  // HDP: padded head dim in shared memory (128 or 256)
 __global__ void __launch_bounds__(256, HDP == 128 ? 2 : 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, AttnParams p) {
-  constexpr int KB = HDP / 64;                   // 64-column blocks of the head dim
-  constexpr int Q_BYTES = AQ * HDP * 2, K_BYTES = KT * HDP * 2, V_BYTES = K_BYTES, P_BYTES = AQ * KT * 2;
-  constexpr int S_COL = 0, O_COL = KT;           // TMEM columns
-  constexpr int TMEM_NEED = KT + HDP, TMEM_ALLOC = TMEM_NEED <= 256 ? 256 : 512;  // 256 lets two CTAs share an SM
+  constexpr int KT = 64, KB = HDP / 64;          // keys per tile, 64-column blocks of the head dim
+  constexpr int Q_BYTES = AQ * HDP * 2, K_BYTES = KT * HDP * 2;
+  constexpr int O_COL = 2 * KT;                  // TMEM columns: S (and P over it) of even / odd tiles, then O
+  constexpr int TMEM_ALLOC = O_COL + HDP <= 256 ? 256 : 512;  // 256 lets two CTAs share an SM
   constexpr int FMT = std::is_same<T, bf16>::value ? 1 : 0;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  // K/V tiles are double-buffered: tile it+1 is requested as soon as S(it) has been issued, so its TMA latency hides
-  // behind the softmax of tile it instead of heading every step of the chain
-  const uint32_t s_q = base, s_kv = s_q + Q_BYTES, s_p = s_kv + 2 * (K_BYTES + V_BYTES);
-  auto s_k = [&](int bf) { return s_kv + bf * (K_BYTES + V_BYTES); };
-  auto s_v = [&](int bf) { return s_kv + bf * (K_BYTES + V_BYTES) + K_BYTES; };
-  const uint32_t bars = s_p + P_BYTES;
-  const uint32_t bar_q = bars, bar_kv0 = bars + 8, bar_s = bars + 16, bar_sfree = bars + 24, bar_p = bars + 32,
-                 bar_o = bars + 40, bar_kv1 = bars + 48, tmem_slot = bars + 56;
-  auto bar_kv = [&](int bf) { return bf ? bar_kv1 : bar_kv0; };
+  const uint32_t s_q = base, s_k0 = s_q + Q_BYTES, s_v0 = s_k0 + 2 * K_BYTES, bars = s_v0 + 2 * K_BYTES;
+  auto s_k = [&](int t) { return s_k0 + (t & 1) * K_BYTES; };
+  auto s_v = [&](int t) { return s_v0 + (t & 1) * K_BYTES; };
+  // one barrier per buffer: tile t completes phase t >> 1 of barrier t & 1
+  const uint32_t bar_q = bars, tmem_slot = bars + 88;
+  auto bar_k = [&](int t) { return bars + 8 + 8 * (t & 1); };         // K(t) has landed
+  auto bar_v = [&](int t) { return bars + 24 + 8 * (t & 1); };        // V(t) has landed
+  auto bar_s = [&](int t) { return bars + 40 + 8 * (t & 1); };        // S(t) is computed
+  auto bar_p = [&](int t) { return bars + 56 + 8 * (t & 1); };        // P(t) is stored (and O rescaled)
+  auto bar_o = [&](int t) { return bars + 72 + 8 * (t & 1); };        // P(t) V(t) has been added to O
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-  uint8_t* p_ptr = smem_raw + (s_p - smem_u32(smem_raw));
+  __shared__ int s_fail;
+  volatile int* fail = &s_fail;
+  if (threadIdx.x == 0) s_fail = 0;
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -72,8 +68,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int k_steps = (p.hd + 15) / 16;          // 16-wide K steps of QK^T that hold real data
 
   if (warp == 1 && lane == 0) {
-    mbar_init(bar_q, 1); mbar_init(bar_kv0, 1); mbar_init(bar_kv1, 1); mbar_init(bar_s, 1); mbar_init(bar_sfree, 128);
-    mbar_init(bar_p, 128); mbar_init(bar_o, 1);
+    mbar_init(bar_q, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_k(i), 1); mbar_init(bar_v(i), 1); mbar_init(bar_s(i), 1); mbar_init(bar_p(i), 128); mbar_init(bar_o(i), 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -84,107 +82,132 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  auto wait = [&](uint32_t bar, int t) { return mbar_wait_lim(bar, (t >> 1) & 1, fail); };
   pdl_wait();  // q / k / v, lengths and page tables come from the preceding kernels
   const int T_len = p.kv_len_dev ? (p.kv_len_dev[b] + p.kv_len_add) : p.kv_len_const;
   const int n_tiles = (T_len + KT - 1) / KT;
 
   if (warp == 0 && lane == 0) {
-    // ===================== TMA + MMA issuer (one thread) =====================
-    const uint32_t idesc_s = umma_idesc(FMT, AQ, KT);
-    const uint32_t idesc_o = umma_idesc(FMT, AQ, nv) | (1u << 16);  // B (= V) is MN-major
-    mbar_expect_tx(bar_q, Q_BYTES);
-    for (int kb = 0; kb < KB; ++kb)
-      tma_load_2d(s_q + kb * (AQ * 128), &map_q, bar_q, p.q_col0 + h * p.hd_stride + kb * 64, b * p.q_len + qb * AQ);
-    // request K (and V in pass 1) of flat step i into buffer i & 1
-    const int total = 2 * n_tiles;
-    auto request = [&](int i) {
-      const int pass = i >= n_tiles ? 1 : 0, t = pass ? i - n_tiles : i, bf = i & 1;
-      const int row = p.page_table ? p.page_table[(size_t)b * p.pt_stride + t] * KT
-                                   : (int)(b * p.kv_batch_rows) + t * KT;
-      mbar_expect_tx(bar_kv(bf), pass == 1 ? K_BYTES + V_BYTES : K_BYTES);
+    // ===================== TMA producer =====================
+    if (n_tiles > 0) {
+      mbar_expect_tx(bar_q, Q_BYTES);
       for (int kb = 0; kb < KB; ++kb)
-        tma_load_2d(s_k(bf) + kb * (KT * 128), &map_k, bar_kv(bf), p.k_col0 + kvh * p.hd_stride + kb * 64, row);
-      if (pass == 1)
-        for (int kb = 0; kb < KB; ++kb)
-          tma_load_2d(s_v(bf) + kb * (KT * 128), &map_v, bar_kv(bf), p.v_col0 + kvh * p.hd_stride + kb * 64, row);
-    };
-    if (total > 0) request(0);
-    mbar_wait(bar_q, 0);
-    for (int it = 0; it < total; ++it) {
-      const int pass = it >= n_tiles ? 1 : 0, t = pass ? it - n_tiles : it, bf = it & 1;
-      if (it > 0) mbar_wait(bar_sfree, (it - 1) & 1);            // S of the previous tile has been read
-      if (pass == 1 && t > 0) mbar_wait(bar_o, (t - 1) & 1);     // previous PV finished with V and P
-      mbar_wait(bar_kv(bf), (it >> 1) & 1);
+        tma_load_2d(s_q + kb * (AQ * 128), &map_q, bar_q, p.q_col0 + h * p.hd_stride + kb * 64, b * p.q_len + qb * AQ);
+    }
+    for (int t = 0; t < n_tiles; ++t) {          // the buffers held tile t - 2: K is free after its S, V after its P V
+      const int row = p.page_table ? p.page_table[(size_t)b * p.pt_stride + t] * KT : (int)(b * p.kv_batch_rows) + t * KT;
+      if (t > 1 && !wait(bar_s(t), t - 2)) break;
+      mbar_expect_tx(bar_k(t), K_BYTES);
+      for (int kb = 0; kb < KB; ++kb)
+        tma_load_2d(s_k(t) + kb * (KT * 128), &map_k, bar_k(t), p.k_col0 + kvh * p.hd_stride + kb * 64, row);
+      if (t > 1 && !wait(bar_o(t), t - 2)) break;
+      mbar_expect_tx(bar_v(t), K_BYTES);
+      for (int kb = 0; kb < KB; ++kb)
+        tma_load_2d(s_v(t) + kb * (KT * 128), &map_v, bar_v(t), p.v_col0 + kvh * p.hd_stride + kb * 64, row);
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ===================== MMA issuer =====================
+    const uint32_t idesc_s = umma_idesc(FMT, AQ, KT);
+    const uint32_t idesc_o = umma_idesc(FMT, AQ, nv) | (1u << 16);   // B (= V) is MN-major
+    auto issue_s = [&](int t) {                                      // S(t) = Q K(t)^T
+      if (!wait(bar_k(t), t)) return false;
       tc_fence_after();
-      for (int ks = 0; ks < k_steps; ++ks) {                     // S = Q K^T
+      for (int ks = 0; ks < k_steps; ++ks) {
         const uint32_t off_q = (ks / 4) * (AQ * 128) + (ks % 4) * 32, off_k = (ks / 4) * (KT * 128) + (ks % 4) * 32;
-        umma(tmem_base + S_COL, umma_desc(s_q + off_q), umma_desc(s_k(bf) + off_k), idesc_s, ks > 0 ? 1u : 0u);
+        umma(tmem_base + (t & 1) * KT, umma_desc(s_q + off_q), umma_desc(s_k(t) + off_k), idesc_s, ks > 0 ? 1u : 0u);
       }
-      umma_commit(bar_s);
-      // the other buffer held step it-1: its K was consumed by S(it-1) (complete: bar_sfree above), its V by PV(it-1)
-      // (complete: bar_o above) -- free for step it+1
-      if (it + 1 < total) request(it + 1);
-      if (pass == 1) {
-        mbar_wait(bar_p, t & 1);                                 // P tile is in shared memory
-        tc_fence_after();
-        for (int ks = 0; ks < KT / 16; ++ks) {                   // O += P V
-          const uint32_t off_p = (ks / 4) * (AQ * 128) + (ks % 4) * 32;
-          umma(tmem_base + O_COL, umma_desc(s_p + off_p), umma_desc_mn(s_v(bf) + ks * 2048, KT * 128), idesc_o,
-               (t > 0 || ks > 0) ? 1u : 0u);
-        }
-        umma_commit(bar_o);
+      umma_commit(bar_s(t));
+      return true;
+    };
+    bool ok = n_tiles > 0 && mbar_wait_lim(bar_q, 0, fail) && issue_s(0);
+    for (int t = 0; ok && t < n_tiles; ++t) {
+      if (t + 1 < n_tiles) {                                         // P(t - 1) lies where S(t + 1) goes
+        if (t > 0 && !wait(bar_o(t - 1), t - 1)) break;
+        if (!issue_s(t + 1)) break;
       }
+      if (!wait(bar_p(t), t) || !wait(bar_v(t), t)) break;
+      tc_fence_after();
+      for (int ks = 0; ks < KT / 16; ++ks)                           // O += P(t) V(t)
+        umma_ts(tmem_base + O_COL, tmem_base + (t & 1) * KT + ks * 8, umma_desc_mn(s_v(t) + ks * 2048, KT * 128), idesc_o,
+                (t > 0 || ks > 0) ? 1u : 0u);
+      umma_commit(bar_o(t));
     }
   } else if (warp >= 4) {
     // ===================== softmax + epilogue: thread <-> query row =====================
     const int qw = warp & 3, r = qw * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
-    float m = -INFINITY, l = 0.f;
-    int it = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int t = 0; t < n_tiles; ++t, ++it) {
-        mbar_wait(bar_s, it & 1);
-        tc_fence_after();
-        if (pass == 1 && t > 0) mbar_wait(bar_o, (t - 1) & 1);     // P buffer is free again
-#pragma unroll 1
-        for (int c = 0; c < KT / 32; ++c) {
-          float s[32];
-          tmem_ld32(t_row + S_COL + c * 32, s);
-          tmem_ld_wait();
+    float m = -INFINITY, l = 0.f;                                    // m in units of log2
+    bool ok = true;
+    for (int t = 0; t < n_tiles; ++t) {
+      if (!wait(bar_s(t), t)) { ok = false; break; }
+      tc_fence_after();
+      float s[KT];
+      tmem_ld32(t_row + (t & 1) * KT, s);
+      tmem_ld32(t_row + (t & 1) * KT + 32, s + 32);
+      tmem_ld_wait();
+      // the scores as the reference materialises them: rounded, scaled, rounded again (an exact scaling needs no rounding)
+      if (p.scale_mul != 0.f) {
+        const float mul = p.scale_mul * LOG2E_F;                     // one rounding instead of two: a power of two is exact
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float x = rnd<T>(s[j]);
-            x = (p.scale_mul != 0.f) ? x * p.scale_mul : rnd<T>(p.scale_mode ? x / p.scale : x * p.scale);
-            s[j] = (t * KT + c * 32 + j < T_len) ? x : -INFINITY;
-          }
-          if (pass == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) m = fmaxf(m, s[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) { s[j] = __expf(s[j] - m); l += s[j]; }
-            // P[r][c*32 .. c*32+31] as bf16 into the K-major SWIZZLE_128B tile: 64-key blocks of 128 rows x 128 B
-            uint8_t* blk = p_ptr + (c / 2) * (AQ * 128) + r * 128;
-#pragma unroll
-            for (int j0 = 0; j0 < 32; j0 += 8) {
-              const int chunk = ((c & 1) * 4 + j0 / 8) ^ (r & 7);
-              *reinterpret_cast<uint4*>(blk + chunk * 16) = pack<T>(s + j0);
-            }
-          }
+        for (int j = 0; j < KT; j += 2) {
+          rnd2<T>(s[j], s[j + 1]);
+          s[j] *= mul;
+          s[j + 1] *= mul;
         }
-        tc_fence_before();
-        if (pass == 1) {
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy smem writes -> UMMA
-          mbar_arrive(bar_p);
+      } else {
+#pragma unroll
+        for (int j = 0; j < KT; ++j) {
+          const float x = rnd<T>(s[j]);
+          s[j] = rnd<T>(p.scale_mode ? x / p.scale : x * p.scale) * LOG2E_F;
         }
-        mbar_arrive(bar_sfree);
       }
+      if ((t + 1) * KT > T_len) {
+#pragma unroll
+        for (int j = 0; j < KT; ++j) s[j] = t * KT + j < T_len ? s[j] : -INFINITY;
+      }
+      float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+      for (int j = 4; j < KT; ++j) mx[j & 3] = fmaxf(mx[j & 3], s[j]);
+      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {            // always for the first tile: it holds a key of every row
+        const float m_new = fmaxf(m, top);
+        if (t > 0) {
+          const float corr = exp2_approx(m - m_new);
+          l *= corr;
+          if (!wait(bar_o(t - 1), t - 1)) { ok = false; break; }     // nothing adds to O until this tile's P is handed over
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c * 16 < nv; ++c) {
+            float o[16];
+            tmem_ld16(t_row + O_COL + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] *= corr;
+            tmem_st16(t_row + O_COL + c * 16, reinterpret_cast<const uint32_t*>(o));
+          }
+        }
+        m = m_new;
+      }
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < KT; ++j) {
+        s[j] = exp2_approx(s[j] - m);
+        sum[j & 3] += s[j];
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      uint32_t pk[KT / 2];
+#pragma unroll
+      for (int j = 0; j < KT / 2; ++j) pk[j] = pack_pair<T>(s[2 * j], s[2 * j + 1]);
+      tmem_st32(t_row + (t & 1) * KT, pk);                           // over the first 32 of this row's S columns
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(bar_p(t));
     }
     if (n_tiles > 0) {
-      mbar_wait(bar_o, (n_tiles - 1) & 1);
+      ok = ok && wait(bar_o(n_tiles - 1), n_tiles - 1);
       tc_fence_after();
       const int qi = qb * AQ + r;
-      const float inv = 1.f / l;
+      const float inv = ok ? 1.f / l : NAN;                          // a wait that gave up shows in the rows it would have written
       T* orow = reinterpret_cast<T*>(p.out) + (size_t)(b * p.q_len + qi) * p.ld_out + (size_t)h * p.hd;
 #pragma unroll 1
       for (int c = 0; c * 32 < p.hd; ++c) {
@@ -206,6 +229,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
+  if (s_fail) {  // let copies and MMAs that are still in flight finish before the shared memory and TMEM go away
+    for (int k = 0; k < 2000; ++k) __nanosleep(1000);
+    __syncthreads();
+  }
   if (warp == 2) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_ALLOC) : "memory");
@@ -236,12 +263,6 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw32(uint32_t smem_addr, uint32
          (1ull << 46) | (6ull << 61);
 }
 __device__ __forceinline__ void vit_softmax_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-constexpr float LOG2E_F = 1.4426950408889634f;
-__device__ __forceinline__ float ex2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(VIT_THREADS, 2)
@@ -372,8 +393,8 @@ attention_vit_kernel(const __grid_constant__ CUtensorMap map64, const __grid_con
           rnd2<T>(x0, x1);
           x0 *= mul; x1 *= mul;
           rnd2<T>(x0, x1);
-          s[j] = ex2_ftz(fmaf(x0, LOG2E_F, neg_m_l2));
-          s[j + 1] = ex2_ftz(fmaf(x1, LOG2E_F, neg_m_l2));
+          s[j] = exp2_approx(fmaf(x0, LOG2E_F, neg_m_l2));
+          s[j + 1] = exp2_approx(fmaf(x1, LOG2E_F, neg_m_l2));
         }
         if (cb + 32 > T_len) {                                 // ragged last chunk only
 #pragma unroll
@@ -456,11 +477,11 @@ static int launch_attn_vit(const CUtensorMap& m64, const CUtensorMap& m16, const
   return launch_tc("attention_vit", kern, dim3(cdiv(p.q_len, AQ), p.n_heads, B), dim3(VIT_THREADS), smem, 1, ctas <= 296, st, m64, m16, p);
 }
 
-template <typename T, int HDP, int KT>
+template <typename T, int HDP>
 static int launch_attn(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int B,
                        cudaStream_t st) {
-  const size_t smem = 1024 + (size_t)(AQ * HDP * 2) + 4 * (size_t)(KT * HDP * 2) + (size_t)(AQ * KT * 2) + 64;
-  auto kern = attention_tc_kernel<T, HDP, KT>;
+  const size_t smem = 1024 + (size_t)(AQ * HDP * 2) + 4 * (size_t)(64 * HDP * 2) + 88 + 8;
+  auto kern = attention_tc_kernel<T, HDP>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     set_error("attention_tc: cannot reserve %zu B of shared memory", smem);
     cudaGetLastError();
@@ -517,6 +538,6 @@ extern "C" int pg_attention_tc(void* out, int ld_out, const void* q, long long q
                  tc::make_map_2d(&mv, v, kv_rows, ld_kv, ld_kv, kt, bf),
              "attention_tc: cuTensorMapEncodeTiled failed");
   PG_REQUIRE(hd == hdp || hd_stride >= ((hd + 63) / 64) * 64 || n_heads == 1, "attention_tc: head rows must be padded to a multiple of 64 columns");
-  if (hdp == 128) return bf ? tc::launch_attn<bf16, 128, 64>(mq, mk, mv, p, B, st) : tc::launch_attn<f16, 128, 64>(mq, mk, mv, p, B, st);
-  return bf ? tc::launch_attn<bf16, 256, 64>(mq, mk, mv, p, B, st) : tc::launch_attn<f16, 256, 64>(mq, mk, mv, p, B, st);
+  if (hdp == 128) return bf ? tc::launch_attn<bf16, 128>(mq, mk, mv, p, B, st) : tc::launch_attn<f16, 128>(mq, mk, mv, p, B, st);
+  return bf ? tc::launch_attn<bf16, 256>(mq, mk, mv, p, B, st) : tc::launch_attn<f16, 256>(mq, mk, mv, p, B, st);
 }
