@@ -316,7 +316,11 @@ int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void*
   PG_REQUIRE(!bias || ((uintptr_t)bias % 16) == 0, "gemm_tc: bias must be 16-byte aligned");
   const bool bf = dtype == PG_BF16;
   const bool dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
-  if (epi == PG_EPI_SWIGLU) goto basic;   // the SiLU pairing lives in the persistent single-CTA kernel only
+  if (epi == PG_EPI_SWIGLU) {             // the SiLU pairing lives in the two row-major kernels only
+    if (!out_f32 && gemm_tc_2cta_wanted(M, N, K, epi))
+      return gemm_tc_2cta(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, st);
+    goto basic;
+  }
   if (gemm_tc_swap_wanted(M, N, K, epi, out_f32, res_mod))  // a prompt's worth of rows: CTA pairs, weights as the M operand
     return gemm_tc_swap(C, A, W, R, M, N, K, lda, ldw, ldc, ldr, epi, dtype, st);
   if (res_mod == 0 && gemm_tc_skinny_wanted(M, N, K, epi))  // a few dozen token rows: stream the weights (swap-AB)
@@ -326,7 +330,7 @@ int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void*
     const int s = gemm_tc_splitk_factor(M, N, K, epi, &sk_bn);  // few tiles, long K: a cluster shares each tile
     if (s) return gemm_tc_splitk(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, sk_bn, s, st);
   }
-  if (gemm_tc_2cta_wanted(M, N, K, epi))  // >= 2 waves of 256 x 256 tiles: CTA pairs (cta_group::2)
+  if (!(dual && out_f32) && gemm_tc_2cta_wanted(M, N, K, epi))  // fewer staged bytes per wave: CTA pairs (cta_group::2)
     return gemm_tc_2cta(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, st);
 basic:
   // 64-wide N tiles when 128-wide ones would occupy well under one wave of the 148 SMs

@@ -83,9 +83,28 @@ __device__ __forceinline__ void epi_apply2(float& x0, float& x1, float b0, float
   if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) { x0 += r0; x1 += r1; rnd2<T>(x0, x1); }
 }
 
+// gelu_tanh(g) u or silu(g) u of two elements, rounded where the single-CTA kernel rounds
+template <typename T, int EPI>
+__device__ __forceinline__ void epi_pair2(float& x0, float& x1, float u0, float u1) {
+  rnd2<T>(x0, x1);
+  rnd2<T>(u0, u1);
+  if (EPI == PG_EPI_GEGLU) { x0 = gelu_tanh_fast(x0); x1 = gelu_tanh_fast(x1); }
+  else { x0 = x0 / (1.f + __expf(-x0)); x1 = x1 / (1.f + __expf(-x1)); }
+  rnd2<T>(x0, x1);
+  x0 *= u0; x1 *= u1;
+  rnd2<T>(x0, x1);
+}
+
+// The gated pairings of a stacked [Wg; Wu]: the pair's first CTA stages 128 gate rows, the second the 128 up rows of the same
+// features, so that the 256-column accumulator of either CTA holds [gate | up] of its token rows and the epilogue pairs
+// column c with column 128 + c.  An output tile is then 256 x 128.
+template <int EPI> constexpr bool g2_dual() { return EPI == PG_EPI_GEGLU || EPI == PG_EPI_SWIGLU; }
+
 template <typename T, int EPI>
 __global__ void __launch_bounds__(G2_THREADS, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, Params2 p) {
+  constexpr bool DUAL = g2_dual<EPI>();
+  constexpr int TILE_N = DUAL ? G2_BN / 2 : G2_BN;   // output columns of a tile
   constexpr uint32_t IDESC = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, G2_BN);
   // a last n-tile with <= 128 real columns (N = 1152: o_proj, fc2) runs N = 128 MMAs: each CTA supplies 64 W rows
   constexpr uint32_t IDESC_HALF = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, G2_BN / 2);
@@ -105,7 +124,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   uint32_t crank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
   const bool leader = crank == 0;
-  const int m_pairs = (((p.M + G2_BM - 1) / G2_BM) + 1) / 2, n_tiles = (p.N + G2_BN - 1) / G2_BN;
+  const int m_pairs = (((p.M + G2_BM - 1) / G2_BM) + 1) / 2, n_tiles = (p.N + TILE_N - 1) / TILE_N;
   const int total_tiles = m_pairs * n_tiles;
   const int sched_first = (int)(blockIdx.x / 2), sched_stride = (int)(gridDim.x / 2);
   const int k_blocks = (p.K + G2_BK - 1) / G2_BK;
@@ -139,13 +158,14 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const int n_blk = p.m_major ? tile % n_tiles : tile / m_pairs;  // neighbouring clusters share A rows or W rows (L2 reuse)
         const int m_blk = 2 * (p.m_major ? tile / n_tiles : tile % m_pairs) + (int)crank;  // a ghost tile past M loads zeros, stores nothing
         const int w_step = (n_blk * G2_BN + G2_BN / 2 >= p.N) ? G2_BN / 4 : G2_BN / 2;  // half tile: 64 rows per CTA
+        const int w_row = n_blk * TILE_N + (int)crank * (DUAL ? p.N : w_step);
         for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(empty_bar(stage), phase ^ 1);
           const uint32_t sa = smem_base + stage * G2_STAGE_BYTES;
           const uint32_t full_leader = mapa_u32(full_bar(stage), 0);
           if (leader) mbar_expect_tx(full_bar(stage), 2 * G2_STAGE_BYTES);  // both CTAs' bytes
           tma_load_2d_cg2(sa, &map_a, full_leader, kb * G2_BK, m_blk * G2_BM);
-          tma_load_2d_cg2(sa + G2_A_BYTES, &map_w, full_leader, kb * G2_BK, n_blk * G2_BN + (int)crank * w_step);
+          tma_load_2d_cg2(sa + G2_A_BYTES, &map_w, full_leader, kb * G2_BK, w_row);
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -160,7 +180,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * G2_BN;
         const int n_blk_mma = p.m_major ? tile % n_tiles : tile / m_pairs;
-        const uint32_t idesc = (n_blk_mma * G2_BN + G2_BN / 2 >= p.N) ? IDESC_HALF : IDESC;
+        const uint32_t idesc = (!DUAL && n_blk_mma * G2_BN + G2_BN / 2 >= p.N) ? IDESC_HALF : IDESC;
         for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(full_bar(stage), phase);
           tc_fence_after();
@@ -194,7 +214,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int row0 = m_blk * G2_BM + q * 32;  // first row of this warp's TMEM lane quarter
       const int m = row0 + lane;
       const int ch_l = lane & 7, r_l = lane >> 3;  // staging <-> global mapping: 8 lanes per 128-byte row segment
-      const int nw0 = n_blk * G2_BN + half * (G2_BN / 2);
+      const int nw0 = n_blk * TILE_N + half * (TILE_N / 2);
       // residual rows of both 64-column slices are requested BEFORE waiting for the accumulator: ordinary loads
       // queue behind ~190 KB of in-flight TMA data per SM, and this wait is where the epilogue warps idle anyway
       uint4 r1[8];
@@ -213,8 +233,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + half * (G2_BN / 2);
-      if (p.out_f32) {
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + half * (TILE_N / 2);
+      if (!DUAL && p.out_f32) {
         // fp32 rows (logits): direct 32-byte stores, thread <-> row
 #pragma unroll 1
         for (int c = 0; c < G2_BN / 64; ++c) {
@@ -242,7 +262,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // 16-bit rows: 64-column slices through a per-warp staging tile so that the residual loads and the output
         // stores are whole 128-byte row segments (4 rows per instruction) instead of 32 scattered 16-byte pieces
 #pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
+        for (int sl = 0; sl < TILE_N / 128; ++sl) {
           const int n0 = nw0 + sl * 64;
           if (n0 >= p.N || row0 >= p.M) break;  // warp-uniform
           if (HAS_RES && sl == 1) {
@@ -255,8 +275,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           }
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
-            float v[32];
+            float v[32], u[DUAL ? 32 : 1];
             tmem_ld32(t_row + sl * 64 + cc * 32, v);
+            if constexpr (DUAL) tmem_ld32(t_row + G2_BN / 2 + cc * 32, u);
             tmem_ld_wait();
 #pragma unroll
             for (int j0 = 0; j0 < 32; j0 += 8) {
@@ -274,7 +295,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int j = 0; j < 8; j += 2) {
                 o[j] = v[j0 + j]; o[j + 1] = v[j0 + j + 1];
-                epi_apply2<T, EPI>(o[j], o[j + 1], bb[j], bb[j + 1], rr[j], rr[j + 1]);
+                if constexpr (DUAL) epi_pair2<T, EPI>(o[j], o[j + 1], u[j0 + j], u[j0 + j + 1]);
+                else epi_apply2<T, EPI>(o[j], o[j + 1], bb[j], bb[j + 1], rr[j], rr[j + 1]);
               }
               *slot = pack<T>(o);
             }
@@ -314,30 +336,39 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const Params2& 
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
-  const int pairs = cdiv(cdiv(p.M, G2_BM), 2) * cdiv(p.N, G2_BN);
+  const int pairs = cdiv(cdiv(p.M, G2_BM), 2) * cdiv(p.N, g2_dual<EPI>() ? G2_BN / 2 : G2_BN);
   return launch_tc("gemm_tcgen05_2cta", kern, dim3(2 * (pairs < 74 ? pairs : 74)), dim3(G2_THREADS), smem, 2, pairs <= 148, st, ma, mw, p);
 }
 
 }  // namespace tc
 
-// CTA-pair GEMM: taken for problems with at least ~2 waves of 256 x 256 tiles (PG_GEMM_2CTA=0 disables it).
+// CTA-pair GEMM against the single-CTA kernel.  Both are paced by what an SM can pull from L2 (about 64 B a clock): a k-block
+// costs the bytes that a CTA stages, 32 KB here for a 256 x 256 tile (256 x 128 when gated), 32 KB there for 128 x 128
+// (48 KB gated, 24 KB with 64 columns), and a GEMM takes that many times the waves of its tiles.  1292 rows: q/k/v (N 2560)
+// 24.2 -> 17.9, o_proj and down_proj together (N 2048, K 2048 and 16384) 176 -> 102, gate/up (F 16384) 149 -> 123 us.
 bool gemm_tc_2cta_wanted(int M, int N, int K, int epi) {
   static const int enabled = env_int("PG_GEMM_2CTA", 1);
   static const int min_pairs = env_int("PG_GEMM_2CTA_MIN_PAIRS", 148);
-  if (!enabled || epi == PG_EPI_GEGLU) return false;
-  return cdiv(cdiv(M, tc::G2_BM), 2) * cdiv(N, tc::G2_BN) >= min_pairs;
+  if (!enabled) return false;
+  const bool dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
+  const int m_tiles = cdiv(M, tc::G2_BM), pairs = cdiv(m_tiles, 2) * cdiv(N, dual ? tc::G2_BN / 2 : tc::G2_BN);
+  if (!dual && pairs >= min_pairs) return true;
+  const int bn = m_tiles * cdiv(N, 128) < 100 ? 64 : 128;      // the single-CTA kernel's tile for this problem
+  const int one = cdiv((long long)m_tiles * cdiv(N, bn), 148) * (16 + (dual ? 2 : 1) * bn / 8);
+  return cdiv(pairs, 74) * 32 < one;
 }
 
 int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                  int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st) {
-  const bool bf = dtype == PG_BF16;
+  const bool bf = dtype == PG_BF16, dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
   CUtensorMap ma, mw;
-  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && tc::make_map_2d(&mw, W, N, K, ldw, tc::G2_BN / 2, bf),
+  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && tc::make_map_2d(&mw, W, dual ? 2 * N : N, K, ldw, tc::G2_BN / 2, bf),
              "gemm_tc2: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, N, K, lda, ldw);
+  PG_REQUIRE(!dual || !out_f32, "gemm_tc2: a gated pairing has no fp32 output");
   // A is re-read once per n-tile (n-major order) or W once per m-pair (m-major): stream the big operand once and
   // keep the small one in L2
   static const int order_env = env_int("PG_GEMM_2CTA_ORDER", -1);
-  const int m_major = order_env >= 0 ? order_env : ((long long)N * K * 2 <= (32ll << 20) ? 1 : 0);
+  const int m_major = order_env >= 0 ? order_env : ((long long)N * K * (dual ? 4 : 2) <= (32ll << 20) ? 1 : 0);
   tc::Params2 p = {C, bias, R, M, N, K, ldc, ldr, res_mod, out_f32, m_major};
 #define PG_TC2(E) return bf ? tc::launch2<bf16, E>(ma, mw, p, st) : tc::launch2<f16, E>(ma, mw, p, st)
   switch (epi) {
@@ -346,6 +377,8 @@ int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const 
     case PG_EPI_BIAS_GELU: PG_TC2(PG_EPI_BIAS_GELU);
     case PG_EPI_BIAS_RES: PG_TC2(PG_EPI_BIAS_RES);
     case PG_EPI_RES: PG_TC2(PG_EPI_RES);
+    case PG_EPI_GEGLU: PG_TC2(PG_EPI_GEGLU);
+    case PG_EPI_SWIGLU: PG_TC2(PG_EPI_SWIGLU);
   }
 #undef PG_TC2
   set_error("gemm_tc2: bad epilogue %d", epi);

@@ -1,0 +1,163 @@
+"""The tensor-core kernels at the edges of their tiles, clusters and splits, against float64 products of the same 16-bit
+operands with the rounding points of the epilogues."""
+import math
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+BF = torch.bfloat16
+
+
+def _cabi():
+    from pg_b200 import _cabi as cabi
+    return cabi, cabi.lib(), cabi.stream()
+
+
+def _randn(gen, *shape, std=1.0, dtype=BF):
+    return (torch.randn(shape, device="cuda", generator=gen) * std).to(dtype)
+
+
+def _rel(got, want):
+    return float((got.to(F64) - want).norm() / want.norm())
+
+
+def _gelu(x):
+    return F.gelu(x, approximate="tanh")
+
+
+# bf16 results: every rounding adds at most 2^-9 relative (rms about 2^-10.8), the hardware tanh 2^-11: three roundings of
+# a pairing stay below 4e-3
+@pytest.mark.parametrize("epi", ["geglu", "swiglu"])
+@pytest.mark.parametrize("M,N,K", [(1292, 2048, 256), (1100, 2056, 128), (513, 4096, 72), (385, 8200, 64)])
+def test_gated_pairs(epi, M, N, K):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, w = _randn(g, M, K), _randn(g, 2 * N, K, std=K ** -0.5)
+    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, None, M, N, K, K, K, N, 0, 0,
+                         cabi.EPI_GEGLU if epi == "geglu" else cabi.EPI_SWIGLU, 0, 2, cabi.PG_BF16, st))
+    z = a.to(F64) @ w.to(F64).T
+    want = (_gelu(z[:, :N]) if epi == "geglu" else F.silu(z[:, :N])) * z[:, N:]
+    assert _rel(out[:M], want) < 5e-3
+    assert bool((out[M] == 0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1292, 2048, 512), (1292, 2560, 200), (700, 2048, 1024), (1025, 264, 4096)])
+def test_row_major_pairs_with_residual(M, N, K):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a, w, r = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N)
+    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr(), M, N, K, K, K, N, N, 0, cabi.EPI_RES, 0, 2,
+                         cabi.PG_BF16, st))
+    assert _rel(out[:M], a.to(F64) @ w.to(F64).T + r.to(F64)) < 4e-3
+    assert bool((out[M] == 0).all())
+
+
+@pytest.mark.parametrize("M", [4, 8, 31, 32, 33, 64])
+@pytest.mark.parametrize("N,K,epi", [(2048, 16384, "res"), (2048, 2048, "res"), (2560, 2048, "none"), (2056, 2048, "bias"), (2048, 4104, "res")])
+def test_few_rows_split_over_clusters(M, N, K, epi):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a, w, r, b = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N), _randn(g, N)
+    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    code = {"res": cabi.EPI_RES, "none": cabi.EPI_NONE, "bias": cabi.EPI_BIAS}[epi]
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr() if epi == "bias" else None,
+                         r.data_ptr() if epi == "res" else None, M, N, K, K, K, N, N if epi == "res" else 0, 0, code, 0, 0, cabi.PG_BF16, st))
+    want = a.to(F64) @ w.to(F64).T + (r.to(F64) if epi == "res" else b.to(F64) if epi == "bias" else 0.0)
+    assert _rel(out[:M], want) < 4e-3
+    assert bool((out[M] == 0).all())
+
+
+@pytest.mark.parametrize("act,rel", [("none", 4e-3), ("silu", 5e-3), ("clamped", 6e-3), ("relu2", 6e-3)])
+@pytest.mark.parametrize("rows", [[1200, 0, 257, 1], [256, 256, 512, 1024], [3000, 5], [3, 1, 0, 2, 0, 1, 4, 5]])
+def test_grouped_products(act, rel, rows):
+    """Experts with many rows (CTA pairs), with none, with one, with a row behind a full tile; a handful of rows in all."""
+    cabi, L, st = _cabi()
+    E, N, K, P = len(rows), 328, 192, sum(rows)
+    g = torch.Generator(device="cuda").manual_seed(P)
+    dual = act in ("silu", "clamped")
+    a, w = _randn(g, P, K), _randn(g, E, 2 * N if dual else N, K, std=K ** -0.5)
+    off = torch.tensor([sum(rows[:e]) for e in range(E + 1)], dtype=torch.int32, device="cuda")
+    out = torch.zeros(P + 1, N, dtype=BF, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    code = {"none": cabi.GLU_NONE, "silu": cabi.GLU_SILU, "clamped": cabi.GLU_CLAMPED, "relu2": cabi.ACT_RELU2}[act]
+    cabi.check(L.pg_moe_gemm_act(out.data_ptr(), N, a.data_ptr(), K, None, w.data_ptr(), off.data_ptr(), P, E, N, K, code, 1.5, 2,
+                                 err.data_ptr(), cabi.PG_BF16, st))
+    want = torch.empty(P, N, dtype=F64, device="cuda")
+    for e in range(E):
+        z = a[off[e]:off[e + 1]].to(F64) @ w[e].to(F64).T
+        if act == "silu":
+            z = F.silu(z[:, :N]) * z[:, N:]
+        elif act == "clamped":
+            gt, up = z[:, :N].clamp(max=1.5), z[:, N:].clamp(-1.5, 1.5)
+            z = gt * torch.sigmoid(1.702 * gt) * (up + 1.0)
+        elif act == "relu2":
+            z = z.clamp_min(0.0) ** 2
+        want[off[e]:off[e + 1]] = z
+    assert int(err) == 0
+    assert _rel(out[:P], want) < rel
+    assert bool((out[P] == 0).all())
+
+
+@pytest.mark.parametrize("B,q,T,H,G,hd", [(1, 16, 16, 8, 1, 256), (2, 130, 193, 8, 1, 256), (1, 260, 260, 8, 1, 256), (1, 33, 1000, 4, 2, 256),
+                                          (3, 128, 64, 2, 2, 256)])
+def test_prompt_attention(B, q, T, H, G, hd):
+    """Unmasked attention over pages; scores that grow along the sequence, so that the reference maximum has to follow."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    cols = -(-T // 64)
+    pages = B * cols + 1
+    kp, vp, qq = _randn(g, pages, 64, G * hd), _randn(g, pages, 64, G * hd), _randn(g, B * q, H * hd)
+    pt = torch.randperm(pages, device="cuda", generator=g)[:B * cols].to(torch.int32).view(B, cols)
+    for b in range(B):
+        for c in range(cols):
+            kp[pt[b, c].long()] *= 0.2 + 1.2 * c
+    kvl = torch.full((B,), T - q if T >= q else 0, dtype=torch.int32, device="cuda")
+    add = T - int(kvl[0])
+    out = torch.zeros(B * q, H * hd, dtype=BF, device="cuda")
+    cabi.check(L.pg_attention_tc(out.data_ptr(), H * hd, qq.data_ptr(), B * q, H * hd, 0, kp.data_ptr(), vp.data_ptr(), pages * 64,
+                                 G * hd, 0, 0, hd, 0, pt.data_ptr(), cols, 64, kvl.data_ptr(), 0, add, B, q, H, G, hd, math.sqrt(hd),
+                                 1, cabi.PG_BF16, st))
+    for b in range(B):
+        k, v = (p[pt[b].long()].reshape(-1, G, hd)[:T].to(F64).repeat_interleave(H // G, 1) for p in (kp, vp))
+        s = torch.einsum("qhd,nhd->hqn", qq[b * q:(b + 1) * q].view(q, H, hd).to(F64), k).to(BF).to(F64) / math.sqrt(hd)
+        want = torch.einsum("hqn,nhd->qhd", torch.softmax(s, -1), v).reshape(q, H * hd)
+        # weights and result are rounded to bf16 (2^-9 each at most); a score that rounds the other way moves its weight
+        assert _rel(out[b * q:(b + 1) * q], want) < 8e-3
+
+
+@pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (128, 128, 12, 1), (256, 256, 8, 1), (256, 192, 5, 1)])
+@pytest.mark.parametrize("window,keep,chunk", [(0, 0, 0), (33, 0, 0), (100, 7, 0), (0, 0, 48)])
+def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
+    """Decode-sized ragged steps: positions at the edges of 16-key chunks, pages, windows, blocks and clusters."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + H)
+    pos = [0, 1, 15, 16, 17, 63, 64, 127, 500, 1535]
+    n, cols = len(pos), 24
+    pages = n * cols + 1
+    kp, vp = _randn(g, pages, 64, G * dim), _randn(g, pages, 64, G * vdim)
+    q, gate = _randn(g, n, H * dim), _randn(g, n, H * vdim)
+    pt = torch.randperm(pages, device="cuda", generator=g)[:n * cols].to(torch.int32).view(n, cols)
+    slopes, sink = torch.rand(H, device="cuda", generator=g) * 0.1, torch.randn(H, device="cuda", generator=g)
+    slot, tp = torch.arange(n, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda")
+    out = torch.zeros(n, H * vdim, dtype=BF, device="cuda")
+    cabi.check(L.pg_attention_ragged_masked(out.data_ptr(), H * vdim, q.data_ptr(), H * dim, gate.data_ptr(), H * vdim, 0, kp.data_ptr(), 0,
+                                            vp.data_ptr(), 0, pt.data_ptr(), cols, 64, slot.data_ptr(), tp.data_ptr(), n, H, G, dim, vdim,
+                                            dim ** -0.5, window, keep, chunk, slopes.data_ptr(), 0, None, sink.data_ptr(), None, 0, 1.0,
+                                            None, 0, cabi.PG_BF16, st))
+    for t, p in enumerate(pos):
+        j = torch.arange(p + 1, device="cuda")
+        seen = torch.ones_like(j, dtype=torch.bool)
+        if window:
+            seen = (p - j < window) | (j < keep)
+        if chunk:
+            seen &= j // chunk == p // chunk
+        k, v = (x[pt[t].long()].reshape(-1, G, w)[:p + 1].to(F64).repeat_interleave(H // G, 1) for x, w in ((kp, dim), (vp, vdim)))
+        s = torch.einsum("hd,nhd->hn", q[t].view(H, dim).to(F64), k) * dim ** -0.5 - slopes.to(F64)[:, None] * (p - j)
+        s = torch.cat([s.masked_fill(~seen, -math.inf), sink.to(F64)[:, None]], 1)
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1)[:, :-1], v).reshape(-1) * torch.sigmoid(gate[t].to(F64))
+        assert _rel(out[t], want) < 4e-3          # one rounding of the result; weights are fp32
