@@ -7,8 +7,13 @@
 // stores are coalesced across the warp (consecutive features of one token).
 //   S == 1 : persistent over the N/128 weight tiles (gate/up with the GeGLU pairing, lm_head), double-buffered
 //            accumulators so the epilogue overlaps the next tile's stream;
-//   S  > 1 : a cluster of S CTAs splits K for one weight tile (q/k/v, o_proj, down_proj have 16-20 tiles only);
-//            partial D^T tiles meet in the leader through distributed shared memory.
+//   S  > 1 : a cluster of S CTAs splits K for one weight tile (q/k/v, o_proj, down_proj have 16-20 tiles only).  Every CTA
+//            leaves its partial D^T in its shared memory and finishes the S-th part of the tokens from all of them
+//            (distributed shared memory, summed in rank order).  With S = 8 a CTA keeps to half an SM's shared memory:
+//            clusters of 8 whole SMs do not all fit the GPCs at once.
+// o_proj and down_proj (K 2048 and 16384) together, launches alone with a cold cache: the pair kernel with a workspace and a
+// reduce launch each (gemm_tcgen05_swap.cu) 41.5 us for 8 rows and 42.4 for 32, this 29.0 and 33.3; 10 and 5 us per layer of
+// a captured step.
 #include "tc_common.cuh"
 
 namespace pg {
@@ -35,16 +40,23 @@ __device__ __forceinline__ float4 sn_ld_dsmem_v4(uint32_t local_addr, uint32_t r
   return v;
 }
 
+template <bool DUAL, int NT, int S>
+constexpr int sn_stages() {
+  constexpr int bytes = (DUAL ? 2 : 1) * SN_BM * SN_BK * 2 + (NT * SN_BK * 2 + 1023) / 1024 * 1024;
+  constexpr int n = (S == 8 ? 100 : 200) * 1024 / bytes;
+  return n > 10 ? 10 : n;
+}
+
 // NT: token columns of the accumulator (multiple of 16, <= 256).  S: K split (cluster size).
 template <typename T, int EPI, int NT, int S>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, S == 8 ? 2 : 1)
 gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, SnParams p) {
   constexpr bool DUAL = (EPI == PG_EPI_GEGLU);
   constexpr int NW = DUAL ? 2 : 1;                               // weight tiles per stage
   constexpr int W_BYTES = SN_BM * SN_BK * 2, X_BYTES = NT * SN_BK * 2;
   constexpr int X_PAD = (X_BYTES + 1023) / 1024 * 1024;          // keep every tile 1024-byte aligned
   constexpr int STAGE_BYTES = NW * W_BYTES + X_PAD;
-  constexpr int NSTAGES = (200 * 1024) / STAGE_BYTES > 10 ? 10 : (200 * 1024) / STAGE_BYTES;
+  constexpr int NSTAGES = sn_stages<DUAL, NT, S>();
   constexpr int ACC_COLS = NW * NT;                              // TMEM columns per accumulator stage
   constexpr int TMEM_COLS = 2 * ACC_COLS <= 32 ? 32 : (2 * ACC_COLS <= 64 ? 64 : (2 * ACC_COLS <= 128 ? 128 : (2 * ACC_COLS <= 256 ? 256 : 512)));
   static_assert(2 * ACC_COLS <= 512, "accumulators do not fit TMEM");
@@ -196,49 +208,60 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   } else {
     const int tile = tile_first;
     const bool have_k = kb1 > kb0;
+    constexpr int NC = NT / S;                       // tokens that this CTA finishes
+    const int m0 = (int)crank * NC, n = tile * SN_BM + r;
+    float res[NC];
     if (warp >= 4) {
-      mbar_wait(tfull_bar(0), 0);   // this CTA's MMAs are complete: accumulator final, stage ring idle
-      tc_fence_after();
-      if (crank != 0) {
-#pragma unroll 1
-        for (int c = 0; c < NT / 16; ++c) {
-          float v[16];
-          tmem_ld16(t_lane + c * 16, v);
-          tmem_ld_wait();
+      // the residual is requested before the accumulator is waited for
 #pragma unroll
-          for (int j = 0; j < 16; j += 4)
-            *reinterpret_cast<float4*>(&part[r * PROW + c * 16 + j]) =
-                have_k ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+      for (int j = 0; j < NC; ++j) {
+        const bool have = (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) && n < p.N && m0 + j < p.M;
+        res[j] = have ? to_f<T>(R[(size_t)(m0 + j) * p.ldr + n]) : 0.f;
       }
-    }
-    tc_fence_before();
-    sn_cluster_sync();
-    if (crank == 0 && warp >= 4) {
+      mbar_wait(tfull_bar(0), 0);   // this CTA's MMAs are complete: accumulator final, stage ring idle
       tc_fence_after();
 #pragma unroll 1
       for (int c = 0; c < NT / 16; ++c) {
-        float v[16], u[DUAL ? 16 : 1];
+        float v[16];
         tmem_ld16(t_lane + c * 16, v);
         tmem_ld_wait();
-        float4 pv[S > 1 ? S - 1 : 1][4];
 #pragma unroll
-        for (int peer = 1; peer < S; ++peer)   // all remote loads in flight before the first add
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            pv[peer - 1][j] = sn_ld_dsmem_v4(smem_base + (uint32_t)((r * PROW + c * 16 + 4 * j) * 4), peer);
-#pragma unroll
-        for (int peer = 1; peer < S; ++peer)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            v[4 * j] += pv[peer - 1][j].x; v[4 * j + 1] += pv[peer - 1][j].y;
-            v[4 * j + 2] += pv[peer - 1][j].z; v[4 * j + 3] += pv[peer - 1][j].w;
-          }
-        finish(tile, v, u, c * 16);
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(&part[r * PROW + c * 16 + j]) =
+              have_k ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
     tc_fence_before();
     sn_cluster_sync();
+    if (warp >= 4 && m0 < p.M) {
+      float v[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] = 0.f;
+#pragma unroll
+      for (int j = 0; j < NC; j += 4) {
+        float4 pv[S];
+#pragma unroll
+        for (int peer = 0; peer < S; ++peer)          // all loads in flight before the first add
+          pv[peer] = sn_ld_dsmem_v4(smem_base + (uint32_t)((r * PROW + m0 + j) * 4), peer);
+#pragma unroll
+        for (int peer = 0; peer < S; ++peer) { v[j] += pv[peer].x; v[j + 1] += pv[peer].y; v[j + 2] += pv[peer].z; v[j + 3] += pv[peer].w; }
+      }
+      if (n < p.N) {
+        float bn = 0.f;
+        if (EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES) bn = to_f<T>(bias[n]);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          const int m = m0 + j;
+          if (m >= p.M) break;
+          float x = rnd<T>(v[j] + bn);
+          if (EPI == PG_EPI_BIAS_GELU) x = rnd<T>(gelu_tanh_fast(x));
+          if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) x = rnd<T>(x + res[j]);
+          if (p.out_f32) Cf[(size_t)m * p.ldc + n] = x;
+          else Ct[(size_t)m * p.ldc + n] = from_f<T>(x);
+        }
+      }
+    }
+    sn_cluster_sync();               // nobody leaves while a peer may still read its shared memory
   }
   tc_fence_before();
   __syncthreads();
@@ -253,7 +276,7 @@ static int launch_sn(const CUtensorMap& mx, const CUtensorMap& mw, const SnParam
   constexpr bool DUAL = (EPI == PG_EPI_GEGLU);
   constexpr int X_PAD = (NT * SN_BK * 2 + 1023) / 1024 * 1024;
   constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * SN_BM * SN_BK * 2 + X_PAD;
-  constexpr int NSTAGES = (200 * 1024) / STAGE_BYTES > 10 ? 10 : (200 * 1024) / STAGE_BYTES;
+  constexpr int NSTAGES = sn_stages<DUAL, NT, S>();
   const size_t smem = 1024 + (size_t)NSTAGES * STAGE_BYTES + 8 * (2 * NSTAGES + 4) + 16;
   auto kern = gemm_tc_skinny_kernel<T, EPI, NT, S>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -286,15 +309,13 @@ static int launch_sn_nt(const CUtensorMap& mx, const CUtensorMap& mw, const SnPa
 }  // namespace tc
 
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
-  // Measured on the batch-32 decode step (tools/kernel_sweep.py, SWEEP_B=32): the swap-AB stream wins where a CTA
-  // owns whole weight tiles (gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us) and for q/k/v (9.9 vs 18.3 us); with a
-  // residual epilogue and a K split (o_proj, down_proj: 16 tiles) the row-major split-K kernel is faster.
+  // Up to 64 rows the swap-AB stream takes every projection; above, where a stage is mostly tokens, the ones whose CTAs own
+  // whole weight tiles (batch 32: gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us, q/k/v 9.9 vs 18.3 us on the row-major kernel).
   static const int mode = env_int("PG_SKINNY", 1);   // 0 off, 1 where it wins, 2 everywhere it applies
   if (!mode || M < 4 || M > 128 || N < 512 || K < 256 || epi < PG_EPI_NONE || epi > PG_EPI_GEGLU) return false;
   if (mode == 2) return true;
   const int n_tiles = cdiv(N, 128);
-  // up to 8 rows the swap-AB stream also wins for the residual projections (batch 8 step: 1.92 vs 2.00 ms)
-  return epi == PG_EPI_GEGLU || epi == PG_EPI_NONE || n_tiles >= 100 || M <= 8;
+  return epi == PG_EPI_GEGLU || epi == PG_EPI_NONE || n_tiles >= 100 || M <= 64;
 }
 
 int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
@@ -302,10 +323,10 @@ int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, cons
   const bool bf = dtype == PG_BF16;
   const int nt = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   const int n_tiles = cdiv(N, tc::SN_BM), kb = cdiv(K, tc::SN_BK);
-  // split K across a cluster until ~148 CTAs stream (each keeps >= 8 K blocks)
+  // split K across a cluster until ~148 CTAs stream (each keeps >= 4 K blocks)
   int s = 1;
   if (epi != PG_EPI_GEGLU)
-    while (s < 4 && n_tiles * s * 2 <= 160 && kb / (s * 2) >= 8) s *= 2;
+    while (s < 8 && n_tiles * s * 2 <= 160 && kb / (s * 2) >= 4) s *= 2;
   CUtensorMap mx, mw;
   const int w_rows = (epi == PG_EPI_GEGLU) ? 2 * N : N;
   PG_REQUIRE(tc::make_map_2d(&mx, A, M, K, lda, nt, bf) && tc::make_map_2d(&mw, W, w_rows, K, ldw, tc::SN_BM, bf),
