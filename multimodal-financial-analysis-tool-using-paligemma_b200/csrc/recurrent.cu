@@ -273,10 +273,11 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //                                       a thread owns rows 4 (m RG + rg) + e of both.  What bounds it is issue slots: a
 //                                       token costs a multiply and two fused multiply-adds per state element, so they run
 //                                       on pairs of rows (fma.rn.f32x2: the same roundings, half the instructions), the
-//                                       q and k a thread reads serve two columns, and the two column sums meet in
-//                                       log2(RG) shuffles together.  The records of the next CH tokens arrive by cp.async
+//                                       q and k a thread reads serve two columns, and a batch of RG / 2 tokens shares
+//                                       its shuffles (a token at a time, each with log2(RG) shuffles behind it, left the
+//                                       warps waiting on one another's latencies: 787 us).  The records of the next CH tokens arrive by cp.async
 //                                       into the other half of a double buffer.  4 x 2048 tokens, 16 heads of 128: one
-//                                       column per thread and scalar arithmetic 842 us, this 787 us.
+//                                       column per thread and scalar arithmetic 842 us, this 638 us.
 //                                       The state is read from and written back to the slot once per launch, which
 //                                       makes a prompt portion and a single decoded token the same case and the
 //                                       result independent of where the sequence was cut.
@@ -562,44 +563,74 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   };
   fetch(0, 0);
   int buf = 0;
-  const bool second = (rg & 1) != 0;                // the column whose sum this lane ends up with
-  const bool writes = rg < 2 && j + rg < vdim;
-  float* orow = out + (size_t)row0 * heads * vdim + (size_t)h * vdim + j + (second ? 1 : 0);
+  // A batch of RG / 2 tokens has as many column sums as a column's lanes: a transposed butterfly (RG - 1 shuffles) leaves lane rg
+  // with the sum of token rg / 2, column rg & 1.  A batch's tokens have no shuffle between them, so their shared-memory
+  // reads and multiplications overlap.
+  constexpr int TB = RG / 2;
+  const int my_c = rg & 1;
+  const bool live = j + my_c < vdim;
+  float* orow = out + (size_t)row0 * heads * vdim + (size_t)h * vdim + j + my_c;
   const size_t ostep = (size_t)heads * vdim;
+  auto token = [&](const float* r, float& c0, float& c1) {         // one token's update and this thread's part of its outputs
+    const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
+    const f32x2 v0 = pair_of(vj.x, vj.x), v1 = pair_of(vj.y, vj.y);
+    const float lam = TD ? r[NV * DMAX + VT] : lam_h;
+    const f32x2 lam2 = pair_of(lam, lam);
+    f32x2 o0[2] = {0ull, 0ull}, o1[2] = {0ull, 0ull};
+#pragma unroll
+    for (int m = 0; m < NG; ++m) {
+      const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(r + 4 * rg + 4 * RG * m);
+      const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(r + DMAX + 4 * rg + 4 * RG * m);
+      ulonglong2 a4 = make_ulonglong2(lam2, lam2);
+      if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r + 2 * DMAX + 4 * rg + 4 * RG * m);   // decays per key channel
+      S[0][2 * m] = fma2(k4.x, v0, mul2(a4.x, S[0][2 * m]));
+      S[0][2 * m + 1] = fma2(k4.y, v0, mul2(a4.y, S[0][2 * m + 1]));
+      S[1][2 * m] = fma2(k4.x, v1, mul2(a4.x, S[1][2 * m]));
+      S[1][2 * m + 1] = fma2(k4.y, v1, mul2(a4.y, S[1][2 * m + 1]));
+      o0[0] = fma2(q4.x, S[0][2 * m], o0[0]);
+      o0[1] = fma2(q4.y, S[0][2 * m + 1], o0[1]);
+      o1[0] = fma2(q4.x, S[1][2 * m], o1[0]);
+      o1[1] = fma2(q4.y, S[1][2 * m + 1], o1[1]);
+    }
+    const float2 a0 = halves_of(o0[0]), a1 = halves_of(o0[1]), b0 = halves_of(o1[0]), b1 = halves_of(o1[1]);
+    c0 = (a0.x + a0.y) + (a1.x + a1.y);
+    c1 = (b0.x + b0.y) + (b1.x + b1.y);
+  };
+  auto gather = [&](float (&c)[RG]) {
+#pragma unroll
+    for (int w = RG / 2; w >= 1; w >>= 1) {
+      const bool up = (rg & w) != 0;
+#pragma unroll
+      for (int i = 0; i < w; ++i) {
+        const float keep = up ? c[i + w] : c[i], send = up ? c[i] : c[i + w];
+        c[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+      }
+    }
+  };
   for (int t0 = 0; t0 < n; t0 += CH, buf ^= 1) {
     const int nt = min(CH, n - t0);
     if (t0 + CH < n) { fetch(t0 + CH, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
     __syncthreads();
-#pragma unroll 4
-    for (int tt = 0; tt < nt; ++tt) {
-      const float* r = sh + ((size_t)buf * CH + tt) * RSZ;
-      const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
-      const f32x2 v0 = pair_of(vj.x, vj.x), v1 = pair_of(vj.y, vj.y);
-      const float lam = TD ? r[NV * DMAX + VT] : lam_h;
-      const f32x2 lam2 = pair_of(lam, lam);
-      f32x2 o0[2] = {0ull, 0ull}, o1[2] = {0ull, 0ull};
+    const float* r0 = sh + (size_t)buf * CH * RSZ;
+    int tt = 0;
+    for (; tt + TB <= nt; tt += TB) {
+      float c[RG];
 #pragma unroll
-      for (int m = 0; m < NG; ++m) {
-        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(r + 4 * rg + 4 * RG * m);
-        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(r + DMAX + 4 * rg + 4 * RG * m);
-        ulonglong2 a4 = make_ulonglong2(lam2, lam2);
-        if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r + 2 * DMAX + 4 * rg + 4 * RG * m);   // decays per key channel
-        S[0][2 * m] = fma2(k4.x, v0, mul2(a4.x, S[0][2 * m]));
-        S[0][2 * m + 1] = fma2(k4.y, v0, mul2(a4.y, S[0][2 * m + 1]));
-        S[1][2 * m] = fma2(k4.x, v1, mul2(a4.x, S[1][2 * m]));
-        S[1][2 * m + 1] = fma2(k4.y, v1, mul2(a4.y, S[1][2 * m + 1]));
-        o0[0] = fma2(q4.x, S[0][2 * m], o0[0]);
-        o0[1] = fma2(q4.y, S[0][2 * m + 1], o0[1]);
-        o1[0] = fma2(q4.x, S[1][2 * m], o1[0]);
-        o1[1] = fma2(q4.y, S[1][2 * m + 1], o1[1]);
+      for (int b = 0; b < TB; ++b) token(r0 + (size_t)(tt + b) * RSZ, c[2 * b], c[2 * b + 1]);
+      gather(c);
+      const int mine = tt + rg / 2;
+      if (live) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
+    }
+    if (tt < nt) {                                  // the last tokens of the segment
+      float c[RG];
+#pragma unroll
+      for (int b = 0; b < TB; ++b) {
+        c[2 * b] = c[2 * b + 1] = 0.f;
+        if (tt + b < nt) token(r0 + (size_t)(tt + b) * RSZ, c[2 * b], c[2 * b + 1]);
       }
-      const float2 a0 = halves_of(o0[0]), a1 = halves_of(o0[1]), b0 = halves_of(o1[0]), b1 = halves_of(o1[1]);
-      const float c0 = (a0.x + a0.y) + (a1.x + a1.y), c1 = (b0.x + b0.y) + (b1.x + b1.y);
-      // lanes with an even rg collect column j, the others column j + 1
-      float o = (second ? c1 : c0) + __shfl_xor_sync(0xffffffffu, second ? c0 : c1, 1);
-#pragma unroll
-      for (int sh_ = 2; sh_ < RG; sh_ <<= 1) o += __shfl_xor_sync(0xffffffffu, o, sh_);
-      if (writes) orow[(size_t)(t0 + tt) * ostep] = fmaf(skip_h, second ? vj.y : vj.x, o);
+      gather(c);
+      const int mine = tt + rg / 2;
+      if (live && mine < nt) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
     }
     __syncthreads();                                // every thread is done with this buffer before it is refilled
   }
