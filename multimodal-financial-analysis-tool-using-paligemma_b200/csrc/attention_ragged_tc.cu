@@ -13,11 +13,11 @@
 // What bounds it: the softmax's instructions (about 8 per score) and the exponentials; the tiles' products and copies
 // run beside them, and the two CTAs of an SM fill each other's waits.  Most tiles lie wholly inside the causal window of
 // all 128 rows and take a loop without masks.  The two-pass form before it (row maximum first, S computed twice, P through
-// shared memory, masks on every score) took 557 us for 4 prompts of 2048 tokens, 16 heads of 128, window 1024; this takes 248 us.
+// shared memory, masks on every score) took 557 us for 4 prompts of 2048 tokens, 16 heads of 128, window 1024; this takes 218 us (246 with
+// the pages walked oldest first).
 // Epilogue: O / sum, times sigmoid(gate), rounded once.  Key width and value width are independent multiples of 64.
 // Extensions (pg_attention_ragged_tc_ex): keep_first > 0 keeps the first keep_first positions visible behind the
-// window: the key tiles are then the pages that hold them (as far as they lie before the window's first page)
-// followed by the window's pages.  sigmoid_weights: p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
+// window: the window's pages are then followed by those that hold them (as far as they lie before the window's first page).  sigmoid_weights: p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
 // gate may be one value per (token, head); the result is multiplied by out_scale before it is rounded.
 // pg_attention_ragged_tc_capped adds a query temperature and a softcap (both fp32, as in attention_ragged.cu; the kernel is
 // instantiated with and without the cap).  A capped score is bounded, so its softmax needs no maximum: with a cap of at
@@ -114,10 +114,12 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;               // first one
   if (p.chunk > 0) lo = max(lo, pos0 / p.chunk * p.chunk);               // the block of the tile's first row
   const int t_lo = lo / WK;
-  // pages of the kept first positions that lie before the window's first page, then the window's pages
+  // The window's pages from the newest to the oldest, then the pages of the kept first positions that lie before them: a distance
+  // bias makes the newest keys the largest, so that a row's reference maximum stands after its own page.  (From the oldest on,
+  // it rises by 92 slope per page: heads with slopes above 0.09 rescaled O on every tile, and 556 -> 248 us was all.)
   const int n_keep = (p.keep_first > 0 && p.window > 0) ? min((p.keep_first + WK - 1) / WK, t_lo) : 0;
-  const int n_tiles = n_keep + hi / WK - t_lo + 1;
-  auto page_of = [&](int t) { return t < n_keep ? t : t_lo + (t - n_keep); };   // key tile -> page of the sequence
+  const int t_hi = hi / WK, n_win = t_hi - t_lo + 1, n_tiles = n_keep + n_win;
+  auto page_of = [&](int t) { return t < n_win ? t_hi - t : t - n_win; };       // key tile -> page of the sequence
   const int32_t* pt_row = p.page_table + (size_t)slot * p.pt_stride;
   const bool sig = p.sigmoid_weights != 0, fixed_max = sig || (CAP && p.bounded);
 
