@@ -303,10 +303,9 @@ int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, cons
 bool gemm_tc_2cta_wanted(int M, int N, int K, int epi);
 int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                  int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st);
-int gemm_tc_splitk_factor(int M, int N, int K, int epi, int* bn_out);
+int gemm_tc_splitk_factor(int M, int N, int K, int epi);
 int gemm_tc_splitk(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int bn, int s,
-                   cudaStream_t st);
+                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int s, cudaStream_t st);
 
 int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
             int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st) {
@@ -326,9 +325,8 @@ int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void*
   if (res_mod == 0 && gemm_tc_skinny_wanted(M, N, K, epi))  // a few dozen token rows: stream the weights (swap-AB)
     return gemm_tc_skinny(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, epi, out_f32, dtype, st);
   {
-    int sk_bn = 0;
-    const int s = gemm_tc_splitk_factor(M, N, K, epi, &sk_bn);  // few tiles, long K: a cluster shares each tile
-    if (s) return gemm_tc_splitk(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, sk_bn, s, st);
+    const int s = gemm_tc_splitk_factor(M, N, K, epi);  // few tiles: a cluster shares each tile
+    if (s) return gemm_tc_splitk(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, s, st);
   }
   if (!(dual && out_f32) && gemm_tc_2cta_wanted(M, N, K, epi))  // fewer staged bytes per wave: CTA pairs (cta_group::2)
     return gemm_tc_2cta(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, st);

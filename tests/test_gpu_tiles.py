@@ -161,3 +161,27 @@ def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
         s = torch.cat([s.masked_fill(~seen, -math.inf), sink.to(F64)[:, None]], 1)
         want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1)[:, :-1], v).reshape(-1) * torch.sigmoid(gate[t].to(F64))
         assert _rel(out[t], want) < 4e-3          # one rounding of the result; weights are fp32
+
+
+@pytest.mark.parametrize("M", [16, 129, 256, 260, 384])
+@pytest.mark.parametrize("N,K,epi", [(1152, 4304, "bias_res"), (2048, 2048, "res"), (2560, 2048, "none"), (1160, 1152, "bias_gelu"),
+                                     (520, 1096, "f32")])
+def test_few_tiles_split_over_clusters(M, N, K, epi):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, w, r, b = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N), _randn(g, N)
+    f32 = epi == "f32"
+    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else BF, device="cuda")
+    code = {"res": cabi.EPI_RES, "bias_res": cabi.EPI_BIAS_RES, "bias_gelu": cabi.EPI_BIAS_GELU}.get(epi, cabi.EPI_NONE)
+    has_b, has_r = epi.startswith("bias"), epi.endswith("res")
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr() if has_b else None, r.data_ptr() if has_r else None, M, N,
+                         K, K, K, N, N if has_r else 0, 0, code, 1 if f32 else 0, 2, cabi.PG_BF16, st))
+    want = a.to(F64) @ w.to(F64).T
+    if has_b:
+        want = want + b.to(F64)
+    if epi == "bias_gelu":
+        want = _gelu(want)
+    if has_r:
+        want = want + r.to(F64)
+    assert _rel(out[:M], want) < 4e-3          # at most three roundings of 2^-9 and the hardware tanh
+    assert bool((out[M] == 0).all())
