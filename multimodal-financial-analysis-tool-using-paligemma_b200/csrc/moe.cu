@@ -11,7 +11,11 @@
 //                   silu(A Wg^T) * (A Wu^T) of stacked [Wg; Wu] weights, or with max(A W^T, 0)^2
 //   pg_moe_combine  x[t] += sum_k w_k * (k-th expert's output, or the token's own input for an identity expert)
 //                           + gate[t] * shared[t]
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pg {
 
@@ -402,37 +406,81 @@ moe_route_topk_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w
   }
 }
 
-// ------------------------------------------------------------------ group the pairs by expert (one CTA)
-__global__ void moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restrict__ sorted_row,
-                                int32_t* __restrict__ pair_pos, const int32_t* __restrict__ topk_idx, int n_pairs,
-                                int top, int n_experts) {
+// ------------------------------------------------------------------ group the pairs by expert (one cluster)
+// A cluster of `CTAs` (1 or 8) takes the pairs in equal consecutive parts.  One shared-memory atomic per pair counts it and gives
+// its place among its CTA's pairs of the expert; the CTAs read each other's counts through distributed shared memory for the
+// first position of every (expert, CTA).  One CTA alone is bound by its own atomics and scattered stores: 16384 pairs of 16
+// experts 15.1 us (16.4 with one atomic per pair on eight counters per expert, 22.9 with lanes grouped by match.any),
+// this 6.7 us with eight.
+constexpr int SORT_ITEMS = 16, SORT_CTAS = 8, SORT_THREADS = 256;
+
+__global__ void __launch_bounds__(SORT_THREADS)
+moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restrict__ sorted_row, int32_t* __restrict__ pair_pos,
+                const int32_t* __restrict__ topk_idx, int n_pairs, int top, int n_experts) {
   extern __shared__ int sm_i[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ctas = (int)gridDim.x, rank = (int)blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
-  int* count = sm_i;                   // [n_experts]
-  int* cursor = sm_i + n_experts;      // [n_experts]
-  for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
+  int* count = sm_i;                   // [n_experts]: this CTA's pairs of an expert (read by the other CTAs)
+  int* first = sm_i + n_experts;       // [n_experts]: position of the first of them
+  for (int e = threadIdx.x; e < n_experts; e += SORT_THREADS) count[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = topk_idx[i];
-    if (e >= 0 && e < n_experts) atomicAdd(&count[e], 1);
+  constexpr int ROUND = SORT_ITEMS * SORT_THREADS;
+  const int per = (n_pairs + ctas - 1) / ctas, begin = rank * per, end = min(n_pairs, begin + per);
+  const bool one_round = per <= ROUND;
+  int ex[SORT_ITEMS], place[SORT_ITEMS];
+  for (int i0 = begin; i0 < end; i0 += ROUND) {
+#pragma unroll
+    for (int k = 0; k < SORT_ITEMS; ++k) {          // a round's loads are in flight together
+      const int i = i0 + k * SORT_THREADS + threadIdx.x;
+      const int e = i < end ? topk_idx[i] : -1;
+      ex[k] = e >= 0 && e < n_experts ? e : -1;     // -1: no place in the grouped order
+    }
+#pragma unroll
+    for (int k = 0; k < SORT_ITEMS; ++k) {
+      const int i = i0 + k * SORT_THREADS + threadIdx.x;
+      place[k] = ex[k] >= 0 ? atomicAdd(&count[ex[k]], 1) : -1;
+      if (!one_round && i < end) pair_pos[i] = place[k];   // this thread takes it up again below
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < n_experts; ++e) { offsets[e] = acc; cursor[e] = acc; acc += count[e]; }
-    offsets[n_experts] = acc;
+  if (ctas > 1) cluster.sync(); else __syncthreads();    // every CTA's counts are complete
+  if (threadIdx.x < 32) {              // prefix over the experts, 32 at a time, and over the CTAs inside an expert
+    const int lane = threadIdx.x;
+    int base = 0;
+    for (int e0 = 0; e0 < n_experts; e0 += 32) {
+      int total = 0, before = 0;
+      if (e0 + lane < n_experts)
+        for (int c = 0; c < ctas; ++c) {
+          const int n = ctas > 1 ? *cluster.map_shared_rank(count + e0 + lane, c) : count[e0 + lane];
+          total += n;
+          if (c < rank) before += n;
+        }
+      int inc = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
+      if (e0 + lane < n_experts) {
+        first[e0 + lane] = base + inc - total + before;
+        if (rank == 0) offsets[e0 + lane] = base + inc - total;
+      }
+      base += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (rank == 0 && lane == 0) offsets[n_experts] = base;
   }
-  __syncthreads();
+  if (ctas > 1) cluster.sync(); else __syncthreads();    // `first` is there; nobody reads another CTA's counts any more
   // the order of the pairs inside a group does not change any result: every output row is computed on its own
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = topk_idx[i];
-    if (e >= 0 && e < n_experts) {
-      const int pos = atomicAdd(&cursor[e], 1);
-      sorted_row[pos] = i / top;
+  for (int i0 = begin; i0 < end; i0 += ROUND) {
+#pragma unroll
+    for (int k = 0; k < SORT_ITEMS; ++k) {
+      const int i = i0 + k * SORT_THREADS + threadIdx.x;
+      if (i >= end) break;
+      if (!one_round) {
+        place[k] = pair_pos[i];
+        ex[k] = place[k] >= 0 ? topk_idx[i] : -1;
+      }
+      const int pos = place[k] >= 0 ? first[ex[k]] + place[k] : -1;
+      if (pos >= 0) sorted_row[pos] = i / top;
       pair_pos[i] = pos;
-    } else {
-      pair_pos[i] = -1;
     }
   }
 }
@@ -442,8 +490,6 @@ __global__ void moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restri
 // grouped before the first layer runs: CTA l handles layer l.  desc[l] = {first entry of the layer's table in `tables`,
 // experts, top, sum of the earlier layers' top, sum of the earlier layers' (experts + 1)}.  Layer l's pair_pos starts at
 // n_tokens * desc[l][3], its offsets at desc[l][4].  An id outside the vocabulary gets no place (-1).
-constexpr int SORT_ITEMS = 16;
-
 __global__ void __launch_bounds__(1024)
 moe_table_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restrict__ pair_pos, const int32_t* __restrict__ tables,
                       const int32_t* __restrict__ desc, const int64_t* __restrict__ ids, int n_tokens, long long vocab,
@@ -749,8 +795,33 @@ extern "C" int pg_moe_route(int32_t* topk_idx, float* topk_w, float* shared_gate
 extern "C" int pg_moe_sort(int32_t* offsets, int32_t* sorted_row, int32_t* pair_pos, const int32_t* topk_idx,
                            int n_pairs, int top, int n_experts, void* stream) {
   PG_REQUIRE(n_experts >= 1 && n_experts <= 4096 && top >= 1, "moe_sort: %d experts, top %d", n_experts, top);
-  return launch_pdl("moe_sort", moe_sort_kernel, dim3(1), dim3(1024), sizeof(int) * 2 * (size_t)n_experts,
-                    (cudaStream_t)stream, offsets, sorted_row, pair_pos, topk_idx, n_pairs, top, n_experts);
+  // eight CTAs from the count on at which one would walk several pairs per thread
+  const int ctas = n_pairs > 4 * SORT_THREADS ? SORT_CTAS : 1;
+  if (ctas == 1)
+    return launch_pdl("moe_sort", moe_sort_kernel, dim3(1), dim3(SORT_THREADS), sizeof(int) * 2 * (size_t)n_experts,
+                      (cudaStream_t)stream, offsets, sorted_row, pair_pos, topk_idx, n_pairs, top, n_experts);
+  static const int pdl = env_int("PG_PDL", 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(SORT_THREADS);
+  cfg.dynamicSmemBytes = sizeof(int) * 2 * (size_t)n_experts;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, moe_sort_kernel, offsets, sorted_row, pair_pos, topk_idx, n_pairs, top, n_experts);
+  if (err != cudaSuccess) {
+    set_error("moe_sort launch: %s", cudaGetErrorString(err));
+    cudaGetLastError();
+    return PG_ERR_CUDA;
+  }
+  return check_launch("moe_sort");
 }
 
 extern "C" int pg_moe_table_sort(int32_t* offsets, int32_t* pair_pos, const int32_t* tables, const int32_t* desc, int n_layers,

@@ -43,20 +43,21 @@ struct TileCursor {
   const int32_t* off;
   int n_experts, n_tiles_n, e, first;   // first = number of the first tile of expert e
   int fixed;                            // > 0: every group has this many rows (off is not read)
-  __device__ __forceinline__ TileCursor(const int32_t* o, int ne, int ntn, int fx = 0)
-      : off(o), n_experts(ne), n_tiles_n(ntn), e(0), first(0), fixed(fx) {}
+  int bm;                               // rows of a tile
+  __device__ __forceinline__ TileCursor(const int32_t* o, int ne, int ntn, int fx = 0, int rows = MG_BM)
+      : off(o), n_experts(ne), n_tiles_n(ntn), e(0), first(0), fixed(fx), bm(rows) {}
   __device__ __forceinline__ int at(int i) const { return fixed > 0 ? i * fixed : off[i]; }
   // -> false when the sequence is exhausted
   __device__ __forceinline__ bool seek(int tile, int& expert, int& m0, int& m_end, int& n_blk) {
     while (e < n_experts) {
       const int rows = at(e + 1) - at(e);
-      const int mt = (rows + MG_BM - 1) / MG_BM;
+      const int mt = (rows + bm - 1) / bm;
       const int cnt = mt * n_tiles_n;
       if (tile < first + cnt) {
         const int i = tile - first;
         expert = e;
         n_blk = i / mt;
-        m0 = at(e) + (i % mt) * MG_BM;
+        m0 = at(e) + (i % mt) * bm;
         m_end = at(e + 1);
         return true;
       }
@@ -66,6 +67,24 @@ struct TileCursor {
     return false;
   }
 };
+
+// One output value from its accumulator(s): the rounding points of moe_gemm_simt_kernel.
+template <typename T, bool DUAL>
+__device__ __forceinline__ float moe_activate(const MoeParams& p, float x, float u) {
+  if (!DUAL && p.act == PG_ACT_RELU2) { x = fmaxf(x, 0.f); return x * x; }
+  x = rnd<T>(x);
+  if (DUAL) {
+    float uu = rnd<T>(u);
+    if (p.act == PG_GLU_CLAMPED) {
+      x = fminf(x, p.limit);
+      uu = fminf(fmaxf(uu, -p.limit), p.limit);
+      x = rnd<T>(x / (1.f + __expf(-1.702f * x))) * (uu + 1.f);
+    } else {
+      x = rnd<T>(rnd<T>(x / (1.f + __expf(-x))) * uu);
+    }
+  }
+  return x;
+}
 
 template <typename T, bool DUAL, int BN>
 __global__ void __launch_bounds__(MG_THREADS, 1)
@@ -198,22 +217,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
             float o[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float x = v[j0 + j];
-              if (!DUAL && p.act == PG_ACT_RELU2) { x = fmaxf(x, 0.f); o[j] = x * x; continue; }
-              x = rnd<T>(x);
-              if (DUAL) {
-                float uu = rnd<T>(u[DUAL ? j0 + j : 0]);
-                if (p.act == PG_GLU_CLAMPED) {
-                  x = fminf(x, p.limit);
-                  uu = fminf(fmaxf(uu, -p.limit), p.limit);
-                  x = rnd<T>(x / (1.f + __expf(-1.702f * x))) * (uu + 1.f);
-                } else {
-                  x = rnd<T>(rnd<T>(x / (1.f + __expf(-x))) * uu);
-                }
-              }
-              o[j] = x;
-            }
+            for (int j = 0; j < 8; ++j) o[j] = moe_activate<T, DUAL>(p, v[j0 + j], u[DUAL ? j0 + j : 0]);
             *reinterpret_cast<uint4*>(out + o_at + n0 + j0) = pack<T>(o);
           }
         }
@@ -252,6 +256,182 @@ static int launch_moe(const CUtensorMap& ma, const CUtensorMap& mw, const MoePar
                    ma, mw, p);
 }
 
+// ------------------------------------------------------------------ many rows per expert: CTA pairs
+// The same grouped product on tcgen05.mma.cta_group::2 for experts with hundreds of rows each: a tile is 256 rows of one expert x
+// 256 weight rows (gated: 128 gate and 128 up rows, the pair's first CTA stages the gate half, the second the up half, so that
+// either accumulator holds [gate | up] of its 128 rows).  An SM is paced by the bytes it pulls from L2: 32 KB per k-block for
+// twice the product of the single-CTA kernel's 32 KB (48 KB gated).  16384 rows of 16 experts, width 2048, ff 2048:
+// gate/up 253 -> 226 us, down 169 -> 106 us.  Eight epilogue warps write whole 128-byte row pieces through a staging tile.
+constexpr int M2_STAGES = 6, M2_THREADS = 384, M2_EPI_WARPS = 8, M2_STG_BYTES = 32 * 128, M2_BN = 256;
+constexpr int M2_W_BYTES = (M2_BN / 2) * MG_BK * 2, M2_STAGE_BYTES = MG_A_BYTES + M2_W_BYTES;
+
+template <typename T, bool DUAL>
+__global__ void __launch_bounds__(M2_THREADS, 1)
+moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, MoeParams p) {
+  constexpr int TILE_N = DUAL ? M2_BN / 2 : M2_BN;   // output columns of a tile
+  constexpr uint32_t IDESC = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * MG_BM, M2_BN);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t stg_base = smem_base + M2_STAGES * M2_STAGE_BYTES;
+  const uint32_t bars = stg_base + M2_EPI_WARPS * M2_STG_BYTES;
+  auto full_bar = [&](int s) { return bars + 8u * s; };                       // used in the leader CTA
+  auto empty_bar = [&](int s) { return bars + 8u * (M2_STAGES + s); };        // one per CTA
+  auto tfull_bar = [&](int a) { return bars + 8u * (2 * M2_STAGES + a); };    // one per CTA
+  auto tempty_bar = [&](int a) { return bars + 8u * (2 * M2_STAGES + 2 + a); };  // used in the leader CTA
+  const uint32_t tmem_slot = bars + 8u * (2 * M2_STAGES + 4);
+  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  __shared__ int s_fail;
+  volatile int* fail = &s_fail;
+  if (threadIdx.x == 0) s_fail = 0;
+
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t crank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+  const bool leader = crank == 0;
+  const int n_tiles_n = (p.N + TILE_N - 1) / TILE_N, k_blocks = (p.K + MG_BK - 1) / MG_BK;
+  const int rows_per_expert = DUAL ? 2 * p.N : p.N;
+  const int sched_first = (int)(blockIdx.x / 2), sched_stride = (int)(gridDim.x / 2);
+
+  if (warp == 0 && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
+  }
+  if (warp == 1 && lane == 0) {
+    for (int s = 0; s < M2_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 2 * M2_EPI_WARPS); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(MG_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer's barriers and TMEM exist before anything lands on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot_ptr;
+  pdl_wait();  // the offsets and the grouped rows come from the preceding kernels
+  int e, m0, m_end, n_blk;
+
+  if (warp == 0 && lane == 0) {
+    // ===================== TMA producer (both CTAs) =====================
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    TileCursor cur(p.offsets, p.n_experts, n_tiles_n, 0, 2 * MG_BM);
+    for (int tile = sched_first; ok && cur.seek(tile, e, m0, m_end, n_blk); tile += sched_stride) {
+      const int w_row = e * rows_per_expert + n_blk * TILE_N + (int)crank * (DUAL ? p.N : M2_BN / 2);
+      const int a_row = m0 + (int)crank * MG_BM;      // rows behind the expert's last one are another's: computed, not stored
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_lim(empty_bar(stage), phase ^ 1, fail)) { ok = false; break; }
+        const uint32_t sa = smem_base + stage * M2_STAGE_BYTES;
+        const uint32_t full_leader = mapa_u32(full_bar(stage), 0);
+        if (leader) mbar_expect_tx(full_bar(stage), 2 * M2_STAGE_BYTES);  // both CTAs' bytes
+        tma_load_2d_cg2(sa, &map_a, full_leader, kb * MG_BK, a_row);
+        tma_load_2d_cg2(sa + MG_A_BYTES, &map_w, full_leader, kb * MG_BK, w_row);
+        if (++stage == M2_STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1 && lane == 0 && leader) {
+    // ===================== MMA issuer (leader CTA only) =====================
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    TileCursor cur(p.offsets, p.n_experts, n_tiles_n, 0, 2 * MG_BM);
+    for (int tile = sched_first; ok && cur.seek(tile, e, m0, m_end, n_blk); tile += sched_stride) {
+      if (!mbar_wait_lim(tempty_bar(acc), acc_phase ^ 1, fail)) break;   // both CTAs' epilogues have drained it
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * M2_BN;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_lim(full_bar(stage), phase, fail)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = smem_base + stage * M2_STAGE_BYTES;
+#pragma unroll
+        for (int k = 0; k < MG_BK / 16; ++k)
+          umma_cg2(d_tmem, umma_desc(sa + k * 32), umma_desc(sa + MG_A_BYTES + k * 32), IDESC, (kb > 0 || k > 0) ? 1u : 0u);
+        umma_commit_cg2(empty_bar(stage), (uint16_t)0x3);  // the stage is free in BOTH CTAs once these MMAs have read it
+        if (++stage == M2_STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      umma_commit_cg2(tfull_bar(acc), (uint16_t)0x3);       // accumulator complete, in both CTAs' TMEM
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+    }
+  } else if (warp >= 4) {
+    // ===================== epilogue: TMEM -> staging -> global (both CTAs) =====================
+    const int q = warp & 3, half = (warp - 4) >> 2;          // TMEM lane quarter, column half
+    const int ch_l = lane & 7, r_l = lane >> 3;              // staging <-> global mapping: 8 lanes per 128-byte row piece
+    uint8_t* wbuf = smem_raw + (stg_base - smem_u32(smem_raw)) + (warp - 4) * M2_STG_BYTES;
+    T* out = reinterpret_cast<T*>(p.out);
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    TileCursor cur(p.offsets, p.n_experts, n_tiles_n, 0, 2 * MG_BM);
+    for (int tile = sched_first; cur.seek(tile, e, m0, m_end, n_blk); tile += sched_stride) {
+      if (!mbar_wait_lim(tfull_bar(acc), acc_phase, fail)) break;
+      tc_fence_after();
+      const int row0 = m0 + (int)crank * MG_BM + q * 32, nw0 = n_blk * TILE_N + half * (TILE_N / 2);
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * M2_BN + half * (TILE_N / 2);
+#pragma unroll
+      for (int sl = 0; sl < TILE_N / 128; ++sl) {
+        const int n0 = nw0 + sl * 64;
+        if (n0 >= p.N || row0 >= m_end) break;  // warp-uniform
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          float v[32], u[DUAL ? 32 : 1];
+          tmem_ld32(t_row + sl * 64 + cc * 32, v);
+          if constexpr (DUAL) tmem_ld32(t_row + M2_BN / 2 + cc * 32, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j0 = 0; j0 < 32; j0 += 8) {
+            float o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = moe_activate<T, DUAL>(p, v[j0 + j], u[DUAL ? j0 + j : 0]);
+            const int ch = cc * 4 + j0 / 8;
+            *reinterpret_cast<uint4*>(wbuf + lane * 128 + ((ch ^ (lane & 7)) << 4)) = pack<T>(o);
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int rr = it * 4 + r_l, m = row0 + rr, col = n0 + ch_l * 8;
+          if (m < m_end && col < p.N)
+            *reinterpret_cast<uint4*>(out + (size_t)m * p.ldo + col) =
+                *reinterpret_cast<const uint4*>(wbuf + rr * 128 + ((ch_l ^ (rr & 7)) << 4));
+        }
+        __syncwarp();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (s_fail) {  // let copies and MMAs that are still in flight finish before the shared memory and TMEM go away
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    if (threadIdx.x == 0 && p.err_flag) *p.err_flag = 2;
+    __syncthreads();
+  }
+  cluster_sync_all();  // the leader's MMAs read this CTA's shared memory, its commits arrive on this CTA's barriers
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(MG_TMEM_COLS) : "memory");
+  }
+}
+
+template <typename T, bool DUAL>
+static int launch_moe_pair(const CUtensorMap& ma, const CUtensorMap& mw, const MoeParams& p, int max_tiles, cudaStream_t st) {
+  const size_t smem = 1024 + (size_t)M2_STAGES * M2_STAGE_BYTES + M2_EPI_WARPS * M2_STG_BYTES + 8 * (2 * M2_STAGES + 4) + 16;
+  auto kern = moe_gemm_pair_kernel<T, DUAL>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    set_error("moe_gemm_pair: cannot reserve %zu B of shared memory", smem);
+    cudaGetLastError();
+    return PG_ERR_CUDA;
+  }
+  return launch_tc("moe_gemm_pair", kern, dim3(2 * (max_tiles < 74 ? max_tiles : 74)), dim3(M2_THREADS), smem, 2, false, st, ma, mw, p);
+}
+
 }  // namespace tc
 
 bool moe_gemm_tc_supported(int ldo, int lda, const int32_t* row_map, int N, int K, int dtype) {
@@ -269,9 +449,21 @@ int moe_gemm_tc(void* out, int ldo, const void* A, int lda, const int32_t* row_m
   PG_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)out % 16) == 0,
              "moe_gemm_tc: operands must be 16-byte aligned");
   const bool bf = dtype == PG_BF16;
-  const int bn = N >= 128 ? 128 : 64;
   const int rows_per_expert = swiglu ? 2 * N : N;
   CUtensorMap ma, mw;
+  // CTA pairs from the row count on at which the last, partly filled 256-row tile of an expert costs less than the halved
+  // operand traffic saves (about two full tiles per expert)
+  static const int pair_rows = env_int("PG_MOE_PAIR_ROWS", 384);
+  if (N >= 128 && n_pairs >= pair_rows * (long long)n_experts) {
+    PG_REQUIRE(tc::make_map_2d(&ma, A, n_pairs, K, lda, tc::MG_BM, bf) &&
+                   tc::make_map_2d(&mw, W, (long long)n_experts * rows_per_expert, K, K, tc::M2_BN / 2, bf),
+               "moe_gemm_pair: cuTensorMapEncodeTiled failed (rows=%d N=%d K=%d)", n_pairs, N, K);
+    tc::MoeParams p = {out, offsets, n_experts, N, K, ldo, err_flag, act, limit, 0, 0, 0, 0};
+    const int max_tiles = (cdiv(n_pairs, 2 * tc::MG_BM) + n_experts) * cdiv(N, swiglu ? tc::M2_BN / 2 : tc::M2_BN);
+    if (swiglu) return bf ? tc::launch_moe_pair<bf16, true>(ma, mw, p, max_tiles, st) : tc::launch_moe_pair<f16, true>(ma, mw, p, max_tiles, st);
+    return bf ? tc::launch_moe_pair<bf16, false>(ma, mw, p, max_tiles, st) : tc::launch_moe_pair<f16, false>(ma, mw, p, max_tiles, st);
+  }
+  const int bn = N >= 128 ? 128 : 64;
   PG_REQUIRE(tc::make_map_2d(&ma, A, n_pairs, K, lda, tc::MG_BM, bf) &&
                  tc::make_map_2d(&mw, W, (long long)n_experts * rows_per_expert, K, K, bn, bf),
              "moe_gemm_tc: cuTensorMapEncodeTiled failed (rows=%d N=%d K=%d)", n_pairs, N, K);
