@@ -99,10 +99,12 @@ __global__ void rmsnorm_kernel(T* __restrict__ out, const T* __restrict__ x, con
   const T* xr = x + (size_t)blockIdx.x * D;
   T* orow = out + (size_t)blockIdx.x * D;
   float f[MAXV][V];
+  uint4 wr[MAXV];             // the weights come in beside the row: behind the reduction they were a second trip to HBM
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
     int c = (j * blockDim.x + threadIdx.x) * V;
+    wr[j] = c < D ? ldg_cached(w + c) : make_uint4(0, 0, 0, 0);
     if (c < D) {
       unpack<T>(ldg_cached(xr + c), f[j]);
 #pragma unroll
@@ -116,7 +118,7 @@ __global__ void rmsnorm_kernel(T* __restrict__ out, const T* __restrict__ x, con
     int c = (j * blockDim.x + threadIdx.x) * V;
     if (c < D) {
       float g[V];
-      unpack<T>(ldg_cached(w + c), g);
+      unpack<T>(wr[j], g);
 #pragma unroll
       for (int i = 0; i < V; ++i) f[j][i] = (f[j][i] * inv) * (1.0f + g[i]);
       *reinterpret_cast<uint4*>(orow + c) = pack<T>(f[j]);
@@ -173,7 +175,11 @@ __global__ void layernorm_kernel(T* __restrict__ out, const T* __restrict__ x, c
 // ------------------------------------------------------------------ warp-per-row norms (many rows)
 // Prefill / vision: thousands of rows of 1152-2048 elements.  One warp per row (8 rows per CTA), the row
 // stays in registers between the statistics and the write, fully coalesced 16-byte accesses.
-template <typename T, int MAXV, bool LAYERNORM>
+// EARLY (up to 1024 rows): the weights are requested together with the row instead of behind the statistics, which are
+// then the only thing between the loads and the stores; with thousands of rows the registers are worth more as rows in flight.
+// Two rows per CTA there, so that 256 rows reach 128 SMs instead of 32.  One image's encode (19 of these among 66 launches) 575 ->
+// 544 us, a 260-token prompt with its image 4855 -> 4674 us.
+template <typename T, int MAXV, bool LAYERNORM, bool EARLY>
 __global__ void __launch_bounds__(256)
 norm_rows_warp_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b,
                       int rows, int D, float eps) {
@@ -181,7 +187,7 @@ norm_rows_warp_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __r
   pdl_wait();               // (launched with the PDL attribute when the grid is small: inputs come from the predecessor)
   constexpr int V = Vec<T>::N;
   const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const T* xr = x + (size_t)row * D;
   T* orow = out + (size_t)row * D;
@@ -192,6 +198,15 @@ norm_rows_warp_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __r
   for (int j = 0; j < MAXV; ++j) {
     const int c = (j * 32 + lane) * V;
     raw[j] = c < D ? ldg_cached(xr + c) : make_uint4(0, 0, 0, 0);
+  }
+  uint4 wr[EARLY ? MAXV : 1], br[EARLY && LAYERNORM ? MAXV : 1];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {
+      const int c = (j * 32 + lane) * V;
+      wr[j] = c < D ? ldg_cached(w + c) : make_uint4(0, 0, 0, 0);
+      if constexpr (LAYERNORM) br[j] = c < D ? ldg_cached(b + c) : make_uint4(0, 0, 0, 0);
+    }
   }
   float s = 0.f;
 #pragma unroll
@@ -226,8 +241,8 @@ norm_rows_warp_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __r
     if (c < D) {
       float f[V], g[V], bb[V];
       unpack<T>(raw[j], f);
-      unpack<T>(ldg_cached(w + c), g);
-      if (LAYERNORM) unpack<T>(ldg_cached(b + c), bb);
+      unpack<T>(EARLY ? wr[EARLY ? j : 0] : ldg_cached(w + c), g);
+      if (LAYERNORM) unpack<T>(EARLY ? br[EARLY && LAYERNORM ? j : 0] : ldg_cached(b + c), bb);
 #pragma unroll
       for (int i = 0; i < V; ++i)
         f[i] = LAYERNORM ? (f[i] - mean) * scale * g[i] + bb[i] : (f[i] * scale) * (1.0f + g[i]);
@@ -495,10 +510,12 @@ int pg_rmsnorm(void* out, const void* x, const void* w, int rows, int D, float e
     PG_REQUIRE(D % V == 0 && D <= 256 * V * 4, "rmsnorm: unsupported D=%d", D);
     const T* none = nullptr;
     if (rows >= 64 && D <= 32 * V * 5)
-      return launch_tc("rmsnorm", norm_rows_warp_kernel<T, 5, false>, dim3(cdiv(rows, 8)), dim3(256), 0, 1, rows <= 4096,
+      return launch_tc("rmsnorm", rows <= 1024 ? norm_rows_warp_kernel<T, 5, false, true> : norm_rows_warp_kernel<T, 5, false, false>,
+                       dim3(cdiv(rows, rows <= 1024 ? 2 : 8)), dim3(rows <= 1024 ? 64 : 256), 0, 1, rows <= 4096,
                        (cudaStream_t)stream, (T*)out, (const T*)x, (const T*)w, none, rows, D, eps);
     if (rows >= 64 && D <= 32 * V * 8)
-      return launch_tc("rmsnorm", norm_rows_warp_kernel<T, 8, false>, dim3(cdiv(rows, 8)), dim3(256), 0, 1, rows <= 4096,
+      return launch_tc("rmsnorm", rows <= 1024 ? norm_rows_warp_kernel<T, 8, false, true> : norm_rows_warp_kernel<T, 8, false, false>,
+                       dim3(cdiv(rows, rows <= 1024 ? 2 : 8)), dim3(rows <= 1024 ? 64 : 256), 0, 1, rows <= 4096,
                        (cudaStream_t)stream, (T*)out, (const T*)x, (const T*)w, none, rows, D, eps);
     return launch_tc("rmsnorm", rmsnorm_kernel<T, 4>, dim3(rows), dim3(256), 0, 1, rows <= 1024, (cudaStream_t)stream, (T*)out,
                      (const T*)x, (const T*)w, D, eps);
@@ -513,10 +530,12 @@ int pg_layernorm(void* out, const void* x, const void* w, const void* b, int row
     constexpr int V = Vec<T>::N;
     PG_REQUIRE(D % V == 0 && D <= 256 * V * 4, "layernorm: unsupported D=%d", D);
     if (rows >= 64 && D <= 32 * V * 5)
-      return launch_tc("layernorm", norm_rows_warp_kernel<T, 5, true>, dim3(cdiv(rows, 8)), dim3(256), 0, 1, rows <= 4096,
+      return launch_tc("layernorm", rows <= 1024 ? norm_rows_warp_kernel<T, 5, true, true> : norm_rows_warp_kernel<T, 5, true, false>,
+                       dim3(cdiv(rows, rows <= 1024 ? 2 : 8)), dim3(rows <= 1024 ? 64 : 256), 0, 1, rows <= 4096,
                        (cudaStream_t)stream, (T*)out, (const T*)x, (const T*)w, (const T*)b, rows, D, eps);
     if (rows >= 64 && D <= 32 * V * 8)
-      return launch_tc("layernorm", norm_rows_warp_kernel<T, 8, true>, dim3(cdiv(rows, 8)), dim3(256), 0, 1, rows <= 4096,
+      return launch_tc("layernorm", rows <= 1024 ? norm_rows_warp_kernel<T, 8, true, true> : norm_rows_warp_kernel<T, 8, true, false>,
+                       dim3(cdiv(rows, rows <= 1024 ? 2 : 8)), dim3(rows <= 1024 ? 64 : 256), 0, 1, rows <= 4096,
                        (cudaStream_t)stream, (T*)out, (const T*)x, (const T*)w, (const T*)b, rows, D, eps);
     return launch_tc("layernorm", layernorm_kernel<T, 4>, dim3(rows), dim3(256), 0, 1, rows <= 1024, (cudaStream_t)stream,
                      (T*)out, (const T*)x, (const T*)w, (const T*)b, D, eps);

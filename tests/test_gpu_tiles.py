@@ -185,3 +185,20 @@ def test_few_tiles_split_over_clusters(M, N, K, epi):
         want = want + r.to(F64)
     assert _rel(out[:M], want) < 4e-3          # at most three roundings of 2^-9 and the hardware tanh
     assert bool((out[M] == 0).all())
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 1023, 1024, 1025])
+@pytest.mark.parametrize("D", [8, 1152, 1288, 2048])
+def test_norm_rows(rows, D):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    x, w, b = _randn(g, rows, D), _randn(g, D), _randn(g, D)
+    out = torch.zeros(rows + 1, D, dtype=BF, device="cuda")
+    xf = x.to(F64)
+    cabi.check(L.pg_rmsnorm(out.data_ptr(), x.data_ptr(), w.data_ptr(), rows, D, 1e-6, cabi.PG_BF16, st))
+    want = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * (1 + w.to(F64))
+    assert _rel(out[:rows], want) < 2.5e-3     # one rounding of the result, statistics in fp32
+    cabi.check(L.pg_layernorm(out.data_ptr(), x.data_ptr(), w.data_ptr(), b.data_ptr(), rows, D, 1e-6, cabi.PG_BF16, st))
+    want = F.layer_norm(xf, (D,), w.to(F64), b.to(F64), 1e-6)
+    assert _rel(out[:rows], want) < 2.5e-3
+    assert bool((out[rows] == 0).all())
