@@ -68,12 +68,28 @@ __device__ __forceinline__ void epi_pair2(float& x0, float& x1, float u0, float 
 // column c with column 128 + c.  An output tile is then 256 x 128.
 template <int EPI> constexpr bool g2_dual() { return EPI == PG_EPI_GEGLU || EPI == PG_EPI_SWIGLU; }
 
-template <typename T, int EPI>
+// TAIL: 257 to 288 rows (an image's 256 tokens and a short text).  A row of tiles for the last 1 to 32
+// rows costs as much as one for 256, so these rows ride along with the full ones: the W tile in shared memory is also a valid
+// M operand, and one more MMA per K step multiplies it with the (up to 32) tail rows as N = 32 columns.  To make room for that
+// accumulator, and for the tail rows in the stage, a tile is 224 columns wide: TMEM holds 2 x (224 + 32) columns, a stage 16 KB of
+// A, 14 of W and 2 of tail rows.  (The M operand reads 128 rows a CTA: 112 of W and the 16 tail rows behind them, whose products
+// with one another land in accumulator rows that nothing reads.)  Gated: either CTA stages 56 gate and 56 up rows of the same
+// features, the accumulator is [g | u | g | u] by 56, and a tail feature meets its partner 56 rows further through shared memory.
+constexpr int G2_TAIL = 32;
+__device__ __forceinline__ void g2_epi_sync() { __syncwarp(); asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+template <typename T, int EPI, bool TAIL>
 __global__ void __launch_bounds__(G2_THREADS, 1)
-gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, Params2 p) {
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                const __grid_constant__ CUtensorMap map_t, Params2 p) {
   constexpr bool DUAL = g2_dual<EPI>();
-  constexpr int TILE_N = DUAL ? G2_BN / 2 : G2_BN;   // output columns of a tile
-  constexpr uint32_t IDESC = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, G2_BN);
+  constexpr int ACC_N = TAIL ? G2_BN - G2_TAIL : G2_BN;   // accumulator columns of a tile
+  constexpr int TILE_N = DUAL ? ACC_N / 2 : ACC_N;        // output columns of a tile
+  constexpr int HALF_N = TILE_N / 2;                      // of which an epilogue warp takes one half
+  constexpr int U_COL = TAIL ? HALF_N : G2_BN / 2;        // gated: from a gate column to its up column
+  constexpr int W_ROWS = ACC_N / 2, W_BYTES = W_ROWS * G2_BK * 2;   // per CTA
+  constexpr uint32_t IDESC = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, ACC_N);
+  constexpr uint32_t IDESC_TAIL = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, G2_TAIL);
   // a last n-tile with <= 128 real columns (N = 1152: o_proj, fc2) runs N = 128 MMAs: each CTA supplies 64 W rows
   constexpr uint32_t IDESC_HALF = umma_idesc(std::is_same<T, bf16>::value ? 1 : 0, 2 * G2_BM, G2_BN / 2);
   extern __shared__ uint8_t smem_raw[];
@@ -92,7 +108,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   uint32_t crank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
   const bool leader = crank == 0;
-  const int m_pairs = (((p.M + G2_BM - 1) / G2_BM) + 1) / 2, n_tiles = (p.N + TILE_N - 1) / TILE_N;
+  const int m_pairs = TAIL ? p.M / (2 * G2_BM) : (((p.M + G2_BM - 1) / G2_BM) + 1) / 2, n_tiles = (p.N + TILE_N - 1) / TILE_N;
   const int total_tiles = m_pairs * n_tiles;
   const int sched_first = (int)(blockIdx.x / 2), sched_stride = (int)(gridDim.x / 2);
   const int k_blocks = (p.K + G2_BK - 1) / G2_BK;
@@ -125,15 +141,21 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       for (int tile = sched_first; tile < total_tiles; tile += sched_stride) {
         const int n_blk = p.m_major ? tile % n_tiles : tile / m_pairs;  // neighbouring clusters share A rows or W rows (L2 reuse)
         const int m_blk = 2 * (p.m_major ? tile / n_tiles : tile % m_pairs) + (int)crank;  // a ghost tile past M loads zeros, stores nothing
-        const int w_step = (n_blk * G2_BN + G2_BN / 2 >= p.N) ? G2_BN / 4 : G2_BN / 2;  // half tile: 64 rows per CTA
-        const int w_row = n_blk * TILE_N + (int)crank * (DUAL ? p.N : w_step);
+        const int w_step = (!TAIL && n_blk * G2_BN + G2_BN / 2 >= p.N) ? G2_BN / 4 : W_ROWS;  // half tile: 64 rows per CTA
+        const int w_row = n_blk * TILE_N + (int)crank * (DUAL ? (TAIL ? HALF_N : p.N) : w_step);
+        const bool tail = TAIL && m_blk / 2 == m_pairs - 1;
         for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(empty_bar(stage), phase ^ 1);
           const uint32_t sa = smem_base + stage * G2_STAGE_BYTES;
           const uint32_t full_leader = mapa_u32(full_bar(stage), 0);
-          if (leader) mbar_expect_tx(full_bar(stage), 2 * G2_STAGE_BYTES);  // both CTAs' bytes
+          if (leader) mbar_expect_tx(full_bar(stage), 2 * (TAIL && !tail ? G2_A_BYTES + W_BYTES : G2_STAGE_BYTES));  // both CTAs' bytes
           tma_load_2d_cg2(sa, &map_a, full_leader, kb * G2_BK, m_blk * G2_BM);
           tma_load_2d_cg2(sa + G2_A_BYTES, &map_w, full_leader, kb * G2_BK, w_row);
+          if constexpr (TAIL) {   // boxes of 56 rows
+            tma_load_2d_cg2(sa + G2_A_BYTES + W_BYTES / 2, &map_w, full_leader, kb * G2_BK, w_row + (DUAL ? p.N : W_ROWS / 2));
+            if (tail)
+              tma_load_2d_cg2(sa + G2_A_BYTES + W_BYTES, &map_t, full_leader, kb * G2_BK, m_pairs * 2 * G2_BM + (int)crank * (G2_TAIL / 2));
+          }
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -148,14 +170,19 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * G2_BN;
         const int n_blk_mma = p.m_major ? tile % n_tiles : tile / m_pairs;
-        const uint32_t idesc = (!DUAL && n_blk_mma * G2_BN + G2_BN / 2 >= p.N) ? IDESC_HALF : IDESC;
+        const bool tail = TAIL && (p.m_major ? tile / n_tiles : tile % m_pairs) == m_pairs - 1;
+        const uint32_t idesc = (!DUAL && !TAIL && n_blk_mma * G2_BN + G2_BN / 2 >= p.N) ? IDESC_HALF : IDESC;
         for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(full_bar(stage), phase);
           tc_fence_after();
           const uint32_t sa = smem_base + stage * G2_STAGE_BYTES;
 #pragma unroll
-          for (int k = 0; k < G2_BK / 16; ++k)
+          for (int k = 0; k < G2_BK / 16; ++k) {
             umma_cg2(d_tmem, umma_desc(sa + k * 32), umma_desc(sa + G2_A_BYTES + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            if (TAIL && tail)
+              umma_cg2(d_tmem + ACC_N, umma_desc(sa + G2_A_BYTES + k * 32), umma_desc(sa + G2_A_BYTES + W_BYTES + k * 32), IDESC_TAIL,
+                       (kb > 0 || k > 0) ? 1u : 0u);
+          }
           umma_commit_cg2(empty_bar(stage), (uint16_t)0x3);  // the stage is free in BOTH CTAs once these MMAs have read it
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
@@ -182,7 +209,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int row0 = m_blk * G2_BM + q * 32;  // first row of this warp's TMEM lane quarter
       const int m = row0 + lane;
       const int ch_l = lane & 7, r_l = lane >> 3;  // staging <-> global mapping: 8 lanes per 128-byte row segment
-      const int nw0 = n_blk * TILE_N + half * (TILE_N / 2);
+      const int nw0 = n_blk * TILE_N + half * HALF_N, n_end = min(p.N, nw0 + HALF_N);   // this warp's columns
       // residual rows of both 64-column slices are requested BEFORE waiting for the accumulator: ordinary loads
       // queue behind ~190 KB of in-flight TMA data per SM, and this wait is where the epilogue warps idle anyway
       uint4 r1[8];
@@ -193,28 +220,28 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const T* rrow = R + (size_t)(p.res_mod > 0 ? (mm % p.res_mod) : mm) * p.ldr;
           uint4 u0 = make_uint4(0, 0, 0, 0);
           r1[it] = make_uint4(0, 0, 0, 0);
-          if (mm < p.M && col < p.N) u0 = ldg_cached(rrow + col);
-          if (mm < p.M && col + 64 < p.N) r1[it] = ldg_cached(rrow + col + 64);
+          if (mm < p.M && col < n_end) u0 = ldg_cached(rrow + col);
+          if (mm < p.M && col + 64 < n_end) r1[it] = ldg_cached(rrow + col + 64);
           *reinterpret_cast<uint4*>(wbuf + rr_ * 128 + ((ch_l ^ (rr_ & 7)) << 4)) = u0;
         }
         __syncwarp();
       }
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + half * (TILE_N / 2);
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + half * (TAIL && DUAL ? ACC_N / 2 : HALF_N);
       if (!DUAL && p.out_f32) {
         // fp32 rows (logits): direct 32-byte stores, thread <-> row
 #pragma unroll 1
-        for (int c = 0; c < G2_BN / 64; ++c) {
+        for (int c = 0; c < (HALF_N + 31) / 32; ++c) {
           float v[32];
           tmem_ld32(t_row + c * 32, v);
           tmem_ld_wait();
-          const int n0 = n_blk * G2_BN + half * (G2_BN / 2) + c * 32;
-          if (m < p.M && n0 < p.N) {
+          const int n0 = nw0 + c * 32;
+          if (m < p.M && n0 < n_end) {
             const int rm = p.res_mod > 0 ? (m % p.res_mod) : m;
 #pragma unroll
             for (int j0 = 0; j0 < 32; j0 += 8) {
-              if (n0 + j0 >= p.N) break;  // N is a multiple of 8 (checked on the host)
+              if (n0 + j0 >= n_end) break;  // N is a multiple of 8 (checked on the host)
               float o[8], bb[8], rr[8];
               if (HAS_BIAS) unpack<T>(ldg_cached(bias + n0 + j0), bb);
               if (HAS_RES) unpack<T>(ldg_cached(R + (size_t)rm * p.ldr + n0 + j0), rr);
@@ -230,9 +257,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // 16-bit rows: 64-column slices through a per-warp staging tile so that the residual loads and the output
         // stores are whole 128-byte row segments (4 rows per instruction) instead of 32 scattered 16-byte pieces
 #pragma unroll
-        for (int sl = 0; sl < TILE_N / 128; ++sl) {
+        for (int sl = 0; sl < (HALF_N + 63) / 64; ++sl) {
           const int n0 = nw0 + sl * 64;
-          if (n0 >= p.N || row0 >= p.M) break;  // warp-uniform
+          if (n0 >= n_end || row0 >= p.M) break;  // warp-uniform
           if (HAS_RES && sl == 1) {
 #pragma unroll
             for (int it = 0; it < 8; ++it) {
@@ -245,7 +272,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int cc = 0; cc < 2; ++cc) {
             float v[32], u[DUAL ? 32 : 1];
             tmem_ld32(t_row + sl * 64 + cc * 32, v);
-            if constexpr (DUAL) tmem_ld32(t_row + G2_BN / 2 + cc * 32, u);
+            if constexpr (DUAL) tmem_ld32(t_row + U_COL + cc * 32, u);
             tmem_ld_wait();
 #pragma unroll
             for (int j0 = 0; j0 < 32; j0 += 8) {
@@ -253,7 +280,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               uint4* slot = reinterpret_cast<uint4*>(wbuf + lane * 128 + ((ch ^ (lane & 7)) << 4));
               float o[8], bb[8], rr[8];
               if (HAS_BIAS) {
-                if (n0 + ch * 8 < p.N) unpack<T>(ldg_cached(bias + n0 + ch * 8), bb);
+                if (n0 + ch * 8 < n_end) unpack<T>(ldg_cached(bias + n0 + ch * 8), bb);
                 else {
 #pragma unroll
                   for (int j = 0; j < 8; ++j) bb[j] = 0.f;
@@ -273,11 +300,50 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
           for (int it = 0; it < 8; ++it) {
             const int rr_ = it * 4 + r_l, mm = row0 + rr_, col = n0 + ch_l * 8;
-            if (mm < p.M && col < p.N)
+            if (mm < p.M && col < n_end)
               *reinterpret_cast<uint4*>(Ct + (size_t)mm * p.ldc + col) =
                   *reinterpret_cast<const uint4*>(wbuf + rr_ * 128 + ((ch_l ^ (rr_ & 7)) << 4));
           }
           __syncwarp();
+        }
+      }
+      if constexpr (TAIL) {
+        if (m_blk / 2 == m_pairs - 1) {   // the tail rows: accumulator row = weight row, column = token
+          const int w = q * 32 + lane, m0 = m_pairs * 2 * G2_BM + half * (G2_TAIL / 2), cnt = min(G2_TAIL / 2, p.M - m0);
+          float v[G2_TAIL / 2];
+          tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + ACC_N + half * (G2_TAIL / 2), v);
+          tmem_ld_wait();
+          if constexpr (DUAL) {
+            float* xch = reinterpret_cast<float*>(smem_raw + (stg_base - smem_u32(smem_raw))) + half * (G2_TAIL / 2) * HALF_N;
+            g2_epi_sync();                 // every warp is done with its staging tile
+            if (w >= HALF_N && w < W_ROWS) {
+#pragma unroll
+              for (int t = 0; t < G2_TAIL / 2; ++t) xch[t * HALF_N + w - HALF_N] = v[t];
+            }
+            g2_epi_sync();
+            const int n = n_blk * TILE_N + (int)crank * HALF_N + w;
+            if (w < HALF_N && n < p.N) {
+#pragma unroll
+              for (int t = 0; t < G2_TAIL / 2; ++t) {
+                float x = v[t], dummy = 0.f;
+                epi_pair2<T, EPI>(x, dummy, xch[t * HALF_N + w], 0.f);
+                if (t < cnt) Ct[(size_t)(m0 + t) * p.ldc + n] = from_f<T>(x);
+              }
+            }
+            g2_epi_sync();                 // before the next tile is staged over the partners
+          } else {
+            const int n = n_blk * TILE_N + (int)crank * W_ROWS + w;
+            if (w < W_ROWS && n < p.N) {
+#pragma unroll
+              for (int t = 0; t < G2_TAIL / 2; ++t) {
+                if (t >= cnt) break;
+                const int mm = m0 + t, rm = p.res_mod > 0 ? mm % p.res_mod : mm;
+                const float x = epi_apply<T, EPI>(v[t], 0.f, HAS_RES ? to_f<T>(R[(size_t)rm * p.ldr + n]) : 0.f);
+                if (p.out_f32) Cf[(size_t)mm * p.ldc + n] = x;
+                else Ct[(size_t)mm * p.ldc + n] = from_f<T>(x);
+              }
+            }
+          }
         }
       }
       tc_fence_before();
@@ -295,17 +361,18 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   }
 }
 
-template <typename T, int EPI>
-static int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const Params2& p, cudaStream_t st) {
+template <typename T, int EPI, bool TAIL>
+static int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mt, const Params2& p, cudaStream_t st) {
   const size_t smem = 1024 + (size_t)G2_STAGES * G2_STAGE_BYTES + G2_EPI_WARPS * G2_STG_BYTES + 8 * (2 * G2_STAGES + 4) + 16;
-  auto kern = gemm_tc2_kernel<T, EPI>;
+  auto kern = gemm_tc2_kernel<T, EPI, TAIL>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     set_error("gemm_tc2: cannot reserve %zu B of shared memory", smem);
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
-  const int pairs = cdiv(cdiv(p.M, G2_BM), 2) * cdiv(p.N, g2_dual<EPI>() ? G2_BN / 2 : G2_BN);
-  return launch_tc("gemm_tcgen05_2cta", kern, dim3(2 * (pairs < 74 ? pairs : 74)), dim3(G2_THREADS), smem, 2, pairs <= 148, st, ma, mw, p);
+  const int acc_n = TAIL ? G2_BN - G2_TAIL : G2_BN;
+  const int pairs = (TAIL ? p.M / (2 * G2_BM) : cdiv(cdiv(p.M, G2_BM), 2)) * cdiv(p.N, g2_dual<EPI>() ? acc_n / 2 : acc_n);
+  return launch_tc("gemm_tcgen05_2cta", kern, dim3(2 * (pairs < 74 ? pairs : 74)), dim3(G2_THREADS), smem, 2, pairs <= 148, st, ma, mw, mt, p);
 }
 
 }  // namespace tc
@@ -314,6 +381,20 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const Params2& 
 // costs the bytes that a CTA stages, 32 KB here for a 256 x 256 tile (256 x 128 when gated), 32 KB there for 128 x 128
 // (48 KB gated, 24 KB with 64 columns), and a GEMM takes that many times the waves of its tiles.  1292 rows: q/k/v (N 2560)
 // 24.2 -> 17.9, o_proj and down_proj together (N 2048, K 2048 and 16384) 176 -> 102, gate/up (F 16384) 149 -> 123 us.
+// Cost of the CTA-pair kernel: waves of tiles x KB staged per k-block; *tail: with 257 to 288 rows the remainder rides along with
+// the first 256 (224-wide tiles, 30 KB and the tail's 2) instead of taking a row of tiles of its own.  260 rows: gate/up (F 16384)
+// 52.2 -> 37.7 us, the fp32 head (N 257152) 463 -> 321 us; a 260-token prompt with its image 4657 -> 4273 us.  From two full row
+// tiles on the remainder is the smaller part and the narrower tiles cost more than it: 1292 rows, gate/up 140 -> 172 us.
+static int g2_cost(int M, int N, int epi, bool* tail) {
+  const bool dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
+  const int rem = M % (2 * tc::G2_BM), acc_t = tc::G2_BN - tc::G2_TAIL;
+  const int plain = cdiv((long long)cdiv(M, 2 * tc::G2_BM) * cdiv(N, dual ? tc::G2_BN / 2 : tc::G2_BN), 74) * 32;
+  const int with = cdiv((long long)(M / (2 * tc::G2_BM)) * cdiv(N, dual ? acc_t / 2 : acc_t), 74) * 30 + 2;
+  static const int enabled = env_int("PG_GEMM_2CTA_TAIL", 1);
+  *tail = enabled && M > 2 * tc::G2_BM && M < 4 * tc::G2_BM && rem > 0 && rem <= tc::G2_TAIL && with < plain && (dual || epi == PG_EPI_NONE || epi == PG_EPI_RES);
+  return *tail ? with : plain;
+}
+
 bool gemm_tc_2cta_wanted(int M, int N, int K, int epi) {
   static const int enabled = env_int("PG_GEMM_2CTA", 1);
   static const int min_pairs = env_int("PG_GEMM_2CTA_MIN_PAIRS", 148);
@@ -323,14 +404,18 @@ bool gemm_tc_2cta_wanted(int M, int N, int K, int epi) {
   if (!dual && pairs >= min_pairs) return true;
   const int bn = m_tiles * cdiv(N, 128) < 100 ? 64 : 128;      // the single-CTA kernel's tile for this problem
   const int one = cdiv((long long)m_tiles * cdiv(N, bn), 148) * (16 + (dual ? 2 : 1) * bn / 8);
-  return cdiv(pairs, 74) * 32 < one;
+  bool tail;
+  return g2_cost(M, N, epi, &tail) < one;
 }
 
 int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                  int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st) {
   const bool bf = dtype == PG_BF16, dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
-  CUtensorMap ma, mw;
-  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && tc::make_map_2d(&mw, W, dual ? 2 * N : N, K, ldw, tc::G2_BN / 2, bf),
+  bool tail;
+  g2_cost(M, N, epi, &tail);
+  CUtensorMap ma, mw, mt;
+  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && tc::make_map_2d(&mt, A, M, K, lda, tc::G2_TAIL / 2, bf) &&
+                 tc::make_map_2d(&mw, W, dual ? 2 * N : N, K, ldw, tail ? (tc::G2_BN - tc::G2_TAIL) / 4 : tc::G2_BN / 2, bf),
              "gemm_tc2: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, N, K, lda, ldw);
   PG_REQUIRE(!dual || !out_f32, "gemm_tc2: a gated pairing has no fp32 output");
   // A is re-read once per n-tile (n-major order) or W once per m-pair (m-major): stream the big operand once and
@@ -338,7 +423,16 @@ int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const 
   static const int order_env = env_int("PG_GEMM_2CTA_ORDER", -1);
   const int m_major = order_env >= 0 ? order_env : ((long long)N * K * (dual ? 4 : 2) <= (32ll << 20) ? 1 : 0);
   tc::Params2 p = {C, bias, R, M, N, K, ldc, ldr, res_mod, out_f32, m_major};
-#define PG_TC2(E) return bf ? tc::launch2<bf16, E>(ma, mw, p, st) : tc::launch2<f16, E>(ma, mw, p, st)
+#define PG_TC2T(E, TL) return bf ? tc::launch2<bf16, E, TL>(ma, mw, mt, p, st) : tc::launch2<f16, E, TL>(ma, mw, mt, p, st)
+#define PG_TC2(E) PG_TC2T(E, false)
+  if (tail) {
+    switch (epi) {
+      case PG_EPI_NONE: PG_TC2T(PG_EPI_NONE, true);
+      case PG_EPI_RES: PG_TC2T(PG_EPI_RES, true);
+      case PG_EPI_GEGLU: PG_TC2T(PG_EPI_GEGLU, true);
+      case PG_EPI_SWIGLU: PG_TC2T(PG_EPI_SWIGLU, true);
+    }
+  }
   switch (epi) {
     case PG_EPI_NONE: PG_TC2(PG_EPI_NONE);
     case PG_EPI_BIAS: PG_TC2(PG_EPI_BIAS);
@@ -349,6 +443,7 @@ int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const 
     case PG_EPI_SWIGLU: PG_TC2(PG_EPI_SWIGLU);
   }
 #undef PG_TC2
+#undef PG_TC2T
   set_error("gemm_tc2: bad epilogue %d", epi);
   return PG_ERR_INVALID;
 }

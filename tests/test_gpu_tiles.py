@@ -202,3 +202,25 @@ def test_norm_rows(rows, D):
     want = F.layer_norm(xf, (D,), w.to(F64), b.to(F64), 1e-6)
     assert _rel(out[:rows], want) < 2.5e-3
     assert bool((out[rows] == 0).all())
+
+
+@pytest.mark.parametrize("M", [256, 257, 272, 273, 288, 289, 516])
+@pytest.mark.parametrize("N,K,kind", [(9480, 136, "geglu"), (9480, 1000, "geglu"), (9472, 136, "swiglu"), (19000, 72, "none"), (18960, 1000, "res"),
+                                      (19000, 1000, "f32")])
+def test_rows_behind_a_multiple_of_256(M, N, K, kind):
+    """257 to 288 rows: the remainder rides along with the full 256; the row counts next to them; ragged last tiles."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    dual, f32 = kind.endswith("glu"), kind == "f32"
+    a, w, r = _randn(g, M, K), _randn(g, 2 * N if dual else N, K, std=K ** -0.5), _randn(g, M, N)
+    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else BF, device="cuda")
+    code = {"geglu": cabi.EPI_GEGLU, "swiglu": cabi.EPI_SWIGLU, "res": cabi.EPI_RES}.get(kind, cabi.EPI_NONE)
+    res = kind == "res"
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr() if res else None, M, N, K, K, K, N, N if res else 0, 0,
+                         code, 1 if f32 else 0, 2, cabi.PG_BF16, st))
+    z = a.to(F64) @ w.to(F64).T
+    want = {"geglu": lambda: _gelu(z[:, :N]) * z[:, N:], "swiglu": lambda: F.silu(z[:, :N]) * z[:, N:], "res": lambda: z + r.to(F64)}.get(kind, lambda: z)()
+    tol = 5e-3                                 # up to three roundings of 2^-9 (the fp32 rows hold values rounded to 16 bits) and the tanh
+    for rows in (slice(0, 256), slice(256, M))[:1 if M == 256 else 2]:
+        assert _rel(out[:M][rows], want[rows]) < tol
+    assert bool((out[M] == 0).all())
