@@ -6,15 +6,15 @@
 // (key tile = page = 64 keys, fetched by TMA from the paged pools; the append kernel has written the step's own keys
 // before this launch).  ONE pass over the key tiles:
 //   S(t) = Q K^T (tcgen05.mma, fp32) into one of two TMEM buffers, issued one tile ahead of the softmax;
-//   thread r owns query row r: z = log2(e) (S * scale - slope_h * (i - j)), masked outside 0 <= i - j < window, in fp32; the row's
+//   two threads own a query row, 32 of the tile's keys each (their maxima meet in shared memory): z = log2(e) (S * scale - slope_h * (i - j)), masked outside 0 <= i - j < window, in fp32; the row's
 //   reference maximum is raised (and O, sum rescaled, after the products that still add to it) only when a tile exceeds it
 //   by more than 2^8; p = exp2(z - m), row sum from the fp32 values, P rounded to the model dtype and stored over the S
 //   columns it came from: O += P V takes P as the TMEM operand and V as an MN-major operand straight from its page.
-// What bounds it: the softmax's instructions (about 8 per score) and the exponentials; the tiles' products and copies
-// run beside them, and the two CTAs of an SM fill each other's waits.  Most tiles lie wholly inside the causal window of
-// all 128 rows and take a loop without masks.  The two-pass form before it (row maximum first, S computed twice, P through
-// shared memory, masks on every score) took 557 us for 4 prompts of 2048 tokens, 16 heads of 128, window 1024; this takes 218 us (246 with
-// the pages walked oldest first).
+// What bounds it: the softmax's instructions and their latencies; the tiles' products and copies run beside them.  Arithmetic is
+// paired (f32x2, the scalar roundings), and two CTAs of eight softmax warps each keep an SM's schedulers fed.  Most tiles lie
+// wholly inside the causal window of all 128 rows and take a loop without masks.  4 prompts of 2048 tokens, 16 heads of 128,
+// window 1024: 557 us in two passes (row maximum first, S computed twice, P through shared memory, masks on every score), 246 in
+// one pass, 219 with the newest pages first, 150 with two threads a row (one: 0.33 instructions a cycle and scheduler).
 // Epilogue: O / sum, times sigmoid(gate), rounded once.  Key width and value width are independent multiples of 64.
 // Extensions (pg_attention_ragged_tc_ex): keep_first > 0 keeps the first keep_first positions visible behind the
 // window: the window's pages are then followed by those that hold them (as far as they lie before the window's first page).  sigmoid_weights: p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
@@ -61,7 +61,7 @@ struct WinParams {
 };
 
 template <typename T, bool CAP>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(320, 2)
 attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, WinParams p) {
   constexpr int FMT = std::is_same<T, bf16>::value ? 1 : 0;
@@ -84,6 +84,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   auto bar_o = [&](int t) { return bars + 72 + 8 * (t & 1); };        // P(t) V(t) has been added to O
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   __shared__ int s_fail;
+  __shared__ float s_half[2][2][WQ];                                  // [tile & 1][half][row]: the halves' maxima, at the end their sums
   volatile int* fail = &s_fail;
   if (threadIdx.x == 0) s_fail = 0;
 
@@ -94,7 +95,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   if (warp == 1 && lane == 0) {
     mbar_init(bar_q, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_k(i), 1); mbar_init(bar_v(i), 1); mbar_init(bar_s(i), 1); mbar_init(bar_p(i), 128); mbar_init(bar_o(i), 1);
+      mbar_init(bar_k(i), 1); mbar_init(bar_v(i), 1); mbar_init(bar_s(i), 1); mbar_init(bar_p(i), 256); mbar_init(bar_o(i), 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -169,9 +170,15 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 (t > 0 || ks > 0) ? 1u : 0u);
       umma_commit(bar_o(t));
     }
-  } else if (warp >= 4) {
-    // ===================== softmax + epilogue: thread <-> query row =====================
-    const int qw = warp & 3, r = qw * 32 + lane;
+  } else if (warp >= 2) {
+    // ===================== softmax + epilogue: two threads per query row, 32 of a tile's keys each =====================
+    // A wait that gave up leaves the loops running (every later wait returns at once): the two halves meet at barriers.
+    const int qw = warp & 3, r = qw * 32 + lane, hf = (warp - 2) >> 2;   // TMEM lane quarter = warp & 3
+    auto meet = [&] {                                              // the two warps of these 32 rows
+      __syncwarp();
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + qw) : "memory");
+    };
+    constexpr int HK = WK / 2;
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
     const int i = pos0 + r;                                        // this row's position
     const float slope = (p.slopes ? p.slopes[h] : 0.f) * LOG2E_F, hbias = (p.head_bias ? p.head_bias[h] : 0.f) * LOG2E_F;
@@ -186,48 +193,57 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const float qs2 = qscale * LOG2E_F;
     bool ok = true;
     for (int t = 0; t < n_tiles; ++t) {
-      if (!wait(bar_s(t), t)) { ok = false; break; }
+      ok = wait(bar_s(t), t) && ok;
       tc_fence_after();
-      const int j0 = page_of(t) * WK;
-      float s[WK];
-      tmem_ld32(t_row + (t & 1) * WK, s);
-      tmem_ld32(t_row + (t & 1) * WK + 32, s + 32);
+      const int page0 = page_of(t) * WK, j0 = page0 + hf * HK;
+      float s[HK];
+      tmem_ld32(t_row + (t & 1) * WK + hf * HK, s);
       tmem_ld_wait();
       if (CAP) {       // cap * tanh(z / cap) = cap - 2 cap / (exp(2 z / cap) + 1): absolute error a few 1e-7 of the cap
 #pragma unroll
-        for (int jj = 0; jj < WK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * LOG2E_F;
+        for (int jj = 0; jj < HK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * LOG2E_F;
       }
       const float d0 = (float)(j0 - i);                            // exact, and so is d0 + jj = j - i
+      f32x2 dd = pair_of(d0, d0 + 1.f);
 #pragma unroll
-      for (int jj = 0; jj < WK; ++jj) {
-        const float z = fmaf(slope, d0 + (float)jj, hbias);
-        s[jj] = CAP ? s[jj] + z : fmaf(s[jj], qs2, z);
+      for (int jj = 0; jj < HK; jj += 2) {
+        const f32x2 z = fma2(pair_of(slope, slope), dd, pair_of(hbias, hbias)), x = pair_of(s[jj], s[jj + 1]);
+        const float2 y = halves_of(CAP ? add2(x, z) : fma2(x, pair_of(qs2, qs2), z));
+        s[jj] = y.x;
+        s[jj + 1] = y.y;
+        dd = add2(dd, pair_of(2.f, 2.f));
       }
       // whole tiles that every row sees need no masks
-      const bool full = j0 + WK - 1 <= pos0 && j0 >= blk_last &&
-                        (p.window <= 0 || pos0 + WQ - 1 - j0 < p.window || j0 + WK <= p.keep_first);
+      const bool full = page0 + WK - 1 <= pos0 && page0 >= blk_last &&
+                        (p.window <= 0 || pos0 + WQ - 1 - page0 < p.window || page0 + WK <= p.keep_first);
       if (!full) {
 #pragma unroll
-        for (int jj = 0; jj < WK; ++jj) {
+        for (int jj = 0; jj < HK; ++jj) {
           const int j = j0 + jj, back = i - j;
           const bool vis = back >= 0 && j >= blk0 && (p.window <= 0 || back < p.window || j < p.keep_first);
           s[jj] = vis ? s[jj] : -INFINITY;
         }
       }
+      float top = -INFINITY;
       if (!fixed_max) {
         float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-        for (int jj = 4; jj < WK; ++jj) mx[jj & 3] = fmaxf(mx[jj & 3], s[jj]);
-        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        for (int jj = 4; jj < HK; ++jj) mx[jj & 3] = fmaxf(mx[jj & 3], s[jj]);
+        top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        s_half[t & 1][hf][r] = top;
+      }
+      meet();                                                      // both have read their scores: P may take S's columns
+      if (!fixed_max) {
+        top = fmaxf(top, s_half[t & 1][hf ^ 1][r]);                // the same in both threads, and so is every decision below
         if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {          // m == -inf: any visible key raises it
           const float m_new = fmaxf(m, top);
           if (t > 0) {
             const float corr = m_new == m ? 1.f : exp2_approx(m - m_new);
             l *= corr;
-            if (!wait(bar_o(t - 1), t - 1)) { ok = false; break; }   // nothing adds to O until this tile's P is handed over
+            ok = wait(bar_o(t - 1), t - 1) && ok;                    // nothing adds to O until this tile's P is handed over
             tc_fence_after();
 #pragma unroll 1
-            for (int c = 0; c < VB * 4; ++c) {
+            for (int c = hf; c < VB * 4; c += 2) {
               float o[16];
               tmem_ld16(t_row + O_COL + c * 16, o);
               tmem_ld_wait();
@@ -241,25 +257,31 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       }
       if (sig) {
 #pragma unroll
-        for (int jj = 0; jj < WK; ++jj) s[jj] = __fdividef(1.f, 1.f + exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
+        for (int jj = 0; jj < HK; ++jj) s[jj] = __fdividef(1.f, 1.f + exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
       } else {
         const float ref = m == -INFINITY ? 0.f : m;                // a row that has seen no key yet
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        f32x2 sum[2] = {pair_of(0.f, 0.f), pair_of(0.f, 0.f)};
 #pragma unroll
-        for (int jj = 0; jj < WK; ++jj) {
-          s[jj] = exp2_approx(s[jj] - ref);
-          sum[jj & 3] += s[jj];
+        for (int jj = 0; jj < HK; jj += 2) {
+          const float2 x = halves_of(add2(pair_of(s[jj], s[jj + 1]), pair_of(-ref, -ref)));
+          s[jj] = exp2_approx(x.x);
+          s[jj + 1] = exp2_approx(x.y);
+          sum[(jj >> 1) & 1] = add2(sum[(jj >> 1) & 1], pair_of(s[jj], s[jj + 1]));
         }
-        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        const float2 a = halves_of(sum[0]), b = halves_of(sum[1]);
+        l += (a.x + a.y) + (b.x + b.y);
       }
-      uint32_t pk[WK / 2];
+      uint32_t pk[HK / 2];
 #pragma unroll
-      for (int jj = 0; jj < WK / 2; ++jj) pk[jj] = pack_pair<T>(s[2 * jj], s[2 * jj + 1]);
-      tmem_st32(t_row + (t & 1) * WK, pk);                         // over the first 32 of this row's S columns
+      for (int jj = 0; jj < HK / 2; ++jj) pk[jj] = pack_pair<T>(s[2 * jj], s[2 * jj + 1]);
+      tmem_st16(t_row + (t & 1) * WK + hf * (HK / 2), pk);         // P takes the first 32 of the row's S columns
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(bar_p(t));
     }
+    s_half[n_tiles & 1][hf][r] = l;
+    meet();
+    l = s_half[n_tiles & 1][0][r] + s_half[n_tiles & 1][1][r];
     if (ok && wait(bar_o(n_tiles - 1), n_tiles - 1)) {
       tc_fence_after();
       if (p.sink && !sig) l += exp2_approx(p.sink[h] * LOG2E_F - m);   // a logit without key or value, counted once
@@ -288,7 +310,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       const float fpos = (float)i;
       if (!p.out_rot) {
 #pragma unroll 1
-        for (int c = 0; c * 32 < p.vdim; ++c) {
+        for (int c = hf; c * 32 < p.vdim; c += 2) {
           float o[32];
           tmem_ld32(t_row + O_COL + c * 32, o);
           tmem_ld_wait();
@@ -298,7 +320,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         }
       } else if (p.out_rot_interleaved) {                          // pairs of neighbours: both halves in one load
 #pragma unroll 1
-        for (int c = 0; c * 32 < p.vdim; ++c) {
+        for (int c = hf; c * 32 < p.vdim; c += 2) {
           float o[32];
           tmem_ld32(t_row + O_COL + c * 32, o);
           tmem_ld_wait();
@@ -315,7 +337,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       } else {                                                     // column m with m + vdim / 2 (vdim is a multiple of 64)
         const int hc = p.vdim / 64;
 #pragma unroll 1
-        for (int c = 0; c < hc; ++c) {
+        for (int c = hf; c < hc; c += 2) {
           float a[32], b[32];
           tmem_ld32(t_row + O_COL + c * 32, a);
           tmem_ld32(t_row + O_COL + (hc + c) * 32, b);
@@ -438,7 +460,7 @@ extern "C" int pg_attention_ragged_tc_capped(void* out, int ld_out, const void* 
   auto run = [&](auto kern) -> int {
     PG_REQUIRE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess,
                "attention_ragged_tc: cannot reserve %zu B of shared memory", smem);
-    return launch_tc("attention_ragged_tc", kern, grid, dim3(256), smem, 1, false, st, mq, mk, mv, p);
+    return launch_tc("attention_ragged_tc", kern, grid, dim3(320), smem, 1, false, st, mq, mk, mv, p);
   };
   if (softcap > 0.f) return bf ? run(tc::attention_window_tc_kernel<bf16, true>) : run(tc::attention_window_tc_kernel<f16, true>);
   return bf ? run(tc::attention_window_tc_kernel<bf16, false>) : run(tc::attention_window_tc_kernel<f16, false>);
