@@ -42,13 +42,31 @@ __device__ __forceinline__ float epi_apply(float x, float b, float r) {
   if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) x = rnd<T>(x + r);
   return x;
 }
+// gelu_tanh_fast of two elements on paired arithmetic (the same roundings, half the instructions)
+// The epilogue of fc1 (K 1152: 18 k-blocks a tile) paces its tiles: 64 images' encode 5563 -> 5493 us.
+__device__ __forceinline__ void gelu_tanh_fast2(float& x0, float& x1) {
+  const f32x2 x = pair_of(x0, x1);
+  const f32x2 inner = mul2(pair_of(0.7978845608028654f, 0.7978845608028654f),
+                           fma2(pair_of(0.044715f, 0.044715f), mul2(mul2(x, x), x), x));
+  float2 t = halves_of(inner);
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(t.x));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(t.y));
+  const float2 y = halves_of(mul2(mul2(pair_of(0.5f, 0.5f), x), add2(pair_of(1.f, 1.f), pair_of(t.x, t.y))));
+  x0 = y.x;
+  x1 = y.y;
+}
+__device__ __forceinline__ void add_pair(float& x0, float& x1, float b0, float b1) {
+  const float2 y = halves_of(add2(pair_of(x0, x1), pair_of(b0, b1)));
+  x0 = y.x;
+  x1 = y.y;
+}
 // two elements at once with packed conversions (keeps the XU pipe for MUFU.TANH)
 template <typename T, int EPI>
 __device__ __forceinline__ void epi_apply2(float& x0, float& x1, float b0, float b1, float r0, float r1) {
-  if (EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES) { x0 += b0; x1 += b1; }
+  if (EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES) add_pair(x0, x1, b0, b1);
   rnd2<T>(x0, x1);
-  if (EPI == PG_EPI_BIAS_GELU) { x0 = gelu_tanh_fast(x0); x1 = gelu_tanh_fast(x1); rnd2<T>(x0, x1); }
-  if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) { x0 += r0; x1 += r1; rnd2<T>(x0, x1); }
+  if (EPI == PG_EPI_BIAS_GELU) { gelu_tanh_fast2(x0, x1); rnd2<T>(x0, x1); }
+  if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) { add_pair(x0, x1, r0, r1); rnd2<T>(x0, x1); }
 }
 
 // gelu_tanh(g) u or silu(g) u of two elements, rounded where the single-CTA kernel rounds
@@ -56,7 +74,7 @@ template <typename T, int EPI>
 __device__ __forceinline__ void epi_pair2(float& x0, float& x1, float u0, float u1) {
   rnd2<T>(x0, x1);
   rnd2<T>(u0, u1);
-  if (EPI == PG_EPI_GEGLU) { x0 = gelu_tanh_fast(x0); x1 = gelu_tanh_fast(x1); }
+  if (EPI == PG_EPI_GEGLU) gelu_tanh_fast2(x0, x1);
   else { x0 = x0 / (1.f + __expf(-x0)); x1 = x1 / (1.f + __expf(-x1)); }
   rnd2<T>(x0, x1);
   x0 *= u0; x1 *= u1;
