@@ -99,7 +99,9 @@ int pg_im2col(void* out, const void* pixels, int B, int C, int H, int W, int p, 
  * stores fp32 (lm_head `.float()`, modeling_gemma.py:417-418).  impl: 0 = auto, 1 = SIMT
  * (any dtype), 2 = tcgen05/TMA (bf16/f16 only; picks the CTA-pair, single-CTA, skinny or split-K kernel by shape),
  * 3 = the CTA-pair swap-AB kernel for 129..512 rows (weights as the M operand, split-K through pg_set_workspace;
- * auto takes it for the projections where it measured faster).  Replaces every nn.Linear / matmul call site
+ * auto takes it for the projections where it measured faster).  W is a parameter: the 16-bit kernels for few rows or few
+ * tiles request it before the preceding launches of this library have finished, so W must not be an output of one that is
+ * still in flight (what other work on the stream wrote is seen).  Replaces every nn.Linear / matmul call site
  * of SURVEY.md §2.3 on the prefill and vision paths. */
 int pg_gemm(void* C, const void* A, const void* W, const void* bias, const void* R,
             int M, int N, int K, int lda, int ldw, int ldc, int ldr, int res_mod,
@@ -133,8 +135,8 @@ int pg_attention(void* out, int ld_out, const void* q, int ld_q, const void* k, 
                  int dtype, void* stream);
 
 /* The same attention on the tcgen05 tensor cores (16-bit dtypes; prefill, cache-off recompute, SigLIP):
- * QK^T and PV as tcgen05.mma with TMEM accumulators, Q/K/V tiles by TMA, two-pass softmax (row max, then
- * exp / PV) with one thread per query row.  q, k, v are row-major matrices (`*_rows` x `ld_*`); head h sits
+ * QK^T and PV as tcgen05.mma with TMEM accumulators, Q/K/V tiles by TMA, one-pass softmax (the row's
+ * reference maximum is raised lazily) with one thread per query row.  q, k, v are row-major matrices (`*_rows` x `ld_*`); head h sits
  * at columns *_col0 + h*hd_stride .. +hd, and a head row must be padded (with zeros) to a multiple of 64
  * columns unless hd is 128 or 256.  Paged K/V needs page_size == key tile (128 for hd <= 128, 64 above).
  * Output is packed: head h at column h*hd of [B*q_len, ld_out]. */
