@@ -14,7 +14,8 @@
 // paired (f32x2, the scalar roundings), and two CTAs of eight softmax warps each keep an SM's schedulers fed.  Most tiles lie
 // wholly inside the causal window of all 128 rows and take a loop without masks.  4 prompts of 2048 tokens, 16 heads of 128,
 // window 1024: 557 us in two passes (row maximum first, S computed twice, P through shared memory, masks on every score), 246 in
-// one pass, 219 with the newest pages first, 150 with two threads a row (one: 0.33 instructions a cycle and scheduler).
+// one pass, 219 with the newest pages first, 150 with two threads a row (one: 0.33 instructions a cycle and scheduler),
+// 139 with the long tiles first.
 // Epilogue: O / sum, times sigmoid(gate), rounded once.  Key width and value width are independent multiples of 64.
 // Extensions (pg_attention_ragged_tc_ex): keep_first > 0 keeps the first keep_first positions visible behind the
 // window: the window's pages are then followed by those that hold them (as far as they lie before the window's first page).  sigmoid_weights: p = sigmoid(s + head_bias[h]), no maximum, no sum.  The
@@ -90,7 +91,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, kvh = h / p.kv_group;
+  const int h = blockIdx.x % p.H, kvh = h / p.kv_group;
 
   if (warp == 1 && lane == 0) {
     mbar_init(bar_q, 1);
@@ -109,7 +110,9 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   const uint32_t tmem_base = *tmem_slot_ptr;
   auto wait = [&](uint32_t bar, int t) { return mbar_wait_lim(bar, (t >> 1) & 1, fail); };
   pdl_wait();  // q, the pools, the tile list and the page table come from the preceding kernels / copies
-  const int32_t* tile = p.tiles + 4 * (size_t)blockIdx.x;
+  // A prompt's later tiles see more keys: the list is walked from its end, the heads of a tile side by side, so that the CTAs
+  // of the last, partly filled wave are short ones: 149 -> 139 us (head by head, tiles in list order, SMs were idle 14 % of it).
+  const int32_t* tile = p.tiles + 4 * (size_t)((gridDim.x - 1 - blockIdx.x) / p.H);
   const int row0 = tile[0], rows = tile[1], slot = tile[2], pos0 = tile[3];
   const int hi = pos0 + rows - 1;                                        // last key position any row can see
   int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;               // first one
@@ -456,7 +459,8 @@ extern "C" int pg_attention_ragged_tc_capped(void* out, int ld_out, const void* 
   const size_t smem = 1024 + (size_t)tc::WQ * kb * 128 + 2 * (size_t)tc::WK * kb * 128 +
                       (tied ? 0 : 2 * (size_t)tc::WK * vb * 128) + 88 + 8;
   cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(n_tiles, n_heads);
+  PG_REQUIRE(n_heads <= 65535 && (long long)n_tiles * n_heads < (1ll << 31), "attention_ragged_tc: %d tiles of %d heads", n_tiles, n_heads);
+  dim3 grid((unsigned)n_tiles * n_heads);
   auto run = [&](auto kern) -> int {
     PG_REQUIRE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess,
                "attention_ragged_tc: cannot reserve %zu B of shared memory", smem);
