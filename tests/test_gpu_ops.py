@@ -430,9 +430,9 @@ def test_attention_tc_gemma_paged(dtype, B, q, T, nq):
 @pytest.mark.parametrize("dtype", [torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [(4096, 4304, 1152), (4100, 2560, 512), (16384, 1152, 4304)])
 @pytest.mark.parametrize("epi", ["bias", "bias_gelu", "bias_res", "f32"])
-def test_gemm_tcgen05_large_m_multicast_pairs(dtype, M, N, K, epi):
-    """Large-M shapes take the 128x256 tiles with 2-CTA clusters and TMA-multicast W halves (odd m-tile counts
-    exercise the ghost tile of the last pair)."""
+def test_gemm_tcgen05_large_m_pairs(dtype, M, N, K, epi):
+    """Large-M shapes take the 256x256 tiles of the CTA-pair kernel (odd m-tile counts exercise the ghost tile of the
+    last pair)."""
     a = gen(M, K, dtype=dtype)
     w = gen(N, K, seed=1, scale=1.0 / math.sqrt(K), dtype=dtype)
     bias, res = gen(N, seed=3, scale=0.1, dtype=dtype), gen(M, N, seed=4, dtype=dtype)

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Time pg_gemm (tcgen05 paths) on the SigLIP batch-64 / prefill shapes; TFLOP/s per shape.
-Tunables come from the environment (PG_GEMM_2CTA, PG_GEMM_MCAST, PG_GEMM_BN ...)."""
+Tunables come from the environment (PG_GEMM_2CTA, PG_GEMM_BN ...)."""
 import json
 import os
 import sys
