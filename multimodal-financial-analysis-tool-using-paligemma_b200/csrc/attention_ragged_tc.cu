@@ -285,7 +285,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     s_half[n_tiles & 1][hf][r] = l;
     meet();
     l = s_half[n_tiles & 1][0][r] + s_half[n_tiles & 1][1][r];
-    if (ok && wait(bar_o(n_tiles - 1), n_tiles - 1)) {
+    if (__all_sync(0xffffffffu, wait(bar_o(n_tiles - 1), n_tiles - 1) && ok)) {   // the loads below take the whole warp
       tc_fence_after();
       if (p.sink && !sig) l += exp2_approx(p.sink[h] * LOG2E_F - m);   // a logit without key or value, counted once
       float inv = (sig ? 1.f : 1.f / l) * p.out_scale;

@@ -134,12 +134,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
   } else if (warp >= 4) {
     // ===================== softmax + epilogue: thread <-> query row =====================
+    // A wait that gave up leaves the loop running (every later wait returns at once): votes, loads and stores of TMEM take
+    // the whole warp.
     const int qw = warp & 3, r = qw * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
     float m = -INFINITY, l = 0.f;                                    // m in units of log2
     bool ok = true;
     for (int t = 0; t < n_tiles; ++t) {
-      if (!wait(bar_s(t), t)) { ok = false; break; }
+      ok = wait(bar_s(t), t) && ok;
       tc_fence_after();
       float s[KT];
       tmem_ld32(t_row + (t & 1) * KT, s);
@@ -174,7 +176,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (t > 0) {
           const float corr = exp2_approx(m - m_new);
           l *= corr;
-          if (!wait(bar_o(t - 1), t - 1)) { ok = false; break; }     // nothing adds to O until this tile's P is handed over
+          ok = wait(bar_o(t - 1), t - 1) && ok;                      // nothing adds to O until this tile's P is handed over
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c * 16 < nv; ++c) {
@@ -204,7 +206,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_arrive(bar_p(t));
     }
     if (n_tiles > 0) {
-      ok = ok && wait(bar_o(n_tiles - 1), n_tiles - 1);
+      ok = wait(bar_o(n_tiles - 1), n_tiles - 1) && ok;
       tc_fence_after();
       const int qi = qb * AQ + r;
       const float inv = ok ? 1.f / l : NAN;                          // a wait that gave up shows in the rows it would have written

@@ -192,7 +192,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     TileCursor cur(p.offsets, p.n_experts, n_tiles_n, p.group_rows);
     int e, m0, m_end, n_blk;
     for (int tile = blockIdx.x; cur.seek(tile, e, m0, m_end, n_blk); tile += gridDim.x) {
-      if (!mbar_wait_lim(tfull_bar(acc), acc_phase, fail)) break;
+      if (!mbar_wait_lim_warp(tfull_bar(acc), acc_phase, fail)) break;
       tc_fence_after();
       const int m = m0 + q * 32 + lane;
       // where this thread's row goes: the grouped row itself, or (per-head mode) its token row at the head's columns
@@ -367,7 +367,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint32_t acc_phase = 0;
     TileCursor cur(p.offsets, p.n_experts, n_tiles_n, 0, 2 * MG_BM);
     for (int tile = sched_first; cur.seek(tile, e, m0, m_end, n_blk); tile += sched_stride) {
-      if (!mbar_wait_lim(tfull_bar(acc), acc_phase, fail)) break;
+      if (!mbar_wait_lim_warp(tfull_bar(acc), acc_phase, fail)) break;
       tc_fence_after();
       const int row0 = m0 + (int)crank * MG_BM + q * 32, nw0 = n_blk * TILE_N + half * (TILE_N / 2);
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * M2_BN + half * (TILE_N / 2);

@@ -110,6 +110,10 @@ __device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity, vol
   *fail = 1;
   return false;
 }
+// The same for a whole warp that goes on to warp-wide instructions (tcgen05.ld, votes): its lanes agree on the outcome.
+__device__ __forceinline__ bool mbar_wait_lim_warp(uint32_t bar, uint32_t parity, volatile int* fail) {
+  return __all_sync(0xffffffffu, mbar_wait_lim(bar, parity, fail));
+}
 
 // A (the weights) from TMEM: 128 lanes, two 16-bit values of a row per column
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
