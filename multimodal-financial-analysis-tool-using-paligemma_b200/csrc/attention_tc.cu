@@ -171,10 +171,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
       for (int j = 4; j < KT; ++j) mx[j & 3] = fmaxf(mx[j & 3], s[j]);
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {            // always for the first tile: it holds a key of every row
+      if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {            // m == -inf: any finite score raises it
         const float m_new = fmaxf(m, top);
         if (t > 0) {
-          const float corr = exp2_approx(m - m_new);
+          const float corr = m_new == m ? 1.f : exp2_approx(m - m_new);
           l *= corr;
           ok = wait(bar_o(t - 1), t - 1) && ok;                      // nothing adds to O until this tile's P is handed over
           tc_fence_after();
@@ -190,10 +190,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         m = m_new;
       }
+      const float ref = m == -INFINITY ? 0.f : m;                    // every score so far is -inf (fp16: products below -65504)
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < KT; ++j) {
-        s[j] = exp2_approx(s[j] - m);
+        s[j] = exp2_approx(s[j] - ref);
         sum[j & 3] += s[j];
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);

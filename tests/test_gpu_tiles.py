@@ -130,6 +130,32 @@ def test_prompt_attention(B, q, T, H, G, hd):
         assert _rel(out[b * q:(b + 1) * q], want) < 8e-3
 
 
+@pytest.mark.parametrize("q,T,low", [(3, 70, 64), (130, 260, 128), (16, 200, 130), (5, 40, 40)])
+def test_prompt_attention_scores_below_the_type(q, T, low):
+    """The first `low` scores of some rows round to -inf in fp16: those keys weigh nothing, and only a row without any other
+    key is undefined, as the reference's softmax has it."""
+    cabi, L, st = _cabi()
+    H, hd, dt = 4, 256, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(T + low)
+    cols = -(-T // 64)
+    kp, vp, qq = (_randn(g, *s, std=std, dtype=dt) for s, std in (((cols, 64, hd), 0.01), ((cols, 64, hd), 1.0), ((q, H * hd), 0.3)))
+    kp.view(-1, hd)[:low] = -30.0
+    qq.view(q, H, hd)[::2, 1:] = 30.0            # 256 x 30 x -30: below -65504
+    pt = torch.arange(cols, dtype=torch.int32, device="cuda").view(1, cols)
+    kvl = torch.full((1,), T - q, dtype=torch.int32, device="cuda")
+    out = torch.zeros(q, H * hd, dtype=dt, device="cuda")
+    cabi.check(L.pg_attention_tc(out.data_ptr(), H * hd, qq.data_ptr(), q, H * hd, 0, kp.data_ptr(), vp.data_ptr(), cols * 64, hd, 0, 0, hd,
+                                 0, pt.data_ptr(), cols, 64, kvl.data_ptr(), 0, q, 1, q, H, 1, hd, math.sqrt(hd), 1, cabi.PG_F16, st))
+    k, v = (p.view(-1, hd)[:T].to(F64) for p in (kp, vp))
+    s = torch.einsum("qhd,nd->hqn", qq.view(q, H, hd).to(F64), k).to(dt).to(F64) / math.sqrt(hd)
+    assert bool(torch.isinf(s).any())
+    want = torch.einsum("hqn,nd->qhd", torch.softmax(s, -1), v).reshape(q, H * hd)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and bool(torch.isnan(want).any()) == (low == T)
+    sure = ~torch.isnan(want)
+    # weights and result are rounded to fp16 (2^-12 each at most); a score that rounds the other way moves its weight
+    assert float((out.to(F64) - want)[sure].norm() / want[sure].norm()) < 2e-3
+
+
 @pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (128, 128, 12, 1), (256, 256, 8, 1), (256, 192, 5, 1)])
 @pytest.mark.parametrize("window,keep,chunk", [(0, 0, 0), (33, 0, 0), (100, 7, 0), (0, 0, 48)])
 def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
