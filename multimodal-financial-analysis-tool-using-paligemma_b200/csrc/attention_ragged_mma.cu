@@ -112,11 +112,11 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
         float mx = fmaxf(w[h], w[h + 2]);
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float mn = fmaxf(m[h], mx);
-        corr[h] = expf(m[h] - mn);
+        const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;   // -inf: no key so far has any weight
+        corr[h] = expf(m[h] - ref);
         m[h] = mn;
-        w[h] = expf(w[h] - mn);
-        w[h + 2] = expf(w[h + 2] - mn);
+        w[h] = expf(w[h] - ref);
+        w[h + 2] = expf(w[h + 2] - ref);
         l[h] = l[h] * corr[h] + (w[h] + w[h + 2]);          // this lane's keys; the lanes meet at the end
       }
     }
@@ -171,6 +171,7 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     float L = 0.f;
     for (int k = 0; k < busy; ++k) {
+      if (s_m[k][hh] == -INFINITY) continue;                // a warp whose keys have no weight
       const float f = expf(s_m[k][hh] - M);
       const float4 v = *reinterpret_cast<const float4*>(&s_acc[k][hh][d]);
       a.x = fmaf(f, v.x, a.x); a.y = fmaf(f, v.y, a.y); a.z = fmaf(f, v.z, a.z); a.w = fmaf(f, v.w, a.w);
@@ -198,7 +199,7 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
     float a = 0.f, L = 0.f;
 #pragma unroll
     for (int i = 0; i < RM_MAX_CTAS; ++i)
-      if (i < n_cta) {
+      if (i < n_cta && pm[i] != -INFINITY) {
         const float f = expf(pm[i] - M);
         a = fmaf(f, pa[i], a);
         L = fmaf(f, pl[i], L);

@@ -462,11 +462,11 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
       float mx = fmaxf(p[h], p[h + 2]);
 #pragma unroll
       for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float mn = fmaxf(m[h], mx);
-      corr[h] = __expf(m[h] - mn);
+      const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;   // -inf: no key so far has any weight
+      corr[h] = __expf(m[h] - ref);
       m[h] = mn;
-      p[h] = __expf(p[h] - mn);
-      p[h + 2] = __expf(p[h + 2] - mn);
+      p[h] = __expf(p[h] - ref);
+      p[h + 2] = __expf(p[h + 2] - ref);
       l[h] = l[h] * corr[h] + (p[h] + p[h + 2]);              // this lane's tokens; the lanes meet at the end
     }
     uint32_t pb[3][2];                                        // three 16-bit terms of the weights, as B fragments
@@ -520,6 +520,7 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     float L = 0.f;
     for (int w = 0; w < busy; ++w) {
+      if (s_m[w][g] == -INFINITY) continue;                   // a warp whose tokens have no weight
       const float f = __expf(s_m[w][g] - M);
       const float4 v = *reinterpret_cast<const float4*>(&s_acc[w][g][d]);
       a.x = fmaf(f, v.x, a.x); a.y = fmaf(f, v.y, a.y); a.z = fmaf(f, v.z, a.z); a.w = fmaf(f, v.w, a.w);
@@ -549,7 +550,7 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
     float a = 0.f, L = 0.f;
 #pragma unroll
     for (int i = 0; i < NS; ++i)
-      if (i < n_cta) {
+      if (i < n_cta && pm[i] != -INFINITY) {
         const float w = __expf(pm[i] - M);
         a = fmaf(w, pa[i], a);
         L = fmaf(w, pl[i], L);

@@ -37,3 +37,26 @@ def test_chunks_pages_and_clusters(dtype, rel, B, T, G, nkv, page):
         got = out[b].to(F64)
         # one rounding of the result (2^-9 and 2^-12 relative at most) and the odd score that rounds the other way
         assert float((got - want).norm() / want.norm()) < rel
+
+
+@pytest.mark.parametrize("T,lo,hi", [(262, 0, 16), (262, 32, 70), (1345, 1024, 1345), (600, 5, 600), (40, 0, 40)])
+def test_scores_below_the_type(T, lo, hi):
+    """fp16 scores of the tokens [lo, hi) round to -inf for half of the heads: those tokens weigh nothing there, wherever
+    the chunks, warps and clusters cut, and a head without any other token is undefined."""
+    from pg_b200 import _cabi as cabi
+    hd, G, page, dt = 256, 8, 64, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(T + lo)
+    cols = -(-T // page)
+    kp, vp = ((torch.randn(cols, page, hd, device="cuda", generator=g) * std).to(dt) for std in (0.01, 1.0))
+    q = (torch.randn(G, hd, device="cuda", generator=g) * 0.3).to(dt)
+    kp.view(-1, hd)[lo:hi] = -30.0
+    q[::2] = 30.0
+    pt = torch.arange(cols, dtype=torch.int32, device="cuda")
+    out, kvl = torch.zeros(G, hd, dtype=dt, device="cuda"), torch.tensor([T], dtype=torch.int32, device="cuda")
+    cabi.check(cabi.lib().pg_decode_attention(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page,
+                                              kvl.data_ptr(), 0, 1, G, 1, hd, 16.0, None, None, 0, cabi.PG_F16, cabi.stream()))
+    k, v = (p.view(-1, hd)[:T].to(F64) for p in (kp, vp))
+    want = torch.softmax((q.to(F64) @ k.T).to(dt).to(F64) / 16.0, -1) @ v
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and bool(torch.isnan(want).any()) == (hi - lo == T)
+    sure = ~torch.isnan(want)
+    assert float((out.to(F64) - want)[sure].norm() / want[sure].norm()) < 6e-4      # as above

@@ -189,6 +189,38 @@ def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
         assert _rel(out[t], want) < 4e-3          # one rounding of the result; weights are fp32
 
 
+def _single_tokens(q, kp, vp, pos, H, G, dim, vdim, scale, head_bias=None, sigmoid=0):
+    cabi, L, st = _cabi()
+    n, dt = q.shape[0], q.dtype
+    cols = kp.shape[0] // n
+    pt = torch.arange(n * cols, dtype=torch.int32, device="cuda")
+    slot, tp = torch.arange(n, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda")
+    out, ws = torch.zeros(n, H * vdim, dtype=dt, device="cuda"), torch.empty(1 << 20, device="cuda")
+    cabi.check(L.pg_attention_ragged_ex(out.data_ptr(), H * vdim, q.data_ptr(), H * dim, None, 0, 0, kp.data_ptr(), vp.data_ptr(),
+                                        pt.data_ptr(), cols, 64, slot.data_ptr(), tp.data_ptr(), n, H, G, dim, vdim, scale, 0, 0, None, sigmoid,
+                                        None if head_bias is None else head_bias.data_ptr(), 1.0, ws.data_ptr(), ws.numel(),
+                                        cabi.DTYPE_CODE[dt], st))
+    return out
+
+
+@pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (256, 192, 5, 1), (256, 256, 8, 1)])
+@pytest.mark.parametrize("lo,hi", [(0, 16), (16, 48), (100, 1000)])
+def test_single_tokens_scores_of_minus_infinity(dim, vdim, H, G, lo, hi):
+    """Keys [lo, hi) whose scores are -inf weigh nothing, wherever the chunks, warps and clusters cut."""
+    g = torch.Generator(device="cuda").manual_seed(dim + lo)
+    pos, cols = [47, 63, 200, 1279], 20
+    kp, vp = _randn(g, 4 * cols, 64, G * dim, std=1e-20), _randn(g, 4 * cols, 64, G * vdim)
+    q = torch.full((4, H * dim), 1e20, dtype=BF, device="cuda")
+    kp.view(4, -1, G * dim)[:, lo:hi] = -1e20                    # products of -1e40
+    out = _single_tokens(q, kp, vp, pos, H, G, dim, vdim, dim ** -0.5)
+    for t, p in enumerate(pos):
+        k, v = (x.view(4, -1, G, w)[t, :p + 1].to(F64).repeat_interleave(H // G, 1) for x, w in ((kp, dim), (vp, vdim)))
+        s = torch.einsum("hd,nhd->hn", q[t].view(H, dim).to(F64), k) * dim ** -0.5
+        s[:, lo:hi] = -math.inf
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1), v).reshape(-1)
+        assert _rel(out[t], want) < 4e-3                         # one rounding of the result; weights are fp32
+
+
 @pytest.mark.parametrize("M", [16, 129, 256, 260, 384])
 @pytest.mark.parametrize("N,K,epi", [(1152, 4304, "bias_res"), (2048, 2048, "res"), (2560, 2048, "none"), (1160, 1152, "bias_gelu"),
                                      (520, 1096, "f32")])
