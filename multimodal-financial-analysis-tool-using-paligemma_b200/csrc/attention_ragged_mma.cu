@@ -7,7 +7,8 @@
 // every key and value row is read once for the whole group, straight into fragments with 16-byte loads: the contraction index of
 // S^T is permuted (lane j of a quad owns 8 consecutive columns of every 32), and so are the rows of O^T (lane group r owns 8
 // consecutive columns of every 64).  Q K^T multiplies the stored 16-bit operands; the weights stay fp32 and enter P V as three
-// 16-bit terms, so that the product is the fp32 one.  (m, l, O) of the warps meet in shared memory and those of the CTAs in
+// 16-bit terms (mma_frag.cuh), so that the product is the fp32 one; fp16 sigmoid weights, which no maximum normalises, stay with
+// the fp32 kernels.  (m, l, O) of the warps meet in shared memory and those of the CTAs in
 // distributed shared memory, in a fixed order: one launch, no workspace.
 // The key-slice kernel of attention_ragged.cu gives a whole key row to one lane (32 rows of 16 bytes per load), keeps the query
 // in shared memory and needs a second launch to merge: 8 tokens x 1024 keys, 16 heads over 4, 128 wide: 30.2 + 9.7 us, this
@@ -120,6 +121,8 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
         l[h] = l[h] * corr[h] + (w[h] + w[h + 2]);          // this lane's keys; the lanes meet at the end
       }
     }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] *= split_scale<T>();
     uint32_t pb[3][2];                                      // three 16-bit terms of the weights, as B fragments
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -157,9 +160,7 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
       if (r == 0) { s_m[wid][2 * j + h] = m[h]; s_l[wid][2 * j + h] = l[h]; }
 #pragma unroll
       for (int vb = 0; vb < VB; ++vb) {
-        float4* dst = reinterpret_cast<float4*>(&s_acc[wid][2 * j + h][vb * 64 + r * 8]);
-        dst[0] = make_float4(acc[vb][0][h], acc[vb][0][h + 2], acc[vb][1][h], acc[vb][1][h + 2]);
-        dst[1] = make_float4(acc[vb][2][h], acc[vb][2][h + 2], acc[vb][3][h], acc[vb][3][h + 2]);
+        store_acc<T>(&s_acc[wid][2 * j + h][vb * 64 + r * 8], acc[vb], h);
       }
     }
   }
@@ -264,9 +265,10 @@ static int launch_rm(const RagAttnParams& p, cudaStream_t st) {
   return check_launch("attention_ragged_mma");
 }
 
-// (key width, value width) pairs the kernel is built for; everything it loads in 16 bytes lies on 16-byte boundaries
+// (key width, value width) pairs the kernel is built for, weights its 16-bit terms hold (mma_frag.cuh); everything it loads in
+// 16 bytes lies on 16-byte boundaries
 bool attention_ragged_mma_wanted(const RagAttnParams& p, int dtype) {
-  if (dtype != PG_BF16 && dtype != PG_F16) return false;
+  if (dtype != PG_BF16 && (dtype != PG_F16 || p.sigmoid_weights)) return false;
   const bool square = p.dim == p.vdim && (p.dim == 64 || p.dim == 128 || p.dim == 256);
   if (!square && !(p.dim == 256 && p.vdim == 192)) return false;
   if (p.ld_q % 8 || p.ld_k % 8 || p.ld_v % 8 || (((uintptr_t)p.q | (uintptr_t)p.k_pool | (uintptr_t)p.v_pool) & 15)) return false;

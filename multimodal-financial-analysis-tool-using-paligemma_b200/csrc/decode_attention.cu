@@ -374,8 +374,7 @@ static int launch_da(void* out, const void* q, const void* k_pool, const void* v
 // A warp takes 16 tokens at a time and all operands go from global memory straight into fragments with 16-byte loads: the
 // contraction index of S^T is permuted (lane j of a quad owns 8 consecutive columns of every 32) and so are the rows of O^T
 // (lane group r owns 8 consecutive columns of every 64), which neither product notices.  The weights stay fp32: they enter
-// as three 16-bit terms (8 + 8 + 8 mantissa bits in bf16), so that P V is the fp32 product; only QK^T's operands are 16-bit,
-// as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
+// as three 16-bit terms (mma_frag.cuh), so that P V is the fp32 product; only QK^T's operands are 16-bit, as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
 // Measured (launch alone, cold cache): 1 sequence x 262 tokens 13.5 -> 9.5 us, 8 x 1345 39.7 -> 14.2 us, 32 x 389 23.6 -> 12.1 us;
 // inside the captured step 4.0, 23 and 5.1 us per layer less.
 constexpr int DM_WARPS = 4, DM_HD = 256, DM_G = 8;
@@ -469,6 +468,8 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
       p[h + 2] = __expf(p[h + 2] - ref);
       l[h] = l[h] * corr[h] + (p[h] + p[h + 2]);              // this lane's tokens; the lanes meet at the end
     }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[e] *= split_scale<T>();
     uint32_t pb[3][2];                                        // three 16-bit terms of the weights, as B fragments
 #pragma unroll
     for (int n = 0; n < 3; ++n) {
@@ -506,9 +507,7 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
       if (r == 0) { s_m[wid][2 * j + h] = m[h]; s_l[wid][2 * j + h] = l[h]; }
 #pragma unroll
       for (int vb = 0; vb < VB; ++vb) {
-        float4* dst = reinterpret_cast<float4*>(&s_acc[wid][2 * j + h][vb * 64 + r * 8]);
-        dst[0] = make_float4(acc[vb][0][h], acc[vb][0][h + 2], acc[vb][1][h], acc[vb][1][h + 2]);
-        dst[1] = make_float4(acc[vb][2][h], acc[vb][2][h + 2], acc[vb][3][h], acc[vb][3][h + 2]);
+        store_acc<T>(&s_acc[wid][2 * j + h][vb * 64 + r * 8], acc[vb], h);
       }
     }
   }

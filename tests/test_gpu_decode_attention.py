@@ -60,3 +60,23 @@ def test_scores_below_the_type(T, lo, hi):
     assert torch.equal(torch.isnan(out), torch.isnan(want)) and bool(torch.isnan(want).any()) == (hi - lo == T)
     sure = ~torch.isnan(want)
     assert float((out.to(F64) - want)[sure].norm() / want[sure].norm()) < 6e-4      # as above
+
+
+@pytest.mark.parametrize("dtype,rel", [(torch.bfloat16, 4e-3), (torch.float16, 6e-4)])
+@pytest.mark.parametrize("T,low", [(4097, -15.0), (700, -11.5), (65, -9.25)])
+def test_many_small_weights(dtype, rel, T, low):
+    """One token of weight 1 and value 0, T - 1 of weight exp(low) and value 1: the small weights make up the result."""
+    from pg_b200 import _cabi as cabi
+    hd, G, page = 256, 8, 64
+    cols = -(-T // page)
+    kp, vp = torch.zeros(cols, page, hd, dtype=dtype, device="cuda"), torch.ones(cols, page, hd, dtype=dtype, device="cuda")
+    kp.view(-1, hd)[1:, 0] = 16.0 * low
+    vp.view(-1, hd)[0] = 0.0
+    q = torch.zeros(G, hd, dtype=dtype, device="cuda")
+    q[:, 0] = 1.0
+    pt = torch.arange(cols, dtype=torch.int32, device="cuda")
+    out, kvl = torch.zeros(G, hd, dtype=dtype, device="cuda"), torch.tensor([T], dtype=torch.int32, device="cuda")
+    cabi.check(cabi.lib().pg_decode_attention(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page,
+                                              kvl.data_ptr(), 0, 1, G, 1, hd, 16.0, None, None, 0, cabi.DTYPE_CODE[dtype], cabi.stream()))
+    small = (T - 1) * math.exp(low)
+    assert float((out.to(F64) / (small / (1.0 + small)) - 1.0).abs().max()) < rel     # one rounding of the result

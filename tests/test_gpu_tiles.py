@@ -221,6 +221,27 @@ def test_single_tokens_scores_of_minus_infinity(dim, vdim, H, G, lo, hi):
         assert _rel(out[t], want) < 4e-3                         # one rounding of the result; weights are fp32
 
 
+@pytest.mark.parametrize("dtype,rel", [(BF, 4e-3), (torch.float16, 6e-4)])
+@pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (256, 192, 5, 1), (256, 256, 8, 1)])
+@pytest.mark.parametrize("sigmoid,low", [(0, -15.0), (0, -9.25), (1, -14.0), (1, -17.5), (1, -2.0)])
+def test_single_tokens_small_weights(dtype, rel, dim, vdim, H, G, sigmoid, low):
+    """Softmax: one key of weight 1 and value 0 beside many of weight exp(low) and value 1.  Sigmoid: nothing but weights of
+    sigmoid(low), of which fp16 itself would hold a few bits or none."""
+    n, cols, pos = 3, 40, [1, 700, 2559]
+    new = lambda f, *s: torch.full(s, f, dtype=dtype, device="cuda")  # noqa: E731
+    kp, vp, q = new(0.0, n * cols, 64, G * dim), new(1.0, n * cols, 64, G * vdim), new(0.0, n, H * dim)
+    q.view(n, H, dim)[:, :, 0] = 1.0
+    if not sigmoid:
+        kp.view(n, -1, G, dim)[:, 1:, :, 0] = low
+        vp.view(n, -1, G * vdim)[:, 0] = 0.0
+    out = _single_tokens(q, kp, vp, pos, H, G, dim, vdim, 1.0, torch.full((H,), low, device="cuda") if sigmoid else None, sigmoid)
+    for t, p in enumerate(pos):
+        small = p * math.exp(low)
+        want = (p + 1) / (1.0 + math.exp(-low)) if sigmoid else small / (1.0 + small)
+        # one rounding of the result (below 2^-14 an fp16 result is a multiple of 2^-24), up to 2560 fp32 additions
+        assert float((out[t].to(F64) - want).abs().max()) < rel * want + (2.0 ** -25 if dtype == torch.float16 else 0.0)
+
+
 @pytest.mark.parametrize("M", [16, 129, 256, 260, 384])
 @pytest.mark.parametrize("N,K,epi", [(1152, 4304, "bias_res"), (2048, 2048, "res"), (2560, 2048, "none"), (1160, 1152, "bias_gelu"),
                                      (520, 1096, "f32")])
