@@ -57,15 +57,8 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
   const float qscale = query_scale(p, pos);
   const T* kpool = reinterpret_cast<const T*>(p.k_pool) + (size_t)g * DIM + j * 8;
   const T* vpool = reinterpret_cast<const T*>(p.v_pool) + (size_t)g * VDIM + r * 8;
-  float acc[VB][4][4];
-#pragma unroll
-  for (int vb = 0; vb < VB; ++vb)
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
   const float m_init = p.sigmoid_weights ? 0.f : -INFINITY;
-  float m[2] = {m_init, m_init}, l[2] = {0.f, 0.f};       // the same in every lane group
+  float acc[VB][4][4], m[2], l[2];                        // m, l: the same in every lane group
 
   const int chunks = (kr.count + 15) / 16, stride = ns * RM_WARPS;
   // lane L looks up key L % 16 of a chunk (positions behind the last key repeat it, with weight 0): its position and pool row
@@ -74,6 +67,15 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
     key = kr.key(min(16 * c + (lane & 15), kr.count - 1));
     row = pt_row[key / p.page_size] * p.page_size + key % p.page_size;
   };
+  for (bool in_fp32 = false;; in_fp32 = true) {
+#pragma unroll
+  for (int vb = 0; vb < VB; ++vb)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
+  m[0] = m[1] = m_init;
+  l[0] = l[1] = 0.f;
   int c = rank + ns * wid;
   if (c < chunks) look_up(c);
   for (; c < chunks; c += stride) {
@@ -90,7 +92,7 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
       va[vb][0] = ldg_cached(vpool + v0 + vb * 64); va[vb][1] = ldg_cached(vpool + v1 + vb * 64);
       va[vb][2] = ldg_cached(vpool + v2 + vb * 64); va[vb][3] = ldg_cached(vpool + v3 + vb * 64);
     }
-    if (c + stride < chunks) look_up(c + stride);          // the next chunk's pages come in beside this one's rows
+    if (!in_fp32 && c + stride < chunks) look_up(c + stride);   // the next chunk's pages come in beside this one's rows
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int kb = 0; kb < KB; ++kb) {
@@ -123,29 +125,14 @@ attention_ragged_mma_kernel(RagAttnParams p, int head_chunks) {
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) w[e] *= split_scale<T>();
-    uint32_t pb[3][2];                                      // three 16-bit terms of the weights, as B fragments
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      pb[k][0] = transpose_8x8(split_pair<T>(w[0], w[1]));
-      pb[k][1] = transpose_8x8(split_pair<T>(w[2], w[3]));
+    if (!in_fp32) {
+      add_values<T, VB>(acc, va, w, corr);
+    } else {
+      add_values_fp32<T, VB>(acc, [&](int k) { return vpool + (size_t)__shfl_sync(0xffffffffu, row, k) * p.ld_v; }, w, corr, n);
+      if (c + stride < chunks) look_up(c + stride);
     }
-#pragma unroll
-    for (int vb = 0; vb < VB; ++vb) {
-      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&va[vb][0]);
-      const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&va[vb][1]);
-      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&va[vb][2]);
-      const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&va[vb][3]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // rows r and r + 8 of this product: columns 64 vb + 8 r + 2 i and + 1
-        const uint32_t a0 = __byte_perm(w0[i], w1[i], 0x5410), a1 = __byte_perm(w0[i], w1[i], 0x7632);
-        const uint32_t a2 = __byte_perm(w2[i], w3[i], 0x5410), a3 = __byte_perm(w2[i], w3[i], 0x7632);
-        float (&o)[4] = acc[vb][i];
-        o[0] *= corr[0]; o[1] *= corr[1]; o[2] *= corr[0]; o[3] *= corr[1];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) mma_16816<T>(o, a0, a1, a2, a3, pb[k][0], pb[k][1]);
-      }
-    }
+  }
+  if (in_fp32 || !any_nan(acc)) break;                      // an infinity among the values: once more
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h)

@@ -408,18 +408,20 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
 #pragma unroll
     for (int kb = 0; kb < KB; ++kb) qf[kb] = r < G ? ldg_cached(qr + kb * 32) : make_uint4(0, 0, 0, 0);
   }
-  float acc[VB][4][4];
+  float acc[VB][4][4], m[2], l[2];                          // m, l: heads 2j and 2j + 1, the same in every lane group
+  __syncthreads();
+
+  const int chunks = (T_len + 15) / 16;
+  const size_t row_elems = (size_t)nkv * DM_HD;
+  for (bool in_fp32 = false;; in_fp32 = true) {
 #pragma unroll
   for (int vb = 0; vb < VB; ++vb)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // heads 2j and 2j + 1, the same in every lane group
-  __syncthreads();
-
-  const int chunks = (T_len + 15) / 16;
-  const size_t row_elems = (size_t)nkv * DM_HD;
+  m[0] = m[1] = -INFINITY;
+  l[0] = l[1] = 0.f;
   // chunk c: CTA c % NS first, so that a short context spreads over the SMs before it stacks up in one
   for (int c = rank + NS * wid; c < chunks; c += NS * DM_WARPS) {
     const int t0 = c * 16, pi = t0 / page_size;               // page_size is a multiple of 16: one page per chunk
@@ -470,29 +472,10 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) p[e] *= split_scale<T>();
-    uint32_t pb[3][2];                                        // three 16-bit terms of the weights, as B fragments
-#pragma unroll
-    for (int n = 0; n < 3; ++n) {
-      pb[n][0] = transpose_8x8(split_pair<T>(p[0], p[1]));
-      pb[n][1] = transpose_8x8(split_pair<T>(p[2], p[3]));
-    }
-#pragma unroll
-    for (int vb = 0; vb < VB; ++vb) {
-      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&va[vb][0]);
-      const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&va[vb][1]);
-      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&va[vb][2]);
-      const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&va[vb][3]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // rows r and r + 8 of this product: columns 64 vb + 8 r + 2 i and + 1
-        const uint32_t a0 = __byte_perm(w0[i], w1[i], 0x5410), a1 = __byte_perm(w0[i], w1[i], 0x7632);
-        const uint32_t a2 = __byte_perm(w2[i], w3[i], 0x5410), a3 = __byte_perm(w2[i], w3[i], 0x7632);
-        float (&o)[4] = acc[vb][i];
-        o[0] *= corr[0]; o[1] *= corr[1]; o[2] *= corr[0]; o[3] *= corr[1];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) mma_16816<T>(o, a0, a1, a2, a3, pb[n][0], pb[n][1]);
-      }
-    }
+    if (!in_fp32) add_values<T, VB>(acc, va, p, corr);
+    else add_values_fp32<T, VB>(acc, [&](int k) { return vp + k * row_elems; }, p, corr, last + 1);
+  }
+  if (in_fp32 || !any_nan(acc)) break;                        // an infinity among the values: once more
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h)

@@ -80,3 +80,27 @@ def test_many_small_weights(dtype, rel, T, low):
                                               kvl.data_ptr(), 0, 1, G, 1, hd, 16.0, None, None, 0, cabi.DTYPE_CODE[dtype], cabi.stream()))
     small = (T - 1) * math.exp(low)
     assert float((out.to(F64) / (small / (1.0 + small)) - 1.0).abs().max()) < rel     # one rounding of the result
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [1, 37, 262, 1345])
+def test_infinite_values(dtype, T):
+    """An infinity in a value row makes its column infinite for every head that gives the token weight, and no other column."""
+    from pg_b200 import _cabi as cabi
+    hd, G, page = 256, 8, 64
+    g = torch.Generator(device="cuda").manual_seed(T)
+    cols = -(-T // page)
+    kp, vp, q = (torch.randn(s, device="cuda", generator=g).to(dtype) * std for s, std in (((cols, page, hd), 0.3), ((cols, page, hd), 1.0),
+                                                                                          ((G, hd), 0.3)))
+    for token, col, value in ((0, 3, math.inf), (T // 2, 130, -math.inf), (T - 1, 70, math.inf)):
+        vp.view(-1, hd)[token, col] = value
+    pt = torch.arange(cols, dtype=torch.int32, device="cuda")
+    out, kvl = torch.zeros(G, hd, dtype=dtype, device="cuda"), torch.tensor([T], dtype=torch.int32, device="cuda")
+    cabi.check(cabi.lib().pg_decode_attention(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page,
+                                              kvl.data_ptr(), 0, 1, G, 1, hd, 16.0, None, None, 0, cabi.DTYPE_CODE[dtype], cabi.stream()))
+    k, v = (p.view(-1, hd)[:T].to(F64) for p in (kp, vp))
+    w = torch.softmax((q.to(F64) @ k.T).to(dtype).to(F64) / 16.0, -1)
+    fine = torch.isfinite(v).all(0)
+    assert bool((out[:, 3] == math.inf).all()) and bool((out[:, 130] == -math.inf).all()) and bool((out[:, 70] == math.inf).all())
+    want = w @ v[:, fine]
+    assert float((out[:, fine].to(F64) - want).norm() / want.norm()) < 4e-3      # the bound of bf16 above

@@ -242,6 +242,28 @@ def test_single_tokens_small_weights(dtype, rel, dim, vdim, H, G, sigmoid, low):
         assert float((out[t].to(F64) - want).abs().max()) < rel * want + (2.0 ** -25 if dtype == torch.float16 else 0.0)
 
 
+@pytest.mark.parametrize("dtype", [BF, torch.float16])
+@pytest.mark.parametrize("sigmoid", [0, 1])
+@pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (256, 192, 5, 1), (256, 256, 8, 1)])
+def test_single_tokens_infinite_values(dtype, sigmoid, dim, vdim, H, G):
+    """An infinity in a value row makes its column infinite for the tokens that see the key, and no other column."""
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    pos, cols = [0, 20, 300, 1279], 20
+    kp, vp, q = (_randn(g, *s, dtype=dtype) for s in ((4 * cols, 64, G * dim), (4 * cols, 64, G * vdim), (4, H * dim)))
+    v4 = vp.view(4, -1, G, vdim)
+    for t, p in enumerate(pos):
+        v4[t, 0, :, 3], v4[t, p // 2, :, 40], v4[t, p, :, 50] = math.inf, -math.inf, math.inf
+    out = _single_tokens(q, kp, vp, pos, H, G, dim, vdim, dim ** -0.5, torch.full((H,), -3.0, device="cuda") if sigmoid else None, sigmoid)
+    for t, p in enumerate(pos):
+        k, v = (x.view(4, -1, G, w)[t, :p + 1].to(F64).repeat_interleave(H // G, 1) for x, w in ((kp, dim), (vp, vdim)))
+        s = torch.einsum("hd,nhd->hn", q[t].view(H, dim).to(F64), k) * dim ** -0.5
+        w = torch.sigmoid(s - 3.0) if sigmoid else torch.softmax(s, -1)
+        o, fine = out[t].view(H, vdim), torch.isfinite(v).all(0).all(0)
+        assert bool((o[:, 3] == math.inf).all()) and bool((o[:, 40] == -math.inf).all()) and bool((o[:, 50] == math.inf).all())
+        want = torch.einsum("hn,nhd->hd", w, v[:, :, fine])
+        assert _rel(o[:, fine], want) < 4e-3      # one rounding of the result; weights are fp32
+
+
 @pytest.mark.parametrize("M", [16, 129, 256, 260, 384])
 @pytest.mark.parametrize("N,K,epi", [(1152, 4304, "bias_res"), (2048, 2048, "res"), (2560, 2048, "none"), (1160, 1152, "bias_gelu"),
                                      (520, 1096, "f32")])
