@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(256)
 im2col_rows_kernel(T* __restrict__ out, const T* __restrict__ px, int C, int H, int W, int p, int ld_out, int n_rows) {
   struct alignas(2 * sizeof(T)) P { T a, b; };
   const int G = W / p, per_tok = C * p;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n_rows; idx += gridDim.x * blockDim.x) {
+  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < n_rows; at += (long long)gridDim.x * blockDim.x) {
+    const int idx = (int)at;             // rows are counted in 32 bits; the step behind the last one may not fit
     // neighbouring threads take the same row of neighbouring patches: their loads are consecutive
     const int gx = idx % G, k = idx / G, ky = k % p, k2 = k / p, c = k2 % C, k3 = k2 / C, gy = k3 % (H / p), b = k3 / (H / p);
     const P* src = reinterpret_cast<const P*>(px + (((size_t)b * C + c) * H + gy * p + ky) * W + gx * p);

@@ -325,3 +325,15 @@ def test_rows_behind_a_multiple_of_256(M, N, K, kind):
     for rows in (slice(0, 256), slice(256, M))[:1 if M == 256 else 2]:
         assert _rel(out[:M][rows], want[rows]) < tol
     assert bool((out[M] == 0).all())
+
+
+def test_im2col_rows_at_the_end_of_32_bits():
+    """The last patch rows below 2^31: one channel of 2 x 2 pixels is one patch of 2 rows, so the output equals the input."""
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 2 x 8.6 GB beside its comparison")
+    cabi, L, st = _cabi()
+    B = 2 ** 30 - 8                                              # 2^31 - 16 patch rows
+    x = torch.empty(4 * B, dtype=torch.int16, device="cuda").random_(0, 2 ** 15 - 1)
+    out = torch.zeros_like(x)
+    cabi.check(L.pg_im2col(out.data_ptr(), x.data_ptr(), B, 1, 2, 2, 2, 4, cabi.PG_BF16, st))
+    assert all(torch.equal(a, b) for a, b in zip(out.split(1 << 30), x.split(1 << 30)))
