@@ -99,10 +99,11 @@ int pg_im2col(void* out, const void* pixels, int B, int C, int H, int W, int p, 
  * stores fp32 (lm_head `.float()`, modeling_gemma.py:417-418).  impl: 0 = auto, 1 = SIMT
  * (any dtype), 2 = tcgen05/TMA (bf16/f16 only; picks the CTA-pair, single-CTA, skinny or split-K kernel by shape),
  * 3 = the CTA-pair swap-AB kernel for 129..512 rows (weights as the M operand, split-K through pg_set_workspace;
- * auto takes it for the projections where it measured faster).  W is a parameter: the 16-bit kernels for few rows or few
- * tiles request it before the preceding launches of this library have finished, so W must not be an output of one that is
- * still in flight (what other work on the stream wrote is seen).  Replaces every nn.Linear / matmul call site
- * of SURVEY.md §2.3 on the prefill and vision paths. */
+ * auto takes it for the projections where it measured faster).  impl | PG_GEMM_W_PARAM: W is a parameter, written long before
+ * this call; the 16-bit kernels for few rows or few tiles then request it before the preceding launches of this library have
+ * finished.  Without the flag W may be an output of any of them, as A, bias and R may.  Replaces every nn.Linear / matmul
+ * call site on the prefill and vision paths. */
+#define PG_GEMM_W_PARAM 16
 int pg_gemm(void* C, const void* A, const void* W, const void* bias, const void* R,
             int M, int N, int K, int lda, int ldw, int ldc, int ldr, int res_mod,
             int epilogue, int out_f32, int impl, int dtype, void* stream);

@@ -270,19 +270,19 @@ bool gemm_tc_supported(int M, int N, int K, int lda, int ldw, int ldc, int epi, 
 
 bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod);
 int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, int N, int K, int lda, int ldw, int ldc,
-                 int ldr, int epi, int dtype, cudaStream_t st);
+                 int ldr, int epi, int dtype, bool w_param, cudaStream_t st);
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi);
 int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, cudaStream_t st);
+                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st);
 bool gemm_tc_2cta_wanted(int M, int N, int K, int epi);
 int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                  int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st);
 int gemm_tc_splitk_factor(int M, int N, int K, int epi);
 int gemm_tc_splitk(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int s, cudaStream_t st);
+                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int s, bool w_param, cudaStream_t st);
 
 int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-            int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st) {
+            int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st) {
   PG_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)C % 16) == 0,
              "gemm_tc: operands must be 16-byte aligned");
   PG_REQUIRE(!R || (((uintptr_t)R % 16) == 0 && ldr % 8 == 0), "gemm_tc: residual must be 16-byte aligned rows");
@@ -295,12 +295,12 @@ int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void*
     goto basic;
   }
   if (gemm_tc_swap_wanted(M, N, K, epi, out_f32, res_mod))  // a prompt's worth of rows: CTA pairs, weights as the M operand
-    return gemm_tc_swap(C, A, W, R, M, N, K, lda, ldw, ldc, ldr, epi, dtype, st);
+    return gemm_tc_swap(C, A, W, R, M, N, K, lda, ldw, ldc, ldr, epi, dtype, w_param, st);
   if (res_mod == 0 && gemm_tc_skinny_wanted(M, N, K, epi))  // a few dozen token rows: stream the weights (swap-AB)
-    return gemm_tc_skinny(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, epi, out_f32, dtype, st);
+    return gemm_tc_skinny(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, epi, out_f32, dtype, w_param, st);
   {
     const int s = gemm_tc_splitk_factor(M, N, K, epi);  // few tiles: a cluster shares each tile
-    if (s) return gemm_tc_splitk(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, s, st);
+    if (s) return gemm_tc_splitk(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, s, w_param, st);
   }
   if (!(dual && out_f32) && gemm_tc_2cta_wanted(M, N, K, epi))  // fewer staged bytes per wave: CTA pairs (cta_group::2)
     return gemm_tc_2cta(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, res_mod, epi, out_f32, dtype, st);

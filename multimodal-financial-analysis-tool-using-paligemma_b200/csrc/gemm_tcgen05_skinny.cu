@@ -26,6 +26,7 @@ struct SnParams {
   const void* bias;
   const void* R;
   int M, N, K, ldc, ldr, out_f32;
+  int w_param;   // W is no output of a preceding launch: it may be requested before the dependency wait
 };
 
 __device__ __forceinline__ void sn_cluster_sync() {
@@ -102,8 +103,9 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   if (warp == 0 && lane == 0) {
     // ===================== TMA producer: weight tile(s) + the token block =====================
     // flat item index i -> (tile, k block).  The first NSTAGES items' WEIGHT tiles are requested before
-    // griddepcontrol.wait: weights never depend on the preceding kernel, so ~150 KB per SM is already in flight
+    // griddepcontrol.wait: a parameter does not depend on the preceding kernel, so ~150 KB per SM is already in flight
     // when the predecessor's activations become visible; the token blocks follow the wait.
+    if (!p.w_param) pdl_wait();
     const int nk = kb1 - kb0;
     const int my_tiles = tile_first < n_tiles ? (n_tiles - tile_first + tile_stride - 1) / tile_stride : 0;
     const int items = my_tiles * nk;
@@ -319,7 +321,7 @@ bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
 }
 
 int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, cudaStream_t st) {
+                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st) {
   const bool bf = dtype == PG_BF16;
   const int nt = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   const int n_tiles = cdiv(N, tc::SN_BM), kb = cdiv(K, tc::SN_BK);
@@ -331,7 +333,7 @@ int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, cons
   const int w_rows = (epi == PG_EPI_GEGLU) ? 2 * N : N;
   PG_REQUIRE(tc::make_map_2d(&mx, A, M, K, lda, nt, bf) && tc::make_map_2d(&mw, W, w_rows, K, ldw, tc::SN_BM, bf),
              "gemm_tc_skinny: cuTensorMapEncodeTiled failed");
-  tc::SnParams p = {C, bias, R, M, N, K, ldc, ldr, out_f32};
+  tc::SnParams p = {C, bias, R, M, N, K, ldc, ldr, out_f32, w_param};
 #define PG_SN(E) return bf ? tc::launch_sn_nt<bf16, E>(mx, mw, p, nt, s, st) : tc::launch_sn_nt<f16, E>(mx, mw, p, nt, s, st)
   switch (epi) {
     case PG_EPI_NONE: PG_SN(PG_EPI_NONE);

@@ -18,6 +18,7 @@ struct SkParams {
   const void* bias;
   const void* R;
   int M, N, K, ldc, ldr, res_mod, out_f32;
+  int w_param;   // W is no output of a preceding launch: it may be requested before the dependency wait
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -74,7 +75,8 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0 && lane == 0) {
-    // the weights never depend on the preceding kernels: the ring's first weight tiles go out before the dependency wait
+    // a parameter does not depend on the preceding kernels: the ring's first weight tiles go out before the dependency wait
+    if (!p.w_param) pdl_wait();
     const int pre = min(SK_STAGES, max(0, kb1 - kb0));
     for (int i = 0; i < pre; ++i) {
       mbar_expect_tx(full_bar(i), STAGE_BYTES);
@@ -224,12 +226,12 @@ int gemm_tc_splitk_factor(int M, int N, int K, int epi) {
 }
 
 int gemm_tc_splitk(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int s, cudaStream_t st) {
+                   int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, int s, bool w_param, cudaStream_t st) {
   const bool bf = dtype == PG_BF16;
   CUtensorMap ma, mw;
   PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::SK_BM, bf) && tc::make_map_2d(&mw, W, N, K, ldw, 64, bf),
              "gemm_tc_splitk: cuTensorMapEncodeTiled failed");
-  tc::SkParams p = {C, bias, R, M, N, K, ldc, ldr, res_mod, out_f32};
+  tc::SkParams p = {C, bias, R, M, N, K, ldc, ldr, res_mod, out_f32, w_param};
 #define PG_SK(E) return bf ? tc::launch_sk_pick<bf16, E>(ma, mw, p, s, st) : tc::launch_sk_pick<f16, E>(ma, mw, p, s, st)
   switch (epi) {
     case PG_EPI_NONE: PG_SK(PG_EPI_NONE);

@@ -30,6 +30,7 @@ struct ParamsSw {
   int M, N, K;         // tokens, output features, reduction length
   int NT, n_t;         // token tile width (multiple of 16, <= 256) and number of tiles (1 or 2)
   int splits, kb_per_split, stages;
+  int w_param;         // W is no output of a preceding launch: it may be requested before the dependency wait
   int dbg;             // PG_SWAP_DBG bit 0: skip the partial stores (timing experiments only)
 };
 
@@ -117,6 +118,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool waited = false;
+      if (!p.w_param) { pdl_wait(); waited = true; }
       for (int item = first; item < items; item += stride) {
         const int ft = item / p.splits, sp = item % p.splits;
         const int kb0 = sp * p.kb_per_split, kb1 = min(k_blocks, kb0 + p.kb_per_split);
@@ -129,7 +131,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           const uint32_t sa = smem_base + stage * stage_bytes;
           const uint32_t full_leader = sw_mapa(full_bar(stage), 0);
           if (leader) mbar_expect_tx(full_bar(stage), 2 * stage_bytes);  // both CTAs' bytes
-          // the weights never depend on the preceding kernels: their loads go out before the dependency wait
+          // a parameter does not depend on the preceding kernels: its first load goes out before the dependency wait
           sw_tma_cg2(sa, &map_w, full_leader, kb * SW_BK, ft * 2 * SW_WROWS + (int)crank * SW_WROWS);
           if (!waited) { pdl_wait(); waited = true; }   // the token rows come from the predecessor
           for (int t = 0; t < p.n_t; ++t)
@@ -307,12 +309,13 @@ bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod)
 }
 
 int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, int N, int K, int lda, int ldw, int ldc,
-                 int ldr, int epi, int dtype, cudaStream_t st) {
+                 int ldr, int epi, int dtype, bool w_param, cudaStream_t st) {
   const bool bf = dtype == PG_BF16;
   const int n_w = epi == PG_EPI_GEGLU ? 2 * N : N;
   tc::ParamsSw p;
   swap_plan(M, n_w, K, &p);
   p.P = reinterpret_cast<float*>(g_ws_ptr);
+  p.w_param = w_param;
   CUtensorMap mw, mx;
   PG_REQUIRE(tc::make_map_2d(&mw, W, n_w, K, ldw, tc::SW_WROWS, bf) && tc::make_map_2d(&mx, A, M, K, lda, p.NT / 2, bf),
              "gemm_swap: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, n_w, K, lda, ldw);

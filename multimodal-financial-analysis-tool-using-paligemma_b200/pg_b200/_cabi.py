@@ -14,6 +14,7 @@ LIB_PATH = os.environ.get("PG_LIB_PATH") or os.path.join(_HERE, "libpg_b200.so")
 
 PG_F32, PG_BF16, PG_F16 = 0, 1, 2
 EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RES, EPI_RES, EPI_GEGLU, EPI_SWIGLU = 0, 1, 2, 3, 4, 5, 6
+GEMM_W_PARAM = 16               # pg_gemm(impl | ...): W is no output of a launch that may still run
 GLU_NONE, GLU_SILU, GLU_CLAMPED, ACT_RELU2 = 0, 1, 2, 3      # pairings / activation of pg_moe_gemm_act
 EMB_NONE, EMB_INIT, EMB_ADD = 0, 1, 2          # what pg_residual_layernorm does with the embedding row
 MAX_DECODE_BATCH = 8            # rows one launch of the GEMV kernels can take

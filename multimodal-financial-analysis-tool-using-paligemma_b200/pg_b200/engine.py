@@ -324,7 +324,7 @@ class PaliGemmaEngine(PagePool):
         ldc = out.stride(0) if ldc is None else ldc
         cabi.check(cabi.lib().pg_gemm(ptr(out), ptr(a), ptr(w), ptr(bias), ptr(res), M, N, K, lda,
                                       w.stride(0), ldc, 0 if res is None else res.stride(0), res_mod, epi,
-                                      1 if out_f32 else 0, self.gemm_impl, self.dt, cabi.stream()), "gemm")
+                                      1 if out_f32 else 0, self.gemm_impl | cabi.GEMM_W_PARAM, self.dt, cabi.stream()), "gemm")
         return out
 
     def _new(self, *shape, dtype=None):

@@ -213,7 +213,7 @@ class RaggedEngine(PagePool):
                 cabi.check(pair(ptr(out), ptr(gu), M, N, self.dt, st), "gated pairing")
                 return out
         cabi.check(L.pg_gemm(ptr(out), ptr(a), ptr(w), None, None, M, N, K, a.stride(0), w.stride(0), out.stride(0), 0, 0,
-                             epi, 1 if out_f32 else 0, self.gemm_impl, self.dt, st), "gemm")
+                             epi, 1 if out_f32 else 0, self.gemm_impl | cabi.GEMM_W_PARAM, self.dt, st), "gemm")
         return out
 
     def _moe_experts(self, h: torch.Tensor, idx: torch.Tensor, n_experts: int, top: int, ff: int, w_gu: torch.Tensor,

@@ -337,3 +337,23 @@ def test_im2col_rows_at_the_end_of_32_bits():
     out = torch.zeros_like(x)
     cabi.check(L.pg_im2col(out.data_ptr(), x.data_ptr(), B, 1, 2, 2, 2, 4, cabi.PG_BF16, st))
     assert all(torch.equal(a, b) for a, b in zip(out.split(1 << 30), x.split(1 << 30)))
+
+
+@pytest.mark.parametrize("M", [8, 40, 100, 260])
+@pytest.mark.parametrize("N,K,epi", [(2048, 2048, "none"), (1152, 4304, "res"), (1024, 1024, "bias")])
+def test_weights_written_by_the_launch_before(M, N, K, epi):
+    """W = U V^T comes from a pg_gemm right in front of the one that multiplies with it, over the rest of another W."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    u, v, a, r, b = _randn(g, N, 512, std=512 ** -0.5), _randn(g, K, 512), _randn(g, M, K, std=K ** -0.5), _randn(g, M, N), _randn(g, N)
+    w, out = torch.empty(N, K, dtype=BF, device="cuda"), torch.empty(M, N, dtype=BF, device="cuda")
+    code = {"res": cabi.EPI_RES, "bias": cabi.EPI_BIAS, "none": cabi.EPI_NONE}[epi]
+    z = a.to(F64) @ (u.to(F64) @ v.to(F64).T).to(BF).to(F64).T
+    want = z + (r.to(F64) if epi == "res" else b.to(F64) if epi == "bias" else 0.0)
+    for _ in range(20):
+        w.fill_(1e4)
+        cabi.check(L.pg_gemm(w.data_ptr(), u.data_ptr(), v.data_ptr(), None, None, N, K, 512, 512, 512, K, 0, 0, 0, 0, 0, cabi.PG_BF16, st))
+        cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr(), M, N, K, K, K, N, N, 0, code, 0, 0,
+                             cabi.PG_BF16, st))
+        # W's elements round either way at their ties with the exact product (2^-9 of a few), the result is rounded once or twice
+        assert _rel(out, want) < 6e-3
