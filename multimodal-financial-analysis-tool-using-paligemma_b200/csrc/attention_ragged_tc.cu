@@ -260,7 +260,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       }
       if (sig) {
 #pragma unroll
-        for (int jj = 0; jj < HK; ++jj) s[jj] = __fdividef(1.f, 1.f + exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
+        for (int jj = 0; jj < HK; ++jj) s[jj] = 1.f / (1.f + exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
       } else {
         const float ref = m == -INFINITY ? 0.f : m;                // a row that has seen no key yet
         f32x2 sum[2] = {pair_of(0.f, 0.f), pair_of(0.f, 0.f)};
@@ -304,7 +304,7 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
             float v = o[q0 + jj];
-            if (grow) v *= __fdividef(1.f, 1.f + __expf(-gt[jj]));
+            if (grow) v *= 1.f / (1.f + __expf(-gt[jj]));
             w[jj] = v;
           }
           *reinterpret_cast<uint4*>(orow + c * 32 + q0) = pack<T>(w);

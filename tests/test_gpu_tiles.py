@@ -357,3 +357,25 @@ def test_weights_written_by_the_launch_before(M, N, K, epi):
                              cabi.PG_BF16, st))
         # W's elements round either way at their ties with the exact product (2^-9 of a few), the result is rounded once or twice
         assert _rel(out, want) < 6e-3
+
+
+@pytest.mark.parametrize("sigmoid", [0, 1])
+def test_window_gates_and_weights_near_the_smallest_number(sigmoid):
+    """sigmoid(-87.5) is 1e-38: times values of 1e38 that is an ordinary number, for the gate and for a sigmoid weight."""
+    cabi, L, st = _cabi()
+    n, H, d, at = 70, 2, 64, -87.5
+    new = lambda f, *s: torch.full(s, f, dtype=BF, device="cuda")  # noqa: E731
+    q, kp, vp, gate = new(0.0, n, H * d), new(0.0, 2, 64, H * d), new(1e38, 2, 64, H * d), new(at, n, H * d)
+    pt = torch.tensor([[1, 0]], dtype=torch.int32, device="cuda")
+    tiles = torch.tensor([[0, n, 0, 0]], dtype=torch.int32, device="cuda")
+    bias, err = torch.full((H,), at, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(n, H * d, dtype=BF, device="cuda")
+    cabi.check(L.pg_attention_ragged_tc_ex(out.data_ptr(), H * d, q.data_ptr(), H * d, None if sigmoid else gate.data_ptr(), H * d, 0,
+                                           kp.data_ptr(), vp.data_ptr(), 128, pt.data_ptr(), 2, 64, tiles.data_ptr(), 1, n, H, H, d, d,
+                                           1.0, 1, 0, None, sigmoid, bias.data_ptr() if sigmoid else None, 1.0, err.data_ptr(),
+                                           cabi.PG_BF16, st))
+    want = float(vp[0, 0, 0]) * math.exp(at)
+    assert int(err) == 0
+    # exp(87.5) as 2^x: the exponent's rounding, 2^-18 of 126, is 3e-4 of the result; a weight of 1e-38 keeps 8 bits or, if the
+    # type's subnormal numbers are meant, 7; one rounding of the result
+    assert float((out.to(F64) - want).abs().max()) < 1.2e-2 * want
