@@ -425,7 +425,7 @@ class PaliGemmaForConditionalGeneration(nn.Module):
     def _decode_one(self, eng: PaliGemmaEngine, paged: PagedKV, input_ids, position: int,
                     mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         """One cached step through the graph-captured decode kernels (vision tower skipped: a
-        single new token has no image slot to fill, SURVEY.md Q5).  `mask` (already known to be a
+        single new token has no image slot to fill).  `mask` (already known to be a
         contiguous CUDA tensor of a supported dtype) is checked for padding by the same launch
         that stages ids / positions; a violation raises AssertionError at the next forward()."""
         ds = eng.decode_state(paged.batch)

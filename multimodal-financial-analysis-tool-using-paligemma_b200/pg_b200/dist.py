@@ -1,4 +1,4 @@
-"""Tensor-parallel plumbing for the Gemma decoder (SURVEY.md §8e; the reference itself is single-device).
+"""Tensor-parallel plumbing for the Gemma decoder (the reference itself is single-device).
 
 Sharding (tp = world size, one process per GPU):
   q_proj rows by query head, o_proj columns by query head   -> sum over ranks of (B*q, D) after o_proj

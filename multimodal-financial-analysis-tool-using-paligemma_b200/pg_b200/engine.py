@@ -5,10 +5,10 @@ PyTorch is used for device memory, streams and CUDA-graph capture only; every FL
 hot path runs in libpg_b200.so through the C ABI of include/pg_b200.h.  There is no CPU or
 PyTorch-op fallback: a missing library or a non-CUDA tensor raises.
 
-Reference semantics reproduced (SURVEY.md Appendix A): attention is never masked (Q1);
-prefill positions 0..N-1 (Q2); cached steps use position = attention-mask length, i.e.
-N+t, skipping N (Q3); a q_len>1 forward on a non-empty cache gives every new token that
-same position (Q6, patched merge); pad ids embed to zero rows (Q8); the sqrt(D)
+Reference semantics reproduced: attention is never masked;
+prefill positions 0..N-1; cached steps use position = attention-mask length, i.e.
+N+t, skipping N; a q_len>1 forward on a non-empty cache gives every new token that
+same position (patched merge); pad ids embed to zero rows; the sqrt(D)
 normaliser is rounded to the model dtype while image features are divided by the exact
 float (Q9); RoPE inv_freq is rounded to the model dtype by `model.to(dtype)`.
 """
@@ -304,7 +304,7 @@ class PaliGemmaEngine(PagePool):
         self.img_div = float(torch.tensor(d.hidden_size ** 0.5, dtype=torch.float32))
 
     def weight_bytes_per_decode_step(self) -> int:
-        """Algorithmic HBM bytes one decode step must read from the weights (SURVEY.md §8d)."""
+        """Algorithmic HBM bytes one decode step must read from the weights."""
         d, e = self.dims, torch.tensor([], dtype=self.dtype).element_size()
         per_layer = ((self.nq_l + 2 * d.nkv) * d.hd * d.D + d.D * self.nq_l * d.hd + 3 * self.F_l * d.D + 2 * d.D)
         return e * (d.L * per_layer + self.V_l * d.D + d.D)
@@ -547,7 +547,7 @@ class PaliGemmaEngine(PagePool):
                 kv.release()
 
     def encode_images_dp(self, pixels: torch.Tensor) -> torch.Tensor:
-        """Batch-level data parallelism for the vision tower (SURVEY.md §8e): every rank encodes its contiguous share
+        """Batch-level data parallelism for the vision tower: every rank encodes its contiguous share
         of the images (SigLIP + projector, modeling_gemma.py:568-571) and the (B, P, D) features are all-gathered
         over NCCL, 1 MB per image in bf16.  Fewer images than ranks: every rank encodes them all (replicated)."""
         tp = self.tp
@@ -861,7 +861,7 @@ class DecodeState:
                 yield ("all_reduce", x)
 
     def _step_batched_gen(self, kv: PagedKV, sample: Optional[tuple], advance: bool):
-        """Decode step for batches above the GEMV tile (batch 32): the projections run as
+        """Decode step for batches above the GEMV tile (32 sequences, for one): the projections run as
         skinny GEMMs (tcgen05 for 16-bit dtypes: weights stream through TMA once for the whole batch), attention
         stays the cluster kernel.  Same rounding points as the GEMV path; capturable (static buffers).
         Tensor parallel: the o_proj / down_proj GEMMs leave fp32 partials in local memory, pg_tp_push hands them to

@@ -1,4 +1,4 @@
-"""Continuous batching around the decode graph (SURVEY.md §8f item 1).
+"""Continuous batching around the decode graph.
 
 The reference serves one request at a time (`inference.py:34-85`: batch 1, one image, the processor asserts a
 single prompt, `processing_paligemma.py:80`).  Here requests of different prompt lengths share ONE captured decode

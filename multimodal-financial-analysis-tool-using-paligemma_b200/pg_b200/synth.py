@@ -2,12 +2,12 @@
 
 Every tensor is drawn from its own seeded CPU generator keyed by the HF
 state-dict name, so any subset of the checkpoint can be produced on any box
-and is bit-identical between this container, the GPU box, the oracle and the
+and is bit-identical on every machine, in the oracle and in the
 golden-vector script.  Key names follow the reference's `state_dict()`
-(SURVEY.md §2.3 census; reference `modeling_gemma.py:429-456`,
+(reference `modeling_gemma.py:429-456`,
 `modeling_siglip.py:36-255`).
 
-Distribution (SURVEY.md §8d): Linear/Conv weight ~ N(0, 0.05), bias ~ N(0, 0.02);
+Distribution: Linear/Conv weight ~ N(0, 0.05), bias ~ N(0, 0.02);
 token embedding ~ N(0, 0.05); position embedding ~ N(0, 0.02); LayerNorm
 w = 1 + N(0, 0.1), b ~ N(0, 0.02); RMSNorm w ~ N(0, 0.1).  The default torch init
 makes the tied lm_head echo its input token, which would make greedy-token

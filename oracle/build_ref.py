@@ -1,16 +1,16 @@
 #!/usr/bin/env python
 """Recipe for `oracle/_ref/`: the reference's own Python files for the hot path, taken UNMODIFIED from
-/root/reference (read-only, present in the build container only).  TEST INFRASTRUCTURE ONLY.
+its own tree (read-only, not present everywhere).  TEST INFRASTRUCTURE ONLY.
 
 The reference is pure Python, so there is nothing to compile: "building" it means staging the five files the path
-consists of where the GPU box can import them (`oracle/_ref/` is git-ignored -- no reference source enters the
-history -- but travels with the gpurun snapshot, like the built .so):
+consists of where the tests can import them (`oracle/_ref/` is git-ignored -- no reference source enters the
+history -- but travels with the working tree, like the built .so):
 
   modeling_gemma.py, modeling_siglip.py      the model the CPU baseline / `bench.py --impl reference` times
   processing_paligemma.py                    its processor
   ablation_study_fixed.py, inference.py      the two drivers tests/test_gpu_reference_drivers.py runs against the drop-ins
 
-    python oracle/build_ref.py        (also run by __graft_entry__.build() when /root/reference exists)
+    python oracle/build_ref.py        (also run by __graft_entry__.build() when the reference is there)
 """
 import hashlib
 import os

@@ -1,10 +1,10 @@
-"""Generate tests/golden/*.npz by running the UNMODIFIED reference (imported from
-/root/reference) on the seeded synthetic weights/inputs of pg_b200.synth.
+"""Generate tests/golden/*.npz by running the UNMODIFIED reference (imported
+from its own tree) on the seeded synthetic weights/inputs of pg_b200.synth.
 
-TEST INFRASTRUCTURE ONLY.  Run in the build container (the GPU box has no
-/root/reference):   python oracle/make_golden.py [tiny] [small] [full] [full_bf16]
+TEST INFRASTRUCTURE ONLY.  Run where the reference is
+(PG_REFERENCE, or its usual place):   python oracle/make_golden.py [tiny] [small] [full] [full_bf16]
 
-The reference ships no golden vectors (SURVEY.md §4); these are the vectors the
+The reference ships no golden vectors; these are the vectors the
 oracle restatement and the CUDA path are pinned to.
 """
 from __future__ import annotations
@@ -283,7 +283,7 @@ def golden_full_decode_bf16(steps: int = 16, probe_step: int = 4, probe_layers=(
 
 @torch.no_grad()
 def golden_vision_batch_bf16(batch: int = 64):
-    """BASELINE configs[2]: SigLIP tower + projector over a batch of 64 synthetic images in bf16 through the
+    """SigLIP tower + projector over a batch of 64 synthetic images in bf16 through the
     reference modules; a strided subsample of every image's projected features (and the fp32 reference run of the
     first 4 images as the truth for the noise yardstick)."""
     cfg = synth.CONFIGS["paligemma-3b-pt-224"]

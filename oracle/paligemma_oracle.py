@@ -11,9 +11,9 @@ rounding points are the reference's: fp32 islands inside RMSNorm and the two
 softmaxes, RoPE cos/sin rounded to the model dtype before the multiply, fp32
 logits on return.
 
-Pinning: the reference has no tests and ships no golden vectors (SURVEY.md §4),
-so this oracle is pinned against outputs of the reference itself, run in the
-build container by `oracle/make_golden.py` (which imports /root/reference) on
+Pinning: the reference has no tests and ships no golden vectors,
+so this oracle is pinned against outputs of the reference itself, run
+by `oracle/make_golden.py` (which imports it from its own tree) on
 the same seeded synthetic weights; the vectors live in `tests/golden/` and
 `tests/test_oracle_golden.py` checks them without the reference present.
 """

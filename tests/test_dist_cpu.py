@@ -1,4 +1,4 @@
-"""CPU checks of the tensor-parallel host plumbing added in round 2 (no GPU, no torch.distributed):
+"""CPU checks of the tensor-parallel host plumbing (no GPU, no torch.distributed):
 the `pg_tp_exchange` ctypes mirror against the header, the exchange-buffer layout arithmetic, the lockstep driver that
 emulates N ranks in one process, TP.run driving a launch generator, the vision batch shares and the static page table
 of PagedKV."""

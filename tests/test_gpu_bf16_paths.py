@@ -4,8 +4,8 @@ oracle/make_golden.py from the unmodified reference) -- full PaliGemma-3B-pt-224
   * cached decode through the CUDA-graph step (what bench.py's `value` times), teacher-forced for 16 steps,
   * single decoder layers of the GEMV step and of the tensor-core (batched) step fed the REFERENCE's own layer inputs
     and K/V caches: elementwise rtol 2e-2 (no amplification through the stack to hide a kernel bug),
-  * SigLIP + projector at batch 64 (BASELINE configs[2]),
-and on the `small` shapes the batched decode step of configs[3] / configs[4] (batch 32 greedy, batch 8 top-p)
+  * SigLIP + projector at batch 64,
+and on the `small` shapes the batched decode step (batch 32 greedy, batch 8 top-p)
 against the CPU oracle."""
 import os
 
@@ -140,7 +140,7 @@ def test_full_size_bf16_single_layers_with_reference_inputs(full_bf16, golden_di
 
 # ------------------------------------------------------------------------------- vision tower, batch 64
 def test_vision_batch64_bf16_features(full_bf16, golden_dir):
-    """BASELINE configs[2]: SigLIP So400m/14 + projector over 64 synthetic images in bf16, against the reference modules
+    """SigLIP So400m/14 + projector over 64 synthetic images in bf16, against the reference modules
     run in bf16 (strided subsample of every image's features); fp32 reference of the first four images as truth."""
     model, cfg, eng = full_bf16
     g = golden(golden_dir, "vision_b64_bf16.npz")
@@ -168,7 +168,7 @@ def test_vision_batch64_bf16_features(full_bf16, golden_dir):
     assert d1 <= 2.5 * rms(ref_p[:4] - tr_p), d1
 
 
-# ------------------------------------------------------------------------------- batched decode step (configs[3], configs[4])
+# ------------------------------------------------------------------------------- batched decode step
 @pytest.mark.parametrize("batch", [8, 32])
 def test_batched_step_bf16_against_oracle(batch):
     """`_step_batched_gen` (skinny tcgen05 GEMMs) on the small shapes, teacher-forced with the oracle's bf16 greedy tokens
@@ -202,7 +202,7 @@ def test_batched_step_fp32_tokens_exact():
 
 
 def test_batched_top_p_draws_from_the_reference_nucleus():
-    """configs[4]'s sampling path on the batched step (batch 8, temperature 0.8, top_p 0.9): teacher-forced with the
+    """The sampling path on the batched step (batch 8, temperature 0.8, top_p 0.9): teacher-forced with the
     oracle's tokens, every token the engine draws lies in the nucleus the reference rule (inference.py:15-24) builds from
     the ORACLE's logits widened by the bf16 band, and logits match as in the greedy case."""
     dtype = torch.bfloat16

@@ -264,7 +264,7 @@ def test_reduced_precision_teacher_forced(name, dtype, golden_dir):
 # ------------------------------------------------------------------------------- full size
 @pytest.mark.slow
 def test_full_size_fp32_tokens_bit_exact(golden_dir):
-    """PaliGemma-3B-pt-224 shapes, fp32 verification mode, config 1 of BASELINE.json: 32 greedy
+    """PaliGemma-3B-pt-224 shapes, fp32 verification mode: 32 greedy
     tokens identical to the reference; logits within 1e-4."""
     g = golden(golden_dir, "full_fp32.npz")
     model, cfg = build_model("paligemma-3b-pt-224", torch.float32)
@@ -314,7 +314,7 @@ def test_tensor_parallel_two_gpus():
     import subprocess
     import sys
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-m", "torch.distributed.run", "--nnodes=1", "--nproc-per-node", "2",
                         "--master-addr", "127.0.0.1", "--master-port", "29611", os.path.join(root, "tests", "tp_check.py")],
@@ -324,7 +324,7 @@ def test_tensor_parallel_two_gpus():
 
 def test_decode_batch_larger_than_kernel_tile(golden_dir):
     """Batch 10 (> the 8-row decode tile: kernels are issued per sub-batch) against the CPU oracle, patched
-    batch semantics (SURVEY Q7), fp32."""
+    batch semantics, fp32."""
     model, cfg = build_model("tiny", torch.float32)
     sd = synth.synth_state_dict(cfg)
     ids = synth.synth_prompt_ids(cfg, batch=10, prefix_len=5)

@@ -1,8 +1,8 @@
 """Tensor-parallel decoder parity on ONE GPU: N rank engines share the device and are advanced one kernel at a time
 (dist.LockstepGroup), so the peer-memory exchange fused into the decode kernels (csrc/tp_exchange.cuh) runs exactly as
 it does across GPUs -- every rank's producer stores into every rank's buffer, every consumer sums what it finds -- and
-its results are checked against the reference's golden vectors and the CPU oracle.  The driver's 1-GPU test box
-therefore sees the tensor-parallel path too; tests/tp_check.py repeats the fp32 cases on real GPUs."""
+its results are checked against the reference's golden vectors and the CPU oracle.  A machine with one GPU
+therefore tests the tensor-parallel path too; tests/tp_check.py repeats the fp32 cases on real GPUs."""
 import os
 
 import numpy as np
@@ -34,7 +34,7 @@ def test_tp_fp32_tokens_match_the_reference(name, tp, golden_dir):
 
 
 def test_tp_fp32_batch3_patched_semantics(golden_dir):
-    """Batch 3 (patched batch>1 semantics, SURVEY Q7) through the exchange: words of three rows per slot."""
+    """Batch 3 (patched batch>1 semantics) through the exchange: words of three rows per slot."""
     g = np.load(os.path.join(golden_dir, "tiny_fp32.npz"))
     engines, cfg = build_engines("tiny", torch.float32, 2)
     ids = synth.synth_prompt_ids(cfg, batch=3, prefix_len=6)

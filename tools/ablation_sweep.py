@@ -5,7 +5,7 @@ and of the cache-off loop (SigLIP + projector + full-prefix recompute per token)
 (`:23,210`; the whole run for shorter sequences), peak decode-phase device memory (statistics reset after the prefill,
 `:202,255`).  Random-init weights of the exact PaliGemma-3B-pt-224 shapes, bf16, one synthetic image + 'caption en'.
 
-  python tools/ablation_sweep.py [--lengths 16,32,64,128,256] [--runs 2] [--out gpurun_out/ablation_n1.json]
+  python tools/ablation_sweep.py [--lengths 16,32,64,128,256] [--runs 2] [--out ablation_n1.json]
   torchrun --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 tools/ablation_sweep.py ...      (N = 2, 4, 8)
 
 N > 1: the cache-on loop runs ONE sequence on the tensor-parallel decoder (latency falls with N); the cache-off loop has
