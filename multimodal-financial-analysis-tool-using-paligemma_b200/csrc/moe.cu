@@ -297,14 +297,22 @@ moe_route_tile_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w
   }
 }
 
-// The tile kernel takes 16-byte loads of both operands and pays from the token count on at which its warps fill the chip;
-// below that a CTA per token, a warp per routed output, has the shorter chain (8 tokens in one go there).
+// The tile kernel takes 16-byte loads of both operands and pays where its warps fill the chip (16 tokens a CTA) or a CTA per token
+// reads the router often enough; its own time hardly depends on the tokens before the chip is full.  us, CTA per token against
+// tile: 512 tokens, 16 experts, width 2048 12 : 20 (128 experts 63 : 94), 1024 tokens 23 : 20 (124 : 93), 4 experts 9 : 12, 3072
+// tokens 54 : 34 (303 : 137).  `line`: experts x width from which 1024 tokens are enough.
 template <typename T>
-static bool route_tile_wanted(const void* h, int ldh, const void* w_router, const void* w_sg, int n_tokens, int D, size_t smem) {
+static bool route_tile_wanted(const void* h, int ldh, const void* w_router, const void* w_sg, int n_tokens, int D, int n_route, int line,
+                              size_t smem) {
   constexpr int V = Vec<T>::N;
-  return n_tokens >= 512 && D % V == 0 && ldh % V == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0 &&
+  return (n_tokens >= 3072 || (n_tokens >= 1024 && (long long)n_route * D >= line)) && D % V == 0 && ldh % V == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(w_router) & 15) == 0 && (reinterpret_cast<uintptr_t>(w_sg) & 15) == 0 && smem <= 96 * 1024;
 }
+
+// Warps of a CTA per token.  A warp per routed output is one short chain for a few tokens; from about two CTAs per SM on it leaves
+// fewer tokens side by side and the idle warps of the choice cost more (16 experts, width 2048: 256 tokens 7 us, 8 warps 12;
+// 32 experts: 13 and 19; 768 tokens 34 and 23).
+static int route_warps(int n_tokens, int outputs) { return max(4, min(n_tokens <= 256 ? 32 : 8, outputs)); }
 
 // ------------------------------------------------------------------ router whose weights are a softmax over the chosen logits
 // z = h W_router^T + bias in fp32; the `top` largest z are chosen (ties: lowest index) and weighted by the softmax over the
@@ -775,12 +783,12 @@ extern "C" int pg_moe_route(int32_t* topk_idx, float* topk_w, float* shared_gate
                             int D, int n_route, int top, float scale, int dtype, void* stream) {
   if (n_tokens <= 0) return PG_OK;
   PG_REQUIRE(top >= 1 && top <= n_route && n_route <= 4096, "moe_route: top %d of %d routed outputs", top, n_route);
-  const int warps = n_route + 1 < 4 ? 4 : (n_route + 1 < 32 ? n_route + 1 : 32);   // a warp per routed output: one short chain
+  const int warps = route_warps(n_tokens, n_route + 1);
   const size_t smem = sizeof(float) * ((size_t)D + 2 * (size_t)n_route);
   PG_REQUIRE(smem <= 200 * 1024, "moe_route: D=%d with %d routed outputs does not fit shared memory", D, n_route);
   PG_DISPATCH_DTYPE(dtype, T, {
     const size_t tile_smem = sizeof(float) * (size_t)RT_WARPS * RT_TOK * 2 * n_route;
-    if (route_tile_wanted<T>(h, ldh, w_router, w_shared_gate, n_tokens, D, tile_smem))
+    if (route_tile_wanted<T>(h, ldh, w_router, w_shared_gate, n_tokens, D, n_route, 32768, tile_smem))
       return launch_pdl("moe_route", moe_route_tile_kernel<T, false>, dim3(cdiv(n_tokens, RT_WARPS * RT_TOK)), dim3(RT_WARPS * 32),
                         tile_smem, (cudaStream_t)stream, topk_idx, topk_w, shared_gate, (const T*)h, ldh, (const T*)w_router,
                         (const T*)correction, (const T*)w_shared_gate, n_tokens, D, n_route, top, scale, 1, 1);
@@ -871,12 +879,12 @@ extern "C" int pg_moe_route_grouped(int32_t* topk_idx, float* topk_w, const void
   PG_REQUIRE(n_groups >= 1 && n_route % n_groups == 0 && keep >= 1 && keep <= n_groups &&
                  (long long)keep * (n_route / n_groups) >= top,
              "moe_route: %d groups over %d experts, %d kept, top %d", n_groups, n_route, keep, top);
-  const int warps = n_route < 4 ? 4 : (n_route < 32 ? n_route : 32);   // a warp per routed output: one short chain
+  const int warps = route_warps(n_tokens, n_route);
   const size_t smem = sizeof(float) * ((size_t)D + 2 * (size_t)n_route + n_groups);
   PG_REQUIRE(smem <= 200 * 1024, "moe_route: D=%d with %d routed outputs does not fit shared memory", D, n_route);
   PG_DISPATCH_DTYPE(dtype, T, {
     const size_t tile_smem = sizeof(float) * (size_t)RT_WARPS * RT_TOK * (2 * n_route + n_groups);
-    if (route_tile_wanted<T>(h, ldh, w_router, nullptr, n_tokens, D, tile_smem))
+    if (route_tile_wanted<T>(h, ldh, w_router, nullptr, n_tokens, D, n_route, 65536, tile_smem))
       return launch_pdl("moe_route_grouped", moe_route_tile_kernel<T, true>, dim3(cdiv(n_tokens, RT_WARPS * RT_TOK)),
                         dim3(RT_WARPS * 32), tile_smem, (cudaStream_t)stream, topk_idx, topk_w, (float*)nullptr, (const T*)h, ldh,
                         (const T*)w_router, (const T*)correction, (const T*)nullptr, n_tokens, D, n_route, top, 1.f, n_groups, keep);

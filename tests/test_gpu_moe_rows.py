@@ -29,7 +29,10 @@ def _check_choice(idx, got_w, choice, weights, top):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,D,E,top,sg", [(512, 264, 16, 2, True), (513, 1024, 5, 5, False), (515, 2048, 18, 2, True),
-                                          (700, 136, 33, 4, True), (511, 264, 40, 3, False)])
+                                          (700, 136, 33, 4, True), (511, 264, 40, 3, False),
+                                          # from 3072 tokens, or 1024 and 32768 experts x width, several tokens per warp
+                                          (3072, 264, 16, 2, True), (3073, 1024, 5, 5, False), (3075, 136, 33, 4, True), (1023, 2048, 18, 2, True),
+                                          (1026, 2048, 18, 2, True), (1024, 1024, 32, 4, False), (256, 264, 40, 3, True), (257, 264, 40, 3, True)])
 def test_softmax_router_tiles(dtype, T, D, E, top, sg):
     cabi, L, st = _setup()
     h, w = _randn(T, D + 8, seed=1, dtype=dtype), _randn(E, D, seed=2, dtype=dtype, std=D ** -0.5)
@@ -49,7 +52,8 @@ def test_softmax_router_tiles(dtype, T, D, E, top, sg):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("T,D,E,top,groups,keep", [(512, 264, 16, 2, 4, 2), (514, 1024, 8, 3, 1, 1), (601, 2048, 24, 4, 3, 2)])
+@pytest.mark.parametrize("T,D,E,top,groups,keep", [(512, 264, 16, 2, 4, 2), (514, 1024, 8, 3, 1, 1), (601, 2048, 24, 4, 3, 2),
+                                                    (3074, 264, 16, 2, 4, 2), (1025, 2048, 32, 4, 4, 2), (1024, 2048, 30, 3, 3, 2), (257, 264, 40, 4, 4, 3)])
 def test_grouped_router_tiles(dtype, T, D, E, top, groups, keep):
     cabi, L, st = _setup()
     h, w = _randn(T, D, seed=5, dtype=dtype), _randn(E, D, seed=6, dtype=dtype, std=D ** -0.5)
