@@ -1,4 +1,4 @@
-// Skinny GEMM for batched decode (4 <= M <= 128 token rows, BASELINE configs[3]): out[M,N] = X[M,K] W[N,K]^T.
+// Skinny GEMM for batched decode (4 <= M <= 128 token rows): out[M,N] = X[M,K] W[N,K]^T.
 // With so few rows the problem is a weight stream, so the operands are swapped: the WEIGHT tile is the 128-row
 // A operand of tcgen05.mma and the tokens are the N dimension (N_mma = M rounded up to 16).  A pipeline stage is
 // then 16 KB of weights + a few KB of activations, so 8-10 stages (~150 KB of weights) are in flight per SM —
@@ -311,13 +311,17 @@ static int launch_sn_nt(const CUtensorMap& mx, const CUtensorMap& mw, const SnPa
 }  // namespace tc
 
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
-  // Up to 64 rows the swap-AB stream takes every projection; above, where a stage is mostly tokens, the ones whose CTAs own
-  // whole weight tiles (batch 32: gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us, q/k/v 9.9 vs 18.3 us on the row-major kernel).
+  // Up to 32 rows the swap-AB stream takes every projection (gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us, q/k/v 9.9 vs 18.3
+  // us on the row-major kernel).  Up to 64 rows it does so for long K; with K 2048 its token-heavy stages and the merge of 64 columns
+  // cost more than the stream gains (64 rows, weights out of HBM: N 2560 13.8 us, the row-major kernel 11.9; N 2048 with a
+  // residual 11.5, the pair kernel 10.2; N 1152, K 4304 13.2, row-major 10.9).  Above, only where CTAs own whole weight tiles or
+  // there are 32 of them (128 rows: N = K = 4096 16.1 us, row-major 17.2; N 2560, K 2048 21.6 and 11.9).
   static const int mode = env_int("PG_SKINNY", 1);   // 0 off, 1 where it wins, 2 everywhere it applies
   if (!mode || M < 4 || M > 128 || N < 512 || K < 256 || epi < PG_EPI_NONE || epi > PG_EPI_GEGLU) return false;
   if (mode == 2) return true;
   const int n_tiles = cdiv(N, 128);
-  return epi == PG_EPI_GEGLU || epi == PG_EPI_NONE || n_tiles >= 100 || M <= 64;
+  if (epi == PG_EPI_GEGLU || n_tiles >= 100 || M <= 32) return true;
+  return M <= 64 ? K >= (epi == PG_EPI_NONE ? 4096 : 8192) : epi == PG_EPI_NONE && n_tiles >= 32 && K >= 4096;
 }
 
 int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
@@ -325,10 +329,11 @@ int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, cons
   const bool bf = dtype == PG_BF16;
   const int nt = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   const int n_tiles = cdiv(N, tc::SN_BM), kb = cdiv(K, tc::SN_BK);
-  // split K across a cluster until ~148 CTAs stream (each keeps >= 4 K blocks)
+  // split K across a cluster until ~148 CTAs stream (each keeps >= 4 K blocks).  A CTA of a cluster of 4 takes an SM's whole
+  // shared memory, and no more than 32 such clusters find room at once (N 4304, K 1152, 8 rows: 34 clusters 11.3 us, pairs 7.7)
   int s = 1;
   if (epi != PG_EPI_GEGLU)
-    while (s < 8 && n_tiles * s * 2 <= 160 && kb / (s * 2) >= 4) s *= 2;
+    while (s < 8 && n_tiles * s * 2 <= (s == 2 ? 128 : 160) && kb / (s * 2) >= 4) s *= 2;
   CUtensorMap mx, mw;
   const int w_rows = (epi == PG_EPI_GEGLU) ? 2 * N : N;
   PG_REQUIRE(tc::make_map_2d(&mx, A, M, K, lda, nt, bf) && tc::make_map_2d(&mw, W, w_rows, K, ldw, tc::SN_BM, bf),

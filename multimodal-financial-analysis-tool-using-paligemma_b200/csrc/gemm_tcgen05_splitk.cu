@@ -214,14 +214,17 @@ static int launch_sk_pick(const CUtensorMap& ma, const CUtensorMap& mw, const Sk
 
 // Split factor for a problem (0 = do not split): up to three m-tiles whose 64-wide tiles leave room for the split within one
 // wave of two CTAs per SM, and at least 8 K blocks per CTA.  One image's encode (256 rows: every GEMM
-// of its layers; unsplit but for fc2 before) 625 -> 577 us, a 260-token prompt with its image 5021 -> 4915 us.  Gated pairings
-// stay out: two accumulators a tile already fill the wave.
+// of its layers; unsplit but for fc2 before) 625 -> 577 us, a 260-token prompt with its image 5021 -> 4915 us.  By 4 with fewer
+// than 16 K blocks a CTA, the second CTA of an SM costs more than the halved chain gains (256 rows, N = K = 2048, weights out of
+// HBM: 12.6 us, by 2 11.4).  By 2 it pays in a chain, for the weights that are on their way early, although a row of equal
+// products is no faster (N 3456, K 1152 by 2 10.0 us, whole 9.6; but one image's encode 544 and 558 us).  Gated pairings stay
+// out: two accumulators a tile already fill the wave.
 int gemm_tc_splitk_factor(int M, int N, int K, int epi) {
   static const int mode = env_int("PG_SPLITK", -1);   // 0 never, 2 / 4: that factor wherever it fits
   if (mode == 0 || epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU || M > 3 * tc::SK_BM) return 0;
   const int kb = cdiv(K, tc::SK_BK), tiles = cdiv(M, tc::SK_BM) * cdiv(N, 64);
   for (int s = mode > 1 ? mode : 4; s >= 2; s /= 2)
-    if (kb / s >= 8 && tiles * s <= 288) return s;
+    if (kb / s >= 8 && tiles * s <= (s >= 4 && kb / s < 16 ? 192 : 288)) return s;
   return 0;
 }
 

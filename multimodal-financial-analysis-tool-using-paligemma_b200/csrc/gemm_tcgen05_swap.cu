@@ -290,13 +290,13 @@ bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod)
   static const int min_m = env_int("PG_GEMM_SWAP_MIN_M", 4);
   if ((!enabled && !g_force_swap) || out_f32 || res_mod != 0 || M < min_m || M > 512) return false;
   if (epi != PG_EPI_NONE && epi != PG_EPI_RES && epi != PG_EPI_GEGLU) return false;
-  // which projections take this kernel (measured per projection, profiles/README.md): bit 0 q/k/v (no epilogue),
+  // which projections take this kernel (measured per projection): bit 0 q/k/v (no epilogue),
   // bit 1 o_proj (residual, K < 8192), bit 2 down_proj (residual, K >= 8192), bit 3 gate/up (GeGLU)
   // measured: prompt-sized rows (129..512) -- down_proj only (prefill 4.16 -> 3.45 ms; q/k/v, o_proj and gate/up are
-  // faster on the row-major kernels); batched-decode rows (65..128) -- o_proj and down_proj (up to 64 rows the cluster
-  // split of gemm_tcgen05_skinny.cu needs no workspace round trip)
+  // faster on the row-major kernels); batched-decode rows (33..128) -- o_proj and down_proj (up to 32 rows, and up to 64 with
+  // a long K, the cluster split of gemm_tcgen05_skinny.cu is faster: it needs no workspace round trip)
   static const int mask_large = env_int("PG_SWAP_MASK", 4), mask_small = env_int("PG_SWAP_MASK_SMALL", 6);
-  if (M <= 64 && !g_force_swap) return false;
+  if ((M <= 32 || (M <= 64 && K >= 8192)) && !g_force_swap) return false;
   const int mask = M > 128 ? mask_large : mask_small;
   const int kind = epi == PG_EPI_NONE ? 1 : (epi == PG_EPI_GEGLU ? 8 : (K >= 8192 ? 4 : 2));
   if (!(mask & kind) && !g_force_swap) return false;
