@@ -31,7 +31,6 @@ struct ParamsSw {
   int NT, n_t;         // token tile width (multiple of 16, <= 256) and number of tiles (1 or 2)
   int splits, kb_per_split, stages;
   int w_param;         // W is no output of a preceding launch: it may be requested before the dependency wait
-  int dbg;             // PG_SWAP_DBG bit 0: skip the partial stores (timing experiments only)
 };
 
 __device__ __forceinline__ uint32_t sw_mapa(uint32_t addr, uint32_t rank) {
@@ -124,7 +123,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const int kb0 = sp * p.kb_per_split, kb1 = min(k_blocks, kb0 + p.kb_per_split);
         // every pair walks its k-blocks from a different starting point: at any moment the pairs read different
         // token slices, so the few hundred L2 lines of one slice are not requested by all 148 SMs at once
-        const int nkb = kb1 - kb0, rot = (p.dbg & 2) ? 0 : (first * 5) % nkb;
+        const int nkb = kb1 - kb0, rot = (first * 5) % nkb;
         for (int i = 0; i < nkb; ++i) {
           const int kb = kb0 + (i + rot) % nkb;
           mbar_wait(empty_bar(stage), phase ^ 1);
@@ -185,7 +184,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         float v[16];
         tmem_ld16(t_lane + t * 256 + cc * 16, v);
         tmem_ld_wait();
-        if (f < p.N && !(p.dbg & 1)) {
+        if (f < p.N) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int tok = t * p.NT + cc * 16 + j;
@@ -280,8 +279,7 @@ static void swap_plan(int M, int N, int K, tc::ParamsSw* p) {
   const int stage_bytes = tc::SW_W_BYTES + p->n_t * (p->NT / 2) * tc::SW_BK * 2;
   int stages = (tc::SW_SMEM_BUDGET - 1024 - 256) / stage_bytes;
   p->stages = stages > 8 ? 8 : stages;
-  static const int dbg = env_int("PG_SWAP_DBG", 0), max_stages = env_int("PG_SWAP_STAGES", 8);
-  p->dbg = dbg;
+  static const int max_stages = env_int("PG_SWAP_STAGES", 8);
   if (p->stages > max_stages) p->stages = max_stages;
 }
 
