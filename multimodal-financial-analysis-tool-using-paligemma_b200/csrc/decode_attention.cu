@@ -576,13 +576,15 @@ template <typename T>
 static int launch_dm_ns(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
                         int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
                         cudaStream_t st) {
-  // as many CTAs per (sequence, kv head) as keep the launch within one wave of two per SM (16 is a non-portable size)
+  // As many CTAs per (sequence, kv head) as keep the launch within one wave of two per SM (16 is a non-portable size), as far as
+  // the GPCs have room for whole clusters: 14 of 16, 33 of 8, 70 of 4.  One cluster more takes a second wave
+  // (262 cached tokens: 14 sequences 8.9 us, 15 with clusters of 16 14.3).
   const int seqs = B * nkv;
 #define PG_DM(N_) \
   return launch_dm<T, N_>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st)
-  if (seqs <= 18) PG_DM(16);
-  if (seqs <= 37) PG_DM(8);
-  if (seqs <= 74) PG_DM(4);
+  if (seqs <= 14) PG_DM(16);
+  if (seqs <= 33) PG_DM(8);
+  if (seqs <= 70) PG_DM(4);
   if (seqs <= 148) PG_DM(2);
   PG_DM(1);
 #undef PG_DM
