@@ -374,7 +374,8 @@ static int launch_da(void* out, const void* q, const void* k_pool, const void* v
 // A warp takes 16 tokens at a time and all operands go from global memory straight into fragments with 16-byte loads: the
 // contraction index of S^T is permuted (lane j of a quad owns 8 consecutive columns of every 32) and so are the rows of O^T
 // (lane group r owns 8 consecutive columns of every 64), which neither product notices.  The weights stay fp32: they enter
-// as three 16-bit terms (mma_frag.cuh), so that P V is the fp32 product; only QK^T's operands are 16-bit, as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
+// as three 16-bit terms (mma_frag.cuh; all their 24 bits in bf16, 2^-39 of the largest weight in fp16); only QK^T's operands are
+// 16-bit, as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
 // Measured (launch alone, cold cache): 1 sequence x 262 tokens 13.5 -> 9.5 us, 8 x 1345 39.7 -> 14.2 us, 32 x 389 23.6 -> 12.1 us;
 // inside the captured step 4.0, 23 and 5.1 us per layer less.
 constexpr int DM_WARPS = 4, DM_HD = 256, DM_G = 8;
@@ -413,70 +414,72 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
 
   const int chunks = (T_len + 15) / 16;
   const size_t row_elems = (size_t)nkv * DM_HD;
-  for (bool in_fp32 = false;; in_fp32 = true) {
+  auto attend = [&](auto in_fp32) {                           // this warp's chunks
+    constexpr bool fp32 = decltype(in_fp32)::value;
 #pragma unroll
-  for (int vb = 0; vb < VB; ++vb)
+    for (int vb = 0; vb < VB; ++vb)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
-  m[0] = m[1] = -INFINITY;
-  l[0] = l[1] = 0.f;
-  // chunk c: CTA c % NS first, so that a short context spreads over the SMs before it stacks up in one
-  for (int c = rank + NS * wid; c < chunks; c += NS * DM_WARPS) {
-    const int t0 = c * 16, pi = t0 / page_size;               // page_size is a multiple of 16: one page per chunk
-    const int page = pi < pt_n ? s_pt[pi] : pt[pi];
-    const size_t base = ((size_t)page * page_size + t0 % page_size) * row_elems + (size_t)kvh * DM_HD;
-    const int last = T_len - 1 - t0;                          // rows behind the last token repeat it with weight 0
-    const T* kp = k_pool + base + j * 8;
-    const T* vp = v_pool + base + r * 8;
-    const size_t k0 = (size_t)min(r, last) * row_elems, k1 = (size_t)min(r + 8, last) * row_elems;
-    const size_t v0 = (size_t)min(2 * j, last) * row_elems, v1 = (size_t)min(2 * j + 1, last) * row_elems;
-    const size_t v2 = (size_t)min(2 * j + 8, last) * row_elems, v3 = (size_t)min(2 * j + 9, last) * row_elems;
-    uint4 ka[KB], kc[KB], va[VB][4];
+        for (int e = 0; e < 4; ++e) acc[vb][i][e] = 0.f;
+    m[0] = m[1] = -INFINITY;
+    l[0] = l[1] = 0.f;
+    // chunk c: CTA c % NS first, so that a short context spreads over the SMs before it stacks up in one
+    for (int c = rank + NS * wid; c < chunks; c += NS * DM_WARPS) {
+      const int t0 = c * 16, pi = t0 / page_size;               // page_size is a multiple of 16: one page per chunk
+      const int page = pi < pt_n ? s_pt[pi] : pt[pi];
+      const size_t base = ((size_t)page * page_size + t0 % page_size) * row_elems + (size_t)kvh * DM_HD;
+      const int last = T_len - 1 - t0;                          // rows behind the last token repeat it with weight 0
+      const T* kp = k_pool + base + j * 8;
+      const T* vp = v_pool + base + r * 8;
+      const size_t k0 = (size_t)min(r, last) * row_elems, k1 = (size_t)min(r + 8, last) * row_elems;
+      const size_t v0 = (size_t)min(2 * j, last) * row_elems, v1 = (size_t)min(2 * j + 1, last) * row_elems;
+      const size_t v2 = (size_t)min(2 * j + 8, last) * row_elems, v3 = (size_t)min(2 * j + 9, last) * row_elems;
+      uint4 ka[KB], kc[KB], va[VB][4];
 #pragma unroll
-    for (int kb = 0; kb < KB; ++kb) { ka[kb] = ldg_cached(kp + k0 + kb * 32); kc[kb] = ldg_cached(kp + k1 + kb * 32); }
+      for (int kb = 0; kb < KB; ++kb) { ka[kb] = ldg_cached(kp + k0 + kb * 32); kc[kb] = ldg_cached(kp + k1 + kb * 32); }
 #pragma unroll
-    for (int vb = 0; vb < VB; ++vb) {
-      va[vb][0] = ldg_cached(vp + v0 + vb * 64); va[vb][1] = ldg_cached(vp + v1 + vb * 64);
-      va[vb][2] = ldg_cached(vp + v2 + vb * 64); va[vb][3] = ldg_cached(vp + v3 + vb * 64);
+      for (int vb = 0; vb < VB; ++vb) {
+        va[vb][0] = ldg_cached(vp + v0 + vb * 64); va[vb][1] = ldg_cached(vp + v1 + vb * 64);
+        va[vb][2] = ldg_cached(vp + v2 + vb * 64); va[vb][3] = ldg_cached(vp + v3 + vb * 64);
+      }
+      float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb) {
+        mma_16816<T>(s0, ka[kb].x, kc[kb].x, ka[kb].y, kc[kb].y, qf[kb].x, qf[kb].y);
+        mma_16816<T>(s1, ka[kb].z, kc[kb].z, ka[kb].w, kc[kb].w, qf[kb].z, qf[kb].w);
+      }
+      // s[0], s[1]: token r, heads 2j, 2j + 1;  s[2], s[3]: token r + 8
+      float p[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // matmul output rounded to the model dtype, then "/ sqrt(head_dim)" (modeling_gemma.py:266); a power-of-two divisor is
+        // applied as an exact multiply
+        const float sr = rnd<T>(s0[e] + s1[e]);
+        const float sc = (scale_mul != 0.f) ? sr * scale_mul : rnd<T>(sr / scale_div);
+        p[e] = (e < 2 ? r : r + 8) <= last ? sc : -INFINITY;
+      }
+      float corr[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float mx = fmaxf(p[h], p[h + 2]);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;   // -inf: no key so far has any weight
+        corr[h] = __expf(m[h] - ref);
+        m[h] = mn;
+        p[h] = __expf(p[h] - ref);
+        p[h + 2] = __expf(p[h + 2] - ref);
+        l[h] = l[h] * corr[h] + (p[h] + p[h + 2]);              // this lane's tokens; the lanes meet at the end
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[e] *= split_scale<T>();
+      if constexpr (!fp32) add_values<T, VB>(acc, va, p, corr);
+      else add_values_fp32<T, VB>(acc, [&](int k) { return vp + k * row_elems; }, p, corr, last + 1);
     }
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int kb = 0; kb < KB; ++kb) {
-      mma_16816<T>(s0, ka[kb].x, kc[kb].x, ka[kb].y, kc[kb].y, qf[kb].x, qf[kb].y);
-      mma_16816<T>(s1, ka[kb].z, kc[kb].z, ka[kb].w, kc[kb].w, qf[kb].z, qf[kb].w);
-    }
-    // s[0], s[1]: token r, heads 2j, 2j + 1;  s[2], s[3]: token r + 8
-    float p[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // matmul output rounded to the model dtype, then "/ sqrt(head_dim)" (modeling_gemma.py:266); a power-of-two divisor is
-      // applied as an exact multiply
-      const float sr = rnd<T>(s0[e] + s1[e]);
-      const float sc = (scale_mul != 0.f) ? sr * scale_mul : rnd<T>(sr / scale_div);
-      p[e] = (e < 2 ? r : r + 8) <= last ? sc : -INFINITY;
-    }
-    float corr[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float mx = fmaxf(p[h], p[h + 2]);
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;   // -inf: no key so far has any weight
-      corr[h] = __expf(m[h] - ref);
-      m[h] = mn;
-      p[h] = __expf(p[h] - ref);
-      p[h + 2] = __expf(p[h + 2] - ref);
-      l[h] = l[h] * corr[h] + (p[h] + p[h + 2]);              // this lane's tokens; the lanes meet at the end
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) p[e] *= split_scale<T>();
-    if (!in_fp32) add_values<T, VB>(acc, va, p, corr);
-    else add_values_fp32<T, VB>(acc, [&](int k) { return vp + k * row_elems; }, p, corr, last + 1);
-  }
-  if (in_fp32 || !any_nan(acc)) break;                        // an infinity among the values: once more
-  }
+  };
+  attend(std::false_type{});
+  if (any_nan(acc)) attend(std::true_type{});                 // an infinity among the values: once more
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
