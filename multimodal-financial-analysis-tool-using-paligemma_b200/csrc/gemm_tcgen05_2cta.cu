@@ -431,8 +431,8 @@ int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const 
   const bool bf = dtype == PG_BF16, dual = epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU;
   bool tail;
   g2_cost(M, N, epi, &tail);
-  CUtensorMap ma, mw, mt;
-  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && tc::make_map_2d(&mt, A, M, K, lda, tc::G2_TAIL / 2, bf) &&
+  CUtensorMap ma, mw, mt = {};   // mt: read by the tail kernels only
+  PG_REQUIRE(tc::make_map_2d(&ma, A, M, K, lda, tc::G2_BM, bf) && (!tail || tc::make_map_2d(&mt, A, M, K, lda, tc::G2_TAIL / 2, bf)) &&
                  tc::make_map_2d(&mw, W, dual ? 2 * N : N, K, ldw, tail ? (tc::G2_BN - tc::G2_TAIL) / 4 : tc::G2_BN / 2, bf),
              "gemm_tc2: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, N, K, lda, ldw);
   PG_REQUIRE(!dual || !out_f32, "gemm_tc2: a gated pairing has no fp32 output");
