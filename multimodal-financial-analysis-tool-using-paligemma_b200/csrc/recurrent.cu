@@ -269,15 +269,17 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //     S <- decay_h S + k v^T,        o = S^T q
 // lightning_prep_kernel  (elementwise)  the activations in fp32, one packed record [q | k | v] per (token, head) with
 //                                       q, k padded to dp = dim rounded up to 4 floats and v to vp likewise (zeros).
-// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): RG lanes share two value columns,
-//                                       a thread owns rows 4 (m RG + rg) + e of both.  What bounds it is issue slots: a
-//                                       token costs a multiply and two fused multiply-adds per state element, so they run
-//                                       on pairs of rows (fma.rn.f32x2: the same roundings, half the instructions), the
-//                                       q and k a thread reads serve two columns, and a batch of RG / 2 tokens shares
-//                                       its shuffles (a token at a time, each with log2(RG) shuffles behind it, left the
-//                                       warps waiting on one another's latencies: 787 us).  The records of the next CH tokens arrive by cp.async
-//                                       into the other half of a double buffer.  4 x 2048 tokens, 16 heads of 128: one
-//                                       column per thread and scalar arithmetic 842 us, this 638 us.
+// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): RG lanes share one or two value
+//                                       columns, a thread owns rows 4 (m RG + rg) + e of them.  What bounds it is latency:
+//                                       a token's update waits for the one before, a CTA has few warps, and each of them
+//                                       also issues the copies of the next CH tokens (cp.async into the other half of a
+//                                       double buffer).  So the arithmetic runs on pairs of rows (fma.rn.f32x2: the same
+//                                       roundings, half the instructions), a batch of tokens shares its shuffles (a token
+//                                       at a time, each with log2(RG) shuffles behind it, took 787 us at the size below),
+//                                       and with many columns the q and k that a thread reads serve two of them.
+//                                       4 x 2048 tokens, 16 heads of 128: one column per thread and scalar arithmetic
+//                                       842 us, this 638 us.  One sequence of 512 tokens: 148, two columns a thread 258,
+//                                       one 105 us.
 //                                       The state is read from and written back to the slot once per launch, which
 //                                       makes a prompt portion and a single decoded token the same case and the
 //                                       result independent of where the sequence was cut.
@@ -492,12 +494,12 @@ __global__ void retention_prep_kernel(float* __restrict__ rec, const T* __restri
 //                                       mixer's direct term, with v its unscaled input).
 enum { DECAY_HEAD = 0, DECAY_TOKEN = 1, DECAY_CHANNEL = 2 };
 
-template <int DMAX, int RG, int CH, int DK>
+template <int DMAX, int RG, int CH, int DK, int COLS>   // COLS: value columns per thread, 1 or 2
 __global__ void __launch_bounds__(256)
 lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ rec,
                  const float* __restrict__ decay, const float* __restrict__ skip, const int32_t* __restrict__ segs,
                  int heads, int dim, int vdim, int dp, int vp) {
-  constexpr int NG = DMAX / (4 * RG);               // groups of four rows per thread (RG lanes share two value columns)
+  constexpr int NG = DMAX / (4 * RG);               // groups of four rows per thread (RG lanes share COLS value columns)
   extern __shared__ __align__(16) float sh[];       // [2][CH][q DMAX | k DMAX | (decays DMAX) | v VT | (decay)]
   pdl_launch_dependents();
   pdl_wait();
@@ -506,14 +508,14 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   if (n <= 0) return;
   constexpr bool TD = DK == DECAY_TOKEN, CD = DK == DECAY_CHANNEL;
   constexpr int XP = TD ? 4 : 0, NV = CD ? 3 : 2;   // NV: vectors of key width in a record
-  const int VT = 2 * (blockDim.x / RG), RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP;
-  const int h = blockIdx.y, j0 = blockIdx.z * VT, jl = 2 * (threadIdx.x / RG), j = j0 + jl, rg = threadIdx.x % RG;
+  const int VT = COLS * (blockDim.x / RG), RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP;
+  const int h = blockIdx.y, j0 = blockIdx.z * VT, jl = COLS * (threadIdx.x / RG), j = j0 + jl, rg = threadIdx.x % RG;
   const float lam_h = DK == DECAY_HEAD ? decay[h] : 0.f, skip_h = skip ? skip[h] : 0.f;
   for (int idx = threadIdx.x; idx < 2 * CH * RSZ; idx += blockDim.x) sh[idx] = 0.f;   // padding the copies never write
-  f32x2 S[2][NG * 2];                               // [column][pair of rows]
+  f32x2 S[COLS][NG * 2];                            // [column][pair of rows]
   float* st = state + ((size_t)slot * heads + h) * dim * vdim;
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
+  for (int c = 0; c < COLS; ++c)
 #pragma unroll
     for (int m = 0; m < NG; ++m)
 #pragma unroll
@@ -540,46 +542,58 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   };
   fetch(0, 0);
   int buf = 0;
-  // A batch of RG / 2 tokens has as many column sums as a column's lanes: a transposed butterfly (RG - 1 shuffles) leaves lane rg
-  // with the sum of token rg / 2, column rg & 1.  A batch's tokens have no shuffle between them, so their shared-memory
-  // reads and multiplications overlap.
-  constexpr int TB = RG / 2;
-  const int my_c = rg & 1;
-  const bool live = j + my_c < vdim;
+  // A batch of TB tokens has SUMS column sums.  A transposed butterfly halves their number with every step while there are
+  // several, so that lane rg ends up with sum rg / REP: token rg / REP / COLS, column rg / REP % COLS.  A batch's tokens have no
+  // shuffle between them: their shared-memory reads and multiplications overlap.
+  constexpr int TB = RG / COLS < CH ? RG / COLS : CH, SUMS = TB * COLS, REP = RG / SUMS;
+  const int my_sum = rg / REP, my_t = my_sum / COLS, my_c = my_sum % COLS;
+  const bool live = j + my_c < vdim && rg % REP == 0;
   float* orow = out + (size_t)row0 * heads * vdim + (size_t)h * vdim + j + my_c;
   const size_t ostep = (size_t)heads * vdim;
-  auto token = [&](const float* r, float& c0, float& c1) {         // one token's update and this thread's part of its outputs
-    const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
-    const f32x2 v0 = pair_of(vj.x, vj.x), v1 = pair_of(vj.y, vj.y);
+  auto token = [&](const float* r, float* sums) {                  // one token's update and this thread's part of its outputs
+    f32x2 v[COLS], o[COLS][2];
+    if constexpr (COLS == 2) {
+      const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
+      v[0] = pair_of(vj.x, vj.x);
+      v[1] = pair_of(vj.y, vj.y);
+    } else {
+      v[0] = pair_of(r[NV * DMAX + jl], r[NV * DMAX + jl]);
+    }
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) o[c][0] = o[c][1] = 0ull;
     const float lam = TD ? r[NV * DMAX + VT] : lam_h;
     const f32x2 lam2 = pair_of(lam, lam);
-    f32x2 o0[2] = {0ull, 0ull}, o1[2] = {0ull, 0ull};
 #pragma unroll
     for (int m = 0; m < NG; ++m) {
       const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(r + 4 * rg + 4 * RG * m);
       const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(r + DMAX + 4 * rg + 4 * RG * m);
       ulonglong2 a4 = make_ulonglong2(lam2, lam2);
       if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r + 2 * DMAX + 4 * rg + 4 * RG * m);   // decays per key channel
-      S[0][2 * m] = fma2(k4.x, v0, mul2(a4.x, S[0][2 * m]));
-      S[0][2 * m + 1] = fma2(k4.y, v0, mul2(a4.y, S[0][2 * m + 1]));
-      S[1][2 * m] = fma2(k4.x, v1, mul2(a4.x, S[1][2 * m]));
-      S[1][2 * m + 1] = fma2(k4.y, v1, mul2(a4.y, S[1][2 * m + 1]));
-      o0[0] = fma2(q4.x, S[0][2 * m], o0[0]);
-      o0[1] = fma2(q4.y, S[0][2 * m + 1], o0[1]);
-      o1[0] = fma2(q4.x, S[1][2 * m], o1[0]);
-      o1[1] = fma2(q4.y, S[1][2 * m + 1], o1[1]);
-    }
-    const float2 a0 = halves_of(o0[0]), a1 = halves_of(o0[1]), b0 = halves_of(o1[0]), b1 = halves_of(o1[1]);
-    c0 = (a0.x + a0.y) + (a1.x + a1.y);
-    c1 = (b0.x + b0.y) + (b1.x + b1.y);
-  };
-  auto gather = [&](float (&c)[RG]) {
 #pragma unroll
-    for (int w = RG / 2; w >= 1; w >>= 1) {
+      for (int c = 0; c < COLS; ++c) {
+        S[c][2 * m] = fma2(k4.x, v[c], mul2(a4.x, S[c][2 * m]));
+        S[c][2 * m + 1] = fma2(k4.y, v[c], mul2(a4.y, S[c][2 * m + 1]));
+        o[c][0] = fma2(q4.x, S[c][2 * m], o[c][0]);
+        o[c][1] = fma2(q4.y, S[c][2 * m + 1], o[c][1]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+      const float2 a = halves_of(o[c][0]), b = halves_of(o[c][1]);
+      sums[c] = (a.x + a.y) + (b.x + b.y);
+    }
+  };
+  auto gather = [&](float (&c)[SUMS]) {             // the order of the additions is that of the lanes, whatever SUMS is
+#pragma unroll
+    for (int w = RG / 2, k = SUMS / 2; w >= 1; w >>= 1, k >>= 1) {
+      if (k == 0) {
+        c[0] += __shfl_xor_sync(0xffffffffu, c[0], w);
+        continue;
+      }
       const bool up = (rg & w) != 0;
 #pragma unroll
-      for (int i = 0; i < w; ++i) {
-        const float keep = up ? c[i + w] : c[i], send = up ? c[i] : c[i + w];
+      for (int i = 0; i < k; ++i) {
+        const float keep = up ? c[i + k] : c[i], send = up ? c[i] : c[i + k];
         c[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
       }
     }
@@ -591,28 +605,29 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
     const float* r0 = sh + (size_t)buf * CH * RSZ;
     int tt = 0;
     for (; tt + TB <= nt; tt += TB) {
-      float c[RG];
+      float c[SUMS];
 #pragma unroll
-      for (int b = 0; b < TB; ++b) token(r0 + (size_t)(tt + b) * RSZ, c[2 * b], c[2 * b + 1]);
+      for (int b = 0; b < TB; ++b) token(r0 + (size_t)(tt + b) * RSZ, c + COLS * b);
       gather(c);
-      const int mine = tt + rg / 2;
+      const int mine = tt + my_t;
       if (live) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
     }
     if (tt < nt) {                                  // the last tokens of the segment
-      float c[RG];
+      float c[SUMS];
 #pragma unroll
       for (int b = 0; b < TB; ++b) {
-        c[2 * b] = c[2 * b + 1] = 0.f;
-        if (tt + b < nt) token(r0 + (size_t)(tt + b) * RSZ, c[2 * b], c[2 * b + 1]);
+#pragma unroll
+        for (int e = 0; e < COLS; ++e) c[COLS * b + e] = 0.f;
+        if (tt + b < nt) token(r0 + (size_t)(tt + b) * RSZ, c + COLS * b);
       }
       gather(c);
-      const int mine = tt + rg / 2;
+      const int mine = tt + my_t;
       if (live && mine < nt) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
     }
     __syncthreads();                                // every thread is done with this buffer before it is refilled
   }
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
+  for (int c = 0; c < COLS; ++c) {
     if (j + c >= vdim) continue;
 #pragma unroll
     for (int m = 0; m < NG; ++m)
@@ -626,29 +641,44 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   }
 }
 
-template <int DMAX, int RG, int CH>
-static int launch_lightning(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
-                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+template <int DMAX, int RG, int CH, int COLS>
+static int launch_lightning_cols(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
+                                 const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
   const int dp = (dim + 3) / 4 * 4, vp = (vdim + 3) / 4 * 4;
   // value columns per CTA: as many as 256 threads hold (every CTA of a head fetches all of q and k), fewer while the CTAs do
   // not fill the SMs; a CTA keeps a whole warp
-  int vt = 512 / RG;
-  while (vt > 64 / RG && vt > 8 && (vt / 2 >= vdim || (long long)n_segs * heads * cdiv(vdim, vt) < 148)) vt /= 2;
+  constexpr int WARP_COLS = 32 / RG * COLS;
+  int vt = 256 / RG * COLS;
+  while (vt > WARP_COLS && vt > 8 && (vt / 2 >= vdim || (long long)n_segs * heads * cdiv(vdim, vt) < (COLS == 1 ? 100 : 148))) vt /= 2;
   static const int vt_env = env_int("PG_LIGHTNING_VT", 0);
-  if (vt_env >= 8 && vt_env >= 64 / RG && vt_env <= 512 / RG && (vt_env & (vt_env - 1)) == 0) vt = vt_env;
+  if (vt_env >= 8 && vt_env >= WARP_COLS && vt_env <= 256 / RG * COLS && (vt_env & (vt_env - 1)) == 0) vt = vt_env;
   const size_t smem = sizeof(float) * 2 * CH * ((dk == DECAY_CHANNEL ? 3 : 2) * DMAX + vt + (dk == DECAY_TOKEN ? 4 : 0));
   // An ordinary launch, not a programmatic dependent one: CTAs that become resident while the preceding kernel still
   // fills the machine are placed on the few SMs with room, and a recurrence of a few hundred long-lived CTAs then runs
   // on a fraction of the GPU (measured at 4 x 2048 tokens, 8 heads of 128: 2.06 ms against 0.88 ms).
-  auto kern = dk == DECAY_CHANNEL ? lightning_kernel<DMAX, RG, CH, DECAY_CHANNEL>
-                                  : (dk == DECAY_TOKEN ? lightning_kernel<DMAX, RG, CH, DECAY_TOKEN> : lightning_kernel<DMAX, RG, CH, DECAY_HEAD>);
+  auto kern = dk == DECAY_CHANNEL ? lightning_kernel<DMAX, RG, CH, DECAY_CHANNEL, COLS>
+                                  : (dk == DECAY_TOKEN ? lightning_kernel<DMAX, RG, CH, DECAY_TOKEN, COLS> : lightning_kernel<DMAX, RG, CH, DECAY_HEAD, COLS>);
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     set_error("lightning: cannot reserve %zu B of shared memory", smem);
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
-  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3(vt / 2 * RG), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim, dp, vp);
+  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3(vt / COLS * RG), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim, dp, vp);
   return check_launch("lightning");
+}
+
+template <int DMAX, int RG, int CH>
+static int launch_lightning(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
+                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+  // Two columns per thread halve the reads of q and k but also the warps: from 1536 warps of the one-column form on (3072 where a
+  // warp's work is small, never up to 32 key channels).  512 tokens, 128 channels, us with one and two: 4096 columns 121 and 167,
+  // 6144 189 and 160, 16384 372 and 239; 64 channels: 8192 columns 119 and 121, 16384 105 and 77 (256 tokens);
+  // 256 channels: 2048 columns 185 and 281, 4096 263 and 240.
+  if constexpr (DMAX > 32) {
+    if ((long long)n_segs * heads * vdim * RG >= (DMAX > 64 ? 1536 : 3072) * 32)
+      return launch_lightning_cols<DMAX, RG, CH, 2>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
+  }
+  return launch_lightning_cols<DMAX, RG, CH, 1>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
 }
 
 template <int DMAX, int CH>

@@ -379,3 +379,48 @@ def test_window_gates_and_weights_near_the_smallest_number(sigmoid):
     # exp(87.5) as 2^x: the exponent's rounding, 2^-18 of 126, is 3e-4 of the result; a weight of 1e-38 keeps 8 bits or, if the
     # type's subnormal numbers are meant, 7; one rounding of the result
     assert float((out.to(F64) - want).abs().max()) < 1.2e-2 * want
+
+
+@pytest.mark.parametrize("dim,vdim", [(20, 128), (32, 136), (64, 130), (100, 131), (128, 256), (200, 132), (256, 128)])
+@pytest.mark.parametrize("per_channel", [0, 1])
+def test_linear_scan_alone_and_in_a_batch(dim, vdim, per_channel):
+    """One value column per thread for a few sequences, two for many: the same sums in the same order, to the bit."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    H, lens = 16, [70, 1, 3, 16, 33, 8]
+    S, T, dp, vp = len(lens), sum(lens), -(-dim // 4) * 4, -(-vdim // 4) * 4
+    nq = 3 if per_channel else 2
+    rec = torch.zeros(T, H, nq * dp + vp, device="cuda")
+    q, k, v = (torch.randn(T, H, w, device="cuda", generator=g) for w in (dim, dim, vdim))
+    decay = torch.rand(T, H, dim, device="cuda", generator=g) if per_channel else torch.linspace(0.5, 0.99, H, device="cuda")
+    rec[:, :, :dim], rec[:, :, dp:dp + dim], rec[:, :, nq * dp:nq * dp + vdim] = q, k, v
+    if per_channel:
+        rec[:, :, 2 * dp:2 * dp + dim] = decay
+    start = torch.randn(S, H, dim, vdim, device="cuda", generator=g)
+    first = [sum(lens[:b]) for b in range(S)]
+
+    def scan(segs, state):
+        out = torch.full((T, H, vdim), 7.0, device="cuda")
+        sg = torch.tensor(segs, dtype=torch.int32, device="cuda")
+        if per_channel:
+            cabi.check(L.pg_gla_attention(out.data_ptr(), state.data_ptr(), rec.data_ptr(), sg.data_ptr(), len(segs), H, dim, vdim, st))
+        else:
+            cabi.check(L.pg_lightning_attention(out.data_ptr(), state.data_ptr(), rec.data_ptr(), decay.data_ptr(), sg.data_ptr(), len(segs), H,
+                                                dim, vdim, st))
+        torch.cuda.synchronize()
+        return out, state
+
+    out, state = scan([[b, first[b], lens[b]] for b in range(S)], start.clone())
+    # two columns from 1536 warps of the one-column form on (64 channels: 3072; up to 32: never); 8 lanes a column, above 128 channels 16
+    lanes = 16 if dim > 128 else 8
+    assert dim <= 32 or S * H * vdim * lanes >= 32 * (1536 if dim > 64 else 3072) > H * vdim * lanes
+    for b in range(S):
+        rows = slice(first[b], first[b] + lens[b])
+        o1, s1 = scan([[b, first[b], lens[b]]], start.clone())
+        assert torch.equal(o1[rows], out[rows]) and torch.equal(s1[b], state[b])
+        x, want = start[b].to(F64), []
+        for t in range(rows.start, rows.stop):
+            a = decay[t].to(F64)[:, :, None] if per_channel else decay.to(F64)[:, None, None]
+            x = a * x + k[t].to(F64)[:, :, None] * v[t].to(F64)[:, None, :]
+            want.append(torch.einsum("hd,hdv->hv", q[t].to(F64), x))
+        assert _rel(out[rows], torch.stack(want)) < 2e-6 and _rel(state[b], x) < 2e-6   # fp32 sums of up to 256 products
