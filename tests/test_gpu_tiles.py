@@ -9,6 +9,7 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 F64 = torch.float64
 BF = torch.bfloat16
+TYPES = [BF, torch.float16]
 
 
 def _cabi():
@@ -24,69 +25,79 @@ def _rel(got, want):
     return float((got.to(F64) - want).norm() / want.norm())
 
 
+def _tol(dtype, bf16, tanh=False):
+    """The same roundings cost fp16 an eighth of bf16's; the hardware tanh (2^-11) stays what it is."""
+    return bf16 if dtype == BF else bf16 / 8 + (2.0 ** -11 if tanh else 0.0)
+
+
 def _gelu(x):
     return F.gelu(x, approximate="tanh")
 
 
 # bf16 results: every rounding adds at most 2^-9 relative (rms about 2^-10.8), the hardware tanh 2^-11: three roundings of
 # a pairing stay below 4e-3
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("epi", ["geglu", "swiglu"])
 @pytest.mark.parametrize("M,N,K", [(1292, 2048, 256), (1100, 2056, 128), (513, 4096, 72), (385, 8200, 64)])
-def test_gated_pairs(epi, M, N, K):
+def test_gated_pairs(epi, M, N, K, dtype):
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(M)
-    a, w = _randn(g, M, K), _randn(g, 2 * N, K, std=K ** -0.5)
-    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    a, w = _randn(g, M, K, dtype=dtype), _randn(g, 2 * N, K, std=K ** -0.5, dtype=dtype)
+    out = torch.zeros(M + 1, N, dtype=dtype, device="cuda")
     cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, None, M, N, K, K, K, N, 0, 0,
-                         cabi.EPI_GEGLU if epi == "geglu" else cabi.EPI_SWIGLU, 0, 2, cabi.PG_BF16, st))
+                         cabi.EPI_GEGLU if epi == "geglu" else cabi.EPI_SWIGLU, 0, 2, cabi.DTYPE_CODE[dtype], st))
     z = a.to(F64) @ w.to(F64).T
     want = (_gelu(z[:, :N]) if epi == "geglu" else F.silu(z[:, :N])) * z[:, N:]
-    assert _rel(out[:M], want) < 5e-3
+    assert _rel(out[:M], want) < _tol(dtype, 5e-3, epi == "geglu")
     assert bool((out[M] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("M,N,K", [(1292, 2048, 512), (1292, 2560, 200), (700, 2048, 1024), (1025, 264, 4096)])
-def test_row_major_pairs_with_residual(M, N, K):
+def test_row_major_pairs_with_residual(M, N, K, dtype):
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(N)
-    a, w, r = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N)
-    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    a, w, r = _randn(g, M, K, dtype=dtype), _randn(g, N, K, std=K ** -0.5, dtype=dtype), _randn(g, M, N, dtype=dtype)
+    out = torch.zeros(M + 1, N, dtype=dtype, device="cuda")
     cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr(), M, N, K, K, K, N, N, 0, cabi.EPI_RES, 0, 2,
-                         cabi.PG_BF16, st))
-    assert _rel(out[:M], a.to(F64) @ w.to(F64).T + r.to(F64)) < 4e-3
+                         cabi.DTYPE_CODE[dtype], st))
+    assert _rel(out[:M], a.to(F64) @ w.to(F64).T + r.to(F64)) < _tol(dtype, 4e-3)
     assert bool((out[M] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("M", [4, 8, 31, 32, 33, 64])
 @pytest.mark.parametrize("N,K,epi", [(2048, 16384, "res"), (2048, 2048, "res"), (2560, 2048, "none"), (2056, 2048, "bias"), (2048, 4104, "res")])
-def test_few_rows_split_over_clusters(M, N, K, epi):
+def test_few_rows_split_over_clusters(M, N, K, epi, dtype):
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(M + K)
-    a, w, r, b = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N), _randn(g, N)
-    out = torch.zeros(M + 1, N, dtype=BF, device="cuda")
+    a, w = _randn(g, M, K, dtype=dtype), _randn(g, N, K, std=K ** -0.5, dtype=dtype)
+    r, b = _randn(g, M, N, dtype=dtype), _randn(g, N, dtype=dtype)
+    out = torch.zeros(M + 1, N, dtype=dtype, device="cuda")
     code = {"res": cabi.EPI_RES, "none": cabi.EPI_NONE, "bias": cabi.EPI_BIAS}[epi]
     cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr() if epi == "bias" else None,
-                         r.data_ptr() if epi == "res" else None, M, N, K, K, K, N, N if epi == "res" else 0, 0, code, 0, 0, cabi.PG_BF16, st))
+                         r.data_ptr() if epi == "res" else None, M, N, K, K, K, N, N if epi == "res" else 0, 0, code, 0, 0, cabi.DTYPE_CODE[dtype], st))
     want = a.to(F64) @ w.to(F64).T + (r.to(F64) if epi == "res" else b.to(F64) if epi == "bias" else 0.0)
-    assert _rel(out[:M], want) < 4e-3
+    assert _rel(out[:M], want) < _tol(dtype, 4e-3)
     assert bool((out[M] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("act,rel", [("none", 4e-3), ("silu", 5e-3), ("clamped", 6e-3), ("relu2", 6e-3)])
 @pytest.mark.parametrize("rows", [[1200, 0, 257, 1], [256, 256, 512, 1024], [3000, 5], [3, 1, 0, 2, 0, 1, 4, 5]])
-def test_grouped_products(act, rel, rows):
+def test_grouped_products(act, rel, rows, dtype):
     """Experts with many rows (CTA pairs), with none, with one, with a row behind a full tile; a handful of rows in all."""
     cabi, L, st = _cabi()
     E, N, K, P = len(rows), 328, 192, sum(rows)
     g = torch.Generator(device="cuda").manual_seed(P)
     dual = act in ("silu", "clamped")
-    a, w = _randn(g, P, K), _randn(g, E, 2 * N if dual else N, K, std=K ** -0.5)
+    a, w = _randn(g, P, K, dtype=dtype), _randn(g, E, 2 * N if dual else N, K, std=K ** -0.5, dtype=dtype)
     off = torch.tensor([sum(rows[:e]) for e in range(E + 1)], dtype=torch.int32, device="cuda")
-    out = torch.zeros(P + 1, N, dtype=BF, device="cuda")
+    out = torch.zeros(P + 1, N, dtype=dtype, device="cuda")
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     code = {"none": cabi.GLU_NONE, "silu": cabi.GLU_SILU, "clamped": cabi.GLU_CLAMPED, "relu2": cabi.ACT_RELU2}[act]
     cabi.check(L.pg_moe_gemm_act(out.data_ptr(), N, a.data_ptr(), K, None, w.data_ptr(), off.data_ptr(), P, E, N, K, code, 1.5, 2,
-                                 err.data_ptr(), cabi.PG_BF16, st))
+                                 err.data_ptr(), cabi.DTYPE_CODE[dtype], st))
     want = torch.empty(P, N, dtype=F64, device="cuda")
     for e in range(E):
         z = a[off[e]:off[e + 1]].to(F64) @ w[e].to(F64).T
@@ -99,7 +110,7 @@ def test_grouped_products(act, rel, rows):
             z = z.clamp_min(0.0) ** 2
         want[off[e]:off[e + 1]] = z
     assert int(err) == 0
-    assert _rel(out[:P], want) < rel
+    assert _rel(out[:P], want) < _tol(dtype, rel)
     assert bool((out[P] == 0).all())
 
 
@@ -157,24 +168,25 @@ def test_prompt_attention_scores_below_the_type(q, T, low):
 
 
 @pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 4, 4), (128, 128, 16, 4), (128, 128, 12, 1), (256, 256, 8, 1), (256, 192, 5, 1)])
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("window,keep,chunk", [(0, 0, 0), (33, 0, 0), (100, 7, 0), (0, 0, 48)])
-def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
+def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk, dtype):
     """Decode-sized ragged steps: positions at the edges of 16-key chunks, pages, windows, blocks and clusters."""
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(dim + H)
     pos = [0, 1, 15, 16, 17, 63, 64, 127, 500, 1535]
     n, cols = len(pos), 24
     pages = n * cols + 1
-    kp, vp = _randn(g, pages, 64, G * dim), _randn(g, pages, 64, G * vdim)
-    q, gate = _randn(g, n, H * dim), _randn(g, n, H * vdim)
+    kp, vp = _randn(g, pages, 64, G * dim, dtype=dtype), _randn(g, pages, 64, G * vdim, dtype=dtype)
+    q, gate = _randn(g, n, H * dim, dtype=dtype), _randn(g, n, H * vdim, dtype=dtype)
     pt = torch.randperm(pages, device="cuda", generator=g)[:n * cols].to(torch.int32).view(n, cols)
     slopes, sink = torch.rand(H, device="cuda", generator=g) * 0.1, torch.randn(H, device="cuda", generator=g)
     slot, tp = torch.arange(n, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda")
-    out = torch.zeros(n, H * vdim, dtype=BF, device="cuda")
+    out = torch.zeros(n, H * vdim, dtype=dtype, device="cuda")
     cabi.check(L.pg_attention_ragged_masked(out.data_ptr(), H * vdim, q.data_ptr(), H * dim, gate.data_ptr(), H * vdim, 0, kp.data_ptr(), 0,
                                             vp.data_ptr(), 0, pt.data_ptr(), cols, 64, slot.data_ptr(), tp.data_ptr(), n, H, G, dim, vdim,
                                             dim ** -0.5, window, keep, chunk, slopes.data_ptr(), 0, None, sink.data_ptr(), None, 0, 1.0,
-                                            None, 0, cabi.PG_BF16, st))
+                                            None, 0, cabi.DTYPE_CODE[dtype], st))
     for t, p in enumerate(pos):
         j = torch.arange(p + 1, device="cuda")
         seen = torch.ones_like(j, dtype=torch.bool)
@@ -186,7 +198,7 @@ def test_single_tokens_over_the_cache(dim, vdim, H, G, window, keep, chunk):
         s = torch.einsum("hd,nhd->hn", q[t].view(H, dim).to(F64), k) * dim ** -0.5 - slopes.to(F64)[:, None] * (p - j)
         s = torch.cat([s.masked_fill(~seen, -math.inf), sink.to(F64)[:, None]], 1)
         want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1)[:, :-1], v).reshape(-1) * torch.sigmoid(gate[t].to(F64))
-        assert _rel(out[t], want) < 4e-3          # one rounding of the result; weights are fp32
+        assert _rel(out[t], want) < _tol(dtype, 4e-3)    # one rounding of the result; weights are fp32
 
 
 def _single_tokens(q, kp, vp, pos, H, G, dim, vdim, scale, head_bias=None, sigmoid=0):
@@ -264,19 +276,21 @@ def test_single_tokens_infinite_values(dtype, sigmoid, dim, vdim, H, G):
         assert _rel(o[:, fine], want) < 4e-3      # one rounding of the result; weights are fp32
 
 
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("M", [16, 129, 256, 260, 384])
 @pytest.mark.parametrize("N,K,epi", [(1152, 4304, "bias_res"), (2048, 2048, "res"), (2560, 2048, "none"), (1160, 1152, "bias_gelu"),
                                      (520, 1096, "f32")])
-def test_few_tiles_split_over_clusters(M, N, K, epi):
+def test_few_tiles_split_over_clusters(M, N, K, epi, dtype):
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(M + N)
-    a, w, r, b = _randn(g, M, K), _randn(g, N, K, std=K ** -0.5), _randn(g, M, N), _randn(g, N)
+    a, w = _randn(g, M, K, dtype=dtype), _randn(g, N, K, std=K ** -0.5, dtype=dtype)
+    r, b = _randn(g, M, N, dtype=dtype), _randn(g, N, dtype=dtype)
     f32 = epi == "f32"
-    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else BF, device="cuda")
+    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else dtype, device="cuda")
     code = {"res": cabi.EPI_RES, "bias_res": cabi.EPI_BIAS_RES, "bias_gelu": cabi.EPI_BIAS_GELU}.get(epi, cabi.EPI_NONE)
     has_b, has_r = epi.startswith("bias"), epi.endswith("res")
     cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr() if has_b else None, r.data_ptr() if has_r else None, M, N,
-                         K, K, K, N, N if has_r else 0, 0, code, 1 if f32 else 0, 2, cabi.PG_BF16, st))
+                         K, K, K, N, N if has_r else 0, 0, code, 1 if f32 else 0, 2, cabi.DTYPE_CODE[dtype], st))
     want = a.to(F64) @ w.to(F64).T
     if has_b:
         want = want + b.to(F64)
@@ -284,7 +298,7 @@ def test_few_tiles_split_over_clusters(M, N, K, epi):
         want = _gelu(want)
     if has_r:
         want = want + r.to(F64)
-    assert _rel(out[:M], want) < 4e-3          # at most three roundings of 2^-9 and the hardware tanh
+    assert _rel(out[:M], want) < _tol(dtype, 4e-3, epi == "bias_gelu")    # at most three roundings of 2^-9 and the hardware tanh
     assert bool((out[M] == 0).all())
 
 
@@ -305,23 +319,24 @@ def test_norm_rows(rows, D):
     assert bool((out[rows] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("M", [256, 257, 272, 273, 288, 289, 516])
 @pytest.mark.parametrize("N,K,kind", [(9480, 136, "geglu"), (9480, 1000, "geglu"), (9472, 136, "swiglu"), (19000, 72, "none"), (18960, 1000, "res"),
                                       (19000, 1000, "f32")])
-def test_rows_behind_a_multiple_of_256(M, N, K, kind):
+def test_rows_behind_a_multiple_of_256(M, N, K, kind, dtype):
     """257 to 288 rows: the remainder rides along with the full 256; the row counts next to them; ragged last tiles."""
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(M + K)
     dual, f32 = kind.endswith("glu"), kind == "f32"
-    a, w, r = _randn(g, M, K), _randn(g, 2 * N if dual else N, K, std=K ** -0.5), _randn(g, M, N)
-    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else BF, device="cuda")
+    a, w, r = _randn(g, M, K, dtype=dtype), _randn(g, 2 * N if dual else N, K, std=K ** -0.5, dtype=dtype), _randn(g, M, N, dtype=dtype)
+    out = torch.zeros(M + 1, N, dtype=torch.float32 if f32 else dtype, device="cuda")
     code = {"geglu": cabi.EPI_GEGLU, "swiglu": cabi.EPI_SWIGLU, "res": cabi.EPI_RES}.get(kind, cabi.EPI_NONE)
     res = kind == "res"
     cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr() if res else None, M, N, K, K, K, N, N if res else 0, 0,
-                         code, 1 if f32 else 0, 2, cabi.PG_BF16, st))
+                         code, 1 if f32 else 0, 2, cabi.DTYPE_CODE[dtype], st))
     z = a.to(F64) @ w.to(F64).T
     want = {"geglu": lambda: _gelu(z[:, :N]) * z[:, N:], "swiglu": lambda: F.silu(z[:, :N]) * z[:, N:], "res": lambda: z + r.to(F64)}.get(kind, lambda: z)()
-    tol = 5e-3                                 # up to three roundings of 2^-9 (the fp32 rows hold values rounded to 16 bits) and the tanh
+    tol = _tol(dtype, 5e-3, kind == "geglu")    # up to three roundings of 2^-9 (the fp32 rows hold values rounded to 16 bits) and the tanh
     for rows in (slice(0, 256), slice(256, M))[:1 if M == 256 else 2]:
         assert _rel(out[:M][rows], want[rows]) < tol
     assert bool((out[M] == 0).all())
@@ -379,6 +394,34 @@ def test_window_gates_and_weights_near_the_smallest_number(sigmoid):
     # exp(87.5) as 2^x: the exponent's rounding, 2^-18 of 126, is 3e-4 of the result; a weight of 1e-38 keeps 8 bits or, if the
     # type's subnormal numbers are meant, 7; one rounding of the result
     assert float((out.to(F64) - want).abs().max()) < 1.2e-2 * want
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("dim,vdim,H,G", [(64, 64, 2, 1), (64, 192, 4, 2), (128, 144, 2, 1), (72, 136, 2, 2), (256, 192, 2, 1), (256, 256, 2, 1)])
+@pytest.mark.parametrize("window", [0, 65, 200])
+def test_window_prompts(dim, vdim, H, G, window, dtype):
+    """Prompt tiles of 128 and 72 rows behind 30 cached tokens, at value widths on both sides of what 256 columns of TMEM hold."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    past, T, cols = 30, 200, 4
+    kp, vp = _randn(g, cols + 1, 64, G * dim, dtype=dtype), _randn(g, cols + 1, 64, G * vdim, dtype=dtype)
+    q, gate = _randn(g, T, H * dim, dtype=dtype), _randn(g, T, H * vdim, dtype=dtype)
+    pt = torch.randperm(cols + 1, device="cuda", generator=g)[:cols].to(torch.int32).view(1, cols)
+    tiles = torch.tensor([[0, 128, 0, past], [128, 72, 0, past + 128]], dtype=torch.int32, device="cuda")
+    slopes, err = torch.rand(H, device="cuda", generator=g) * 0.2, torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(T + 1, H * vdim, dtype=dtype, device="cuda")
+    cabi.check(L.pg_attention_ragged_tc_capped(out.data_ptr(), H * vdim, q.data_ptr(), H * dim, gate.data_ptr(), H * vdim, 0, kp.data_ptr(), 0,
+                                               vp.data_ptr(), 0, (cols + 1) * 64, pt.data_ptr(), cols, 64, tiles.data_ptr(), 2, T, H, G, dim,
+                                               vdim, dim ** -0.5, window, 0, 0, slopes.data_ptr(), 0, None, None, 0.0, 0.0, 0, None, 0, 1.0,
+                                               err.data_ptr(), cabi.DTYPE_CODE[dtype], st))
+    i, j = torch.arange(T, device="cuda")[:, None] + past, torch.arange(past + T, device="cuda")[None]
+    seen = (j <= i) & ((i - j < window) if window else (j >= 0))
+    k, v = (x[pt[0].long()].reshape(-1, G, w)[:past + T].to(F64).repeat_interleave(H // G, 1) for x, w in ((kp, dim), (vp, vdim)))
+    s = torch.einsum("qhd,nhd->hqn", q.view(T, H, dim).to(F64), k) * dim ** -0.5 - slopes.to(F64)[:, None, None] * (i - j)
+    want = torch.einsum("hqn,nhd->qhd", torch.softmax(s.masked_fill(~seen, -math.inf), -1), v).reshape(T, -1) * torch.sigmoid(gate.to(F64))
+    assert int(err) == 0
+    assert _rel(out[:T], want) < _tol(dtype, 5e-3)      # weights and result are rounded once each
+    assert bool((out[T] == 0).all())
 
 
 @pytest.mark.parametrize("dim,vdim", [(20, 128), (32, 136), (64, 130), (100, 131), (128, 256), (200, 132), (256, 128)])
