@@ -1,7 +1,7 @@
 /* pg_b200 — C ABI of the B200-native PaliGemma hot path.
  *
  * The reference (PhilipWilliamVentura/multimodal-financial-analysis-tool-using-paligemma)
- * is pure Python/PyTorch and has no FFI of its own (SURVEY.md §8b): its boundary is the
+ * is pure Python/PyTorch and has no FFI of its own: its boundary is the
  * Python class surface of modeling_gemma.py / modeling_siglip.py.  Our drop-in modules of
  * the same names call these entry points (ctypes); every entry names
  * the reference code it replaces.
@@ -35,8 +35,8 @@ enum {
   PG_EPI_SWIGLU = 6     /* C = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu]       gated experts */
 };
 
-/* One exchange of the tensor-parallel decoder over NVLink peer memory (csrc/tp_exchange.cuh; SURVEY.md §8e: the
- * reference is single-device, the sharding is the north star's).  The PRODUCER kernel stores this rank's fp32 partial
+/* One exchange of the tensor-parallel decoder over NVLink peer memory (csrc/tp_exchange.cuh; the
+ * reference is single-device).  The PRODUCER kernel stores this rank's fp32 partial
  * as {value, sequence number} words into slot (parity, rank) of EVERY rank's buffer; the CONSUMER kernel waits for all
  * `size` slots of its local buffer and sums them in rank order.  Passed by pointer (host memory, read at launch);
  * NULL means "not tensor parallel" everywhere a parameter of this type appears. */
@@ -139,7 +139,7 @@ int pg_attention(void* out, int ld_out, const void* q, int ld_q, const void* k, 
  * QK^T and PV as tcgen05.mma with TMEM accumulators, Q/K/V tiles by TMA, one-pass softmax (the row's
  * reference maximum is raised lazily) with one thread per query row.  q, k, v are row-major matrices (`*_rows` x `ld_*`); head h sits
  * at columns *_col0 + h*hd_stride .. +hd, and a head row must be padded (with zeros) to a multiple of 64
- * columns unless hd is 128 or 256.  Paged K/V needs page_size == key tile (128 for hd <= 128, 64 above).
+ * columns unless hd is 128 or 256.  Paged K/V needs page_size == key tile (64).
  * Output is packed: head h at column h*hd of [B*q_len, ld_out]. */
 int pg_attention_tc(void* out, int ld_out, const void* q, long long q_rows, int ld_q, int q_col0,
                     const void* k, const void* v, long long kv_rows, int ld_kv, int k_col0, int v_col0,

@@ -7,12 +7,13 @@
 // every key and value row is read once for the whole group, straight into fragments with 16-byte loads: the contraction index of
 // S^T is permuted (lane j of a quad owns 8 consecutive columns of every 32), and so are the rows of O^T (lane group r owns 8
 // consecutive columns of every 64).  Q K^T multiplies the stored 16-bit operands; the weights stay fp32 and enter P V as three
-// 16-bit terms (mma_frag.cuh), so that the product is the fp32 one; fp16 sigmoid weights, which no maximum normalises, stay with
-// the fp32 kernels.  (m, l, O) of the warps meet in shared memory and those of the CTAs in
+// 16-bit terms (mma_frag.cuh): all their 24 bits in bf16, 2^-39 of the largest weight in fp16; fp16 sigmoid weights, which no
+// maximum normalises, stay with the fp32 kernels.  (m, l, O) of the warps meet in shared memory and those of the CTAs in
 // distributed shared memory, in a fixed order: one launch, no workspace.
 // The key-slice kernel of attention_ragged.cu gives a whole key row to one lane (32 rows of 16 bytes per load), keeps the query
 // in shared memory and needs a second launch to merge: 8 tokens x 1024 keys, 16 heads over 4, 128 wide: 30.2 + 9.7 us, this
-// kernel 13.7 us (launch alone, cold cache; 31.9 -> 9.6 us in a row of steps), the bytes alone 2.6 us: what is left is the chain tile -> page -> rows -> merge.
+// kernel 13.7 us (launch alone, cold cache; 31.9 -> 9.6 us in a row of steps), the bytes alone 2.6 us: what is left is the chain
+// token -> page -> rows -> merge.
 #include <cooperative_groups.h>
 
 #include "attention_ragged.cuh"

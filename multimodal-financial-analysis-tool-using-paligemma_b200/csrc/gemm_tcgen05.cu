@@ -10,7 +10,7 @@
 //   warp 2  TMEM allocator    512 columns = 2 accumulator stages x (1 or 2) x 128 columns
 //   warps 4-7 epilogue        TMEM -> registers -> global, overlapped with the next tile's MMAs
 // Used by the prefill / cache-off recompute / SigLIP / projector / lm_head(all positions) GEMMs of
-// the reference (every nn.Linear of SURVEY.md §2.3 with more than a handful of rows).
+// the reference (every nn.Linear with more than a handful of rows).
 #include "tc_common.cuh"
 
 namespace pg {

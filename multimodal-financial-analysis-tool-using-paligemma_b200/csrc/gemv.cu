@@ -1,7 +1,7 @@
 // Decode-path weight-streaming kernels (q_len == 1): every weight byte is read exactly once per
 // step with 128-bit loads, fp32 accumulation, and the reference's elementwise neighbours fused
 // in: RMSNorm prologue, RoPE + KV-append / GeGLU / residual / logits+argmax epilogues.
-// HBM-bound: bytes per step = the weight bytes (SURVEY.md §8d).
+// HBM-bound: bytes per step = the weight bytes.
 //
 // Latency structure (what matters at batch 1, where a layer is five ~3-25 us kernels):
 //  * a stage is U x R independent 128-bit loads per lane, 24-32 warps per SM keep > 100 KB in flight;

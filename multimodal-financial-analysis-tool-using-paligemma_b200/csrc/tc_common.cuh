@@ -158,8 +158,9 @@ template <> __device__ __forceinline__ uint32_t pack_pair<f16>(float lo, float h
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 constexpr float LOG2E_F = 1.4426950408889634f;
-constexpr float MAX_RAISE = 8.f;  // one-pass softmax: a row's reference maximum follows when a score exceeds it by more than 2^8
-                                  // (weights of at most 256 keep their relative precision in 16 bits)
+// One-pass softmax: a row's reference maximum follows only when a score exceeds it by more than 2^8 (the conditional rescaling
+// published with FlashAttention-4; weights of at most 256 keep their relative precision in 16 bits).
+constexpr float MAX_RAISE = 8.f;
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- CTA pairs (cta_group::2)

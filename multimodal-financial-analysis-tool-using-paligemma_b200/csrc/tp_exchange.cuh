@@ -1,4 +1,4 @@
-// Tensor-parallel exchange over NVLink peer memory, fused into the decode kernels (SURVEY.md §8e).
+// Tensor-parallel exchange over NVLink peer memory, fused into the decode kernels.
 //
 // The tensor-parallel Gemma decoder needs the sum over ranks of the (B, D) partial outputs of o_proj and
 // down_proj, 2 x 18 times per token.  Instead of a collective launch between the kernels, the PRODUCER
