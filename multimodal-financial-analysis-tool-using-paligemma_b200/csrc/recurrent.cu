@@ -25,6 +25,7 @@
 // headnorm_gate_kernel (warp per (token, head)): o / rms(o) per head, times a weight (may be absent), times sigmoid(gate)
 //                                         or silu(gate), times a constant, rounded to the model dtype as the output projection's operand.
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace pg {
 
@@ -269,20 +270,25 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //     S <- decay_h S + k v^T,        o = S^T q
 // lightning_prep_kernel  (elementwise)  the activations in fp32, one packed record [q | k | v] per (token, head) with
 //                                       q, k padded to dp = dim rounded up to 4 floats and v to vp likewise (zeros).
-// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): RG lanes share one or two value
-//                                       columns, a thread owns rows 4 (m RG + rg) + e of them.  What bounds it is latency:
-//                                       a token's update waits for the one before, a CTA has few warps, and each of them
-//                                       also issues the copies of the next CH tokens (cp.async into the other half of a
-//                                       double buffer).  So the arithmetic runs on pairs of rows (fma.rn.f32x2: the same
-//                                       roundings, half the instructions), a batch of tokens shares its shuffles (a token
-//                                       at a time, each with log2(RG) shuffles behind it, took 787 us at the size below),
-//                                       and with many columns the q and k that a thread reads serve two of them.
-//                                       4 x 2048 tokens, 16 heads of 128: one column per thread and scalar arithmetic
-//                                       842 us, this 638 us.  One sequence of 512 tokens: 148, two columns a thread 258,
-//                                       one 105 us.
+// lightning_kernel       (CTA per (sequence segment, head, slice of VT value columns)): a step is four tokens.  With S the state
+//                                       before them, E_i the product of the decays up to token i, G_j of those behind token j:
+//                                           o_i = (E_i q_i)^T S + sum over j <= i of (q_i . (decays between them) k_j) v_j
+//                                           S  <- E_3 S + sum over j of (G_j k_j) v_j^T
+//                                       which is nine multiply-adds per state element and step for twelve, and no token of a
+//                                       step waits for the one before.  Decays are only multiplied, never divided by, so any
+//                                       value keeps its meaning; a token reads nothing of a later one, infinities neither.
+//                                       Two warps copy the records (cp.async, several steps ahead), scale q and k and take
+//                                       the ten products of a step; up to four hold the state, RG lanes sharing one, two or
+//                                       four value columns, a thread rows 4 (m RG + rg) + e of them.  The arithmetic runs on
+//                                       pairs of rows (fma.rn.f32x2; 2.4 cycles an SM quarter, 3 from a single warp).
+//                                       Bound by those and by the shared-memory reads of q and k: of a step's 1480 cycles
+//                                       (64 columns of 128 rows) 890 issue and about 700 multiply.
+//                                       4 x 2048 tokens, 16 heads of 128: token by token with the copies in every warp 620
+//                                       us, this 373; one sequence of 512 tokens 105 and 62, 8 heads of it 150 and 49; 128 single
+//                                       tokens 96 and 86.
 //                                       The state is read from and written back to the slot once per launch, which
-//                                       makes a prompt portion and a single decoded token the same case and the
-//                                       result independent of where the sequence was cut.
+//                                       makes a prompt portion and a single decoded token the same case; where a sequence
+//                                       is cut decides which tokens share a step, and with it the last bits.
 template <typename T>
 __global__ void lightning_prep_kernel(float* __restrict__ rec, const T* __restrict__ proj, int ld, int q_col0, int k_col0,
                                       int v_col0, long long n_tokens, int heads, int dim, int vdim, int dp, int vp) {
@@ -494,192 +500,500 @@ __global__ void retention_prep_kernel(float* __restrict__ rec, const T* __restri
 //                                       mixer's direct term, with v its unscaled input).
 enum { DECAY_HEAD = 0, DECAY_TOKEN = 1, DECAY_CHANNEL = 2 };
 
-template <int DMAX, int RG, int CH, int DK, int COLS>   // COLS: value columns per thread, 1 or 2
-__global__ void __launch_bounds__(256)
+constexpr int SCAN_TB = 4, SCAN_AUX = 2;                  // tokens per step, warps that prepare steps
+constexpr int SCAN_SIDE = 20;                             // floats beside a step: weights [4][4], the step's whole decay
+
+// A thread's part of a state: COLS value columns from j on, rows 4 (m RG + rg) + e (m < NG, e < 4) of them, in pairs of rows.
+template <int RG, int NG, int COLS>
+struct ScanState {
+  f32x2 S[COLS][NG * 2];
+  static __device__ __forceinline__ void load_row(float* x, const float* p) {
+    if constexpr (COLS == 4) *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(p);
+    else if constexpr (COLS == 2) *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(p);
+    else x[0] = p[0];
+  }
+  static __device__ __forceinline__ void store_row(float* p, const float* x) {
+    if constexpr (COLS == 4) *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(x);
+    else if constexpr (COLS == 2) *reinterpret_cast<float2*>(p) = *reinterpret_cast<const float2*>(x);
+    else p[0] = x[0];
+  }
+  // wide: whole aligned groups of columns; with all rows there too, nothing is asked per row (a branch for each delays the next
+  // one's load)
+  __device__ __forceinline__ void load(const float* st, int dim, int vdim, int j, int rg, bool wide) {
+    if (wide && dim == 4 * NG * RG) {
+      float x[NG * 4][COLS];
+#pragma unroll
+      for (int m = 0; m < NG; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) load_row(x[m * 4 + e], st + (size_t)(4 * (m * RG + rg) + e) * vdim + j);
+#pragma unroll
+      for (int y = 0; y < NG * 2; ++y)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) S[c][y] = pair_of(x[2 * y][c], x[2 * y + 1][c]);
+      return;
+    }
+#pragma unroll
+    for (int m = 0; m < NG; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          const int i = 4 * (m * RG + rg) + e;
+          const float* p = st + (size_t)i * vdim + j + c;
+          const bool col = j + c < vdim;
+          S[c][m * 2 + e / 2] = pair_of(col && i < dim ? p[0] : 0.f, col && i + 1 < dim ? p[vdim] : 0.f);
+        }
+  }
+  __device__ __forceinline__ void store(float* st, int dim, int vdim, int j, int rg, bool wide) const {
+    const bool whole = wide && dim == 4 * NG * RG;
+#pragma unroll
+    for (int m = 0; m < NG; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 4 * (m * RG + rg) + e;
+        float* p = st + (size_t)i * vdim + j;
+        float x[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) { const float2 y = halves_of(S[c][m * 2 + e / 2]); x[c] = e & 1 ? y.y : y.x; }
+        if (whole) store_row(p, x);
+        else
+#pragma unroll
+          for (int c = 0; c < COLS; ++c) if (i < dim && j + c < vdim) p[c] = x[c];
+      }
+  }
+  // A few tokens, one after the other, from the records themselves (r: the first one's, tok floats apart).
+  template <int DK>
+  __device__ __forceinline__ void tokens(float* out, const float* r, size_t tok, int n, const float* decay, int h, int heads, float skip_h,
+                                         int vdim, int dp, int vp, int j, int rg) {
+    constexpr bool TD = DK == DECAY_TOKEN, CD = DK == DECAY_CHANNEL;
+    constexpr int NV = CD ? 3 : 2;
+    for (int t = 0; t < n; ++t, r += tok, out += (size_t)heads * vdim) {
+      const float lam = TD ? __ldg(r + NV * dp + vp) : (CD ? 1.f : decay[h]);
+      float v[COLS];
+      f32x2 v2[COLS], o[COLS];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        v[c] = j + c < vp ? __ldg(r + NV * dp + j + c) : 0.f;
+        v2[c] = pair_of(v[c], v[c]);
+        o[c] = 0ull;
+      }
+#pragma unroll
+      for (int m = 0; m < NG; ++m) {
+        const int i = 4 * (m * RG + rg);
+        const ulonglong2 z = make_ulonglong2(0ull, 0ull);
+        const ulonglong2 q4 = i < dp ? __ldg(reinterpret_cast<const ulonglong2*>(r + i)) : z;
+        const ulonglong2 k4 = i < dp ? __ldg(reinterpret_cast<const ulonglong2*>(r + dp + i)) : z;
+        ulonglong2 a4 = make_ulonglong2(pair_of(lam, lam), pair_of(lam, lam));
+        if (CD) a4 = i < dp ? __ldg(reinterpret_cast<const ulonglong2*>(r + 2 * dp + i)) : z;
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          S[c][2 * m] = fma2(k4.x, v2[c], mul2(a4.x, S[c][2 * m]));
+          S[c][2 * m + 1] = fma2(k4.y, v2[c], mul2(a4.y, S[c][2 * m + 1]));
+          o[c] = fma2(q4.x, S[c][2 * m], o[c]);
+          o[c] = fma2(q4.y, S[c][2 * m + 1], o[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        const float2 x = halves_of(o[c]);
+        float y = x.x + x.y;
+#pragma unroll
+        for (int w = RG / 2; w >= 1; w >>= 1) y += __shfl_xor_sync(0xffffffffu, y, w);
+        if (rg == c % RG && j + c < vdim) out[(size_t)h * vdim + j + c] = fmaf(skip_h, v[c], y);
+      }
+    }
+  }
+};
+
+// The wait of a whole warp: a phase that is over costs one try and a vote (the loop with its limit: 200 cycles).
+__device__ __forceinline__ bool scan_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
+  if (__all_sync(0xffffffffu, tc::mbar_try_wait(bar, parity))) return true;
+  return tc::mbar_wait_lim_warp(bar, parity, fail);
+}
+
+// p = a b with its rounding error (exact while p is a normal number)
+__device__ __forceinline__ void two_prod(float a, float b, float& p, float& err) { p = a * b; err = fmaf(a, b, -p); }
+
+// steps in shared memory: those of a warp are requested this many rounds ahead, less one
+template <int DMAX, int DK> constexpr int SCAN_AHEAD = DMAX <= 128 ? 4 : (DK == DECAY_CHANNEL ? 2 : 3);
+
+constexpr int scan_lanes(int dmax) { return dmax == 32 ? 4 : (dmax <= 128 ? 8 : 16); }   // lanes that share value columns
+
+template <int DMAX, int DK, int COLS>           // COLS: value columns per thread, 1, 2 or 4
+__global__ void __launch_bounds__((4 + SCAN_AUX) * 32, 2)
 lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ rec,
                  const float* __restrict__ decay, const float* __restrict__ skip, const int32_t* __restrict__ segs,
-                 int heads, int dim, int vdim, int dp, int vp) {
-  constexpr int NG = DMAX / (4 * RG);               // groups of four rows per thread (RG lanes share COLS value columns)
-  extern __shared__ __align__(16) float sh[];       // [2][CH][q DMAX | k DMAX | (decays DMAX) | v VT | (decay)]
+                 int heads, int dim, int vdim, int dp, int vp, int vec) {
+  constexpr int AHEAD = SCAN_AHEAD<DMAX, DK>, SCAN_RING = AHEAD * SCAN_AUX;
+  constexpr int RG = scan_lanes(DMAX), NG = DMAX / (4 * RG), TB = SCAN_TB;   // RG lanes share COLS value columns, NG groups of four rows each
+  extern __shared__ __align__(16) float sh[];         // [ring][TB][q DMAX | k DMAX | (decays DMAX) | v VT | (decay)] | [ring][side]
+  __shared__ __align__(8) uint64_t bars[2 * SCAN_RING];
+  __shared__ int fail;
   pdl_launch_dependents();
   pdl_wait();
   const int32_t* sg = segs + 3 * (size_t)blockIdx.x;
   const int slot = sg[0], row0 = sg[1], n = sg[2];
   if (n <= 0) return;
   constexpr bool TD = DK == DECAY_TOKEN, CD = DK == DECAY_CHANNEL;
-  constexpr int XP = TD ? 4 : 0, NV = CD ? 3 : 2;   // NV: vectors of key width in a record
-  const int VT = COLS * (blockDim.x / RG), RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP;
-  const int h = blockIdx.y, j0 = blockIdx.z * VT, jl = COLS * (threadIdx.x / RG), j = j0 + jl, rg = threadIdx.x % RG;
-  const float lam_h = DK == DECAY_HEAD ? decay[h] : 0.f, skip_h = skip ? skip[h] : 0.f;
-  // padding the copies never write, of the tokens that there are (128 single tokens, 16 heads of 128: all of it 103 us, this 96)
-  for (int idx = threadIdx.x; idx < min(n, 2 * CH) * RSZ; idx += blockDim.x) sh[idx] = 0.f;
-  f32x2 S[COLS][NG * 2];                            // [column][pair of rows]
-  float* st = state + ((size_t)slot * heads + h) * dim * vdim;
+  constexpr int XP = TD ? 4 : 0, NV = CD ? 3 : 2;     // NV: vectors of key width in a record
+  const int nw = (int)(blockDim.x >> 5) - SCAN_AUX, VT = COLS * (32 / RG) * nw;
+  const int RSZ = NV * DMAX + VT + XP, rs = NV * dp + vp + XP, steps = (n + TB - 1) / TB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, j0 = blockIdx.z * VT;
+  const float* head_rec = rec + ((size_t)row0 * heads + h) * (size_t)rs;   // token t's record: + t * heads * rs
+  const size_t tok_step = (size_t)heads * rs;
+  float* side = sh + (size_t)SCAN_RING * TB * RSZ;
+  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
+  auto ready = [&](int s) { return bar0 + 8u * s; };                      // the step is prepared
+  auto empty = [&](int s) { return bar0 + 8u * (SCAN_RING + s); };        // every warp has used it
+  const bool direct = n < TB;                         // a few tokens: no ring, each state warp reads the records itself
+  if (direct) {
+    if (warp >= nw) return;
+  } else {
+    if (threadIdx.x == 0) {
+      for (int s = 0; s < SCAN_RING; ++s) { tc::mbar_init(ready(s), 1); tc::mbar_init(empty(s), nw); }
+      fail = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+  }
+
+  if (warp >= nw) {
+    // ---- a step's records and what it needs besides, by one warp: with E_i the product of the decays up to token i and G_j of
+    // those behind token j, q_i <- E_i q_i, k_j <- G_j k_j, and the weight of v_j in token i's output, w_ij = q_i . (the decays
+    // between them) k_j.  Tokens behind the segment's last are zeros that decay by 1.  The copies run AHEAD - 1 of this warp's
+    // steps ahead (plain loads into registers shared their scoreboards with the shuffles: 3000 cycles a step instead of 600).
+    constexpr int F4 = (DMAX / 4 + 31) / 32;
+    const float lam_h = DK == DECAY_HEAD ? decay[h] : 1.f;
+    // values: 16-byte pieces of the step's tokens, V4 per lane (VT / 4 is a power of two up to 32)
+    constexpr int V4 = (COLS * (32 / RG) * 4 + 31) / 32;
+    const int v_len = min(VT, vp - j0), v_pieces = VT / 4, v_tok = lane / v_pieces, v_col = 4 * (lane % v_pieces), v_tstep = 32 / v_pieces;
+    float carry[CD ? F4 : 1][4];                        // what the roundings of the whole decays have added up to (relative)
 #pragma unroll
-  for (int c = 0; c < COLS; ++c)
+    for (int f = 0; f < (CD ? F4 : 1); ++f)
 #pragma unroll
-    for (int m = 0; m < NG; ++m)
+      for (int e = 0; e < 4; ++e) carry[f][e] = 0.f;
+    auto request = [&](int it) {
+      if (it < steps) {
+        const int s = it % SCAN_RING, nv = min(TB, n - it * TB);
+        const float* src = head_rec + (size_t)it * TB * tok_step;
+        float* dst = sh + (size_t)s * TB * RSZ;
+        // the state's warps have read the slot (in a first round nobody has to); a wait that ran out shows at this warp's next one
+        if (it >= SCAN_RING) scan_wait(empty(s), (it / SCAN_RING - 1) & 1, &fail);
 #pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int i = 4 * (m * RG + rg) + e;
-        S[c][m * 2 + e / 2] = pair_of((j + c < vdim && i < dim) ? st[(size_t)i * vdim + j + c] : 0.f,
-                                      (j + c < vdim && i + 1 < dim) ? st[(size_t)(i + 1) * vdim + j + c] : 0.f);
+        for (int t = 0; t < TB; ++t) {
+          const float* p = src + t * tok_step;
+          float* d = dst + t * RSZ;
+#pragma unroll
+          for (int f = 0; f < F4; ++f) {
+            const int c = 4 * (lane + 32 * f);
+            const bool have = t < nv && c < dp;
+#pragma unroll
+            for (int x = 0; x < NV; ++x) if (have) cp_async16(d + x * DMAX + c, p + x * dp + c);
+          }
+          if (TD && lane == 31 && t < nv) cp_async16(d + NV * DMAX + VT, p + NV * dp + vp);
+        }
+#pragma unroll
+        for (int x = 0; x < V4; ++x)
+          if (v_tok + x * v_tstep < nv && v_col < v_len)
+            cp_async16(dst + (v_tok + x * v_tstep) * RSZ + NV * DMAX + v_col, src + (v_tok + x * v_tstep) * tok_step + NV * dp + j0 + v_col);
       }
-  __syncthreads();
-  const int qk_pieces = dp / 4, v_pieces = min(VT, vp - j0) / 4, pieces = NV * qk_pieces + v_pieces + (TD ? 1 : 0);
-  auto fetch = [&](int t0, int buf) {               // records of tokens [t0, t0 + CH) of this head -> buffer buf
-    const int nt = min(CH, n - t0);
-    for (int idx = threadIdx.x; idx < nt * pieces; idx += blockDim.x) {
-      const int tt = idx / pieces, pc = idx % pieces;
-      const float* src = rec + (((size_t)row0 + t0 + tt) * heads + h) * (size_t)rs;
-      float* dst = sh + ((size_t)buf * CH + tt) * RSZ;
-      if (pc < qk_pieces) cp_async16(dst + pc * 4, src + pc * 4);
-      else if (pc < 2 * qk_pieces) cp_async16(dst + DMAX + (pc - qk_pieces) * 4, src + dp + (pc - qk_pieces) * 4);
-      else if (CD && pc < 3 * qk_pieces) cp_async16(dst + 2 * DMAX + (pc - 2 * qk_pieces) * 4, src + 2 * dp + (pc - 2 * qk_pieces) * 4);
-      else if (pc < NV * qk_pieces + v_pieces) cp_async16(dst + NV * DMAX + (pc - NV * qk_pieces) * 4, src + NV * dp + j0 + (pc - NV * qk_pieces) * 4);
-      else cp_async16(dst + NV * DMAX + VT, src + NV * dp + vp);
-    }
-    cp_async_commit();
-  };
-  fetch(0, 0);
-  int buf = 0;
-  // A batch of TB tokens has SUMS column sums.  A transposed butterfly halves their number with every step while there are
-  // several, so that lane rg ends up with sum rg / REP: token rg / REP / COLS, column rg / REP % COLS.  A batch's tokens have no
-  // shuffle between them: their shared-memory reads and multiplications overlap.
-  constexpr int TB = RG / COLS < CH ? RG / COLS : CH, SUMS = TB * COLS, REP = RG / SUMS;
-  const int my_sum = rg / REP, my_t = my_sum / COLS, my_c = my_sum % COLS;
-  const bool live = j + my_c < vdim && rg % REP == 0;
-  float* orow = out + (size_t)row0 * heads * vdim + (size_t)h * vdim + j + my_c;
-  const size_t ostep = (size_t)heads * vdim;
-  auto token = [&](const float* r, float* sums) {                  // one token's update and this thread's part of its outputs
-    f32x2 v[COLS], o[COLS][2];
-    if constexpr (COLS == 2) {
-      const float2 vj = *reinterpret_cast<const float2*>(r + NV * DMAX + jl);
-      v[0] = pair_of(vj.x, vj.x);
-      v[1] = pair_of(vj.y, vj.y);
-    } else {
-      v[0] = pair_of(r[NV * DMAX + jl], r[NV * DMAX + jl]);
-    }
+      cp_async_commit();
+    };
+    const int first = warp - nw;
+#pragma unroll 1
+    for (int i = 0; i < AHEAD - 1; ++i) request(first + i * SCAN_AUX);
+    for (int it = first; it < steps; it += SCAN_AUX) {
+      cp_async_wait<AHEAD - 2>();
+      __syncwarp();
+      if (*(volatile int*)&fail) break;
+      const int s = it % SCAN_RING, nv = min(TB, n - it * TB);
+      float* base = sh + (size_t)s * TB * RSZ;
+      float* sd = side + (size_t)s * SCAN_SIDE;
+      float q[F4][TB][4], k[F4][TB][4], a[CD ? F4 : 1][TB][4], lam[TB];
 #pragma unroll
-    for (int c = 0; c < COLS; ++c) o[c][0] = o[c][1] = 0ull;
-    const float lam = TD ? r[NV * DMAX + VT] : lam_h;
-    const f32x2 lam2 = pair_of(lam, lam);
+      for (int t = 0; t < TB; ++t) {
+        lam[t] = t >= nv ? 1.f : (TD ? base[t * RSZ + NV * DMAX + VT] : lam_h);
+#pragma unroll
+        for (int f = 0; f < F4; ++f) {
+          const int c = 4 * (lane + 32 * f);
+          const bool have = t < nv && c < dp;
+          const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+          const float* p = base + t * RSZ + c;
+          *reinterpret_cast<float4*>(q[f][t]) = have ? *reinterpret_cast<const float4*>(p) : z;
+          *reinterpret_cast<float4*>(k[f][t]) = have ? *reinterpret_cast<const float4*>(p + DMAX) : z;
+          if constexpr (CD) *reinterpret_cast<float4*>(a[f][t]) = have ? *reinterpret_cast<const float4*>(p + 2 * DMAX) : one;
+        }
+        if (t >= nv)
+          for (int c = lane; c < VT; c += 32) base[t * RSZ + NV * DMAX + c] = 0.f;
+      }
+      float w[16];                                      // the weights of token pairs j <= i, at i (i + 1) / 2 + j
+#pragma unroll
+      for (int x = 0; x < 16; ++x) w[x] = 0.f;
+      // The whole decay of a step multiplies the state once per step: rounded the same way every time its error would add up over
+      // the steps (a constant decay near 1 above all), so the part that the last roundings lost is put back into the next one.
+      auto whole = [&](float p, float err, float& carry) {
+        const float fix = fmaf(p, carry, err), d = p + fix;
+        carry = p > 1e-30f ? ((p - d) + fix) / p : 0.f;
+        return d;
+      };
+      float E[TB], G[TB], D = 1.f;
+      if constexpr (!CD) {
+        float p = lam[0], err = 0.f;
+        E[0] = p;
+#pragma unroll
+        for (int i = 1; i < TB; ++i) {
+          float x, y;
+          two_prod(p, lam[i], x, y);
+          err = fmaf(err, lam[i], y);
+          p = x;
+          E[i] = p + err;
+        }
+        D = whole(p, err, carry[0][0]);
+        G[TB - 1] = 1.f;
+        p = 1.f; err = 0.f;
+#pragma unroll
+        for (int i = TB - 2; i >= 0; --i) {
+          float x, y;
+          two_prod(p, lam[i + 1], x, y);
+          err = fmaf(err, lam[i + 1], y);
+          p = x;
+          G[i] = p + err;
+        }
+      }
+#pragma unroll
+      for (int f = 0; f < F4; ++f) {
+        const int c = 4 * (lane + 32 * f);
+        if (c >= DMAX) break;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float p = 1.f, err = 0.f;
+#pragma unroll
+          for (int i = 0; i < TB; ++i) {
+            const float ai = CD ? a[f][i][e] : lam[i];
+#pragma unroll
+            for (int j = 0; j <= i; ++j) {
+              // token j's key decayed up to token i
+              if (CD && j < i) k[f][j][e] *= ai;
+              w[i * (i + 1) / 2 + j] = fmaf(q[f][i][e], k[f][j][e], w[i * (i + 1) / 2 + j]);
+            }
+            if constexpr (CD) {
+              float x, y;
+              two_prod(p, ai, x, y);
+              err = fmaf(err, ai, y);
+              p = x;
+              q[f][i][e] *= p + err;
+            } else {
+              q[f][i][e] *= E[i];
+            }
+          }
+          if constexpr (CD) {
+            a[f][0][e] = whole(p, err, carry[f][e]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < TB - 1; ++j) k[f][j][e] *= G[j];
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < TB; ++t) {
+          *reinterpret_cast<float4*>(base + t * RSZ + c) = *reinterpret_cast<const float4*>(q[f][t]);
+          *reinterpret_cast<float4*>(base + t * RSZ + DMAX + c) = *reinterpret_cast<const float4*>(k[f][t]);
+        }
+        if constexpr (CD) *reinterpret_cast<float4*>(base + 2 * DMAX + c) = *reinterpret_cast<const float4*>(a[f][0]);
+      }
+      float between[TB][TB];                            // the decays between two tokens, where one number per token does
+      if constexpr (!CD) {
+#pragma unroll
+        for (int j = 0; j < TB; ++j) {
+          between[j][j] = 1.f;
+#pragma unroll
+          for (int i = j + 1; i < TB; ++i) between[i][j] = between[i - 1][j] * lam[i];
+        }
+      }
+#pragma unroll
+      for (int o = 16, m = 8; o >= 2; o >>= 1, m >>= 1) {   // a transposed butterfly: lane L ends up with half of sum L / 2
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int x = 0; x < m; ++x) {
+          const float keep = up ? w[x + m] : w[x], send = up ? w[x] : w[x + m];
+          w[x] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], 1);
+      // one store for the warp, chosen without branches (a branch per weight cost 2400 cycles a step)
+      float mine = lane == 31 ? D : w[0];
+      int at = lane == 31 ? 16 : 17;                    // 17: nobody's
+#pragma unroll
+      for (int i = 0; i < TB; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+          const bool is = lane == 2 * (i * (i + 1) / 2 + j);
+          if (!CD && j < i) mine = is ? mine * between[i][j] : mine;
+          at = is ? 4 * i + j : at;
+        }
+      sd[at] = mine;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(ready(s));
+      request(it + (AHEAD - 1) * SCAN_AUX);
+    }
+    return;
+  }
+
+  // ---- the state's warps
+  const int jl = COLS * (threadIdx.x / RG), j = j0 + jl, rg = threadIdx.x % RG;
+  const float skip_h = skip ? skip[h] : 0.f;
+  float* st = state + ((size_t)slot * heads + h) * dim * vdim;
+  const bool wide = vec && j + COLS <= vdim;
+  ScanState<RG, NG, COLS> mine;
+  auto& S = mine.S;                                   // [column][pair of rows]
+  mine.load(st, dim, vdim, j, rg, wide);
+  if (direct) {
+    mine.template tokens<DK>(out + (size_t)row0 * heads * vdim, head_rec, tok_step, n, decay, h, heads, skip_h, vdim, dp, vp, j, rg);
+    mine.store(st, dim, vdim, j, rg, wide);
+    return;
+  }
+  // A step has SUMS column sums.  A transposed butterfly halves their number with every exchange while there are several: lane rg
+  // ends up with the PER sums from rg * PER on, or (more lanes than sums) with sum rg / REP.  Sum x: token x / COLS, column x % COLS.
+  constexpr int SUMS = TB * COLS, PER = SUMS >= RG ? SUMS / RG : 1, REP = SUMS >= RG ? 1 : RG / SUMS;
+  static_assert(COLS % PER == 0, "the sums of a lane belong to one token");
+  const int sum0 = rg * PER / REP, my_t = sum0 / COLS, my_c = sum0 % COLS;
+  float* orow = out + ((size_t)row0 + my_t) * heads * vdim + (size_t)h * vdim + j + my_c;
+  const size_t ostep = (size_t)TB * heads * vdim;
+  bool ok = true;
+  for (int it = 0; it < steps; ++it, orow += ostep) {
+    const int s = it % SCAN_RING;
+    if (!scan_wait(ready(s), (it / SCAN_RING) & 1, &fail)) { ok = false; break; }
+    const float* r0 = sh + (size_t)s * TB * RSZ;
+    const float* sd = side + (size_t)s * SCAN_SIDE;
+    // what the step's tokens read from the state before it
+    f32x2 o[TB][COLS];
+    ulonglong2 x4[2][TB];                             // the next group's rows are requested before this one's are used
+    auto rows = [&](int which, int m, ulonglong2 (&x)[TB]) {
+#pragma unroll
+      for (int t = 0; t < TB; ++t) x[t] = *reinterpret_cast<const ulonglong2*>(r0 + t * RSZ + which * DMAX + 4 * rg + 4 * RG * m);
+    };
+    rows(0, 0, x4[0]);
 #pragma unroll
     for (int m = 0; m < NG; ++m) {
-      const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(r + 4 * rg + 4 * RG * m);
-      const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(r + DMAX + 4 * rg + 4 * RG * m);
-      ulonglong2 a4 = make_ulonglong2(lam2, lam2);
-      if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r + 2 * DMAX + 4 * rg + 4 * RG * m);   // decays per key channel
+      if (m + 1 < NG) rows(0, m + 1, x4[(m + 1) & 1]);
+      else rows(1, 0, x4[NG & 1]);
 #pragma unroll
-      for (int c = 0; c < COLS; ++c) {
-        S[c][2 * m] = fma2(k4.x, v[c], mul2(a4.x, S[c][2 * m]));
-        S[c][2 * m + 1] = fma2(k4.y, v[c], mul2(a4.y, S[c][2 * m + 1]));
-        o[c][0] = fma2(q4.x, S[c][2 * m], o[c][0]);
-        o[c][1] = fma2(q4.y, S[c][2 * m + 1], o[c][1]);
-      }
+      for (int t = 0; t < TB; ++t)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          o[t][c] = m ? fma2(x4[m & 1][t].x, S[c][2 * m], o[t][c]) : mul2(x4[0][t].x, S[c][0]);
+          o[t][c] = fma2(x4[m & 1][t].y, S[c][2 * m + 1], o[t][c]);
+        }
     }
+    float c_sum[SUMS];
 #pragma unroll
-    for (int c = 0; c < COLS; ++c) {
-      const float2 a = halves_of(o[c][0]), b = halves_of(o[c][1]);
-      sums[c] = (a.x + a.y) + (b.x + b.y);
-    }
-  };
-  auto gather = [&](float (&c)[SUMS]) {             // the order of the additions is that of the lanes, whatever SUMS is
+    for (int t = 0; t < TB; ++t)
 #pragma unroll
-    for (int w = RG / 2, k = SUMS / 2; w >= 1; w >>= 1, k >>= 1) {
+      for (int c = 0; c < COLS; ++c) { const float2 x = halves_of(o[t][c]); c_sum[t * COLS + c] = x.x + x.y; }
+#pragma unroll
+    for (int w = RG / 2, k = SUMS / 2; w >= 1; w >>= 1, k >>= 1) {   // the order of the additions is that of the lanes
       if (k == 0) {
-        c[0] += __shfl_xor_sync(0xffffffffu, c[0], w);
+        c_sum[0] += __shfl_xor_sync(0xffffffffu, c_sum[0], w);
         continue;
       }
       const bool up = (rg & w) != 0;
 #pragma unroll
       for (int i = 0; i < k; ++i) {
-        const float keep = up ? c[i + k] : c[i], send = up ? c[i] : c[i + k];
-        c[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        const float keep = up ? c_sum[i + k] : c_sum[i], send = up ? c_sum[i] : c_sum[i + k];
+        c_sum[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
       }
     }
-  };
-  for (int t0 = 0; t0 < n; t0 += CH, buf ^= 1) {
-    const int nt = min(CH, n - t0);
-    if (t0 + CH < n) { fetch(t0 + CH, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-    __syncthreads();
-    const float* r0 = sh + (size_t)buf * CH * RSZ;
-    int tt = 0;
-    for (; tt + TB <= nt; tt += TB) {
-      float c[SUMS];
+    // the state behind the step
+    f32x2 v[TB][COLS];
 #pragma unroll
-      for (int b = 0; b < TB; ++b) token(r0 + (size_t)(tt + b) * RSZ, c + COLS * b);
-      gather(c);
-      const int mine = tt + my_t;
-      if (live) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
+    for (int t = 0; t < TB; ++t) {
+      float x[COLS];
+      const float* vs = r0 + t * RSZ + NV * DMAX + jl;
+      if constexpr (COLS == 4) *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vs);
+      else if constexpr (COLS == 2) *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(vs);
+      else x[0] = vs[0];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) v[t][c] = pair_of(x[c], x[c]);
     }
-    if (tt < nt) {                                  // the last tokens of the segment
-      float c[SUMS];
+    const float whole = CD ? 1.f : sd[16];
+    const f32x2 d2 = pair_of(whole, whole);
 #pragma unroll
-      for (int b = 0; b < TB; ++b) {
+    for (int m = 0; m < NG; ++m) {
+      ulonglong2 a4 = make_ulonglong2(d2, d2);
+      if (CD) a4 = *reinterpret_cast<const ulonglong2*>(r0 + 2 * DMAX + 4 * rg + 4 * RG * m);
 #pragma unroll
-        for (int e = 0; e < COLS; ++e) c[COLS * b + e] = 0.f;
-        if (tt + b < nt) token(r0 + (size_t)(tt + b) * RSZ, c + COLS * b);
+      for (int c = 0; c < COLS; ++c) { S[c][2 * m] = mul2(a4.x, S[c][2 * m]); S[c][2 * m + 1] = mul2(a4.y, S[c][2 * m + 1]); }
+      if (m + 1 < NG) rows(1, m + 1, x4[(NG + m + 1) & 1]);
+#pragma unroll
+      for (int t = 0; t < TB; ++t)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          S[c][2 * m] = fma2(x4[(NG + m) & 1][t].x, v[t][c], S[c][2 * m]);
+          S[c][2 * m + 1] = fma2(x4[(NG + m) & 1][t].y, v[t][c], S[c][2 * m + 1]);
+        }
+    }
+    // the step's own tokens, up to this lane's one, and the direct term
+    {
+      const float* vs = r0 + NV * DMAX + jl + my_c;
+      const bool writes = rg % REP == 0 && it * TB + my_t < n;
+#pragma unroll
+      for (int x = 0; x < PER; ++x) {
+        float y = c_sum[x];
+#pragma unroll
+        for (int t = 0; t < TB; ++t) y = t <= my_t ? fmaf(sd[4 * my_t + t], vs[t * RSZ + x], y) : y;
+        if (writes && j + my_c + x < vdim) orow[x] = fmaf(skip_h, vs[my_t * RSZ + x], y);
       }
-      gather(c);
-      const int mine = tt + my_t;
-      if (live && mine < nt) orow[(size_t)(t0 + mine) * ostep] = fmaf(skip_h, r0[(size_t)mine * RSZ + NV * DMAX + jl + my_c], c[0]);
     }
-    __syncthreads();                                // every thread is done with this buffer before it is refilled
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(empty(s));
   }
+  if (!ok) {                                          // a wait ran out: the state shows it
+    const float nan = __int_as_float(0x7fffffff);
 #pragma unroll
-  for (int c = 0; c < COLS; ++c) {
-    if (j + c >= vdim) continue;
+    for (int c = 0; c < COLS; ++c)
 #pragma unroll
-    for (int m = 0; m < NG; ++m)
-#pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int i = 4 * (m * RG + rg) + e;
-        const float2 v = halves_of(S[c][m * 2 + e / 2]);
-        if (i < dim) st[(size_t)i * vdim + j + c] = v.x;
-        if (i + 1 < dim) st[(size_t)(i + 1) * vdim + j + c] = v.y;
-      }
+      for (int x = 0; x < NG * 2; ++x) S[c][x] = pair_of(nan, nan);
   }
+  mine.store(st, dim, vdim, j, rg, wide);
 }
 
-template <int DMAX, int RG, int CH, int COLS>
-static int launch_lightning_cols(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
-                                 const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+template <int DMAX, int COLS>
+static int launch_scan_cols(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
+                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
   const int dp = (dim + 3) / 4 * 4, vp = (vdim + 3) / 4 * 4;
-  // value columns per CTA: as many as 256 threads hold (every CTA of a head fetches all of q and k), fewer while the CTAs do
-  // not fill the SMs; a CTA keeps a whole warp
-  constexpr int WARP_COLS = 32 / RG * COLS;
-  int vt = 256 / RG * COLS;
-  while (vt > WARP_COLS && vt > 8 && (vt / 2 >= vdim || (long long)n_segs * heads * cdiv(vdim, vt) < (COLS == 1 ? 100 : 148))) vt /= 2;
-  static const int vt_env = env_int("PG_LIGHTNING_VT", 0);
-  if (vt_env >= 8 && vt_env >= WARP_COLS && vt_env <= 256 / RG * COLS && (vt_env & (vt_env - 1)) == 0) vt = vt_env;
-  const size_t smem = sizeof(float) * 2 * CH * ((dk == DECAY_CHANNEL ? 3 : 2) * DMAX + vt + (dk == DECAY_TOKEN ? 4 : 0));
+  // value columns per CTA: those of four warps, of fewer while the CTAs do not fill the SMs or the columns are fewer
+  constexpr int WARP_COLS = 32 / scan_lanes(DMAX) * COLS;
+  int nw = 4;
+  while (nw > 1 && (nw / 2) * WARP_COLS >= 4 && ((nw / 2) * WARP_COLS >= vdim || (long long)n_segs * heads * cdiv(vdim, nw * WARP_COLS) < 100))
+    nw /= 2;
+  const int vt = nw * WARP_COLS;
+  const int ring = SCAN_AUX * (dk == DECAY_CHANNEL ? SCAN_AHEAD<DMAX, DECAY_CHANNEL> : SCAN_AHEAD<DMAX, DECAY_HEAD>);
+  const size_t smem = sizeof(float) * ring * (SCAN_TB * ((dk == DECAY_CHANNEL ? 3 : 2) * DMAX + vt + (dk == DECAY_TOKEN ? 4 : 0)) + SCAN_SIDE);
   // An ordinary launch, not a programmatic dependent one: CTAs that become resident while the preceding kernel still
   // fills the machine are placed on the few SMs with room, and a recurrence of a few hundred long-lived CTAs then runs
   // on a fraction of the GPU (measured at 4 x 2048 tokens, 8 heads of 128: 2.06 ms against 0.88 ms).
-  auto kern = dk == DECAY_CHANNEL ? lightning_kernel<DMAX, RG, CH, DECAY_CHANNEL, COLS>
-                                  : (dk == DECAY_TOKEN ? lightning_kernel<DMAX, RG, CH, DECAY_TOKEN, COLS> : lightning_kernel<DMAX, RG, CH, DECAY_HEAD, COLS>);
+  auto kern = dk == DECAY_CHANNEL ? lightning_kernel<DMAX, DECAY_CHANNEL, COLS>
+                                  : (dk == DECAY_TOKEN ? lightning_kernel<DMAX, DECAY_TOKEN, COLS> : lightning_kernel<DMAX, DECAY_HEAD, COLS>);
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     set_error("lightning: cannot reserve %zu B of shared memory", smem);
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
-  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3(vt / COLS * RG), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim, dp, vp);
+  const int vec = COLS == 1 || (vdim % COLS == 0 && (uintptr_t)state % 16 == 0);
+  kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3((nw + SCAN_AUX) * 32), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim,
+                                                                                        dp, vp, vec);
   return check_launch("lightning");
 }
 
-template <int DMAX, int RG, int CH>
-static int launch_lightning(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
-                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
-  // Two columns per thread halve the reads of q and k but also the warps: from 1536 warps of the one-column form on (3072 where a
-  // warp's work is small, never up to 32 key channels).  512 tokens, 128 channels, us with one and two: 4096 columns 121 and 167,
-  // 6144 189 and 160, 16384 372 and 239; 64 channels: 8192 columns 119 and 121, 16384 105 and 77 (256 tokens);
-  // 256 channels: 2048 columns 185 and 281, 4096 263 and 240.
-  if constexpr (DMAX > 32) {
-    if ((long long)n_segs * heads * vdim * RG >= (DMAX > 64 ? 1536 : 3072) * 32)
-      return launch_lightning_cols<DMAX, RG, CH, 2>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
-  }
-  return launch_lightning_cols<DMAX, RG, CH, 1>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
+template <int DMAX>
+static int launch_scan(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
+                       const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+  // Value columns per thread: more of them share a token's reads of q and k, but are fewer warps.  By the warps of the one-column
+  // form; 512 tokens, us with one, two and four: 128 channels, 1024 columns 49, 60, 92; 4096 98, 76, 92; 8192 193, 113, 107;
+  // 64 channels, 4096 72, 58, 55; 256 channels (twice the lanes a column), 2048 113, 84, 91; 4096 220, 126, 117.
+  const long long warps = (long long)n_segs * heads * vdim * scan_lanes(DMAX) / 32;
+  if (warps >= 1536) return launch_scan_cols<DMAX, 4>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
+  if (warps >= 768) return launch_scan_cols<DMAX, 2>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
+  return launch_scan_cols<DMAX, 1>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
 }
 
 template <int DMAX, int CH>
@@ -805,19 +1119,11 @@ static int lightning_any(float* out, float* state, const float* rec, const float
   PG_REQUIRE(out && state && rec && segs, "lightning_attention: bad arguments");
   PG_REQUIRE(dim > 0 && dim <= 256 && vdim > 0, "lightning_attention: key size %d (1..256), value size %d", dim, vdim);
   cudaStream_t st = (cudaStream_t)stream;
-  // lanes per value column: a thread keeps DMAX / RG state elements, and a token is that many fused multiply-adds
-  // twice plus log2(RG) shuffle steps on the critical path of the recurrence
-  if (dim <= 32) return launch_lightning<32, 4, 16>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  // tokens per buffer: the next buffer's records must be on their way for longer than a DRAM round trip while this
-  // one is consumed (16 tokens of 64..128 key channels; 8 left the recurrence waiting on every refill)
-  static const int deep = env_int("PG_LIGHTNING_DEEP", 1);
-  if (dim <= 64)
-    return deep ? launch_lightning<64, 8, 16>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st)
-                : launch_lightning<64, 8, 8>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  if (dim <= 128)
-    return deep ? launch_lightning<128, 8, 16>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st)
-                : launch_lightning<128, 8, 8>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  return launch_lightning<256, 16, 4>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
+  // lanes per value column: a thread keeps DMAX / RG rows of the state
+  if (dim <= 32) return launch_scan<32>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
+  if (dim <= 64) return launch_scan<64>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
+  if (dim <= 128) return launch_scan<128>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
+  return launch_scan<256>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
 }
 
 extern "C" int pg_lightning_attention_ex(float* out, float* state, const float* rec, const float* decay, const float* skip,

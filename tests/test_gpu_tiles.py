@@ -467,3 +467,61 @@ def test_linear_scan_alone_and_in_a_batch(dim, vdim, per_channel):
             x = a * x + k[t].to(F64)[:, :, None] * v[t].to(F64)[:, None, :]
             want.append(torch.einsum("hd,hdv->hv", q[t].to(F64), x))
         assert _rel(out[rows], torch.stack(want)) < 2e-6 and _rel(state[b], x) < 2e-6   # fp32 sums of up to 256 products
+
+
+@pytest.mark.parametrize("kind", ["head", "token", "channel"])
+@pytest.mark.parametrize("H,dim,vdim,lens", [(2, 32, 20, [1, 2, 3, 4, 5, 31, 32, 33, 300]), (3, 128, 36, [7, 64, 129]),
+                                             (2, 256, 130, [3, 70]), (16, 128, 128, [1, 3, 4, 2, 9] * 13)])
+def test_linear_scan_steps_of_four(kind, H, dim, vdim, lens):
+    """Whole and partial steps of four tokens, the ring of prepared steps and its second round, short segments and many of
+    them, a decay of 0, of 1 and just below it, and a later token's infinity."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    S, T, dp, vp = len(lens), sum(lens), -(-dim // 4) * 4, -(-vdim // 4) * 4
+    nq, tail = (3, 0) if kind == "channel" else (2, 4 if kind == "token" else 0)
+    q, k, v = (torch.randn(T, H, w, device="cuda", generator=g) for w in (dim, dim, vdim))
+    by_head = torch.linspace(0.99, 0.999, H, device="cuda")
+    by_head[0] = 0.0
+    a = {"head": lambda: by_head.view(1, H, 1).expand(T, H, dim), "channel": lambda: torch.rand(T, H, dim, device="cuda", generator=g) ** 0.1,
+         "token": lambda: (torch.rand(T, H, 1, device="cuda", generator=g) ** 0.1).expand(T, H, dim)}[kind]().clone()
+    if kind != "head":
+        a[1:3] = 1.0
+    rec = torch.zeros(T, H, nq * dp + vp + tail, device="cuda")
+    rec[:, :, :dim], rec[:, :, dp:dp + dim], rec[:, :, nq * dp:nq * dp + vdim] = q, k, v
+    if kind == "channel":
+        rec[:, :, 2 * dp:2 * dp + dim] = a
+    if kind == "token":
+        rec[:, :, nq * dp + vp] = a[:, :, 0]
+    skip = torch.randn(H, device="cuda", generator=g) if kind == "token" else None
+    first = [sum(lens[:b]) for b in range(S)]
+    segs = torch.tensor([[b, first[b], lens[b]] for b in range(S)] + [[0, 0, 0]], dtype=torch.int32, device="cuda")
+    start = torch.randn(S, H, dim, vdim, device="cuda", generator=g)
+
+    def scan(rec):
+        out, state = torch.full((T, H, vdim), 7.0, device="cuda"), start.clone()
+        if kind == "channel":
+            cabi.check(L.pg_gla_attention(out.data_ptr(), state.data_ptr(), rec.data_ptr(), segs.data_ptr(), S + 1, H, dim, vdim, st))
+        else:
+            cabi.check(L.pg_lightning_attention_ex(out.data_ptr(), state.data_ptr(), rec.data_ptr(), by_head.data_ptr() if kind == "head" else None,
+                                                   None if skip is None else skip.data_ptr(), segs.data_ptr(), S + 1, H, dim, vdim, st))
+        torch.cuda.synchronize()
+        return out, state
+
+    out, state = scan(rec)
+    want, end = torch.empty(T, H, vdim, dtype=F64, device="cuda"), start.to(F64)
+    for b in range(S):
+        x = end[b]
+        for t in range(first[b], first[b] + lens[b]):
+            x = a[t].to(F64)[:, :, None] * x + k[t].to(F64)[:, :, None] * v[t].to(F64)[:, None, :]
+            want[t] = torch.einsum("hd,hdv->hv", q[t].to(F64), x) + (0 if skip is None else skip.to(F64)[:, None] * v[t].to(F64))
+        end[b] = x
+    # a product of dim terms and a state of some hundred: a few roundings of 2^-24 each, in quadrature
+    assert _rel(out, want) < 1e-6 and _rel(state, end) < 1e-6
+    if lens[0] > 1 or lens[1] > 2:
+        at = first[-1] + lens[-1] - 1                     # the last token of the last segment: nothing before it may notice
+        bad = rec.clone()
+        bad[at, :, nq * dp:nq * dp + vdim] = float("inf")
+        out2, state2 = scan(bad)
+        keep = torch.arange(T, device="cuda") != at
+        assert torch.equal(out2[keep], out[keep]) and not bool(torch.isfinite(out2[at]).any())
+        assert torch.equal(state2[:-1], state[:-1]) and not bool(torch.isfinite(state2[-1, :, :dim]).any())
