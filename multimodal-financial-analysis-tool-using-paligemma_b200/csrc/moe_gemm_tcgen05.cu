@@ -434,6 +434,10 @@ static int launch_moe_pair(const CUtensorMap& ma, const CUtensorMap& mw, const M
 
 }  // namespace tc
 
+bool moe_gemm_few_wanted(int n_pairs, int K);
+int moe_gemm_few(void* out, int ldo, const void* A, int lda, const void* W, const int32_t* offsets, int n_pairs, int n_experts, int N,
+                 int K, int act, float limit, int dtype, cudaStream_t st);
+
 bool moe_gemm_tc_supported(int ldo, int lda, const int32_t* row_map, int N, int K, int dtype) {
   static const int enabled = env_int("PG_MOE_TC", 1);
   if (!enabled || (dtype != PG_BF16 && dtype != PG_F16) || row_map != nullptr) return false;
@@ -449,6 +453,8 @@ int moe_gemm_tc(void* out, int ldo, const void* A, int lda, const int32_t* row_m
   PG_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)out % 16) == 0,
              "moe_gemm_tc: operands must be 16-byte aligned");
   const bool bf = dtype == PG_BF16;
+  if (moe_gemm_few_wanted(n_pairs, K))
+    return moe_gemm_few(out, ldo, A, lda, W, offsets, n_pairs, n_experts, N, K, act, limit, dtype, st);
   const int rows_per_expert = swiglu ? 2 * N : N;
   CUtensorMap ma, mw;
   // CTA pairs from the row count on at which the last, partly filled 256-row tile of an expert costs less than the halved

@@ -128,3 +128,37 @@ def test_weighted_sum(dtype, T, D, top, shared, pad):
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6      # one rounding of the result
     assert bool(((out[:, :D].cpu().to(F64) - want).abs() <= eps * want.abs() + 1e-5).all())
     assert bool((out[:, D:] == 0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["silu", "clamped", "none", "relu2"])
+@pytest.mark.parametrize("counts,N,K", [([0, 1, 0, 3], 8, 8), ([2, 0, 9], 24, 72), ([17, 0, 1, 16, 30], 40, 1032), ([1] * 40, 16, 520),
+                                        ([0, 0, 12], 1200, 1024), ([5, 11, 0, 0], 2056, 2048)])
+def test_few_rows_per_expert(dtype, kind, counts, N, K):
+    """Row blocks of up to 16 rows (an expert with more, experts without), features that end inside a unit, columns that end inside
+    and behind a chunk of 1024, fewer and more units than CTAs; rows behind the last expert's are not written."""
+    cabi, L, st = _setup()
+    E, P, dual = len(counts), sum(counts) + 1, kind in ("silu", "clamped")
+    off = torch.tensor([0] + counts).cumsum(0).to(torch.int32)
+    a, w = _randn(P, K + 8, seed=21, dtype=dtype), _randn(E, (2 if dual else 1) * N, K, seed=22, dtype=dtype, std=K ** -0.5)
+    a[-1] = float("nan")                                 # nobody's row
+    ad, wd, offd = a.cuda(), w.cuda(), off.cuda()
+    out = torch.full((P, N + 8), 7.0, dtype=dtype, device="cuda")
+    code = {"silu": cabi.GLU_SILU, "clamped": cabi.GLU_CLAMPED, "none": cabi.GLU_NONE, "relu2": cabi.ACT_RELU2}[kind]
+    cabi.check(L.pg_moe_gemm_act(out.data_ptr(), N + 8, ad.data_ptr(), K + 8, None, wd.data_ptr(), offd.data_ptr(), P, E, N, K, code, 1.5, 2,
+                                 None, cabi.DTYPE_CODE[dtype], st))
+    e = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    y = torch.einsum("pk,pnk->pn", a[:-1, :K].to(F64), w.to(F64)[e])
+    g, u = y[:, :N], y[:, N:]
+    if kind == "silu":
+        y = g * torch.sigmoid(g) * u
+    elif kind == "clamped":
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        y = g * torch.sigmoid(1.702 * g) * (u + 1)
+    elif kind == "relu2":
+        y = g.clamp(min=0) ** 2
+    got = out[:-1, :N].cpu().to(F64)
+    # up to five roundings of values of about 1, each within half a step of the type
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert float((got - y).norm() / y.norm()) < 2 * eps and float((got - y).abs().max()) < 6 * eps * float(y.abs().max())
+    assert bool((out[-1] == 7).all()) and bool((out[:, N:] == 7).all())
