@@ -186,6 +186,13 @@ __device__ __forceinline__ uint4 ldg_cached(const void* p) {
   return __ldg(reinterpret_cast<const uint4*>(p));
 }
 
+// 16 bytes from global to shared memory, in groups that the thread waits for
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 template <typename T> __device__ __forceinline__ void unpack(const uint4& u, float* f);
 template <> __device__ __forceinline__ void unpack<float>(const uint4& u, float* f) {
   f[0] = __uint_as_float(u.x); f[1] = __uint_as_float(u.y);

@@ -274,6 +274,9 @@ int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, in
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi);
 int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                    int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st);
+bool gemm_stream_wanted(int M, int N, int K, int epi);
+int gemm_stream(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda, int ldw, int ldc,
+                int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st);
 bool gemm_tc_2cta_wanted(int M, int N, int K, int epi);
 int gemm_tc_2cta(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
                  int ldw, int ldc, int ldr, int res_mod, int epi, int out_f32, int dtype, cudaStream_t st);
@@ -296,6 +299,8 @@ int gemm_tc(void* C, const void* A, const void* W, const void* bias, const void*
   }
   if (gemm_tc_swap_wanted(M, N, K, epi, out_f32, res_mod))  // a prompt's worth of rows: CTA pairs, weights as the M operand
     return gemm_tc_swap(C, A, W, R, M, N, K, lda, ldw, ldc, ldr, epi, dtype, w_param, st);
+  if (res_mod == 0 && gemm_stream_wanted(M, N, K, epi))    // a few token rows: every SM streams as many weight rows
+    return gemm_stream(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, epi, out_f32, dtype, w_param, st);
   if (res_mod == 0 && gemm_tc_skinny_wanted(M, N, K, epi))  // a few dozen token rows: stream the weights (swap-AB)
     return gemm_tc_skinny(C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, epi, out_f32, dtype, w_param, st);
   {

@@ -15,6 +15,9 @@
 
 namespace pg {
 
+bool gemv_stream_wanted(int B, int N, int K);
+int gemv_stream(void* out, const void* x, const void* W, const void* R, int B, int N, int K, int dtype, cudaStream_t st);
+
 #ifndef PG_GEMV_THREADS
 #define PG_GEMV_THREADS 256
 #endif
@@ -552,6 +555,8 @@ int pg_gemv_res(void* out, const void* x, const void* W, const void* R, int B, i
   const TpEx tex = tp_ex_from(ex);
   PG_REQUIRE(!ex || (tex.tp >= 2 && tex.tp <= TP_MAX_RANKS && (long long)B * N * 8 <= tex.slot_bytes),
              "gemv_res: bad tensor-parallel exchange");
+  if (!ex && pf.bytes == 0 && (dtype == PG_BF16 || dtype == PG_F16) && gemv_stream_wanted(B, N, K))
+    return gemv_stream(out, x, W, R, B, N, K, dtype, (cudaStream_t)stream);
   PG_DISPATCH_DTYPE(dtype, T, {
     PG_REQUIRE(K % Vec<T>::N == 0, "gemv_res: K=%d not vector aligned", K);
     return dispatch_nb(B, [&](auto nb) {

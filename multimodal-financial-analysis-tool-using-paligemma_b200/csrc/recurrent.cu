@@ -113,12 +113,6 @@ delta_prep_kernel(float* __restrict__ rec, const T* __restrict__ proj, int ld, i
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // segs: [n_segs][3] = {state slot, first token row, tokens}; the tokens of a segment are consecutive rows of one
 // sequence in position order.  A segment with 0 tokens is skipped (the list is padded to a fixed length so that a
 // captured launch stays valid).  Shared memory: two buffers of CH records.

@@ -525,3 +525,35 @@ def test_linear_scan_steps_of_four(kind, H, dim, vdim, lens):
         keep = torch.arange(T, device="cuda") != at
         assert torch.equal(out2[keep], out[keep]) and not bool(torch.isfinite(out2[at]).any())
         assert torch.equal(state2[:-1], state[:-1]) and not bool(torch.isfinite(state2[-1, :, :dim]).any())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(4, 8, 8), (7, 1184, 72), (8, 1192, 1024), (9, 2368, 1032), (16, 2376, 2048), (17, 2048, 2048), (32, 1000, 2040),
+                                   (12, 9472, 520), (5, 2048, 16384), (16, 2048, 8200), (1, 2367, 72), (2, 2048, 16384), (3, 1001, 4104)])
+def test_streamed_rows(M, N, K, dtype):
+    """Every SM's share of weight rows: fewer rows than CTAs, shares of 8, 9, 16 and 17 rows (a second group), four groups, columns that
+    end inside a lane's step and behind a chunk; one to three rows of a decode step, features that are no multiple of 8."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    pad = 8 if M > 3 else 0
+    a, w = _randn(g, M, K + pad, dtype=dtype), _randn(g, N, K + pad, std=K ** -0.5, dtype=dtype)
+    b, r = _randn(g, N, dtype=dtype), _randn(g, M, N + pad, dtype=dtype)
+    y = a[:, :K].to(F64) @ w[:, :K].to(F64).T
+    y_b, res = y + b.to(F64), r[:, :N].to(F64)
+    want = {cabi.EPI_NONE: y, cabi.EPI_RES: y + res, cabi.EPI_BIAS: y_b, cabi.EPI_BIAS_RES: y_b + res,
+            cabi.EPI_BIAS_GELU: torch.nn.functional.gelu(y_b, approximate="tanh")}
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for epi, ref in want.items():
+        for f32 in (0, 1) if M > 3 else (0,):
+            out = torch.full((M + 1, N + pad), 7.0, dtype=torch.float32 if f32 else dtype, device="cuda")
+            if M > 3:
+                cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr(), M, N, K, K + pad, K + pad, N + pad,
+                                     N + pad, 0, epi, f32, 2 | cabi.GEMM_W_PARAM, cabi.DTYPE_CODE[dtype], st))
+            elif epi in (cabi.EPI_NONE, cabi.EPI_RES):
+                cabi.check(L.pg_gemv_res(out.data_ptr(), a.data_ptr(), w.data_ptr(), r.data_ptr() if epi == cabi.EPI_RES else None, M, N, K, None,
+                                         cabi.DTYPE_CODE[dtype], st))
+            else:
+                continue
+            # up to three roundings (product, activation, sum) of half a step of the type each, and the fast tanh's 2^-11
+            assert _rel(out[:M, :N], ref) < 1.5 * eps + 2.0 ** -11 and float((out[:M, :N].to(F64) - ref).abs().max()) < 4 * eps * float(ref.abs().max())
+            assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())
