@@ -7,16 +7,19 @@
 // before this launch).  ONE pass over the key tiles:
 //   S(t) = Q K^T (tcgen05.mma, fp32) into one of two TMEM buffers, issued one tile ahead of the softmax;
 //   two threads own a query row, 32 of the tile's keys each (their maxima meet in shared memory):
-//   z = log2(e) (S * scale - slope_h * (i - j)), masked outside 0 <= i - j < window, in fp32; the row's
-//   reference maximum is raised (and O, sum rescaled, after the products that still add to it) only when a tile exceeds it
-//   by more than 2^8; p = exp2(z - m), row sum from the fp32 values, P rounded to the model dtype and stored over the S
+//   z = log2(e) (S * scale - slope_h * (i - j)) - m, masked outside 0 <= i - j < window, in fp32; the row's
+//   reference maximum m is raised (and O, sum rescaled, after the products that still add to it) only when a tile exceeds it
+//   by more than 2^8; p = exp2(z), row sum from the fp32 values, P rounded to the model dtype and stored over the S
 //   columns it came from: O += P V takes P as the TMEM operand and V as an MN-major operand straight from its page.
-// What bounds it: the softmax's instructions and their latencies; the tiles' products and copies run beside them.  Arithmetic is
-// paired (f32x2, the scalar roundings), and two CTAs of eight softmax warps each keep an SM's schedulers fed.  Most tiles lie
-// wholly inside the causal window of all 128 rows and take a loop without masks.  4 prompts of 2048 tokens, 16 heads of 128,
-// window 1024: 557 us in two passes (row maximum first, S computed twice, P through shared memory, masks on every score), 246 in
-// one pass, 219 with the newest pages first, 150 with two threads a row (one: 0.33 instructions a cycle and scheduler),
-// 139 with the long tiles first.
+// What bounds it: the latencies of the softmax's chain (accumulators out of TMEM, the halves' barrier, exponentials, weights into
+// TMEM), which four warps on each of an SM's schedulers hide to 40 % of its issue slots; the tiles' products and copies run
+// beside it.  So its steps are few: the reference is part of the score's constant, so that the usual tile, which does not raise it,
+// subtracts nothing, and distance and scale are two scalar multiply-adds with the key's place as an immediate (in pairs, f32x2, they
+// took as many cycles and registers for every constant twice: 231 multiply-add and 213 integer instructions a warp and tile, now
+// 184 and 141).  Most tiles lie wholly inside the causal window of all 128 rows and take no masks.  4 prompts of 2048 tokens, 16
+// heads of 128, window 1024: 557 us in two passes (row maximum first, S computed twice, P through shared memory, masks on every score),
+// 246 in one pass, 219 with the newest pages first, 150 with two threads a row (one: 0.33 instructions a cycle and
+// scheduler), 139 with the long tiles first, 141 with exact reciprocals, 124 with the score's constant as above.
 // Epilogue: O / sum, times sigmoid(gate), rounded once.  Key width and value width are independent multiples of 64.
 // Extensions (pg_attention_ragged_tc_ex): keep_first > 0 keeps the first keep_first positions visible behind the
 // window: the window's pages are then followed by those that hold them (as far as they lie before the window's first page).
@@ -199,7 +202,8 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const uint32_t t_row = tmem_base + ((uint32_t)(qw * 32) << 16);
     const int i = pos0 + r;                                        // this row's position
     const float slope = (p.slopes ? p.slopes[h] : 0.f) * LOG2E_F, hbias = (p.head_bias ? p.head_bias[h] : 0.f) * LOG2E_F;
-    const int blk0 = p.chunk > 0 ? i / p.chunk * p.chunk : 0;      // first position of this row's block
+    // the first position that this row sees but for kept ones: its window's, and its block's
+    const int first = max(p.chunk > 0 ? i / p.chunk * p.chunk : 0, p.window > 0 ? i - p.window + 1 : 0);
     const int blk_last = p.chunk > 0 ? (pos0 + WQ - 1) / p.chunk * p.chunk : 0;
     float m = -INFINITY, l = 0.f;                                  // m in units of log2
     if (CAP && p.bounded) m = (p.sink ? fmaxf(p.sink[h], 0.f) : 0.f) * LOG2E_F;  // any value near the scores does: they are bounded
@@ -220,26 +224,22 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll
         for (int jj = 0; jj < HK; ++jj) s[jj] = (p.softcap - __fdividef(cap_out, __expf(s[jj] * cap_in) + 1.f)) * LOG2E_F;
       }
-      const float d0 = (float)(j0 - i);                            // exact, and so is d0 + jj = j - i
-      f32x2 dd = pair_of(d0, d0 + 1.f);
+      // slope (j - i) + bias - the row's reference, from its value at the thread's first key
+      const float ref = m == -INFINITY ? 0.f : m;                  // a row that has seen no key yet
+      const float z0 = fmaf(slope, (float)(j0 - i), hbias - ref);
 #pragma unroll
-      for (int jj = 0; jj < HK; jj += 2) {
-        const f32x2 z = fma2(pair_of(slope, slope), dd, pair_of(hbias, hbias)), x = pair_of(s[jj], s[jj + 1]);
-        const float2 y = halves_of(CAP ? add2(x, z) : fma2(x, pair_of(qs2, qs2), z));
-        s[jj] = y.x;
-        s[jj + 1] = y.y;
-        dd = add2(dd, pair_of(2.f, 2.f));
+      for (int jj = 0; jj < HK; ++jj) {
+        const float z = fmaf(slope, (float)jj, z0);
+        s[jj] = CAP ? s[jj] + z : fmaf(s[jj], qs2, z);
       }
       // whole tiles that every row sees need no masks
       const bool full = page0 + WK - 1 <= pos0 && page0 >= blk_last &&
                         (p.window <= 0 || pos0 + WQ - 1 - page0 < p.window || page0 + WK <= p.keep_first);
-      if (!full) {
+      if (!full) {                                                 // visible: first <= j <= i, or a kept first position up to i
+        const unsigned span = (unsigned)(i - first), at = (unsigned)(j0 - first);
+        const int kept = min(p.keep_first, i + 1) - j0;
 #pragma unroll
-        for (int jj = 0; jj < HK; ++jj) {
-          const int j = j0 + jj, back = i - j;
-          const bool vis = back >= 0 && j >= blk0 && (p.window <= 0 || back < p.window || j < p.keep_first);
-          s[jj] = vis ? s[jj] : -INFINITY;
-        }
+        for (int jj = 0; jj < HK; ++jj) s[jj] = (at + jj <= span || jj < kept) ? s[jj] : -INFINITY;
       }
       float top = -INFINITY;
       if (!fixed_max) {
@@ -252,8 +252,8 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       meet();                                                      // both have read their scores: P may take S's columns
       if (!fixed_max) {
         top = fmaxf(top, s_half[t & 1][hf ^ 1][r]);                // the same in both threads, and so is every decision below
-        if (__any_sync(0xffffffffu, top > m + MAX_RAISE)) {          // m == -inf: any visible key raises it
-          const float m_new = fmaxf(m, top);
+        if (__any_sync(0xffffffffu, top > (m == -INFINITY ? -INFINITY : MAX_RAISE))) {   // m == -inf: any visible key raises it
+          const float m_new = fmaxf(m, top + ref);
           if (t > 0) {
             const float corr = m_new == m ? 1.f : exp2_approx(m - m_new);
             l *= corr;
@@ -270,23 +270,22 @@ attention_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             }
           }
           m = m_new;
+          const float up = (m == -INFINITY ? 0.f : m) - ref;
+#pragma unroll
+          for (int jj = 0; jj < HK; ++jj) s[jj] -= up;
         }
       }
       if (sig) {
 #pragma unroll
         for (int jj = 0; jj < HK; ++jj) s[jj] = inverse_of_1_plus(exp2_approx(-s[jj]));   // exp2(+inf) -> weight 0 when masked
       } else {
-        const float ref = m == -INFINITY ? 0.f : m;                // a row that has seen no key yet
-        f32x2 sum[2] = {pair_of(0.f, 0.f), pair_of(0.f, 0.f)};
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int jj = 0; jj < HK; jj += 2) {
-          const float2 x = halves_of(add2(pair_of(s[jj], s[jj + 1]), pair_of(-ref, -ref)));
-          s[jj] = exp2_approx(x.x);
-          s[jj + 1] = exp2_approx(x.y);
-          sum[(jj >> 1) & 1] = add2(sum[(jj >> 1) & 1], pair_of(s[jj], s[jj + 1]));
+        for (int jj = 0; jj < HK; ++jj) {
+          s[jj] = exp2_approx(s[jj]);
+          sum[jj & 3] += s[jj];
         }
-        const float2 a = halves_of(sum[0]), b = halves_of(sum[1]);
-        l += (a.x + a.y) + (b.x + b.y);
+        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       }
       uint32_t pk[HK / 2];
 #pragma unroll
