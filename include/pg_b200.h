@@ -72,12 +72,6 @@ int pg_embed_merge(void* out, const int64_t* ids, const void* emb, const void* i
 /* GemmaRMSNorm.forward (modeling_gemma.py:114-120) */
 int pg_rmsnorm(void* out, const void* x, const void* w, int rows, int D, float eps,
                int dtype, void* stream);
-/* pg_rmsnorm and the projection behind it in one launch, for the few rows of a decode step: C = epilogue(norm(x) W^T), with
- * epilogue PG_EPI_NONE or PG_EPI_GEGLU (W = [gate; up], 2 N rows), the normed rows rounded to the dtype.  norm_w and W are
- * parameters: no preceding launch writes them.  pg_norm_gemm_ok: 1 where it takes the problem. */
-int pg_norm_gemm_ok(int M, int N, int K, int ldx, int ldw, int ldc, int epilogue, int dtype);
-int pg_norm_gemm(void* C, const void* x, const void* norm_w, const void* W, int M, int N, int K, int ldx, int ldw, int ldc,
-                 float eps, int epilogue, int dtype, void* stream);
 /* nn.LayerNorm (modeling_siglip.py:175,177,234) */
 int pg_layernorm(void* out, const void* x, const void* w, const void* b, int rows, int D,
                  float eps, int dtype, void* stream);

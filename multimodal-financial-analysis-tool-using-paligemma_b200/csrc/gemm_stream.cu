@@ -2,16 +2,14 @@
 //
 // What bounds them is the weight stream.  As tiles of 128 weight rows (gemm_tcgen05_skinny.cu) they are 16 to 20, whose K is cut over
 // clusters that occupy 128 of the 148 SMs and meet through distributed shared memory; as rows of their own for one or two warps
-// (gemv.cu) 512 CTAs do not come out even, and each warp's stream is short.  Here every SM takes the same number of weight rows, to
-// within one: [N b / grid, N (b + 1) / grid), in groups of 16 (gated: the gate and up rows of 8 features).  The 8 warps of a CTA split
-// K, 128 columns of every 1024 each; weights go straight from global memory into mma.m16n8k16 B fragments with 16-byte loads (the contraction index is permuted alike for both
+// (gemv.cu) 512 CTAs do not come out even, and each warp's stream is short.  Here every SM takes the same number of weight rows, to within one: [N b / grid, N (b + 1) / grid), in
+// groups of 16.  The 8 warps of a CTA split K, 128 columns of every 1024 each; weights go
+// straight from global memory into mma.m16n8k16 B fragments with 16-byte loads (the contraction index is permuted alike for both
 // operands: lane j of a quad owns 8 consecutive columns of every 32), about 128 KB of them in flight per SM, the first of them
 // requested before the preceding launch has finished.  The tokens are the A operand, copied to shared memory: as a whole where a CTA
 // has several groups, else each lane's own pieces, as many steps ahead as the weights (without that their trip to L2 bounds a step:
 // K 16384, 8 rows 17.8 us, now 13.8).  Up to three rows take fp32 multiply-adds instead of mma.  The warps' partial sums meet in
 // shared memory, in warp order.
-// With the tokens in shared memory their RMS norm can be taken there, by every CTA for itself (pg_norm_gemm): a layer's two norm launches
-// of a few rows are launch and latency, 2.3 us each in the chain of a captured step.
 #include "common.cuh"
 #include "mma_frag.cuh"
 
@@ -28,45 +26,40 @@ struct StreamParams {
   const void* R;
   int M, N, K, lda, ldw, ldc, ldr, out_f32;
   int w_param;   // W is no output of a preceding launch: it may be requested before the dependency wait
-  const void* norm_w;   // x <- x / rms(x) * (1 + norm_w) first
-  float eps;
 };
 
 template <typename T, int EPI>
-__device__ __forceinline__ float stream_epilogue(const StreamParams& p, float s, float u, int m, int n) {
+__device__ __forceinline__ float stream_epilogue(const StreamParams& p, float s, int m, int n) {
   constexpr bool HAS_BIAS = EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES;
   if (HAS_BIAS) s += to_f<T>(reinterpret_cast<const T*>(p.bias)[n]);
   float x = rnd<T>(s);
   if (EPI == PG_EPI_BIAS_GELU) x = rnd<T>(gelu_tanh_fast(x));
-  if (EPI == PG_EPI_GEGLU) x = rnd<T>(rnd<T>(gelu_tanh_fast(x)) * rnd<T>(u));
   if (EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES) x = rnd<T>(x + to_f<T>(reinterpret_cast<const T*>(p.R)[(size_t)m * p.ldr + n]));
   return x;
 }
 
 constexpr int gs_ring(int mh, bool xs) { return !xs && mh == 4 ? 2 : 4; }
 
-// MH: blocks of 8 token rows (1, 2 or 4).  XS: all tokens' columns are in shared memory, otherwise those of RING items are, each
-// lane's pieces copied by itself.  NB: 0, or so many rows by fp32 multiply-adds instead of mma.
-template <typename T, int EPI, int MH, bool XS, int NB, bool NORM>
+// MH: blocks of 8 token rows (1, 2 or 4).  NB: 0, or so many rows by fp32 multiply-adds instead of mma.  XS: all tokens' columns are in shared memory,
+// otherwise those of RING items are, each lane's pieces copied by itself.
+template <typename T, int EPI, int MH, bool XS, int NB>
 __global__ void __launch_bounds__(GS_WARPS * 32, 1)
 gemm_stream_kernel(StreamParams p) {
-  constexpr bool DUAL = EPI == PG_EPI_GEGLU;
-  constexpr int UF = DUAL ? 8 : 16;                   // features of a group; its second 8 weight rows are the up rows or the next features
   constexpr int RING = gs_ring(MH, XS);               // items (a group's chunks, 2 GS_KB loads of a lane) in flight
   constexpr int MG = (MH + 1) / 2;                    // groups of 16 token rows
   constexpr int PART = GS_WARPS * MH * 8 * 16;
-  extern __shared__ __align__(16) uint8_t smem[];     // part [2][warp][MH 8][16] fp32 | x: [M][K + pad] (| norm_w [K]), or [RING][warp][MH 8][128]
+  extern __shared__ __align__(16) uint8_t smem[];     // part [2][warp][MH 8][16] fp32 | x: [M][K + pad], or [RING][warp][MH 8][128]
   float* part = reinterpret_cast<float*>(smem);
   T* xs = reinterpret_cast<T*>(smem + 2 * PART * sizeof(float));
   const int ldx = p.K + GS_PAD;
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, j = lane & 3;
   const int n0 = (int)((long long)p.N * blockIdx.x / gridDim.x), n1 = (int)((long long)p.N * (blockIdx.x + 1) / gridDim.x);
-  const int chunks = (p.K + GS_CHUNK - 1) / GS_CHUNK, items = (n1 - n0 + UF - 1) / UF * chunks;
+  const int chunks = (p.K + GS_CHUNK - 1) / GS_CHUNK, items = (n1 - n0 + 15) / 16 * chunks;
   const int col_w = warp * 32 * GS_KB + j * 8;        // this lane's first column in a chunk
   const T* W = reinterpret_cast<const T*>(p.W) + (size_t)(n0 + r) * p.ldw + col_w;
   const T* A = reinterpret_cast<const T*>(p.A) + (size_t)r * p.lda + col_w;
-  const size_t second = (size_t)(DUAL ? p.N : 8) * p.ldw;
+  const size_t second = (size_t)8 * p.ldw;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   uint4 ring[RING][2][GS_KB];
   int req = 0, req_chunk = 0, req_n = n0;             // the next item to request
@@ -78,18 +71,15 @@ gemm_stream_kernel(StreamParams p) {
     for (int x = 0; x < 2; ++x)
 #pragma unroll
       for (int b = 0; b < GS_KB; ++b) {
-        const bool in = live && col_w + col + 32 * b < p.K && req_n + r + (DUAL ? 0 : 8 * x) < n1;
+        const bool in = live && col_w + col + 32 * b < p.K && req_n + r + 8 * x < n1;
         w[x][b] = in ? ldg_stream(req_row + x * second + col + 32 * b) : zero;
       }
     ++req;
-    if (++req_chunk == chunks) { req_chunk = 0; req_n += UF; req_row += (size_t)UF * p.ldw; }
+    if (++req_chunk == chunks) { req_chunk = 0; req_n += 16; req_row += (size_t)16 * p.ldw; }
   };
   if (!p.w_param) pdl_wait();
 #pragma unroll
   for (int i = 0; i < RING; ++i) request(ring[i]);
-  T* gs = xs + (size_t)p.M * ldx;
-  if (NORM)                                           // a parameter as well
-    for (int c = threadIdx.x; c < p.K / 8; c += GS_WARPS * 32) cp_async16(gs + 8 * c, reinterpret_cast<const T*>(p.norm_w) + 8 * c);
   pdl_wait();                                         // the tokens, the residual and the output belong to the preceding kernels
   // without XS: piece b of a row in a slot; odd rows start 64 bytes on, so that a quarter-warp meets no bank twice
   auto slot = [&](int s, int row, int b) {
@@ -114,26 +104,6 @@ gemm_stream_kernel(StreamParams p) {
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    if (NORM) {                                       // rounded to T as pg_rmsnorm's result
-      for (int row = warp; row < p.M; row += GS_WARPS) {
-        T* xr = xs + (size_t)row * ldx;
-        float ss = 0.f, f[8], g[8];
-        for (int c = lane; c < vecs; c += 32) {
-          unpack<T>(*reinterpret_cast<const uint4*>(xr + 8 * c), f);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
-        }
-        const float inv = rsqrtf(warp_sum(ss) / (float)p.K + p.eps);
-        for (int c = lane; c < vecs; c += 32) {
-          unpack<T>(*reinterpret_cast<const uint4*>(xr + 8 * c), f);
-          unpack<T>(*reinterpret_cast<const uint4*>(gs + 8 * c), g);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = (f[e] * inv) * (1.0f + g[e]);
-          *reinterpret_cast<uint4*>(xr + 8 * c) = pack<T>(f);
-        }
-      }
-      __syncthreads();
-    }
   } else {
 #pragma unroll
     for (int i = 0; i < RING; ++i) copy(i);
@@ -226,32 +196,29 @@ gemm_stream_kernel(StreamParams p) {
           }
       }
       __syncthreads();                                // the other buffer's readers are through as well
-      for (int i = threadIdx.x; i < p.M * UF; i += GS_WARPS * 32) {
-        const int m = i / UF, f = i % UF;
+      for (int i = threadIdx.x; i < p.M * 16; i += GS_WARPS * 32) {
+        const int m = i / 16, f = i % 16;
         if (n + f >= n1) continue;
         const float* at = part + (size_t)buf * PART + m * 16 + f;
-        float s = 0.f, u = 0.f;
+        float s = 0.f;
 #pragma unroll
-        for (int w = 0; w < GS_WARPS; ++w) {
-          s += at[w * (MH * 8 * 16)];
-          if (DUAL) u += at[w * (MH * 8 * 16) + 8];
-        }
-        const float v = stream_epilogue<T, EPI>(p, s, u, m, n + f);
+        for (int w = 0; w < GS_WARPS; ++w) s += at[w * (MH * 8 * 16)];
+        const float v = stream_epilogue<T, EPI>(p, s, m, n + f);
         if (p.out_f32) reinterpret_cast<float*>(p.C)[(size_t)m * p.ldc + n + f] = v;
         else reinterpret_cast<T*>(p.C)[(size_t)m * p.ldc + n + f] = from_f<T>(v);
       }
       buf ^= 1;
       chunk = 0;
-      n += UF;
+      n += 16;
     }
   }
 }
 
-template <typename T, int EPI, int MH, bool XS, int NB = 0, bool NORM = false>
+template <typename T, int EPI, int MH, bool XS, int NB = 0>
 static int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
-  const size_t x = XS ? (size_t)p.M * (p.K + GS_PAD) + (NORM ? p.K : 0) : (size_t)gs_ring(MH, XS) * MH * 8 * GS_CHUNK;
+  const size_t x = XS ? (size_t)p.M * (p.K + GS_PAD) : (size_t)gs_ring(MH, XS) * MH * 8 * GS_CHUNK;
   const size_t smem = sizeof(float) * 2 * GS_WARPS * MH * 8 * 16 + sizeof(T) * x;
-  return launch_pdl("gemm_stream", gemm_stream_kernel<T, EPI, MH, XS, NB, NORM>, dim3(grid), dim3(GS_WARPS * 32), smem, st, p);
+  return launch_pdl("gemm_stream", gemm_stream_kernel<T, EPI, MH, XS, NB>, dim3(grid), dim3(GS_WARPS * 32), smem, st, p);
 }
 
 static int stream_grid(int N) { return cdiv(N, 8) < 148 ? cdiv(N, 8) : 148; }
@@ -295,14 +262,14 @@ static int gemv_stream_t(const StreamParams& p, int grid, cudaStream_t st) {
 bool gemv_stream_wanted(int B, int N, int K) { return B >= 1 && B <= 3 && K % 8 == 0 && cdiv(N, stream_grid(N)) <= 16; }
 
 int gemv_stream(void* out, const void* x, const void* W, const void* R, int B, int N, int K, int dtype, cudaStream_t st) {
-  const StreamParams p = {out, x, W, nullptr, R, B, N, K, K, K, N, N, 0, 1, nullptr, 0.f};
+  const StreamParams p = {out, x, W, nullptr, R, B, N, K, K, K, N, N, 0, 1};
   return dtype == PG_BF16 ? gemv_stream_t<bf16>(p, stream_grid(N), st) : gemv_stream_t<f16>(p, stream_grid(N), st);
 }
 
 // 16-bit operands, N, K and leading dimensions multiples of 8, 16-byte aligned rows (checked by the caller)
 int gemm_stream(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda, int ldw, int ldc,
                 int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st) {
-  const StreamParams p = {C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, out_f32, w_param ? 1 : 0, nullptr, 0.f};
+  const StreamParams p = {C, A, W, bias, R, M, N, K, lda, ldw, ldc, ldr, out_f32, w_param ? 1 : 0};
 #define PG_ST(E) return dtype == PG_BF16 ? launch_stream_pick<bf16, E>(p, st) : launch_stream_pick<f16, E>(p, st)
   switch (epi) {
     case PG_EPI_NONE: PG_ST(PG_EPI_NONE);
@@ -316,34 +283,4 @@ int gemm_stream(void* C, const void* A, const void* W, const void* bias, const v
   return PG_ERR_INVALID;
 }
 
-template <typename T, int EPI>
-static int norm_stream_t(const StreamParams& p, cudaStream_t st) {
-  const int grid = stream_grid(p.N);
-  static const int m1 = env_int("PG_M1", 1);
-  return p.M <= 8 && (m1 || EPI != PG_EPI_GEGLU) ? launch_stream<T, EPI, 1, true, 0, true>(p, grid, st) : launch_stream<T, EPI, 2, true, 0, true>(p, grid, st);
-}
-
 }  // namespace pg
-
-using namespace pg;
-
-// The norm in the projection pays where the projection streams as fast here as elsewhere: up to 16 rows, gated up to NORM_GATED_MAX.
-extern "C" int pg_norm_gemm_ok(int M, int N, int K, int ldx, int ldw, int ldc, int epilogue, int dtype) {
-  if ((dtype != PG_BF16 && dtype != PG_F16) || (epilogue != PG_EPI_NONE && epilogue != PG_EPI_GEGLU)) return 0;
-  static const int gm = env_int("PG_NORM_GATED", 8);
-  static const int nm = env_int("PG_NORM_MAX", 16);
-  if (M < 4 || M > (epilogue == PG_EPI_GEGLU ? gm : nm) || N <= 0 || K <= 0 || N % 8 || K % 8 || ldx % 8 || ldw % 8) return 0;
-  return 2 * ((size_t)M * (K + GS_PAD) + K) <= 136 * 1024;
-}
-
-extern "C" int pg_norm_gemm(void* C, const void* x, const void* norm_w, const void* W, int M, int N, int K, int ldx, int ldw, int ldc,
-                            float eps, int epilogue, int dtype, void* stream) {
-  PG_REQUIRE(pg_norm_gemm_ok(M, N, K, ldx, ldw, ldc, epilogue, dtype), "norm_gemm: unsupported problem (M=%d N=%d K=%d epilogue %d dtype %d)",
-             M, N, K, epilogue, dtype);
-  PG_REQUIRE(C && x && norm_w && W && ldx >= K && ldw >= K && ldc >= N, "norm_gemm: bad arguments");
-  PG_REQUIRE((((uintptr_t)x | (uintptr_t)norm_w | (uintptr_t)W) & 15) == 0, "norm_gemm: operands must be 16-byte aligned");
-  const StreamParams p = {C, x, W, nullptr, nullptr, M, N, K, ldx, ldw, ldc, 0, 0, 1, norm_w, eps};
-  cudaStream_t st = (cudaStream_t)stream;
-  if (epilogue == PG_EPI_GEGLU) return dtype == PG_BF16 ? norm_stream_t<bf16, PG_EPI_GEGLU>(p, st) : norm_stream_t<f16, PG_EPI_GEGLU>(p, st);
-  return dtype == PG_BF16 ? norm_stream_t<bf16, PG_EPI_NONE>(p, st) : norm_stream_t<f16, PG_EPI_NONE>(p, st);
-}

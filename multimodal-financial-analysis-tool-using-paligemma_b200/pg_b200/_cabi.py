@@ -36,8 +36,6 @@ SIGNATURES = {
     "pg_launch_count": [],
     "pg_embed_merge": [_vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _ll, _i, _f, _f, _vp, _i, _vp],
     "pg_rmsnorm": [_vp, _vp, _vp, _i, _i, _f, _i, _vp],
-    "pg_norm_gemm_ok": [_i] * 8,
-    "pg_norm_gemm": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp],
     "pg_layernorm": [_vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp],
     "pg_im2col": [_vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "pg_resample_u8": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],

@@ -810,20 +810,6 @@ class DecodeState:
         cabi.check(cabi.lib().pg_tp_push(ptr(self.part), self.B * d.D, exref(fab.x(index, 2 * d.L + 2)), cabi.stream()),
                    "tp_push")
 
-    def _norm_gemm_gen(self, out, x, w_norm, w_mat, epi):
-        """RMSNorm and the projection behind it: one launch for a few rows, else two."""
-        eng, d, L, st, dt = self.eng, self.eng.dims, cabi.lib(), cabi.stream(), self.eng.dt
-        N = out.shape[1]
-        if L.pg_norm_gemm_ok(self.B, N, d.D, x.stride(0), w_mat.stride(0), out.stride(0), epi, dt) and eng.gemm_impl in (0, 2):
-            cabi.check(L.pg_norm_gemm(ptr(out), ptr(x), ptr(w_norm), ptr(w_mat), self.B, N, d.D, x.stride(0), w_mat.stride(0), out.stride(0),
-                                      d.eps, epi, dt, st), "norm_gemm")
-            yield
-            return
-        cabi.check(L.pg_rmsnorm(ptr(self.bn), ptr(x), ptr(w_norm), self.B, d.D, d.eps, dt, st), "rmsnorm")
-        yield
-        eng._gemm(out, self.bn, w_mat, None, None, epi)
-        yield
-
     def layer_batched_gen(self, li: int, kv: PagedKV, fab, first: bool):
         """Decoder layer `li` of the tensor-core step (same stream conventions as layer_gemv_gen)."""
         eng, d, L, st = self.eng, self.eng.dims, cabi.lib(), cabi.stream()
@@ -837,11 +823,11 @@ class DecodeState:
         kp, vp = eng.k_pool[li], eng.v_pool[li]
         if fab is not None and not first:
             self._reduce_norm(fab, n, x, x2, w["ln1"], 2 * li)          # x = x2 + sum(down partials of layer li-1)
-            yield
-            eng._gemm(self.bqkv, n, w["qkv"])
-            yield
         else:
-            yield from self._norm_gemm_gen(self.bqkv, x, w["ln1"], w["qkv"], cabi.EPI_NONE)
+            cabi.check(L.pg_rmsnorm(ptr(n), ptr(x), ptr(w["ln1"]), B, d.D, d.eps, dt, st), "rmsnorm")
+        yield
+        eng._gemm(self.bqkv, n, w["qkv"])
+        yield
         cabi.check(L.pg_rope_append(ptr(self.q), ptr(self.bqkv), ptr(eng.inv_freq), ptr(self.pos), ptr(kp), ptr(vp),
                                     ptr(kv.page_table), kv.max_pages, eng.page_size, ptr(kv.kv_len), B, 1, nq, d.nkv,
                                     d.hd, d.max_pos, dt, st), "rope_append")
@@ -856,14 +842,15 @@ class DecodeState:
             yield
             self._reduce_norm(fab, n, x2, x, w["ln2"], 2 * li + 1)      # x2 = x + sum(o_proj partials)
             yield
-            eng._gemm(self.g, n, w["gu"], None, None, cabi.EPI_GEGLU)
-            yield
         else:
             eng._gemm(x2, self.att, w["o"], None, x if tp.rank == 0 else None, res_epi)
             yield
             if tp.active:
                 yield ("all_reduce", x2)
-            yield from self._norm_gemm_gen(self.g, x2, w["ln2"], w["gu"], cabi.EPI_GEGLU)
+            cabi.check(L.pg_rmsnorm(ptr(n), ptr(x2), ptr(w["ln2"]), B, d.D, d.eps, dt, st), "rmsnorm")
+            yield
+        eng._gemm(self.g, n, w["gu"], None, None, cabi.EPI_GEGLU)
+        yield
         if fab is not None:
             self._partial_push(fab, self.g, w["down"], 2 * li + 2)
             yield

@@ -557,26 +557,3 @@ def test_streamed_rows(M, N, K, dtype):
             # up to three roundings (product, activation, sum) of half a step of the type each, and the fast tanh's 2^-11
             assert _rel(out[:M, :N], ref) < 1.5 * eps + 2.0 ** -11 and float((out[:M, :N].to(F64) - ref).abs().max()) < 4 * eps * float(ref.abs().max())
             assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())
-
-
-@pytest.mark.parametrize("dtype", TYPES)
-@pytest.mark.parametrize("gated,M,N,K", [(0, 4, 2560, 2048), (0, 9, 1000, 72), (0, 16, 8, 1032), (1, 4, 16384, 2048), (1, 8, 1192, 520), (1, 7, 8, 8)])
-def test_norm_in_the_projection(gated, M, N, K, dtype):
-    """The normed rows are rounded as the norm's own launch rounds them, then multiplied: float64 products of those rows."""
-    cabi, L, st = _cabi()
-    g = torch.Generator(device="cuda").manual_seed(M + N + K)
-    x = _randn(g, M, K + 8, dtype=dtype) * torch.logspace(-2, 2, M, device="cuda", dtype=dtype)[:, None]
-    nw, w = _randn(g, K, std=0.2, dtype=dtype), _randn(g, (1 + gated) * N, K + 8, std=K ** -0.5, dtype=dtype)
-    out = torch.full((M + 1, N + 8), 7.0, dtype=dtype, device="cuda")
-    epi = cabi.EPI_GEGLU if gated else cabi.EPI_NONE
-    assert L.pg_norm_gemm_ok(M, N, K, K + 8, K + 8, N + 8, epi, cabi.DTYPE_CODE[dtype]) == 1
-    cabi.check(L.pg_norm_gemm(out.data_ptr(), x.data_ptr(), nw.data_ptr(), w.data_ptr(), M, N, K, K + 8, K + 8, N + 8, 1e-6, epi,
-                              cabi.DTYPE_CODE[dtype], st))
-    h = x[:, :K].to(F64)
-    h = (h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * (1.0 + nw.to(F64))).to(dtype)
-    z = h.to(F64) @ w[:, :K].to(F64).T
-    want = _gelu(z[:, :N]) * z[:, N:] if gated else z
-    # roundings as in test_gated_pairs; a normed value on the edge of two may round to the other
-    assert _rel(out[:M, :N], want) < _tol(dtype, 5e-3, gated)
-    assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())
-    assert L.pg_norm_gemm_ok(17, N, K, K + 8, K + 8, N + 8, epi, cabi.DTYPE_CODE[dtype]) == 0
