@@ -261,9 +261,16 @@ static int gemv_stream_t(const StreamParams& p, int grid, cudaStream_t st) {
   return launch_stream<T, PG_EPI_NONE, 1, false, 3>(p, grid, st);
 }
 
-// Against two warps a row (gemv_res_kernel), K 16384, N 2048: 13.8 and 12.7 us for one row, 15.6 and 14.2 for two, 27.7 and 16.8 for
-// three; K 2048 6.5 and 6.5, in the chain of a captured step 0.4 us a layer less.
-bool gemv_stream_wanted(int B, int N, int K) { return B >= 1 && B <= 3 && K % 8 == 0 && cdiv(N, stream_grid(N)) <= 16; }
+// Against one warp a row, from K 8192 on two (gemv_res_kernel), weights out of HBM, us there and here.  A short row leaves the warps of
+// a CTA without columns (N = 2048: one row of K 512 2.0 and 2.6, of K 2048 3.5 and 3.3, 4096 6.2 and 4.8; with up to 64 CTAs earlier:
+// N 512, K 768 2.0 and 1.7; three rows, whose products bound a warp, from K 1024: 3.4 and 3.1).  From K 8192 on two and three rows of
+// few features come out faster there (three rows of K 16384: N 1024 14.4 and 15.7, N 2048, more CTAs than find room at once, 28.0
+// and 17.4; two rows: N 256 10.5 and 11.4, N 768 12.6 and 11.7; one row of N 2048 14.2 and 12.3).
+bool gemv_stream_wanted(int B, int N, int K) {
+  if (B < 1 || B > 3 || K % 8 || cdiv(N, stream_grid(N)) > 16) return false;
+  if (K >= 8192) return B == 1 || N >= (B == 2 ? 768 : 148 * 3 * 4);
+  return K >= 2048 || (B == 3 && K >= 1024) || (N <= 512 && K >= 640);
+}
 
 int gemv_stream(void* out, const void* x, const void* W, const void* R, int B, int N, int K, int dtype, cudaStream_t st) {
   const StreamParams p = {out, x, W, nullptr, R, B, N, K, K, K, N, N, 0, 1};

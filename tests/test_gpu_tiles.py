@@ -529,7 +529,8 @@ def test_linear_scan_steps_of_four(kind, H, dim, vdim, lens):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K", [(4, 8, 8), (7, 1184, 72), (8, 1192, 1024), (9, 2368, 1032), (16, 2376, 2048), (17, 2048, 2048), (32, 1000, 2040),
-                                   (12, 9472, 520), (5, 2048, 16384), (16, 2048, 8200), (1, 2367, 72), (2, 2048, 16384), (3, 1001, 4104)])
+                                   (12, 9472, 520), (5, 2048, 16384), (16, 2048, 8200), (1, 2367, 72), (2, 2048, 16384), (3, 1001, 4104),
+                                   (1, 2367, 2056), (2, 504, 648), (2, 776, 8200), (3, 8, 1032), (3, 1784, 8192), (7, 2376, 512), (16, 9472, 4096)])
 def test_streamed_rows(M, N, K, dtype):
     """Every SM's share of weight rows: fewer rows than CTAs, shares of 8, 9, 16 and 17 rows (a second group), four groups, columns that
     end inside a lane's step and behind a chunk; one to three rows of a decode step, features that are no multiple of 8."""
