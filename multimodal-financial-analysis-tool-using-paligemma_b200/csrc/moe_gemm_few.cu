@@ -192,9 +192,13 @@ static int launch_moe_few(const MoeFewParams& p, cudaStream_t st) {
   return launch_pdl("moe_gemm_few", moe_gemm_few_kernel<T, DUAL>, dim3(units < 148 ? (unsigned)units : 148u), dim3(MF_WARPS * 32), smem, st, p);
 }
 
-// The rows' columns leave the loads in flight their 90 KB of L1 up to 136 KB (K 2048: 24 rows 45 and 26 us against 67 and 42, 32
-// rows of all experts 51 and 29 against 56 and 29, 48 rows 91 and 49 against 56 and 29).
-bool moe_gemm_few_wanted(int n_pairs, int K) { return n_pairs <= MF_PAIRS && 2 * (size_t)n_pairs * (K + MF_PAD) <= 136 * 1024; }
+// The rows' columns leave the loads in flight their 90 KB of L1 up to 136 KB, where a row's two products share them, else 128 KB (us,
+// weights out of HBM, the tiles and this.  K 2048: gate/up of 24 rows 67 and 45, 32 rows on 8 experts 35 and 29, 48 rows 56 and 91;
+// down of 24 rows 40 and 26, 32 rows on 8 experts 16.9 and 17.9; K 1024: gate/up of 64 rows on 2 experts, whose weights are read
+// twice each, 20 and 11, down on 16 experts 12.0 and 12.5).
+bool moe_gemm_few_wanted(int n_pairs, int K, bool dual) {
+  return n_pairs <= MF_PAIRS && 2 * (size_t)n_pairs * (K + MF_PAD) <= (dual ? 136 : 128) * 1024;
+}
 
 // 16-bit operands, N and K multiples of 8, 16-byte aligned rows (checked by the caller)
 int moe_gemm_few(void* out, int ldo, const void* A, int lda, const void* W, const int32_t* offsets, int n_pairs, int n_experts, int N,

@@ -434,7 +434,7 @@ static int launch_moe_pair(const CUtensorMap& ma, const CUtensorMap& mw, const M
 
 }  // namespace tc
 
-bool moe_gemm_few_wanted(int n_pairs, int K);
+bool moe_gemm_few_wanted(int n_pairs, int K, bool dual);
 int moe_gemm_few(void* out, int ldo, const void* A, int lda, const void* W, const int32_t* offsets, int n_pairs, int n_experts, int N,
                  int K, int act, float limit, int dtype, cudaStream_t st);
 
@@ -453,7 +453,7 @@ int moe_gemm_tc(void* out, int ldo, const void* A, int lda, const int32_t* row_m
   PG_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)out % 16) == 0,
              "moe_gemm_tc: operands must be 16-byte aligned");
   const bool bf = dtype == PG_BF16;
-  if (moe_gemm_few_wanted(n_pairs, K))
+  if (moe_gemm_few_wanted(n_pairs, K, swiglu != 0))
     return moe_gemm_few(out, ldo, A, lda, W, offsets, n_pairs, n_experts, N, K, act, limit, dtype, st);
   const int rows_per_expert = swiglu ? 2 * N : N;
   CUtensorMap ma, mw;
