@@ -386,6 +386,8 @@ def batched_rows(eng, cfg, quick: bool, world: int, local: int, which=(3, 4)):
                       "bytes_per_rank_per_step": step_bytes,
                       "hbm_frac_per_rank": step_bytes / (total_ms / n * 1e-3) / 1e9 / measured_peaks()["hbm"],
                       "distinct_tokens_sampled": int(toks.unique().numel()),
+                      # random weights draw every id; the engine feeds an image token of its own back as a zero row
+                      "image_tokens_drawn": int((toks == eng.dims.image_token_index).sum()),
                       "parallelism": f"tp{world}" if world > 1 else "single GPU",
                       "sampling": "greedy" if sample is None else f"temperature {sample[0]}, top_p {sample[1]} (pg_top_p_sample)"}
     return rows

@@ -68,6 +68,13 @@ int pg_embed_merge(void* out, const int64_t* ids, const void* emb, const void* i
                    int n_tokens, int D, int64_t vocab, int64_t image_token_id, int64_t pad_id,
                    int n_img_rows, float img_div, float normalizer, int* err_flag,
                    int dtype, void* stream);
+/* The same, with what a caller needs to name the error: info (device-visible, 3 values, may be NULL) receives the first bad token's
+ * id, its place t and *step (device int, may be NULL: -1) before a clear *err_flag is set.  drawn: the ids were picked by
+ * pg_argmax / pg_top_p_sample, not given by a caller; an image token without an image row is then a zero row and no error. */
+int pg_embed_merge_ex(void* out, const int64_t* ids, const void* emb, const void* img_feats,
+                      int n_tokens, int D, int64_t vocab, int64_t image_token_id, int64_t pad_id,
+                      int n_img_rows, float img_div, float normalizer, int* err_flag, int drawn,
+                      const int32_t* step, long long* info, int dtype, void* stream);
 
 /* GemmaRMSNorm.forward (modeling_gemma.py:114-120) */
 int pg_rmsnorm(void* out, const void* x, const void* w, int rows, int D, float eps,

@@ -45,28 +45,50 @@ int check_launch(const char* what) {
 
 // ------------------------------------------------------------------ embed + merge
 // One CTA per token.  The k-th image token (row-major over the flattened ids) takes image row k
-// (masked_scatter order, modeling_gemma.py:498).
+// (masked_scatter order, modeling_gemma.py:498).  The first token that is an error is described in info (id, t, the step's
+// number or -1) before the flag is set.
 template <typename T>
 __global__ void embed_merge_kernel(T* __restrict__ out, const int64_t* __restrict__ ids,
                                    const T* __restrict__ emb, const T* __restrict__ img,
                                    int n_tokens, int D, int64_t vocab, int64_t img_id, int64_t pad_id,
-                                   int n_img_rows, float img_div, float normalizer, int* err_flag) {
+                                   int n_img_rows, float img_div, float normalizer, int* err_flag, int drawn,
+                                   const int32_t* __restrict__ step, long long* info) {
   pdl_launch_dependents();  // a tensor-core kernel launched next may start its prologue now
   constexpr int V = Vec<T>::N;
   __shared__ float red[32];
   const int t = blockIdx.x;
   const int64_t id = ids[t];
   const T* src = nullptr;
-  bool is_img = false;
+  bool is_img = false, bad = false;
   if (id == img_id) {
     float cnt = 0.f;
     for (int i = threadIdx.x; i < t; i += blockDim.x) cnt += (ids[i] == img_id) ? 1.f : 0.f;
     int k = (int)(block_sum(cnt, red) + 0.5f);
     if (img != nullptr && k < n_img_rows) { src = img + (size_t)k * D; is_img = true; }
-    else if (err_flag && threadIdx.x == 0) *err_flag = 1;
+    else bad = drawn == 0;
   } else if (id != pad_id) {
     if (id >= 0 && id < vocab) src = emb + (size_t)id * D;
-    else if (err_flag && threadIdx.x == 0) *err_flag = 1;
+    else bad = true;
+  }
+  if (bad && err_flag) {                                 // rare: is an earlier token the one to name?
+    float outside = 0.f, images = 0.f;
+    for (int i = threadIdx.x; i < t; i += blockDim.x) {
+      const int64_t x = ids[i];
+      if (x == img_id) images += 1.f;
+      else if (x != pad_id && (x < 0 || x >= vocab)) outside += 1.f;
+    }
+    outside = block_sum(outside, red);
+    images = drawn ? 0.f : block_sum(images, red);
+    const int rows = img != nullptr ? n_img_rows : 0;
+    if (threadIdx.x == 0 && outside == 0.f && images <= (float)rows) {
+      if (info && *(volatile int*)err_flag == 0) {
+        info[0] = id;
+        info[1] = t;
+        info[2] = step ? *step : -1;
+        __threadfence_system();
+      }
+      *(volatile int*)err_flag = 1;
+    }
   }
   T* dst = out + (size_t)t * D;
   for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
@@ -494,12 +516,20 @@ int pg_set_next_prefetch(const void* ptr, long long bytes) {
 int pg_embed_merge(void* out, const int64_t* ids, const void* emb, const void* img_feats, int n_tokens,
                    int D, int64_t vocab, int64_t image_token_id, int64_t pad_id, int n_img_rows,
                    float img_div, float normalizer, int* err_flag, int dtype, void* stream) {
+  return pg_embed_merge_ex(out, ids, emb, img_feats, n_tokens, D, vocab, image_token_id, pad_id, n_img_rows, img_div, normalizer,
+                           err_flag, 0, nullptr, nullptr, dtype, stream);
+}
+
+int pg_embed_merge_ex(void* out, const int64_t* ids, const void* emb, const void* img_feats, int n_tokens,
+                      int D, int64_t vocab, int64_t image_token_id, int64_t pad_id, int n_img_rows,
+                      float img_div, float normalizer, int* err_flag, int drawn, const int32_t* step,
+                      long long* info, int dtype, void* stream) {
   if (n_tokens <= 0) return PG_OK;
   PG_DISPATCH_DTYPE(dtype, T, {
     PG_REQUIRE(D % Vec<T>::N == 0, "embed_merge: D=%d not a multiple of %d", D, Vec<T>::N);
     embed_merge_kernel<T><<<n_tokens, 256, 0, (cudaStream_t)stream>>>(
         (T*)out, ids, (const T*)emb, (const T*)img_feats, n_tokens, D, vocab, image_token_id, pad_id,
-        n_img_rows, img_div, normalizer, err_flag);
+        n_img_rows, img_div, normalizer, err_flag, drawn, step, info);
   });
   return check_launch("embed_merge");
 }

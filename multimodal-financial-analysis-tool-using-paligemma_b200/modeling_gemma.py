@@ -366,11 +366,11 @@ class PaliGemmaForConditionalGeneration(nn.Module):
         img = None if image_features is None or image_features.numel() == 0 else \
             image_features.reshape(-1, d.D).to(eng.dtype).contiguous()
         out = torch.empty((B * q, d.D), dtype=eng.dtype, device=eng.device)
-        cabi.check(cabi.lib().pg_embed_merge(out.data_ptr(), ids.data_ptr(), eng.emb.data_ptr(),
-                                             None if img is None else img.data_ptr(), B * q, d.D, d.V,
-                                             d.image_token_index, d.pad_token_id, 0 if img is None else img.shape[0],
-                                             eng.img_div, 1.0, eng.err_flag.data_ptr(), eng.dt, cabi.stream()),
-                   "embed_merge")
+        cabi.check(cabi.lib().pg_embed_merge_ex(out.data_ptr(), ids.data_ptr(), eng.emb.data_ptr(),
+                                                None if img is None else img.data_ptr(), B * q, d.D, d.V,
+                                                d.image_token_index, d.pad_token_id, 0 if img is None else img.shape[0],
+                                                eng.img_div, 1.0, eng.err_flag.data_ptr(), 0, None, eng.err_info.data_ptr(),
+                                                eng.dt, cabi.stream()), "embed_merge")
         cached = 0 if kv_cache is None else kv_cache.num_items()
         mask = torch.zeros((B, 1, q, cached + q), dtype=eng.dtype, device=eng.device)
         if cached > 0:
@@ -441,7 +441,7 @@ class PaliGemmaForConditionalGeneration(nn.Module):
             ds.ids.copy_(input_ids.reshape(-1), non_blocking=True)
             ds.pos.fill_(position)
         ds.want_full_logits = True       # tensor parallel: forward() returns the whole vocabulary row
-        ds.run_steps(paged, 1)
+        ds.run_steps(paged, 1, given=True)
         # a fresh tensor per call, as the reference returns (callers keep earlier steps' logits)
         return ds.logits.clone().view(paged.batch, 1, -1)
 

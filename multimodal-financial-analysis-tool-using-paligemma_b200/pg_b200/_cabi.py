@@ -35,6 +35,7 @@ SIGNATURES = {
     "pg_abi_version": [],
     "pg_launch_count": [],
     "pg_embed_merge": [_vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _ll, _i, _f, _f, _vp, _i, _vp],
+    "pg_embed_merge_ex": [_vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _ll, _i, _f, _f, _vp, _i, _vp, _vp, _i, _vp],
     "pg_rmsnorm": [_vp, _vp, _vp, _i, _i, _f, _i, _vp],
     "pg_layernorm": [_vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp],
     "pg_im2col": [_vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],

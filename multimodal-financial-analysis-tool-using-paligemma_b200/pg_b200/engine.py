@@ -184,6 +184,7 @@ class PaliGemmaEngine(PagePool):
         # pinned, device-mapped: kernels store to it only when they meet a bad id, the host reads it without a sync
         self.err_flag = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._err_np = self.err_flag.numpy()
+        self.err_info = torch.zeros(3, dtype=torch.int64).pin_memory()   # of the token that set it: id, place, step or -1
         self.max_splits = 32
         self._decode_states: Dict[tuple, "DecodeState"] = {}
         # scratch for the split-K prompt GEMMs (fp32 partials; 512 tokens x 2F features is the largest user)
@@ -478,9 +479,10 @@ class PaliGemmaEngine(PagePool):
             img = None if image_features is None or image_features.numel() == 0 else \
                 image_features.reshape(-1, d.D).to(self.dtype).contiguous()
             x = self._new(T, d.D)
-            cabi.check(L.pg_embed_merge(ptr(x), ptr(ids), ptr(self.emb), ptr(img), T, d.D, d.V,
-                                        d.image_token_index, d.pad_token_id, 0 if img is None else img.shape[0],
-                                        self.img_div, self.normalizer, ptr(self.err_flag), self.dt, st), "embed_merge")
+            cabi.check(L.pg_embed_merge_ex(ptr(x), ptr(ids), ptr(self.emb), ptr(img), T, d.D, d.V,
+                                           d.image_token_index, d.pad_token_id, 0 if img is None else img.shape[0],
+                                           self.img_div, self.normalizer, ptr(self.err_flag), 0, None, ptr(self.err_info),
+                                           self.dt, st), "embed_merge")
             nq, tp = self.nq_l, self.tp
             res_epi = cabi.EPI_RES if tp.rank == 0 else cabi.EPI_NONE   # the residual enters the sum once
             nqkv = (nq + 2 * d.nkv) * d.hd
@@ -568,7 +570,8 @@ class PaliGemmaEngine(PagePool):
 
     def check_errors(self, sync: bool = False) -> None:
         """Raise if a kernel flagged an id problem (image token without image rows, id out of range): the reference
-        raises from masked_scatter / embedding for the same inputs.  The flag lives in pinned host memory, so the
+        raises from masked_scatter / embedding for the same inputs.  An image token that the engine drew itself in a decode
+        loop is none: it is fed back as a zero row (the reference's loop feeds the first image feature).  The flag lives in pinned host memory, so the
         check itself never synchronises; callers that are at a synchronisation point anyway (prefill forward, end of
         generate(), the scheduler's per-chunk read-back) pass sync=True to see this call's own kernels, the per-token
         decode path reports at the next call (like the deferred mask check)."""
@@ -579,7 +582,10 @@ class PaliGemmaEngine(PagePool):
             self._err_np[0] = 0
             if lost:
                 raise RuntimeError("tensor-parallel exchange timed out waiting for a peer rank")
-            raise RuntimeError("input_ids held an image token with no image feature left, or an id outside the vocabulary")
+            token, place, step = self.err_info.tolist()
+            where = f"place {place} of the flattened input_ids" if step < 0 else f"row {place} of decode step {step}"
+            raise RuntimeError(f"input_ids held an image token with no image feature left, or an id outside the vocabulary: "
+                               f"token {token} at {where}")
 
     # ------------------------------------------------------------------ decode (q_len == 1)
     def decode_state(self, batch: int) -> "DecodeState":
@@ -636,15 +642,23 @@ class DecodeState:
             cabi.check(cabi.lib().pg_set_next_prefetch(t.data_ptr() + off, n), "set_next_prefetch")
 
     # one decode step: kernels only, no host sync, capturable
-    def launch_step(self, kv: PagedKV, sample: Optional[tuple] = None, advance: bool = True) -> None:
-        self.eng.tp.run(self.step_gen(kv, sample, advance))
+    def launch_step(self, kv: PagedKV, sample: Optional[tuple] = None, advance: bool = True, given: bool = False) -> None:
+        self.eng.tp.run(self.step_gen(kv, sample, advance, given))
 
-    def step_gen(self, kv: PagedKV, sample: Optional[tuple] = None, advance: bool = True):
-        """The step as a launch generator (one `yield` per kernel; see dist.TP.run / dist.LockstepGroup)."""
+    def step_gen(self, kv: PagedKV, sample: Optional[tuple] = None, advance: bool = True, given: bool = False):
+        """The step as a launch generator (one `yield` per kernel; see dist.TP.run / dist.LockstepGroup).  given: the ids come
+        from the caller, not from the step before."""
         if self.B >= self.eng.batched_min:
-            yield from self._step_batched_gen(kv, sample, advance)
+            yield from self._step_batched_gen(kv, sample, advance, given)
         else:
-            yield from self._step_gemv_gen(kv, sample, advance)
+            yield from self._step_gemv_gen(kv, sample, advance, given)
+
+    def _embed(self, given: bool) -> None:
+        eng, d = self.eng, self.eng.dims
+        cabi.check(cabi.lib().pg_embed_merge_ex(ptr(self.x), ptr(self.ids), ptr(eng.emb), None, self.B, d.D, d.V,
+                                                d.image_token_index, d.pad_token_id, 0, eng.img_div, eng.normalizer,
+                                                ptr(eng.err_flag), 0 if given else 1, ptr(self.step), ptr(eng.err_info), eng.dt,
+                                                cabi.stream()), "embed")
 
     def _fabric(self):
         """The peer-memory exchange when this step can use it (rows fit one slot, one GEMV sub-batch)."""
@@ -723,7 +737,7 @@ class DecodeState:
         if tp.active:
             yield ("all_reduce", x)
 
-    def _step_gemv_gen(self, kv: PagedKV, sample: Optional[tuple], advance: bool):
+    def _step_gemv_gen(self, kv: PagedKV, sample: Optional[tuple], advance: bool, given: bool):
         eng, d, L, st = self.eng, self.eng.dims, cabi.lib(), cabi.stream()
         B, dt, MB = self.B, self.eng.dt, cabi.MAX_DECODE_BATCH
         tp = eng.tp
@@ -732,9 +746,7 @@ class DecodeState:
         if fab is not None:
             cabi.check(L.pg_tp_begin_step(ptr(fab.epoch), st), "tp_begin_step")
             yield
-        cabi.check(L.pg_embed_merge(ptr(self.x), ptr(self.ids), ptr(eng.emb), None, B, d.D, d.V,
-                                    d.image_token_index, d.pad_token_id, 0, eng.img_div, eng.normalizer,
-                                    ptr(eng.err_flag), dt, st), "embed")
+        self._embed(given)
         yield
         for li in range(len(eng.t_layers)):
             yield from self.layer_gemv_gen(li, kv, fab, first=li == 0)
@@ -860,7 +872,7 @@ class DecodeState:
             if tp.active:
                 yield ("all_reduce", x)
 
-    def _step_batched_gen(self, kv: PagedKV, sample: Optional[tuple], advance: bool):
+    def _step_batched_gen(self, kv: PagedKV, sample: Optional[tuple], advance: bool, given: bool):
         """Decode step for batches above the GEMV tile (32 sequences, for one): the projections run as
         skinny GEMMs (tcgen05 for 16-bit dtypes: weights stream through TMA once for the whole batch), attention
         stays the cluster kernel.  Same rounding points as the GEMV path; capturable (static buffers).
@@ -875,9 +887,7 @@ class DecodeState:
         if fab is not None:
             cabi.check(L.pg_tp_begin_step(ptr(fab.epoch), st), "tp_begin_step")
             yield
-        cabi.check(L.pg_embed_merge(ptr(self.x), ptr(self.ids), ptr(eng.emb), None, B, d.D, d.V,
-                                    d.image_token_index, d.pad_token_id, 0, eng.img_div, eng.normalizer,
-                                    ptr(eng.err_flag), dt, st), "embed")
+        self._embed(given)
         yield
         for li in range(len(eng.t_layers)):
             yield from self.layer_batched_gen(li, kv, fab, first=li == 0)
@@ -911,16 +921,18 @@ class DecodeState:
         self.step.zero_()
         self.keys.zero_()
 
-    def run_steps(self, kv: PagedKV, n_steps: int, sample: Optional[tuple] = None, use_graph: bool = True) -> None:
-        """Advance n_steps tokens entirely on the device (tokens land in self.history)."""
+    def run_steps(self, kv: PagedKV, n_steps: int, sample: Optional[tuple] = None, use_graph: bool = True,
+                  given: bool = False) -> None:
+        """Advance n_steps tokens entirely on the device (tokens land in self.history).  given: the step's ids come from a
+        caller, so that an image token among them is an error."""
         if n_steps > self.max_hist:
             raise ValueError("too many steps for the history buffer")
         kv.reserve(kv.length + n_steps)
         if not use_graph:
             for _ in range(n_steps):
-                self.launch_step(kv, sample)
+                self.launch_step(kv, sample, given=given)
         else:
-            key = (kv.page_table.data_ptr(), kv.kv_len.data_ptr(), kv.max_pages, sample, self.want_full_logits)
+            key = (kv.page_table.data_ptr(), kv.kv_len.data_ptr(), kv.max_pages, sample, self.want_full_logits) + (("given",) if given else ())
             g = self.graphs.get(key)
             if g is None:
                 # warm up on a side stream (lazy module loading, smem attributes), undo its effects
@@ -928,13 +940,13 @@ class DecodeState:
                 s = torch.cuda.Stream()
                 s.wait_stream(torch.cuda.current_stream())
                 with torch.cuda.stream(s):
-                    self.launch_step(kv, sample)
+                    self.launch_step(kv, sample, given=given)
                 torch.cuda.current_stream().wait_stream(s)
                 for t, v in zip((self.ids, self.pos, self.step, self.keys, kv.kv_len, self.history[:, :1]), saved):
                     t.copy_(v)
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
-                    self.launch_step(kv, sample)
+                    self.launch_step(kv, sample, given=given)
                 for t, v in zip((self.ids, self.pos, self.step, self.keys, kv.kv_len, self.history[:, :1]), saved):
                     t.copy_(v)
                 if len(self.graphs) > 8:

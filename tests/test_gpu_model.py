@@ -337,3 +337,41 @@ def test_decode_batch_larger_than_kernel_tile(golden_dir):
     assert tuple(out.shape) == (10, 4) and int(out.min()) >= 0 and int(out.max()) < cfg["vocab_size"]
     again = model.generate(ids.cuda(), pix.cuda(), 4, do_sample=True, temperature=0.8, top_p=0.9, seed=11).cpu()
     assert out.tolist() == again.tolist()          # counter-based RNG: same seed, same draw
+
+
+@pytest.mark.parametrize("name,dtype,batch", [("tiny", torch.float32, 2), ("small", torch.bfloat16, 5)])
+def test_image_token_behind_the_prompt(name, dtype, batch):
+    """An image token that a caller feeds to a cached step is an error that names it; one that the decode loop drew itself is
+    fed back as a zero row.  An id outside the vocabulary is an error in both."""
+    model, cfg = build_model(name, dtype)
+    eng, image = model._engine_ready(), cfg["image_token_index"]
+    ids, pix = synth.synth_prompt_ids(cfg, batch=batch).cuda(), synth.synth_pixels(cfg, batch=batch).to(dtype).cuda()
+    mask, cache = torch.ones_like(ids), MG.KVCache()
+    with torch.no_grad():
+        model(input_ids=ids, pixel_values=pix, attention_mask=mask, kv_cache=cache)
+        for row, token in ((1, image), (0, cfg["vocab_size"])):
+            mask = torch.cat([mask, torch.ones_like(mask[:, :1])], 1)
+            bad = torch.full((batch, 1), 5, dtype=torch.int64, device="cuda")
+            bad[row] = token
+            model(input_ids=bad, pixel_values=None, attention_mask=mask, kv_cache=cache)
+            torch.cuda.synchronize()
+            with pytest.raises(RuntimeError, match=f"token {token} at row {row} of decode step"):
+                eng.check_errors()
+        with pytest.raises(RuntimeError, match=f"token {image} at place 0 of the flattened input_ids"):
+            model(input_ids=ids, pixel_values=None, attention_mask=torch.ones_like(ids), kv_cache=MG.KVCache())
+        kv = eng.new_kv(batch)
+        try:
+            feats = eng.encode_images(pix)
+            eng.text_forward(ids, feats, kv, logits="last")
+            ds, first = eng.decode_state(batch), torch.full((batch,), 5, dtype=torch.int64, device="cuda")
+            first[batch - 1] = image
+            ds.bind(kv, first, position=ids.shape[1] + 1)
+            ds.run_steps(kv, 2)
+            eng.check_errors(sync=True)
+            assert bool(torch.isfinite(ds.logits).all())
+            ds.ids[0] = -3
+            ds.run_steps(kv, 1)
+            with pytest.raises(RuntimeError, match="token -3 at row 0 of decode step 2"):
+                eng.check_errors(sync=True)
+        finally:
+            kv.release()

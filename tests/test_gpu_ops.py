@@ -86,6 +86,38 @@ def test_embed_merge(dtype):
     assert int(err.item()) == 1
 
 
+@pytest.mark.parametrize("drawn", [0, 1])
+@pytest.mark.parametrize("ids,rows,named", [([7, 40, 3, 41, 41], 1, (41, 4)), ([41, 2, 5, 9, 40], 0, (41, 0)), ([2, 40, 41, -7, 99], 0, (41, 2)),
+                                            ([5, 3, -1, 41, 60], 1, (-1, 2))])
+def test_embed_names_the_first_bad_token(ids, rows, named, drawn):
+    """Id, place and step of the first token that is an error: image tokens (41) behind the last image row, ids outside the
+    vocabulary of 50; tokens the engine drew itself may be image tokens."""
+    D, V, img_id = 64, 50, 41
+    emb, img, x = gen(V, D, dtype=torch.float32), gen(1, D, seed=3, dtype=torch.float32), torch.tensor(ids)
+    out = torch.full((len(ids), D), 7.0, device="cuda")
+    err, info = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((3,), -9, dtype=torch.int64, device="cuda")
+    step = torch.full((1,), 23, dtype=torch.int32, device="cuda")
+
+    def embed(step):
+        cabi.check(cabi.lib().pg_embed_merge_ex(out.data_ptr(), dev(x).data_ptr(), dev(emb).data_ptr(), dev(img).data_ptr() if rows else None,
+                                                len(ids), D, V, img_id, 0, rows, 8.0, 2.0, err.data_ptr(), drawn, cabi.ptr(step),
+                                                info.data_ptr(), 0, st()))
+
+    embed(step)
+    left = [t for t, i in enumerate(ids) if not 0 <= i < V or (i == img_id and ids[:t].count(img_id) >= rows)]
+    errors = [t for t in left if not (drawn and ids[t] == img_id)]
+    assert named[1] == left[0] and int(err) == (1 if errors else 0)
+    assert info.tolist() == ([ids[errors[0]], errors[0], 23] if errors else [-9, -9, -9])
+    assert bool((out[left] == 0).all())
+    if errors:                                       # a flag that nobody has read keeps its token
+        info[0] = -5
+        embed(None)
+        assert info.tolist()[0] == -5
+        err.zero_()
+        embed(None)
+        assert info.tolist() == [ids[errors[0]], errors[0], -1]
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_im2col_patch_embed(dtype):
     B, C, S, p, Hv = 2, 3, 56, 14, 144
