@@ -440,7 +440,9 @@ int pg_glu_clamped(void* out, const void* gate_up, int rows, int F, float limit,
  * projection's columns at q_col0 / k_col0 / v_col0 (heads x dim, heads x dim, heads x vdim):
  *   S <- decay[h] S + k v^T;  o = S^T q.   segs as for pg_delta_rule; out fp32 [n_tokens, heads * vdim].
  * pg_lightning_prep writes rec: pg_lightning_record_floats(n_tokens, heads, dim, vdim) floats (the fp32 activations,
- * one packed record [q | k | v] per (token, head)); pg_lightning_attention runs the recurrence over them. */
+ * one packed record [q | k | v] per (token, head)); pg_lightning_attention runs the recurrence over them, in steps of four tokens
+ * (a segment of up to three token by token): where a sequence is cut into segments decides the last bits of state and outputs,
+ * within 1e-6 of a float64 recurrence either way. */
 long long pg_lightning_record_floats(int n_tokens, int heads, int dim, int vdim);
 int pg_lightning_prep(float* rec, const void* proj, int ld, int q_col0, int k_col0, int v_col0, int n_tokens, int heads,
                       int dim, int vdim, int dtype, void* stream);
@@ -676,6 +678,11 @@ int pg_gla_prep(float* rec, const void* proj, int ld, int q_col0, int k_col0, in
                 const void* b2, float q_scale, float inv_tau, int n_tokens, int heads, int dim, int vdim, int dtype, void* stream);
 int pg_gla_attention(float* out, float* state, const float* rec, const int32_t* segs, int n_segs, int heads, int dim, int vdim,
                      void* stream);
+/* pg_lightning_attention_ex, or with per_channel pg_gla_attention (decay and skip NULL), that says when one of its bounded waits
+ * ran out: *err_flag (device-visible int, may be NULL) becomes 2.  The segment's outputs and state are then NaN, with a flag or
+ * without.  no_wait: every wait counts as run out (segments of up to three tokens wait for nothing). */
+int pg_linear_scan(float* out, float* state, const float* rec, const float* decay, const float* skip, int per_channel,
+                   const int32_t* segs, int n_segs, int heads, int dim, int vdim, int no_wait, int* err_flag, void* stream);
 int pg_conv_qk_append(void* q_out, const void* proj, int ld, int q_col0, int n_heads, int k_col0, int n_kv_heads, int dim,
                       const void* conv, int taps, const float* state, int state_len, int state_cols, const void* q_w,
                       const void* k_w, float eps, const float* freq, int rot_dims, void* k_pool, void* v_pool,

@@ -617,7 +617,7 @@ template <int DMAX, int DK, int COLS>           // COLS: value columns per threa
 __global__ void __launch_bounds__((4 + SCAN_AUX) * 32, 2)
 lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ rec,
                  const float* __restrict__ decay, const float* __restrict__ skip, const int32_t* __restrict__ segs,
-                 int heads, int dim, int vdim, int dp, int vp, int vec) {
+                 int heads, int dim, int vdim, int dp, int vp, int vec, int no_wait, int* __restrict__ err_flag) {
   constexpr int AHEAD = SCAN_AHEAD<DMAX, DK>, SCAN_RING = AHEAD * SCAN_AUX;
   constexpr int RG = scan_lanes(DMAX), NG = DMAX / (4 * RG), TB = SCAN_TB;   // RG lanes share COLS value columns, NG groups of four rows each
   extern __shared__ __align__(16) float sh[];         // [ring][TB][q DMAX | k DMAX | (decays DMAX) | v VT | (decay)] | [ring][side]
@@ -666,13 +666,14 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
     for (int f = 0; f < (CD ? F4 : 1); ++f)
 #pragma unroll
       for (int e = 0; e < 4; ++e) carry[f][e] = 0.f;
+    bool lost = no_wait != 0;                           // the state's warps have stopped
     auto request = [&](int it) {
-      if (it < steps) {
+      // the state's warps have read the slot (in a first round nobody has to)
+      if (it >= SCAN_RING && it < steps) lost = !scan_wait(empty(it % SCAN_RING), (it / SCAN_RING - 1) & 1, &fail);
+      if (it < steps && !lost) {
         const int s = it % SCAN_RING, nv = min(TB, n - it * TB);
         const float* src = head_rec + (size_t)it * TB * tok_step;
         float* dst = sh + (size_t)s * TB * RSZ;
-        // the state's warps have read the slot (in a first round nobody has to); a wait that ran out shows at this warp's next one
-        if (it >= SCAN_RING) scan_wait(empty(s), (it / SCAN_RING - 1) & 1, &fail);
 #pragma unroll
         for (int t = 0; t < TB; ++t) {
           const float* p = src + t * tok_step;
@@ -699,7 +700,7 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
     for (int it = first; it < steps; it += SCAN_AUX) {
       cp_async_wait<AHEAD - 2>();
       __syncwarp();
-      if (*(volatile int*)&fail) break;
+      if (lost) break;
       const int s = it % SCAN_RING, nv = min(TB, n - it * TB);
       float* base = sh + (size_t)s * TB * RSZ;
       float* sd = side + (size_t)s * SCAN_SIDE;
@@ -829,6 +830,15 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
       if (lane == 0) tc::mbar_arrive(ready(s));
       request(it + (AHEAD - 1) * SCAN_AUX);
     }
+    // A wait that ran out, here or in a state's warp (which then waited for one of these two): the flag and the outputs show it.
+    // These warps tell it: values kept for it in the state's loop cost 6 of 380 us at 4 x 2048 tokens.
+    cp_async_wait<0>();
+    if (__any_sync(0xffffffffu, lost || *(volatile int*)&fail)) {
+      if (lane == 0 && err_flag) *err_flag = 2;
+      float* o = out + ((size_t)row0 * heads + h) * vdim + j0;
+      for (int t = 0; t < n; ++t, o += (size_t)heads * vdim)
+        for (int c = lane; c < min(VT, vdim - j0); c += 32) o[c] = __int_as_float(0x7fffffff);
+    }
     return;
   }
 
@@ -852,10 +862,11 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
   const int sum0 = rg * PER / REP, my_t = sum0 / COLS, my_c = sum0 % COLS;
   float* orow = out + ((size_t)row0 + my_t) * heads * vdim + (size_t)h * vdim + j + my_c;
   const size_t ostep = (size_t)TB * heads * vdim;
-  bool ok = true;
-  for (int it = 0; it < steps; ++it, orow += ostep) {
+  const int last = no_wait ? 0 : steps;
+  int it = 0;
+  for (; it < last; ++it, orow += ostep) {
     const int s = it % SCAN_RING;
-    if (!scan_wait(ready(s), (it / SCAN_RING) & 1, &fail)) { ok = false; break; }
+    if (!scan_wait(ready(s), (it / SCAN_RING) & 1, &fail)) break;
     const float* r0 = sh + (size_t)s * TB * RSZ;
     const float* sd = side + (size_t)s * SCAN_SIDE;
     // what the step's tokens read from the state before it
@@ -940,8 +951,9 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(empty(s));
   }
-  if (!ok) {                                          // a wait ran out: the state shows it
+  if (it < steps) {                                   // a wait ran out: the state shows it, and the warps that prepare steps are told
     const float nan = __int_as_float(0x7fffffff);
+    if (lane == 0) *(volatile int*)&fail = 1;
 #pragma unroll
     for (int c = 0; c < COLS; ++c)
 #pragma unroll
@@ -952,7 +964,7 @@ lightning_kernel(float* __restrict__ out, float* __restrict__ state, const float
 
 template <int DMAX, int COLS>
 static int launch_scan_cols(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
-                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+                            const int32_t* segs, int n_segs, int heads, int dim, int vdim, int no_wait, int* err, cudaStream_t st) {
   const int dp = (dim + 3) / 4 * 4, vp = (vdim + 3) / 4 * 4;
   // value columns per CTA: those of four warps, of fewer while the CTAs do not fill the SMs or the columns are fewer
   constexpr int WARP_COLS = 32 / scan_lanes(DMAX) * COLS;
@@ -974,20 +986,20 @@ static int launch_scan_cols(float* out, float* state, const float* rec, const fl
   }
   const int vec = COLS == 1 || (vdim % COLS == 0 && (uintptr_t)state % 16 == 0);
   kern<<<dim3(n_segs, heads, cdiv(vdim, vt)), dim3((nw + SCAN_AUX) * 32), smem, st>>>(out, state, rec, decay, skip, segs, heads, dim, vdim,
-                                                                                        dp, vp, vec);
+                                                                                        dp, vp, vec, no_wait, err);
   return check_launch("lightning");
 }
 
 template <int DMAX>
 static int launch_scan(float* out, float* state, const float* rec, const float* decay, const float* skip, int dk,
-                       const int32_t* segs, int n_segs, int heads, int dim, int vdim, cudaStream_t st) {
+                       const int32_t* segs, int n_segs, int heads, int dim, int vdim, int no_wait, int* err, cudaStream_t st) {
   // Value columns per thread: more of them share a token's reads of q and k, but are fewer warps.  By the warps of the one-column
   // form; 512 tokens, us with one, two and four: 128 channels, 1024 columns 49, 60, 92; 4096 98, 76, 92; 8192 193, 113, 107;
   // 64 channels, 4096 72, 58, 55; 256 channels (twice the lanes a column), 2048 113, 84, 91; 4096 220, 126, 117.
   const long long warps = (long long)n_segs * heads * vdim * scan_lanes(DMAX) / 32;
-  if (warps >= 1536) return launch_scan_cols<DMAX, 4>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
-  if (warps >= 768) return launch_scan_cols<DMAX, 2>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
-  return launch_scan_cols<DMAX, 1>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, st);
+  if (warps >= 1536) return launch_scan_cols<DMAX, 4>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, no_wait, err, st);
+  if (warps >= 768) return launch_scan_cols<DMAX, 2>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, no_wait, err, st);
+  return launch_scan_cols<DMAX, 1>(out, state, rec, decay, skip, dk, segs, n_segs, heads, dim, vdim, no_wait, err, st);
 }
 
 template <int DMAX, int CH>
@@ -1108,27 +1120,34 @@ extern "C" int pg_lightning_attention(float* out, float* state, const float* rec
 }
 
 static int lightning_any(float* out, float* state, const float* rec, const float* decay, const float* skip, int td,
-                         const int32_t* segs, int n_segs, int heads, int dim, int vdim, void* stream) {
+                         const int32_t* segs, int n_segs, int heads, int dim, int vdim, int no_wait, int* err, void* stream) {
   if (n_segs <= 0) return PG_OK;
   PG_REQUIRE(out && state && rec && segs, "lightning_attention: bad arguments");
   PG_REQUIRE(dim > 0 && dim <= 256 && vdim > 0, "lightning_attention: key size %d (1..256), value size %d", dim, vdim);
   cudaStream_t st = (cudaStream_t)stream;
   // lanes per value column: a thread keeps DMAX / RG rows of the state
-  if (dim <= 32) return launch_scan<32>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  if (dim <= 64) return launch_scan<64>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  if (dim <= 128) return launch_scan<128>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
-  return launch_scan<256>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, st);
+  if (dim <= 32) return launch_scan<32>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, no_wait, err, st);
+  if (dim <= 64) return launch_scan<64>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, no_wait, err, st);
+  if (dim <= 128) return launch_scan<128>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, no_wait, err, st);
+  return launch_scan<256>(out, state, rec, decay, skip, td, segs, n_segs, heads, dim, vdim, no_wait, err, st);
 }
 
 extern "C" int pg_lightning_attention_ex(float* out, float* state, const float* rec, const float* decay, const float* skip,
                                          const int32_t* segs, int n_segs, int heads, int dim, int vdim, void* stream) {
   // no constant decay: the records carry one per token
-  return lightning_any(out, state, rec, decay, skip, decay ? DECAY_HEAD : DECAY_TOKEN, segs, n_segs, heads, dim, vdim, stream);
+  return lightning_any(out, state, rec, decay, skip, decay ? DECAY_HEAD : DECAY_TOKEN, segs, n_segs, heads, dim, vdim, 0, nullptr, stream);
 }
 
 extern "C" int pg_gla_attention(float* out, float* state, const float* rec, const int32_t* segs, int n_segs, int heads, int dim,
                                 int vdim, void* stream) {
-  return lightning_any(out, state, rec, nullptr, nullptr, DECAY_CHANNEL, segs, n_segs, heads, dim, vdim, stream);
+  return lightning_any(out, state, rec, nullptr, nullptr, DECAY_CHANNEL, segs, n_segs, heads, dim, vdim, 0, nullptr, stream);
+}
+
+extern "C" int pg_linear_scan(float* out, float* state, const float* rec, const float* decay, const float* skip, int per_channel,
+                              const int32_t* segs, int n_segs, int heads, int dim, int vdim, int no_wait, int* err_flag, void* stream) {
+  PG_REQUIRE(!per_channel || (!decay && !skip), "linear_scan: a decay per channel lies in the records and goes without a direct term");
+  return lightning_any(out, state, rec, decay, skip, per_channel ? DECAY_CHANNEL : (decay ? DECAY_HEAD : DECAY_TOKEN), segs, n_segs,
+                       heads, dim, vdim, no_wait, err_flag, stream);
 }
 
 extern "C" long long pg_gla_record_floats(int n_tokens, int heads, int dim, int vdim) {

@@ -145,6 +145,7 @@ SIGNATURES = {
     "pg_gla_record_floats": [_i, _i, _i, _i],
     "pg_gla_prep": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _f, _i, _i, _i, _i, _i, _vp],
     "pg_gla_attention": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "pg_linear_scan": [_vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "pg_conv_qk_append": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _i, _i, _vp,
                           _vp, _i, _i, _vp],
     "pg_lru_conv": [_vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _i, _i, _i, _vp],

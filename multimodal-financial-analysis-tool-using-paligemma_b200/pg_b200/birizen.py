@@ -238,8 +238,8 @@ class BirizenEngine(LatentAttentionMixin, RaggedEngine):
             cabi.check(L.pg_lightning_prep(ptr(rec), ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], T, a.heads, a.dim,
                                            a.vdim, self.dt, st), "lightning_prep")
         with tm("lightning"):
-            cabi.check(L.pg_lightning_attention(ptr(o), ptr(kv.state.layers[ri]), ptr(rec), ptr(w["decay"]), ptr(inp.segs),
-                                                inp.n_segs, a.heads, a.dim, a.vdim, st), "lightning_attention")
+            cabi.check(L.pg_linear_scan(ptr(o), ptr(kv.state.layers[ri]), ptr(rec), ptr(w["decay"]), None, 0, ptr(inp.segs),
+                                        inp.n_segs, a.heads, a.dim, a.vdim, 0, ptr(self.err_flag), st), "lightning_attention")
         att = self._new(T, nv)
         with tm("headnorm_gate"):       # one RMS over all heads of the token: a single "head" of heads * vdim columns
             cabi.check(L.pg_headnorm_gate(ptr(att), nv, ptr(o), ptr(w["onorm"]), ptr(proj[:, at["g"]:]), proj.stride(0), T, 1,

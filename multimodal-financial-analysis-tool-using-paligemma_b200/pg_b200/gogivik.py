@@ -307,8 +307,8 @@ class GogivikEngine(LatentAttentionMixin, RaggedEngine):
                                                 inp.n_segs, a.channels, a.taps, self.dt, st), "time_conv_state")
         y = self._new(T, a.inner, dtype=torch.float32)
         with tm("ssm_scan"):
-            cabi.check(L.pg_lightning_attention_ex(ptr(y), ptr(kv.state.layers[("ssm", li)]), ptr(rec), None, ptr(w["skip"]),
-                                                   ptr(inp.segs), inp.n_segs, a.heads, a.state, a.vdim, st), "ssm_scan")
+            cabi.check(L.pg_linear_scan(ptr(y), ptr(kv.state.layers[("ssm", li)]), ptr(rec), None, ptr(w["skip"]), 0, ptr(inp.segs),
+                                        inp.n_segs, a.heads, a.state, a.vdim, 0, ptr(self.err_flag), st), "ssm_scan")
         g = self._new(T, a.inner)
         with tm("gate_groupnorm"):
             cabi.check(L.pg_gate_groupnorm(ptr(g), a.inner, ptr(y), ptr(proj), proj.stride(0), ptr(w["gnorm"]), T, a.inner,

@@ -334,8 +334,8 @@ class MutiraxEngine(LatentAttentionMixin, RaggedEngine):
                                      ptr(w["a2_b"]), a.dim ** -0.5, 1.0 / a.tau, T, a.heads, a.dim, a.vdim, self.dt, st), "gla_prep")
         o = self._new(T, nv, dtype=torch.float32)
         with tm("gla"):
-            cabi.check(L.pg_gla_attention(ptr(o), ptr(kv.state.layers[("gla", ri)]), ptr(rec), ptr(inp.segs), inp.n_segs, a.heads,
-                                          a.dim, a.vdim, st), "gla_attention")
+            cabi.check(L.pg_linear_scan(ptr(o), ptr(kv.state.layers[("gla", ri)]), ptr(rec), None, None, 1, ptr(inp.segs), inp.n_segs,
+                                        a.heads, a.dim, a.vdim, 0, ptr(self.err_flag), st), "gla_attention")
         g = self._new(T, nv)
         with tm("headnorm_gate"):
             cabi.check(L.pg_headnorm_gate_ex(ptr(g), nv, ptr(o), ptr(w["onorm"]), ptr(proj[:, at["g"]:]), proj.stride(0), 1, T,

@@ -389,7 +389,7 @@ class RaggedEngine(PagePool):
         """Recurrent state of `slots` sequences (scheduler.SlotState), None for designs without any."""
         return None
 
-    _ERR_TEXT = {2: "a tensor-core kernel gave up waiting on its pipeline (its results are invalid)"}
+    _ERR_TEXT = {2: "a kernel gave up waiting on its pipeline (its results are invalid)"}
 
     def check_errors(self, sync: bool = False) -> None:
         if sync:

@@ -284,8 +284,8 @@ class RanesunEngine(RaggedEngine):
                                            a.vdim, self.dt, st), "retention_prep")
         o = self._new(T, nv, dtype=torch.float32)
         with tm("retention"):
-            cabi.check(L.pg_lightning_attention(ptr(o), ptr(kv.state.layers[ri]), ptr(rec), ptr(w["decay"]), ptr(inp.segs),
-                                                inp.n_segs, a.heads, a.dim, a.vdim, st), "retention")
+            cabi.check(L.pg_linear_scan(ptr(o), ptr(kv.state.layers[ri]), ptr(rec), ptr(w["decay"]), None, 0, ptr(inp.segs),
+                                        inp.n_segs, a.heads, a.dim, a.vdim, 0, ptr(self.err_flag), st), "retention")
         g = self._new(T, nv)
         with tm("headnorm_gate"):
             cabi.check(L.pg_headnorm_gate_ex(ptr(g), nv, ptr(o), None, ptr(proj[:, at["g"]:]), proj.stride(0), 1, T, a.heads,

@@ -527,6 +527,44 @@ def test_linear_scan_steps_of_four(kind, H, dim, vdim, lens):
         assert torch.equal(state2[:-1], state[:-1]) and not bool(torch.isfinite(state2[-1, :, :dim]).any())
 
 
+@pytest.mark.parametrize("per_channel", [0, 1])
+@pytest.mark.parametrize("H,dim,vdim,lens", [(2, 32, 20, [40, 3, 9]), (3, 128, 36, [100, 4, 1]), (16, 64, 128, [5, 2, 70, 33])])
+def test_linear_scan_waits_that_run_out(H, dim, vdim, lens, per_channel):
+    """Waits that count as run out: the flag is set, outputs and states of the segments that wait are NaN, shorter segments have
+    their results; nothing is written outside the segments, and the next call is whole again."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    S, T, dp, vp, nq = len(lens), sum(lens), dim, -(-vdim // 4) * 4, 3 if per_channel else 2
+    rec = torch.rand(T, H, nq * dp + vp, device="cuda", generator=g) * 0.9
+    decay = None if per_channel else torch.linspace(0.5, 0.99, H, device="cuda")
+    first = [sum(lens[:b]) for b in range(S)]
+    segs = torch.tensor([[b, first[b], lens[b]] for b in range(S)], dtype=torch.int32, device="cuda")
+    start = torch.randn(S + 1, H, dim, vdim, device="cuda", generator=g)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def scan(no_wait, flag):
+        out, state = torch.full((T + 1, H, vdim), 7.0, device="cuda"), start.clone()
+        cabi.check(L.pg_linear_scan(out.data_ptr(), state.data_ptr(), rec.data_ptr(), cabi.ptr(decay), None, per_channel, segs.data_ptr(), S, H,
+                                    dim, vdim, no_wait, cabi.ptr(flag), st))
+        torch.cuda.synchronize()
+        return out, state
+
+    out, state = scan(0, err)
+    assert int(err) == 0 and bool(torch.isfinite(out).all()) and bool(torch.isfinite(state).all())
+    for flag in (None, err):
+        lost, gone = scan(1, flag)
+        for b in range(S):
+            rows = slice(first[b], first[b] + lens[b])
+            if lens[b] < 4:
+                assert torch.equal(lost[rows], out[rows]) and torch.equal(gone[b], state[b])
+            else:
+                assert bool(torch.isnan(lost[rows]).all()) and bool(torch.isnan(gone[b]).all())
+        assert bool((lost[T] == 7).all()) and torch.equal(gone[S], start[S])
+    assert int(err) == 2
+    again, state2 = scan(0, None)
+    assert torch.equal(again, out) and torch.equal(state2, state)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K", [(4, 8, 8), (7, 1184, 72), (8, 1192, 1024), (9, 2368, 1032), (16, 2376, 2048), (17, 2048, 2048), (32, 1000, 2040),
                                    (12, 9472, 520), (5, 2048, 16384), (16, 2048, 8200), (1, 2367, 72), (2, 2048, 16384), (3, 1001, 4104),
