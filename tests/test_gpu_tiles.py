@@ -424,10 +424,16 @@ def test_window_prompts(dim, vdim, H, G, window, dtype):
     assert bool((out[T] == 0).all())
 
 
+def _scan_columns(seqs, heads, dim, vdim):
+    """Value columns per thread: by the warps of the one-column form, with 4, 8 or 16 lanes a column."""
+    warps = seqs * heads * vdim * (4 if dim <= 32 else 8 if dim <= 128 else 16) / 32
+    return 4 if warps >= 1536 else 2 if warps >= 768 else 1
+
+
 @pytest.mark.parametrize("dim,vdim", [(20, 128), (32, 136), (64, 130), (100, 131), (128, 256), (200, 132), (256, 128)])
 @pytest.mark.parametrize("per_channel", [0, 1])
 def test_linear_scan_alone_and_in_a_batch(dim, vdim, per_channel):
-    """One value column per thread for a few sequences, two for many: the same sums in the same order, to the bit."""
+    """One or two value columns per thread for a sequence alone, four for the batch: the same sums in the same order, to the bit."""
     cabi, L, st = _cabi()
     g = torch.Generator(device="cuda").manual_seed(dim + vdim)
     H, lens = 16, [70, 1, 3, 16, 33, 8]
@@ -454,9 +460,7 @@ def test_linear_scan_alone_and_in_a_batch(dim, vdim, per_channel):
         return out, state
 
     out, state = scan([[b, first[b], lens[b]] for b in range(S)], start.clone())
-    # two columns from 1536 warps of the one-column form on (64 channels: 3072; up to 32: never); 8 lanes a column, above 128 channels 16
-    lanes = 16 if dim > 128 else 8
-    assert dim <= 32 or S * H * vdim * lanes >= 32 * (1536 if dim > 64 else 3072) > H * vdim * lanes
+    assert _scan_columns(S, H, dim, vdim) == 4 > _scan_columns(1, H, dim, vdim)
     for b in range(S):
         rows = slice(first[b], first[b] + lens[b])
         o1, s1 = scan([[b, first[b], lens[b]]], start.clone())
@@ -525,6 +529,51 @@ def test_linear_scan_steps_of_four(kind, H, dim, vdim, lens):
         keep = torch.arange(T, device="cuda") != at
         assert torch.equal(out2[keep], out[keep]) and not bool(torch.isfinite(out2[at]).any())
         assert torch.equal(state2[:-1], state[:-1]) and not bool(torch.isfinite(state2[-1, :, :dim]).any())
+
+
+@pytest.mark.parametrize("kind", ["head", "token", "channel"])
+@pytest.mark.parametrize("dim", [24, 60, 100, 200])
+@pytest.mark.parametrize("columns,vdim", [(1, 131), (2, 131), (2, 132), (4, 130), (4, 132)])
+def test_linear_scan_value_columns(columns, vdim, dim, kind):
+    """Every form (value columns per thread, key width, kind of decay), whole and partial groups of columns: to the bit what a
+    sequence gives alone, and a float64 recurrence."""
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim + columns)
+    H, n, dp, vp = 8, 10, -(-dim // 4) * 4, -(-vdim // 4) * 4
+    S = columns * (4 if dim <= 32 else 2 if dim <= 128 else 1)
+    assert _scan_columns(S, H, dim, vdim) == columns and _scan_columns(1, H, dim, vdim) == 1
+    nq, tail = (3, 0) if kind == "channel" else (2, 4 if kind == "token" else 0)
+    q, k, v = (torch.randn(S * n, H, w, device="cuda", generator=g) for w in (dim, dim, vdim))
+    by_head = torch.linspace(0.5, 0.99, H, device="cuda")
+    wide = {"head": 1, "token": 1, "channel": dim}[kind]
+    a = by_head.view(1, H, 1).expand(S * n, H, 1) if kind == "head" else torch.rand(S * n, H, wide, device="cuda", generator=g)
+    rec = torch.zeros(S * n, H, nq * dp + vp + tail, device="cuda")
+    rec[:, :, :dim], rec[:, :, dp:dp + dim], rec[:, :, nq * dp:nq * dp + vdim] = q, k, v
+    if kind == "channel":
+        rec[:, :, 2 * dp:2 * dp + dim] = a
+    if kind == "token":
+        rec[:, :, nq * dp + vp] = a[:, :, 0]
+    start = torch.randn(S, H, dim, vdim, device="cuda", generator=g)
+
+    def scan(seqs):
+        out, state = torch.full((S * n, H, vdim), 7.0, device="cuda"), start.clone()
+        segs = torch.tensor([[b, b * n, n] for b in seqs], dtype=torch.int32, device="cuda")
+        cabi.check(L.pg_linear_scan(out.data_ptr(), state.data_ptr(), rec.data_ptr(), by_head.data_ptr() if kind == "head" else None, None,
+                                    1 if kind == "channel" else 0, segs.data_ptr(), len(seqs), H, dim, vdim, 0, None, st))
+        torch.cuda.synchronize()
+        return out, state
+
+    out, state = scan(list(range(S)))
+    x, want = start.to(F64), []
+    q64, k64, v64, a64 = (z.to(F64).view(S, n, H, -1) for z in (q, k, v, a.contiguous()))
+    for t in range(n):
+        x = a64[:, t, :, :, None] * x + k64[:, t, :, :, None] * v64[:, t, :, None, :]
+        want.append(torch.einsum("shd,shdv->shv", q64[:, t], x))
+    # a product of dim terms and a state of some units: a few roundings of 2^-24 each, in quadrature
+    assert _rel(out, torch.stack(want, 1).view(S * n, H, vdim)) < 1e-6 and _rel(state, x) < 1e-6
+    for b in (0, S - 1):
+        o1, s1 = scan([b])
+        assert torch.equal(o1[b * n:(b + 1) * n], out[b * n:(b + 1) * n]) and torch.equal(s1[b], state[b])
 
 
 @pytest.mark.parametrize("per_channel", [0, 1])
