@@ -42,7 +42,7 @@ import torch  # noqa: E402
 MODEL = "paligemma-3b-pt-224"
 METRIC = "decode_tokens_per_s"
 UNIT = "tokens/s"
-FLOP_PER_IMAGE = 2.202e11   # SURVEY.md §8d: SigLIP So400m/14 + projector per 224x224 image
+FLOP_PER_IMAGE = 2.202e11   # SigLIP So400m/14 + projector per 224x224 image
 
 
 def measured_peaks():
@@ -361,7 +361,7 @@ def timed_decode(eng, ids_d, pix_d, B, K, W, world, local, sample=None, dp_visio
 
 
 def batched_rows(eng, cfg, quick: bool, world: int, local: int, which=(3, 4)):
-    """BASELINE.json configs[3] and [4], device-resident (prefill untimed, then CUDA-graph replays timed with CUDA
+    """Batched decode, device-resident (prefill untimed, then CUDA-graph replays timed with CUDA
     events): batch 32 x 256 greedy tokens, and batch 8 with a 320-token prefix x 1024 tokens of top-p sampling
     (temperature 0.8, top_p 0.9: inference.py:92-93) over the paged KV cache.  Tensor parallel when the engine is."""
     from pg_b200 import synth

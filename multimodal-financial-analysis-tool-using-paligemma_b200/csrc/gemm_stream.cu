@@ -2,13 +2,14 @@
 //
 // What bounds them is the weight stream.  As tiles of 128 weight rows (gemm_tcgen05_skinny.cu) they are 16 to 20, whose K is cut over
 // clusters that occupy 128 of the 148 SMs and meet through distributed shared memory; as rows of their own for one or two warps
-// (gemv.cu) 512 CTAs do not come out even, and each warp's stream is short.  Here every SM takes the same number of weight rows, to within one: [N b / grid, N (b + 1) / grid), in
-// groups of 16.  The 8 warps of a CTA split K, 128 columns of every 1024 each; weights go
-// straight from global memory into mma.m16n8k16 B fragments with 16-byte loads (the contraction index is permuted alike for both
+// (gemv.cu) 512 CTAs do not come out even, and each warp's stream is short.  Here every SM takes the same number of weight rows, to
+// within one: [N b / grid, N (b + 1) / grid), in groups of 16.  The 8 warps of a CTA split K, 128 columns of every 1024 each; weights
+// go straight from global memory into mma.m16n8k16 B fragments with 16-byte loads (the contraction index is permuted alike for both
 // operands: lane j of a quad owns 8 consecutive columns of every 32), about 128 KB of them in flight per SM, the first of them
-// requested before the preceding launch has finished.  The tokens are the A operand, copied to shared memory: as a whole where a CTA
+// requested before the preceding launch has finished, as far as that leaves room: a CTA takes three quarters of an SM's registers,
+// so between two streams a small launch (a norm) hides more than fusing it would save.  The tokens are the A operand, copied to shared memory: as a whole where a CTA
 // has several groups, else each lane's own pieces, as many steps ahead as the weights (without that their trip to L2 bounds a step:
-// K 16384, 8 rows 17.8 us, now 13.8).  Up to three rows take fp32 multiply-adds instead of mma.  The warps' partial sums meet in
+// K 16384, 8 rows 17.8 us, now 13.2).  Up to three rows take fp32 multiply-adds instead of mma.  The warps' partial sums meet in
 // shared memory, in warp order.
 #include "common.cuh"
 #include "mma_frag.cuh"

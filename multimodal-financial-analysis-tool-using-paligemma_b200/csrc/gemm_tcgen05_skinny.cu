@@ -311,8 +311,8 @@ static int launch_sn_nt(const CUtensorMap& mx, const CUtensorMap& mw, const SnPa
 }  // namespace tc
 
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
-  // Up to 32 rows the swap-AB stream takes every projection (gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us, q/k/v 9.9 vs 18.3
-  // us on the row-major kernel).  Up to 64 rows it does so for long K; with K 2048 its token-heavy stages and the merge of 64 columns
+  // Up to 32 rows the swap-AB stream takes every projection that gemm_stream.cu leaves (gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us,
+  // q/k/v 9.9 vs 18.3 us on the row-major kernel).  Up to 64 rows it does so for long K; with K 2048 its token-heavy stages and the merge of 64 columns
   // cost more than the stream gains (64 rows, weights out of HBM: N 2560 13.8 us, the row-major kernel 11.9; N 2048 with a
   // residual 11.5, the pair kernel 10.2; N 1152, K 4304 13.2, row-major 10.9).  Above, only where CTAs own whole weight tiles or
   // there are 32 of them (128 rows: N = K = 4096 16.1 us, row-major 17.2; N 2560, K 2048 21.6 and 11.9).

@@ -562,7 +562,8 @@ int pg_gemv_res(void* out, const void* x, const void* W, const void* R, int B, i
     return dispatch_nb(B, [&](auto nb) {
       constexpr int NB = decltype(nb)::value;
       // long rows (down_proj, K 16384): with two warps a row each keeps a longer run of loads in flight and half the partial
-      // sums meet in shared memory.  The batch-1 step: 8 warps a row 1146, 4 1137, 2 1126, 1 (256 rows are too few CTAs) 1284 us
+      // sums meet in shared memory.  The batch-1 step, when all of it took this kernel: 8 warps a row 1146, 4 1137, 2 1126, 1 (256
+      // rows are too few CTAs) 1284 us
       static const int ks_big = env_int("PG_DOWN_KS", 2);
       cudaStream_t st = (cudaStream_t)stream;
       if (K >= 8192 && ks_big == 8) { PG_GR(8); }

@@ -270,7 +270,9 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //                                           S  <- E_3 S + sum over j of (G_j k_j) v_j^T
 //                                       which is nine multiply-adds per state element and step for twelve, and no token of a
 //                                       step waits for the one before.  Decays are only multiplied, never divided by, so any
-//                                       value keeps its meaning; a token reads nothing of a later one, infinities neither.
+//                                       value keeps its meaning; a token reads nothing of a later one, infinities neither.  (A
+//                                       query times a key is taken before the value: where that overflows, or a query is
+//                                       infinite, the token's outputs are not finite, NaN where token by token gave infinity.)
 //                                       Two warps copy the records (cp.async, several steps ahead), scale q and k and take
 //                                       the ten products of a step; up to four hold the state, RG lanes sharing one, two or
 //                                       four value columns, a thread rows 4 (m RG + rg) + e of them.  The arithmetic runs on
@@ -278,8 +280,8 @@ __global__ void headnorm_gate_kernel(T* __restrict__ out, int ld_out, const floa
 //                                       Bound by those and by the shared-memory reads of q and k: of a step's 1480 cycles
 //                                       (64 columns of 128 rows) 890 issue and about 700 multiply.
 //                                       4 x 2048 tokens, 16 heads of 128: token by token with the copies in every warp 620
-//                                       us, this 373; one sequence of 512 tokens 105 and 62, 8 heads of it 150 and 49; 128 single
-//                                       tokens 96 and 86.
+//                                       us, this 375; one sequence of 512 tokens 105 and 62, 8 heads of it 150 and 49; 128 single
+//                                       tokens 96 and 86.  A wait that runs out leaves NaN in state and outputs and sets the flag.
 //                                       The state is read from and written back to the slot once per launch, which
 //                                       makes a prompt portion and a single decoded token the same case; where a sequence
 //                                       is cut decides which tokens share a step, and with it the last bits.

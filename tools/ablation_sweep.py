@@ -160,7 +160,7 @@ def main():
                               "pre-allocated paged KV pool (see the module docstring); with N > 1 each rank holds the "
                               "replicated model for the cache-off loop AND its tensor-parallel shard"}
     if rank == 0:
-        path = args.out or os.path.join(ROOT, "gpurun_out", f"ablation_n{world}.json")
+        path = os.path.abspath(args.out or f"ablation_n{world}.json")
         os.makedirs(os.path.dirname(path), exist_ok=True)
         with open(path, "w") as f:
             json.dump(out, f, indent=1)

@@ -2,7 +2,7 @@
 """Reduce `ncu -i capture.ncu-rep --page raw --csv` (a `--set full` capture: ~2000 columns) to the columns the
 records under profiles/ keep -- the format `bench.py::ncu_traffic_per_launch` reads.
 
-  ncu -i gpurun_out/x.ncu-rep --page raw --csv | python tools/ncu_compact.py > profiles/rNN_ncu_full_x.csv
+  ncu -i x.ncu-rep --page raw --csv | python tools/ncu_compact.py > profiles/ncu_full_x.csv
 """
 import csv
 import sys
