@@ -230,6 +230,27 @@ template <> __device__ __forceinline__ uint4 pack<f16>(const float* f) {
   return u;
 }
 
+// two 16-bit values in one register, the first in the low half
+template <typename T> __device__ __forceinline__ void unpack_pair(uint32_t u, float* f) {
+  if constexpr (std::is_same<T, bf16>::value) {
+    f[0] = __uint_as_float(u << 16);
+    f[1] = __uint_as_float(u & 0xffff0000u);
+  } else {
+    const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&u));
+    f[0] = t.x;
+    f[1] = t.y;
+  }
+}
+template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  if constexpr (std::is_same<T, bf16>::value) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
 // ---------------------------------------------------------------- reductions
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

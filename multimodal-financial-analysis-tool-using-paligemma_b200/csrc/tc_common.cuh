@@ -148,15 +148,6 @@ __device__ __forceinline__ float exp2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack_pair<bf16>(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-template <> __device__ __forceinline__ uint32_t pack_pair<f16>(float lo, float hi) {
-  const __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 constexpr float LOG2E_F = 1.4426950408889634f;
 // One-pass softmax: a row's reference maximum follows only when a score exceeds it by more than 2^8 (the conditional rescaling
 // published with FlashAttention-4; weights of at most 256 keep their relative precision in 16 bits).
