@@ -119,9 +119,9 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
   const bool have_k = kb1 > kb0;
   constexpr int NC = BN / S, HB = BN / 2;                   // columns that this CTA finishes; a half
-  constexpr int LANES = NC / 4, ROWS = 32 / LANES, STEPS = 16 / ROWS;   // per row; rows of a warp at once; steps for its 16 rows
+  constexpr int LANES = NC / 4, ROWS = 32 / LANES, STEPS = 16 / ROWS;   // per row; rows of a warp at once; the warps' steps through 128 rows
   static_assert(HB == 32 && NC % 8 == 0 && STEPS >= 1, "a half is one load of TMEM");
-  const int col = 4 * (lane % LANES), row0 = warp * 16 + lane / LANES, m0 = m_blk * SK_BM + row0, n = n_blk * BN + (int)rank * NC + col;
+  const int col = 4 * (lane % LANES), row0 = warp * ROWS + lane / LANES, m0 = m_blk * SK_BM + row0, n = n_blk * BN + (int)rank * NC + col;
   constexpr bool HAS_BIAS = EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES;
   constexpr bool HAS_RES = EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES;
   uint2 res[STEPS], bia = make_uint2(0, 0);
@@ -129,7 +129,7 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   if (HAS_BIAS && n < p.N) bia = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(p.bias) + n));   // N is a multiple of 8
 #pragma unroll
   for (int i = 0; i < STEPS; ++i) {     // requested before the accumulator is waited for
-    const int m = m0 + i * ROWS, rm = p.res_mod > 0 ? (m % p.res_mod) : m;
+    const int m = m0 + i * (8 * ROWS), rm = p.res_mod > 0 ? (m % p.res_mod) : m;
     res[i] = HAS_RES && m < p.M && n < p.N ? __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(p.R) + (size_t)rm * p.ldr + n))
                                            : make_uint2(0, 0);
   }
@@ -149,16 +149,26 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   cluster_sync_all();         // partial tiles are visible cluster-wide, and nobody reads TMEM any more
   // Whole row pieces by neighbouring lanes: with a row per lane each load of a warp is 32 lines of the peer's shared memory, and the
   // exchange took 3.1 us of the 8.4 between a launch's dependency and its end (256 rows, N 4304, K 1152 by 2).  The cluster is told that the
-  // reads are done before the epilogue's arithmetic.  One image's 9 layers 545 -> 472 us, a 260-token prompt with its image
-  // 4291 -> 4040.
+  // reads are done before the epilogue's arithmetic.  One image's 9 layers 544 -> 470 us, a 260-token prompt with its image
+  // 4285 -> 3985.
   float4 pv[STEPS][S];
+  auto read = [&](int i) {
+    const int at = (row0 + i * (8 * ROWS)) * PROW + (int)rank * NC + col;
 #pragma unroll
-  for (int i = 0; i < STEPS; ++i)
-#pragma unroll
-    for (int peer = 0; peer < S; ++peer) {
-      const int at = (row0 + i * ROWS) * PROW + (int)rank * NC + col;
+    for (int peer = 0; peer < S; ++peer)
       pv[i][peer] = peer == (int)rank ? *reinterpret_cast<const float4*>(part + at) : ld_dsmem_v4(smem_base + (uint32_t)(at * 4), peer);
+  };
+  if ((m_blk + 1) * SK_BM <= p.M) {
+#pragma unroll
+    for (int i = 0; i < STEPS; ++i) read(i);
+  } else {                    // rows that nobody asked for cost the exchange as much as others
+#pragma unroll
+    for (int i = 0; i < STEPS; ++i) {
+#pragma unroll
+      for (int peer = 0; peer < S; ++peer) pv[i][peer] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m0 + i * (8 * ROWS) < p.M) read(i);
     }
+  }
   float o[STEPS][4];
 #pragma unroll
   for (int i = 0; i < STEPS; ++i) {
@@ -179,7 +189,7 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   unpack_pair<T>(bia.y, bb + 2);
 #pragma unroll
   for (int i = 0; i < STEPS; ++i) {
-    const int m = m0 + i * ROWS;
+    const int m = m0 + i * (8 * ROWS);
     if (m >= p.M || n >= p.N) break;
     float rr[4];
     unpack_pair<T>(res[i].x, rr);
