@@ -23,7 +23,8 @@ namespace tc {
 
 constexpr int SW_BK = 64, SW_WROWS = 128, SW_THREADS = 384;
 constexpr int SW_W_BYTES = SW_WROWS * SW_BK * 2;   // 16 KB of weights per CTA per k-block
-constexpr int SW_SMEM_BUDGET = 220 * 1024;
+constexpr int SW_OUT_BYTES = 16 * SW_WROWS * 4;    // 16 tokens' partial sums of a CTA's 128 features
+constexpr int SW_SMEM_BUDGET = 220 * 1024 - 4 * SW_OUT_BYTES;
 
 struct ParamsSw {
   float* P;            // workspace: [splits][M tokens][N features] fp32
@@ -66,13 +67,14 @@ __device__ __forceinline__ void sw_cluster_sync() {
 
 template <int FMT>  // 1 bf16, 0 f16
 __global__ void __launch_bounds__(SW_THREADS, 1)
-gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, ParamsSw p) {
+gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                 const __grid_constant__ CUtensorMap map_p, ParamsSw p) {
   constexpr int MAX_STAGES = 8;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int x_bytes = (p.NT / 2) * SW_BK * 2;                 // one token tile's half per k-block (multiple of 1024)
   const int stage_bytes = SW_W_BYTES + p.n_t * x_bytes;
-  const uint32_t bars = smem_base + p.stages * stage_bytes;
+  const uint32_t out_base = smem_base + p.stages * stage_bytes, bars = out_base + 4 * SW_OUT_BYTES;
   auto full_bar = [&](int s) { return bars + 8u * s; };                      // used in the leader CTA
   auto empty_bar = [&](int s) { return bars + 8u * (MAX_STAGES + s); };      // one per CTA
   const uint32_t tfull_bar = bars + 8u * (2 * MAX_STAGES);                   // one per CTA
@@ -168,28 +170,39 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   } else if (warp >= 4) {
     // ===================== epilogue: TMEM -> fp32 partial [split][token][feature] (both CTAs) =====================
+    // A chunk of 16 tokens goes to shared memory as 16 rows of 128 features and on by one TMA store of the warpgroup's first thread;
+    // two buffers for each of the two warpgroups.  (A feature per lane and a store per token: 6.7 us of the 28 of 260 rows, N 2048, K 16384; a
+    // 260-token prompt with its image, with the reduction below asking for all splits at once, 3985 -> 3920 us.)
     const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter; the two halves interleave 16-column chunks
+    const bool store_thread = q == 0 && lane == 0;
     uint32_t acc_phase = 0;
     const int chunks_per_tile = p.NT / 16, chunks = p.n_t * chunks_per_tile;
+    uint8_t* const out_sm = smem_raw + (out_base - smem_u32(smem_raw)) + half * 2 * SW_OUT_BYTES;
     pdl_wait();  // the workspace may still be read by the predecessor's reduce kernel
+    int buf = 0;
     for (int item = first; item < items; item += stride) {
       const int ft = item / p.splits, sp = item % p.splits;
-      const int f = ft * 2 * SW_WROWS + (int)crank * SW_WROWS + q * 32 + lane;   // this thread's output feature
-      float* prow = p.P + (size_t)sp * p.M * p.N + f;
+      const int f0 = ft * 2 * SW_WROWS + (int)crank * SW_WROWS;   // this CTA's first output feature
       mbar_wait(tfull_bar, acc_phase);
       tc_fence_after();
       const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
-      for (int c = half; c < chunks; c += 2) {
+      for (int c = half; c < chunks; c += 2, buf ^= 1) {
         const int t = c / chunks_per_tile, cc = c % chunks_per_tile;   // token tile t lives at TMEM columns [256 t, 256 t + NT)
         float v[16];
         tmem_ld16(t_lane + t * 256 + cc * 16, v);
+        if (store_thread) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the buffer's last store has read it
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
         tmem_ld_wait();
-        if (f < p.N) {
+        float* row = reinterpret_cast<float*>(out_sm + buf * SW_OUT_BYTES) + q * 32 + lane;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int tok = t * p.NT + cc * 16 + j;
-            if (tok < p.M) prow[(size_t)tok * p.N] = v[j];   // a warp writes 32 consecutive features: one 128-byte row piece
-          }
+        for (int j = 0; j < 16; ++j) row[j * SW_WROWS] = v[j];
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        if (store_thread && f0 < p.N && t * p.NT + cc * 16 < p.M) {
+          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"   // clipped at N and at M
+                       ::"l"(reinterpret_cast<uint64_t>(&map_p)), "r"(out_base + (half * 2 + buf) * SW_OUT_BYTES), "r"(f0),
+                       "r"(t * p.NT + cc * 16), "r"(sp) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
       tc_fence_before();
@@ -197,6 +210,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       if (lane == 0) sw_arrive_cluster(sw_mapa(tempty_bar, 0));
       acc_phase ^= 1;
     }
+    if (store_thread) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -222,13 +236,24 @@ gemm_swap_reduce_kernel(T* __restrict__ out, const float* __restrict__ P, const 
     const int m = (int)(i / vec_per_row), n = (int)(i % vec_per_row) * 4;
     const float* src = P + (size_t)m * Np + n;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), u = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(src + s * split_stride);
-      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
-      if (EPI == PG_EPI_GEGLU) {
-        const float4 w = *reinterpret_cast<const float4*>(src + s * split_stride + Nout);
-        u.x += w.x; u.y += w.y; u.z += w.z; u.w += w.w;
-      }
+    constexpr int AT_ONCE = EPI == PG_EPI_GEGLU ? 4 : 10;      // splits whose loads are in flight together
+    for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
+      float4 v[AT_ONCE], w[EPI == PG_EPI_GEGLU ? AT_ONCE : 1];
+#pragma unroll
+      for (int k = 0; k < AT_ONCE; ++k)
+        if (s0 + k < splits) {
+          v[k] = __ldcg(reinterpret_cast<const float4*>(src + (s0 + k) * split_stride));
+          if (EPI == PG_EPI_GEGLU) w[EPI == PG_EPI_GEGLU ? k : 0] = __ldcg(reinterpret_cast<const float4*>(src + (s0 + k) * split_stride + Nout));
+        }
+#pragma unroll
+      for (int k = 0; k < AT_ONCE; ++k)
+        if (s0 + k < splits) {
+          a.x += v[k].x; a.y += v[k].y; a.z += v[k].z; a.w += v[k].w;
+          if (EPI == PG_EPI_GEGLU) {
+            const float4 x = w[EPI == PG_EPI_GEGLU ? k : 0];
+            u.x += x.x; u.y += x.y; u.z += x.z; u.w += x.w;
+          }
+        }
     }
     float o[4] = {rnd<T>(a.x), rnd<T>(a.y), rnd<T>(a.z), rnd<T>(a.w)};
     if (EPI == PG_EPI_GEGLU) {
@@ -283,6 +308,17 @@ static void swap_plan(int M, int N, int K, tc::ParamsSw* p) {
   if (p->stages > max_stages) p->stages = max_stages;
 }
 
+// the partial sums [splits][M][N] fp32, for stores of 16 tokens x 128 features
+static bool make_map_partials(CUtensorMap* map, void* base, int N, int M, int splits) {
+  tc::EncodeTiledFn fn = tc::encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits};
+  cuuint64_t strides[2] = {(cuuint64_t)N * 4, (cuuint64_t)M * N * 4};
+  cuuint32_t box[3] = {tc::SW_WROWS, 16, 1}, estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod) {
   static const int enabled = env_int("PG_GEMM_SWAP", 1);
   static const int min_m = env_int("PG_GEMM_SWAP_MIN_M", 4);
@@ -303,7 +339,7 @@ bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod)
   tc::ParamsSw p;
   swap_plan(M, n_w, K, &p);
   if (p.stages < 3) return false;
-  return g_ws_ptr && (long long)p.splits * M * n_w * 4 <= g_ws_bytes;
+  return g_ws_ptr && (uintptr_t)g_ws_ptr % 16 == 0 && (long long)p.splits * M * n_w * 4 <= g_ws_bytes;
 }
 
 int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, int N, int K, int lda, int ldw, int ldc,
@@ -314,11 +350,12 @@ int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, in
   swap_plan(M, n_w, K, &p);
   p.P = reinterpret_cast<float*>(g_ws_ptr);
   p.w_param = w_param;
-  CUtensorMap mw, mx;
-  PG_REQUIRE(tc::make_map_2d(&mw, W, n_w, K, ldw, tc::SW_WROWS, bf) && tc::make_map_2d(&mx, A, M, K, lda, p.NT / 2, bf),
+  CUtensorMap mw, mx, mp;
+  PG_REQUIRE(tc::make_map_2d(&mw, W, n_w, K, ldw, tc::SW_WROWS, bf) && tc::make_map_2d(&mx, A, M, K, lda, p.NT / 2, bf) &&
+                 make_map_partials(&mp, p.P, n_w, M, p.splits),
              "gemm_swap: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, n_w, K, lda, ldw);
   const int stage_bytes = tc::SW_W_BYTES + p.n_t * (p.NT / 2) * tc::SW_BK * 2;
-  const size_t smem = 1024 + (size_t)p.stages * stage_bytes + 8 * (2 * 8 + 3) + 16;
+  const size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * tc::SW_OUT_BYTES + 8 * (2 * 8 + 3) + 16;
   auto kern = bf ? tc::gemm_swap_kernel<1> : tc::gemm_swap_kernel<0>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     set_error("gemm_swap: cannot reserve %zu B of shared memory", smem);
@@ -327,7 +364,7 @@ int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, in
   }
   const int items = cdiv(n_w, 2 * tc::SW_WROWS) * p.splits;
   int rc = launch_tc("gemm_tcgen05_swap", kern, dim3(2 * (items < 74 ? items : 74)), dim3(tc::SW_THREADS), smem, 2, true, st,
-                     mw, mx, p);
+                     mw, mx, mp, p);
   if (rc != PG_OK) return rc;
   const long long vecs = (long long)M * (N / 4);
   const int grid = (int)((vecs + 255) / 256 < 148 * 8 ? (vecs + 255) / 256 : 148 * 8);
