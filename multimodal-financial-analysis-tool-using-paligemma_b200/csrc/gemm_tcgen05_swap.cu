@@ -7,8 +7,8 @@
 // chip-wide), not HBM or the tensor pipe, sets the time (gate/up 48 us, down_proj 56 us per layer).  Here:
 //   * the WEIGHT rows are the M = 256 operand of a tcgen05.mma.cta_group::2 (128 rows per CTA of the pair), streamed
 //     from HBM exactly once;
-//   * ALL tokens are the N operand: one accumulator of NT <= 256 columns (<= 256 tokens) or two (<= 512 tokens, the
-//     second at TMEM column 256) in TMEM; the pair SPLITS the token tile (each CTA stages NT/2 token rows per k-block), so the token re-read that
+//   * ALL tokens are the N operand: one accumulator of NT <= 256 columns (<= 256 tokens) or a second one for the rest (<= 512 tokens) at
+//     TMEM column 256; the pair SPLITS the token tile (each CTA stages NT/2 token rows per k-block), so the token re-read that
 //     every weight tile costs is halved against single-CTA swap-AB;
 //   * short-N / long-K problems (o_proj, down_proj, q/k/v: 8-10 weight tiles) are split along K over the 74 pairs;
 //     every work item leaves an fp32 partial [split][token][feature] in a caller-provided workspace (L2-resident) and
@@ -29,7 +29,7 @@ constexpr int SW_SMEM_BUDGET = 220 * 1024 - 4 * SW_OUT_BYTES;
 struct ParamsSw {
   float* P;            // workspace: [splits][M tokens][N features] fp32
   int M, N, K;         // tokens, output features, reduction length
-  int NT, n_t;         // token tile width (multiple of 16, <= 256) and number of tiles (1 or 2)
+  int NT, NT2;         // widths of the first and the second token tile (multiples of 16, <= 256; NT2 may be 0)
   int splits, kb_per_split, stages;
   int w_param;         // W is no output of a preceding launch: it may be requested before the dependency wait
 };
@@ -68,12 +68,12 @@ __device__ __forceinline__ void sw_cluster_sync() {
 template <int FMT>  // 1 bf16, 0 f16
 __global__ void __launch_bounds__(SW_THREADS, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                 const __grid_constant__ CUtensorMap map_p, ParamsSw p) {
+                 const __grid_constant__ CUtensorMap map_x2, const __grid_constant__ CUtensorMap map_p, ParamsSw p) {
   constexpr int MAX_STAGES = 8;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int x_bytes = (p.NT / 2) * SW_BK * 2;                 // one token tile's half per k-block (multiple of 1024)
-  const int stage_bytes = SW_W_BYTES + p.n_t * x_bytes;
+  const int x_bytes = (p.NT / 2) * SW_BK * 2;                 // the first token tile's half per k-block (multiple of 1024)
+  const int stage_bytes = SW_W_BYTES + ((p.NT + p.NT2) / 2) * SW_BK * 2;
   const uint32_t out_base = smem_base + p.stages * stage_bytes, bars = out_base + 4 * SW_OUT_BYTES;
   auto full_bar = [&](int s) { return bars + 8u * s; };                      // used in the leader CTA
   auto empty_bar = [&](int s) { return bars + 8u * (MAX_STAGES + s); };      // one per CTA
@@ -91,7 +91,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const int items = f_tiles * p.splits;
   const int first = (int)(blockIdx.x / 2), stride = (int)(gridDim.x / 2);
   const int k_blocks = (p.K + SW_BK - 1) / SW_BK;
-  const uint32_t idesc = umma_idesc(FMT, 2 * SW_WROWS, p.NT);
+  const uint32_t idesc = umma_idesc(FMT, 2 * SW_WROWS, p.NT), idesc2 = umma_idesc(FMT, 2 * SW_WROWS, p.NT2 ? p.NT2 : 16);
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
@@ -135,8 +135,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           // a parameter does not depend on the preceding kernels: its first load goes out before the dependency wait
           sw_tma_cg2(sa, &map_w, full_leader, kb * SW_BK, ft * 2 * SW_WROWS + (int)crank * SW_WROWS);
           if (!waited) { pdl_wait(); waited = true; }   // the token rows come from the predecessor
-          for (int t = 0; t < p.n_t; ++t)
-            sw_tma_cg2(sa + SW_W_BYTES + t * x_bytes, &map_x, full_leader, kb * SW_BK, t * p.NT + (int)crank * (p.NT / 2));
+          sw_tma_cg2(sa + SW_W_BYTES, &map_x, full_leader, kb * SW_BK, (int)crank * (p.NT / 2));
+          if (p.NT2) sw_tma_cg2(sa + SW_W_BYTES + x_bytes, &map_x2, full_leader, kb * SW_BK, p.NT + (int)crank * (p.NT2 / 2));
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
       }
@@ -157,10 +157,11 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           tc_fence_after();
           const uint32_t sa = smem_base + stage * stage_bytes;
 #pragma unroll
-          for (int k = 0; k < SW_BK / 16; ++k)
-            for (int t = 0; t < p.n_t; ++t)
-              sw_umma_cg2(tmem_base + t * 256, umma_desc(sa + k * 32), umma_desc(sa + SW_W_BYTES + t * x_bytes + k * 32), idesc,
-                          (i > kb0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < SW_BK / 16; ++k) {
+            const uint32_t accumulate = (i > kb0 || k > 0) ? 1u : 0u;
+            sw_umma_cg2(tmem_base, umma_desc(sa + k * 32), umma_desc(sa + SW_W_BYTES + k * 32), idesc, accumulate);
+            if (p.NT2) sw_umma_cg2(tmem_base + 256, umma_desc(sa + k * 32), umma_desc(sa + SW_W_BYTES + x_bytes + k * 32), idesc2, accumulate);
+          }
           sw_commit_cg2(empty_bar(stage), (uint16_t)0x3);  // the stage is free in BOTH CTAs once these MMAs have read it
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -176,7 +177,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter; the two halves interleave 16-column chunks
     const bool store_thread = q == 0 && lane == 0;
     uint32_t acc_phase = 0;
-    const int chunks_per_tile = p.NT / 16, chunks = p.n_t * chunks_per_tile;
+    const int chunks_per_tile = p.NT / 16, chunks = chunks_per_tile + p.NT2 / 16;
     uint8_t* const out_sm = smem_raw + (out_base - smem_u32(smem_raw)) + half * 2 * SW_OUT_BYTES;
     pdl_wait();  // the workspace may still be read by the predecessor's reduce kernel
     int buf = 0;
@@ -187,7 +188,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       tc_fence_after();
       const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
       for (int c = half; c < chunks; c += 2, buf ^= 1) {
-        const int t = c / chunks_per_tile, cc = c % chunks_per_tile;   // token tile t lives at TMEM columns [256 t, 256 t + NT)
+        const int t = c >= chunks_per_tile ? 1 : 0, cc = c - t * chunks_per_tile;   // the second token tile lives from TMEM column 256 on
         float v[16];
         tmem_ld16(t_lane + t * 256 + cc * 16, v);
         if (store_thread) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the buffer's last store has read it
@@ -288,8 +289,8 @@ extern "C" int pg_set_workspace(void* ptr, long long bytes) {
 
 static void swap_plan(int M, int N, int K, tc::ParamsSw* p) {
   p->M = M; p->N = N; p->K = K;
-  p->n_t = M <= 256 ? 1 : 2;
-  p->NT = (((M + p->n_t - 1) / p->n_t) + 15) / 16 * 16;
+  p->NT = M >= 256 ? 256 : (M + 15) / 16 * 16;
+  p->NT2 = (M - (M < 256 ? M : 256) + 15) / 16 * 16;
   const int f_tiles = cdiv(N, 2 * tc::SW_WROWS), k_blocks = cdiv(K, tc::SW_BK);
   // split K until the work items fill the 74 CTA pairs about once (every split keeps >= 2 k-blocks)
   int splits = 1;
@@ -301,7 +302,7 @@ static void swap_plan(int M, int N, int K, tc::ParamsSw* p) {
   splits = cdiv(k_blocks, kbs);           // no empty split
   p->splits = splits;
   p->kb_per_split = kbs;
-  const int stage_bytes = tc::SW_W_BYTES + p->n_t * (p->NT / 2) * tc::SW_BK * 2;
+  const int stage_bytes = tc::SW_W_BYTES + ((p->NT + p->NT2) / 2) * tc::SW_BK * 2;
   int stages = (tc::SW_SMEM_BUDGET - 1024 - 256) / stage_bytes;
   p->stages = stages > 8 ? 8 : stages;
   static const int max_stages = env_int("PG_SWAP_STAGES", 8);
@@ -350,11 +351,12 @@ int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, in
   swap_plan(M, n_w, K, &p);
   p.P = reinterpret_cast<float*>(g_ws_ptr);
   p.w_param = w_param;
-  CUtensorMap mw, mx, mp;
+  CUtensorMap mw, mx, mx2 = {}, mp;
   PG_REQUIRE(tc::make_map_2d(&mw, W, n_w, K, ldw, tc::SW_WROWS, bf) && tc::make_map_2d(&mx, A, M, K, lda, p.NT / 2, bf) &&
+                 (!p.NT2 || tc::make_map_2d(&mx2, A, M, K, lda, p.NT2 / 2, bf)) &&
                  make_map_partials(&mp, p.P, n_w, M, p.splits),
              "gemm_swap: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%d ldw=%d)", M, n_w, K, lda, ldw);
-  const int stage_bytes = tc::SW_W_BYTES + p.n_t * (p.NT / 2) * tc::SW_BK * 2;
+  const int stage_bytes = tc::SW_W_BYTES + ((p.NT + p.NT2) / 2) * tc::SW_BK * 2;
   const size_t smem = 1024 + (size_t)p.stages * stage_bytes + 4 * tc::SW_OUT_BYTES + 8 * (2 * 8 + 3) + 16;
   auto kern = bf ? tc::gemm_swap_kernel<1> : tc::gemm_swap_kernel<0>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -364,7 +366,7 @@ int gemm_tc_swap(void* C, const void* A, const void* W, const void* R, int M, in
   }
   const int items = cdiv(n_w, 2 * tc::SW_WROWS) * p.splits;
   int rc = launch_tc("gemm_tcgen05_swap", kern, dim3(2 * (items < 74 ? items : 74)), dim3(tc::SW_THREADS), smem, 2, true, st,
-                     mw, mx, mp, p);
+                     mw, mx, mx2, mp, p);
   if (rc != PG_OK) return rc;
   const long long vecs = (long long)M * (N / 4);
   const int grid = (int)((vecs + 255) / 256 < 148 * 8 ? (vecs + 255) / 256 : 148 * 8);
