@@ -378,7 +378,13 @@ static int launch_da(void* out, const void* q, const void* k_pool, const void* v
 // 16-bit, as stored.  128 threads per CTA and two CTAs per SM keep a cluster of 16 within 8 SMs.
 // Measured (launch alone, cold cache): 1 sequence x 262 tokens 13.5 -> 9.5 us, 8 x 1345 39.7 -> 14.2 us, 32 x 389 23.6 -> 12.1 us;
 // inside the captured step 4.0, 23 and 5.1 us per layer less.
+// What then bounded it was the tail, 4 to 5 us of 7 to 11 behind the wait: merging the warps (1.6 to 2.8 us), fetching the peers' sums
+// (1.7) and the barrier behind that (0.75).  With the sums handed over by the CTAs that have them, and the rows in L2 before the wait,
+// behind the wait: 1 sequence x 262 tokens 7.0 -> 4.9 us, 8 x 1345 11.3 -> 7.9, 32 x 389 10.5 -> 6.7.
+// (The next chunk's keys requested behind this one's scores: 48 bytes spilled, and no faster.)
 constexpr int DM_WARPS = 4, DM_HD = 256, DM_G = 8;
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
 
 template <typename T, int NS>
 __global__ void __launch_bounds__(DM_WARPS * 32, 2)
@@ -392,15 +398,35 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   l2_prefetch_slice(pf);
   const int rank = (int)cluster.block_rank(), b = blockIdx.y, kvh = blockIdx.z, G = nq / nkv;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, r = lane >> 2, j = lane & 3;
-  __shared__ __align__(16) float s_acc[DM_WARPS][DM_G][DM_HD];
-  __shared__ __align__(16) float c_acc[DM_G][DM_HD];      // CTA-level partial (read by peers)
-  __shared__ float s_m[DM_WARPS][DM_G], s_l[DM_WARPS][DM_G], c_m[DM_G], c_l[DM_G];
+  __shared__ __align__(16) float s_acc[DM_WARPS][DM_G][DM_HD + 4];
+  // what the cluster's CTAs have put here for this CTA's share of the outputs: [CTA][output of the share], [CTA][head]{maximum, sum}
+  __shared__ __align__(16) float r_acc[DM_G * DM_HD];
+  __shared__ float2 r_ml[NS][DM_G];
+  __shared__ float s_m[DM_WARPS][DM_G], s_l[DM_WARPS][DM_G];
   __shared__ int s_pt[DC_MAX_PT];
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before anything goes to another CTA
+  const int32_t* pt = page_table + (size_t)b * pt_stride;
+  const size_t row_elems = (size_t)nkv * DM_HD;
+  {
+    // While the preceding kernel runs (1.5 to 2.5 us in a captured step): this warp's first four chunks into L2.  A hint only: the
+    // length and the page numbers it goes by are read again behind the wait.
+    const int t_end = __ldcg(kv_len + b) + kv_len_add;
+    for (int c = rank + NS * wid, i = 0; i < 4; c += NS * DM_WARPS, ++i) {
+      const int t = c * 16 + (lane >> 1), pi = t / page_size;
+      if (t >= t_end || pi >= pt_stride) break;
+      const int page = __ldcg(pt + pi);
+      if (page < 0) break;
+      const size_t at = ((size_t)page * page_size + t % page_size) * row_elems + (size_t)kvh * DM_HD + (lane & 1) * 128;
+      prefetch_l2(k_pool + at);
+      prefetch_l2(k_pool + at + 64);
+      prefetch_l2(v_pool + at);
+      prefetch_l2(v_pool + at + 64);
+    }
+  }
   pdl_wait();  // q and this step's K/V row come from the preceding qkv kernel
 
   // the length, the page-table row and the query rows are requested together
   const int T_len = kv_len[b] + kv_len_add;
-  const int32_t* pt = page_table + (size_t)b * pt_stride;
   const int pt_n = min(pt_stride, DC_MAX_PT);
   for (int i = threadIdx.x; i < pt_n; i += DM_WARPS * 32) s_pt[i] = pt[i];
   uint4 qf[KB];
@@ -413,7 +439,6 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   __syncthreads();
 
   const int chunks = (T_len + 15) / 16;
-  const size_t row_elems = (size_t)nkv * DM_HD;
   auto attend = [&](auto in_fp32) {                           // this warp's chunks
     constexpr bool fp32 = decltype(in_fp32)::value;
 #pragma unroll
@@ -485,9 +510,19 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], o);
 
-  // ---- merge the warps of this CTA (those that met a chunk)
-  const int busy = min(DM_WARPS, (max(0, chunks - rank) + NS - 1) / NS);
-  if (wid < busy) {
+  // ---- merge the warps of this CTA (those that met a chunk) and hand the sums to the CTAs that finish them.  A CTA writes into its
+  // peers' shared memory and reads only its own: fetched from the peers the sums were 48 loads a thread behind the barrier, and a
+  // second barrier kept everybody until the last one had read.  The weights of a merge are computed once, a lane each, and go
+  // round by shuffle; computed anew for every output they were 4 and 16 exponentials a thread.
+  const int busy = min(DM_WARPS, (max(0, chunks - rank) + NS - 1) / NS), per = G * DM_HD / NS;
+  auto push4 = [&](int e, const float4& v) {                  // outputs e .. e + 3 of this CTA
+    const int to = e / per;
+    *reinterpret_cast<float4*>(cluster.map_shared_rank(r_acc + rank * per + (e - to * per), to)) = v;
+  };
+  auto push_ml = [&](int t, float m_g, float l_g) {           // t: receiving CTA and head
+    *cluster.map_shared_rank(&r_ml[rank][t % G], t / G) = make_float2(m_g, l_g);
+  };
+  if (busy > 1 && wid < busy) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (r == 0) { s_m[wid][2 * j + h] = m[h]; s_l[wid][2 * j + h] = l[h]; }
@@ -497,52 +532,74 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
       }
     }
   }
-  __syncthreads();
-  for (int e = threadIdx.x * 4; e < G * DM_HD; e += DM_WARPS * 32 * 4) {
-    const int g = e / DM_HD, d = e % DM_HD;
-    float M = -INFINITY;
-    for (int w = 0; w < busy; ++w) M = fmaxf(M, s_m[w][g]);
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    float L = 0.f;
-    for (int w = 0; w < busy; ++w) {
-      if (s_m[w][g] == -INFINITY) continue;                   // a warp whose tokens have no weight
-      const float f = __expf(s_m[w][g] - M);
-      const float4 v = *reinterpret_cast<const float4*>(&s_acc[w][g][d]);
-      a.x = fmaf(f, v.x, a.x); a.y = fmaf(f, v.y, a.y); a.z = fmaf(f, v.z, a.z); a.w = fmaf(f, v.w, a.w);
-      L = fmaf(f, s_l[w][g], L);
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");             // every CTA of the cluster is there
+  if (busy == 1) {                                            // one warp met a chunk: its sums are the CTA's
+    if (wid == 0) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int g = 2 * j + h;
+        if (g < G) {
+#pragma unroll
+          for (int vb = 0; vb < VB; ++vb) {
+            float v[8];
+            store_acc<T>(v, acc[vb], h);
+            push4(g * DM_HD + vb * 64 + r * 8, make_float4(v[0], v[1], v[2], v[3]));
+            push4(g * DM_HD + vb * 64 + r * 8 + 4, make_float4(v[4], v[5], v[6], v[7]));
+          }
+          for (int to = r; to < NS; to += 8) push_ml(to * G + g, m[h], l[h]);
+        }
+      }
     }
-    *reinterpret_cast<float4*>(&c_acc[g][d]) = a;
-    if (d == 0) { c_m[g] = M; c_l[g] = L; }
+  } else if (busy > 1) {
+    __syncthreads();
+    for (int g = wid; g < G; g += DM_WARPS) {                 // a warp per head, its lanes' weights by shuffle
+      float mw = lane < busy ? s_m[lane & (DM_WARPS - 1)][g] : -INFINITY, lw = s_l[lane & (DM_WARPS - 1)][g], M = mw;
+#pragma unroll
+      for (int o = 1; o < DM_WARPS; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+      M = __shfl_sync(0xffffffffu, M, 0);
+      const float fw = mw == -INFINITY ? 0.f : __expf(mw - M);             // a warp whose tokens have no weight
+      float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+      float L = 0.f;
+#pragma unroll
+      for (int w = 0; w < DM_WARPS; ++w) {
+        if (w >= busy || __shfl_sync(0xffffffffu, mw, w) == -INFINITY) continue;
+        const float f = __shfl_sync(0xffffffffu, fw, w);
+        const float4 u = *reinterpret_cast<const float4*>(&s_acc[w][g][lane * 4]);
+        const float4 v = *reinterpret_cast<const float4*>(&s_acc[w][g][128 + lane * 4]);
+        L = fmaf(f, __shfl_sync(0xffffffffu, lw, w), L);
+        a0.x = fmaf(f, u.x, a0.x); a0.y = fmaf(f, u.y, a0.y); a0.z = fmaf(f, u.z, a0.z); a0.w = fmaf(f, u.w, a0.w);
+        a1.x = fmaf(f, v.x, a1.x); a1.y = fmaf(f, v.y, a1.y); a1.z = fmaf(f, v.z, a1.z); a1.w = fmaf(f, v.w, a1.w);
+      }
+      push4(g * DM_HD + lane * 4, a0);
+      push4(g * DM_HD + 128 + lane * 4, a1);
+      if (lane < NS) push_ml(lane * G + g, M, L);
+    }
   }
-  cluster.sync();  // every CTA's partial is visible cluster-wide
+  __syncwarp();
+  cluster.sync();  // what was handed over is there; from here on a CTA reads its own shared memory only
 
-  // ---- merge the CTAs that met a chunk: CTA `rank` finalises its slice of the G * 256 outputs through DSMEM
+  // ---- this CTA's share of the G * 256 outputs, from the CTAs that met a chunk
   const int n_cta = min(NS, chunks);
-  const int per = (G * DM_HD + NS - 1) / NS, e_end = min(G * DM_HD, (rank + 1) * per);
-  for (int e = rank * per + threadIdx.x; e < e_end; e += DM_WARPS * 32) {
-    const int g = e / DM_HD, d = e % DM_HD;
-    float pm[NS], pl[NS], pa[NS];
+  for (int e0 = wid * 32; e0 < per; e0 += DM_WARPS * 32) {    // per is a multiple of 16: half a warp has one head
+    const int e = e0 + lane, i = lane & 15, g = min((rank * per + e) / DM_HD, G - 1), d = (rank * per + e) % DM_HD;
+    const float2 ml = i < n_cta ? r_ml[i & (NS - 1)][g] : make_float2(-INFINITY, 0.f);   // lane i: CTA i's
+    float M = ml.x;
 #pragma unroll
-    for (int i = 0; i < NS; ++i) {
-      const bool have = i < n_cta;
-      pm[i] = have ? *cluster.map_shared_rank(&c_m[g], i) : -INFINITY;
-      pl[i] = have ? *cluster.map_shared_rank(&c_l[g], i) : 0.f;
-      pa[i] = have ? *cluster.map_shared_rank(&c_acc[g][d], i) : 0.f;
-    }
-    float M = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) M = fmaxf(M, pm[i]);
+    for (int o = 1; o < NS; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o, 16));
+    const float wi = ml.x == -INFINITY ? 0.f : __expf(ml.x - M);
     float a = 0.f, L = 0.f;
 #pragma unroll
-    for (int i = 0; i < NS; ++i)
-      if (i < n_cta && pm[i] != -INFINITY) {
-        const float w = __expf(pm[i] - M);
-        a = fmaf(w, pa[i], a);
-        L = fmaf(w, pl[i], L);
+    for (int c = 0; c < NS; ++c) {
+      const float mc = __shfl_sync(0xffffffffu, ml.x, c, 16), w = __shfl_sync(0xffffffffu, wi, c, 16);
+      const float lc = __shfl_sync(0xffffffffu, ml.y, c, 16);
+      if (mc != -INFINITY && e < per) {
+        a = fmaf(w, r_acc[c * per + e], a);
+        L = fmaf(w, lc, L);
       }
-    out[((size_t)b * nq + (size_t)kvh * G + g) * DM_HD + d] = from_f<T>(a / L);
+    }
+    if (e < per)
+      out[((size_t)b * nq + (size_t)kvh * G + g) * DM_HD + d] = from_f<T>(a / L);
   }
-  cluster.sync();  // nobody leaves while a peer may still read its shared memory
 }
 
 template <typename T, int NS>
