@@ -386,12 +386,24 @@ constexpr int DM_WARPS = 4, DM_HD = 256, DM_G = 8;
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
 
-template <typename T, int NS>
+// ROPE: the step's rotary embedding and cache row too.  q is then the q/k/v projections [B][nq + 2 nkv][256]: every CTA rotates its
+// heads' query rows (pg_rope_append's arithmetic and rounding) into shared memory, and the one that meets the last chunk writes the
+// new key and value row before it reads the chunk.  As a launch of its own that was 4.3 us for 8 rows of 10 heads, most of it the
+// launch and the chain position -> page -> load -> store; here the loads go out with those of the length and the pages and the angles
+// are there before the wait.  Six layers: 8 sequences x 1345 tokens 406 -> 402 us, 32 x 389 452 -> 437; the two launches stay for
+// what this kernel does not take.
+struct DecodeRope {
+  const float* inv_freq;
+  const int32_t* positions;
+  int max_pos;
+};
+
+template <typename T, int NS, bool ROPE>
 __global__ void __launch_bounds__(DM_WARPS * 32, 2)
-decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_pool,
-                            const T* __restrict__ v_pool, const int32_t* __restrict__ page_table, int pt_stride, int page_size,
+decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const T* k_pool, const T* v_pool,
+                            const int32_t* __restrict__ page_table, int pt_stride, int page_size,
                             const int32_t* __restrict__ kv_len, int kv_len_add, int nq, int nkv, float scale_div,
-                            float scale_mul, Prefetch pf) {
+                            float scale_mul, DecodeRope rope, Prefetch pf) {
   constexpr int KB = DM_HD / 32, VB = DM_HD / 64;
   cg::cluster_group cluster = cg::this_cluster();
   pdl_launch_dependents();
@@ -407,21 +419,37 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before anything goes to another CTA
   const int32_t* pt = page_table + (size_t)b * pt_stride;
   const size_t row_elems = (size_t)nkv * DM_HD;
-  {
-    // While the preceding kernel runs (1.5 to 2.5 us in a captured step): this warp's first four chunks into L2.  A hint only: the
-    // length and the page numbers it goes by are read again behind the wait.
-    const int t_end = __ldcg(kv_len + b) + kv_len_add;
-    for (int c = rank + NS * wid, i = 0; i < 4; c += NS * DM_WARPS, ++i) {
-      const int t = c * 16 + (lane >> 1), pi = t / page_size;
-      if (t >= t_end || pi >= pt_stride) break;
-      const int page = __ldcg(pt + pi);
-      if (page < 0) break;
-      const size_t at = ((size_t)page * page_size + t % page_size) * row_elems + (size_t)kvh * DM_HD + (lane & 1) * 128;
-      prefetch_l2(k_pool + at);
-      prefetch_l2(k_pool + at + 64);
-      prefetch_l2(v_pool + at);
-      prefetch_l2(v_pool + at + 64);
-    }
+  // While the preceding kernel runs (1.5 to 2.5 us in a captured step): this warp's first four chunks into L2.  A hint only: the length
+  // and the page numbers it goes by are read again behind the wait.
+  const int jp = threadIdx.x & 63;
+  int ahead[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ahead[i] = __ldcg(pt + min((rank + NS * (wid + DM_WARPS * i)) * 16 / page_size, pt_stride - 1));
+  const int t_end = __ldcg(kv_len + b) + kv_len_add;
+  // ... and the angles of this thread's columns 2 jp, 2 jp + 1, done again if what they come from is another behind the wait
+  float angle[2] = {0.f, 0.f}, c[2], s[2];
+  auto angles = [&] {
+    const float pos = (float)min(max(__ldcg(rope.positions + b), 0), rope.max_pos - 1);
+    const float2 f = __ldcg(reinterpret_cast<const float2*>(rope.inv_freq) + jp);
+    const float a0 = pos * f.x, a1 = pos * f.y;
+    const bool other = a0 != angle[0] || a1 != angle[1];
+    angle[0] = a0; angle[1] = a1;
+    return other;
+  };
+  if constexpr (ROPE) angles();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = (rank + NS * (wid + DM_WARPS * i)) * 16 + (lane >> 1);
+    if (t >= t_end || ahead[i] < 0) break;
+    const size_t at = ((size_t)ahead[i] * page_size + t % page_size) * row_elems + (size_t)kvh * DM_HD + (lane & 1) * 128;
+    prefetch_l2(k_pool + at);
+    prefetch_l2(k_pool + at + 64);
+    prefetch_l2(v_pool + at);
+    prefetch_l2(v_pool + at + 64);
+  }
+  if constexpr (ROPE) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { c[i] = rnd<T>(cosf(angle[i])); s[i] = rnd<T>(sinf(angle[i])); }
   }
   pdl_wait();  // q and this step's K/V row come from the preceding qkv kernel
 
@@ -430,7 +458,54 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   const int pt_n = min(pt_stride, DC_MAX_PT);
   for (int i = threadIdx.x; i < pt_n; i += DM_WARPS * 32) s_pt[i] = pt[i];
   uint4 qf[KB];
-  {
+  if constexpr (ROPE) {
+    typedef uint32_t u32;
+    constexpr int LD = DM_HD + 32, HALF = DM_HD / 2;          // rows of 144 words: the fragments' 16-byte reads meet no bank twice
+    T* s_q = reinterpret_cast<T*>(s_acc);                     // until the sums need the room
+    const int slot = T_len - 1;
+    const T* row = q + (size_t)b * (nq + 2 * nkv) * DM_HD;
+    const bool newest = (slot / 16) % NS == rank;             // this CTA meets the last chunk
+    u32 lo[DM_G / 2 + 1], hi[DM_G / 2 + 1];
+#pragma unroll
+    for (int i = 0; i <= DM_G / 2; ++i) {                      // its query heads, then the key head
+      const int h = min(2 * i + (int)(threadIdx.x >> 6), G);
+      const T* at = row + (size_t)(h < G ? kvh * G + h : nq + kvh) * DM_HD + 2 * jp;
+      lo[i] = __ldg(reinterpret_cast<const u32*>(at));
+      hi[i] = __ldg(reinterpret_cast<const u32*>(at + HALF));
+    }
+    const u32 nv = __ldg(reinterpret_cast<const u32*>(row + (size_t)(nq + nkv + kvh) * DM_HD + 2 * threadIdx.x));
+    if (angles()) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) { c[i] = rnd<T>(cosf(angle[i])); s[i] = rnd<T>(sinf(angle[i])); }
+    }
+    u32 nk_lo = 0, nk_hi = 0;
+#pragma unroll
+    for (int i = 0; i <= DM_G / 2; ++i) {
+      const int h = 2 * i + (threadIdx.x >> 6);
+      if (h > G) continue;
+      float x[2], y[2];
+      unpack_pair<T>(lo[i], x);
+      unpack_pair<T>(hi[i], y);
+      const u32 l2 = pack_pair<T>(rnd<T>(x[0] * c[0]) + rnd<T>(-y[0] * s[0]), rnd<T>(x[1] * c[1]) + rnd<T>(-y[1] * s[1]));
+      const u32 h2 = pack_pair<T>(rnd<T>(y[0] * c[0]) + rnd<T>(x[0] * s[0]), rnd<T>(y[1] * c[1]) + rnd<T>(x[1] * s[1]));
+      if (h == G) { nk_lo = l2; nk_hi = h2; continue; }
+      *reinterpret_cast<u32*>(s_q + h * LD + 2 * jp) = l2;
+      *reinterpret_cast<u32*>(s_q + h * LD + HALF + 2 * jp) = h2;
+    }
+    __syncthreads();
+    if (newest) {
+      const int pi = slot / page_size, page = pi < pt_n ? s_pt[pi] : pt[pi];
+      const size_t at = ((size_t)page * page_size + slot % page_size) * row_elems + (size_t)kvh * DM_HD;
+      if ((threadIdx.x >> 6) == (G & 1)) {
+        *reinterpret_cast<u32*>(const_cast<T*>(k_pool) + at + 2 * jp) = nk_lo;
+        *reinterpret_cast<u32*>(const_cast<T*>(k_pool) + at + HALF + 2 * jp) = nk_hi;
+      }
+      *reinterpret_cast<u32*>(const_cast<T*>(v_pool) + at + 2 * threadIdx.x) = nv;
+    }
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb)
+      qf[kb] = r < G ? *reinterpret_cast<const uint4*>(s_q + r * LD + kb * 32 + j * 8) : make_uint4(0, 0, 0, 0);
+  } else {
     const T* qr = q + ((size_t)b * nq + (size_t)kvh * G + r) * DM_HD + j * 8;
 #pragma unroll
     for (int kb = 0; kb < KB; ++kb) qf[kb] = r < G ? ldg_cached(qr + kb * 32) : make_uint4(0, 0, 0, 0);
@@ -439,6 +514,10 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   __syncthreads();
 
   const int chunks = (T_len + 15) / 16;
+  auto load_row = [](const T* p) {                            // ROPE: the last row is this kernel's own
+    if constexpr (ROPE) return __ldcg(reinterpret_cast<const uint4*>(p));
+    else return ldg_cached(p);
+  };
   auto attend = [&](auto in_fp32) {                           // this warp's chunks
     constexpr bool fp32 = decltype(in_fp32)::value;
 #pragma unroll
@@ -462,11 +541,11 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
       const size_t v2 = (size_t)min(2 * j + 8, last) * row_elems, v3 = (size_t)min(2 * j + 9, last) * row_elems;
       uint4 ka[KB], kc[KB], va[VB][4];
 #pragma unroll
-      for (int kb = 0; kb < KB; ++kb) { ka[kb] = ldg_cached(kp + k0 + kb * 32); kc[kb] = ldg_cached(kp + k1 + kb * 32); }
+      for (int kb = 0; kb < KB; ++kb) { ka[kb] = load_row(kp + k0 + kb * 32); kc[kb] = load_row(kp + k1 + kb * 32); }
 #pragma unroll
       for (int vb = 0; vb < VB; ++vb) {
-        va[vb][0] = ldg_cached(vp + v0 + vb * 64); va[vb][1] = ldg_cached(vp + v1 + vb * 64);
-        va[vb][2] = ldg_cached(vp + v2 + vb * 64); va[vb][3] = ldg_cached(vp + v3 + vb * 64);
+        va[vb][0] = load_row(vp + v0 + vb * 64); va[vb][1] = load_row(vp + v1 + vb * 64);
+        va[vb][2] = load_row(vp + v2 + vb * 64); va[vb][3] = load_row(vp + v3 + vb * 64);
       }
       float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -500,7 +579,7 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
 #pragma unroll
       for (int e = 0; e < 4; ++e) p[e] *= split_scale<T>();
       if constexpr (!fp32) add_values<T, VB>(acc, va, p, corr);
-      else add_values_fp32<T, VB>(acc, [&](int k) { return vp + k * row_elems; }, p, corr, last + 1);
+      else add_values_fp32<T, VB, ROPE>(acc, [&](int k) { return vp + k * row_elems; }, p, corr, last + 1);
     }
   };
   attend(std::false_type{});
@@ -602,11 +681,11 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   }
 }
 
-template <typename T, int NS>
+template <typename T, int NS, bool ROPE>
 static int launch_dm(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
-                     int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
-                     cudaStream_t st) {
-  auto kern = decode_attention_mma_kernel<T, NS>;
+                     int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, const DecodeRope& rope,
+                     Prefetch pf, cudaStream_t st) {
+  auto kern = decode_attention_mma_kernel<T, NS, ROPE>;
   if (NS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(NS, B, nkv);
@@ -623,7 +702,7 @@ static int launch_dm(void* out, const void* q, const void* k_pool, const void* v
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (T*)out, (const T*)q, (const T*)k_pool, (const T*)v_pool, page_table, pt_stride,
-                                     page_size, kv_len, kv_len_add, nq, nkv, scale_div, exact_reciprocal(scale_div), pf);
+                                     page_size, kv_len, kv_len_add, nq, nkv, scale_div, exact_reciprocal(scale_div), rope, pf);
   if (e != cudaSuccess) {
     set_error("decode_attention launch: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -632,16 +711,16 @@ static int launch_dm(void* out, const void* q, const void* k_pool, const void* v
   return check_launch("decode_attention");
 }
 
-template <typename T>
+template <typename T, bool ROPE = false>
 static int launch_dm_ns(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
                         int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
-                        cudaStream_t st) {
+                        cudaStream_t st, const DecodeRope& rope = {}) {
   // As many CTAs per (sequence, kv head) as keep the launch within one wave of two per SM (16 is a non-portable size), as far as
   // the GPCs have room for whole clusters: 14 of 16, 33 of 8, 70 of 4.  One cluster more takes a second wave
   // (262 cached tokens: 14 sequences 8.9 us, 15 with clusters of 16 14.3).
   const int seqs = B * nkv;
 #define PG_DM(N_) \
-  return launch_dm<T, N_>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st)
+  return launch_dm<T, N_, ROPE>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, rope, pf, st)
   if (seqs <= 14) PG_DM(16);
   if (seqs <= 33) PG_DM(8);
   if (seqs <= 70) PG_DM(4);
@@ -654,7 +733,41 @@ static int launch_dm_ns(void* out, const void* q, const void* k_pool, const void
 
 using namespace pg;
 
+// the mma kernel: 16-bit pools of 256-wide heads in 16-byte aligned rows, whole 16-token chunks inside a page, and query
+// heads that fit its 8 columns; everything else (fp32, other head sizes) stays on the general kernel
+static bool decode_mma_wanted(const void* q, const void* k_pool, const void* v_pool, int page_size, int G, int hd) {
+  const bool aligned = (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+  return hd == DM_HD && (G == 1 || G == 2 || G == 4 || G == DM_G) && page_size > 0 && page_size % 16 == 0 && aligned;
+}
+
 extern "C" {
+
+int pg_rope_append(void* q_out, const void* qkv, const float* inv_freq, const int32_t* positions, void* k_pool, void* v_pool,
+                   const int32_t* page_table, int pt_stride, int page_size, const int32_t* slot_base, int B, int q_len, int nq,
+                   int nkv, int hd, int max_pos, int dtype, void* stream);
+int pg_decode_attention(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
+                        int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, int hd, float scale_div,
+                        float* ws, int* counters, int max_splits, int dtype, void* stream);
+
+// pg_rope_append for one token of each sequence and pg_decode_attention behind it, in one launch where the mma kernel takes them.
+// `q`: room for the rotated queries of the two launches.
+int pg_decode_attention_rope(void* out, void* q, const void* qkv, const float* inv_freq, const int32_t* positions, void* k_pool,
+                             void* v_pool, const int32_t* page_table, int pt_stride, int page_size, const int32_t* kv_len, int B,
+                             int nq, int nkv, int hd, int max_pos, float scale_div, int dtype, void* stream) {
+  PG_REQUIRE(B > 0 && B <= 65535 && nkv > 0 && nq % nkv == 0, "decode_attention_rope: bad shape");
+  const DecodeRope rope{inv_freq, positions, max_pos};
+#define PG_DM_ARGS \
+  out, qkv, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, 1, B, nq, nkv, scale_div, take_prefetch(), (cudaStream_t)stream, rope
+  if (decode_mma_wanted(qkv, k_pool, v_pool, page_size, nq / nkv, hd) && ((uintptr_t)inv_freq & 7) == 0) {
+    if (dtype == PG_BF16) return launch_dm_ns<bf16, true>(PG_DM_ARGS);
+    if (dtype == PG_F16) return launch_dm_ns<f16, true>(PG_DM_ARGS);
+  }
+#undef PG_DM_ARGS
+  const int rc = pg_rope_append(q, qkv, inv_freq, positions, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, B, 1, nq, nkv,
+                                hd, max_pos, dtype, stream);
+  return rc != PG_OK ? rc : pg_decode_attention(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, 1, B, nq, nkv, hd,
+                                                scale_div, nullptr, nullptr, 0, dtype, stream);
+}
 
 long long pg_decode_attention_ws_floats(int, int, int, int) { return 0; }
 
@@ -666,10 +779,7 @@ int pg_decode_attention(void* out, const void* q, const void* k_pool, const void
   PG_REQUIRE(B > 0 && B <= 65535 && nq % nkv == 0, "decode_attention: bad shape");
   const int G = nq / nkv;
   cudaStream_t st = (cudaStream_t)stream;
-  // the mma kernel: 16-bit pools of 256-wide heads in 16-byte aligned rows, whole 16-token chunks inside a page, and query
-  // heads that fit its 8 columns; everything else (fp32, other head sizes) stays on the general kernel
-  const bool aligned = (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
-  if (hd == DM_HD && (G == 1 || G == 2 || G == 4 || G == DM_G) && page_size > 0 && page_size % 16 == 0 && aligned) {
+  if (decode_mma_wanted(q, k_pool, v_pool, page_size, G, hd)) {
 #define PG_DM_ARGS out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st
     if (dtype == PG_BF16) return launch_dm_ns<bf16>(PG_DM_ARGS);
     if (dtype == PG_F16) return launch_dm_ns<f16>(PG_DM_ARGS);

@@ -69,7 +69,7 @@ __device__ __forceinline__ void add_values(float (&acc)[VB][4][4], const uint4 (
 }
 // The same in fp32 multiplications, key by key: an infinite value times a weight's zero or negative second term is NaN above,
 // times the weight itself infinite.  Keys behind the chunk's last one are left out.  values(k): this lane's columns of key k.
-template <typename T, int VB, typename Row>
+template <typename T, int VB, bool OWN_ROWS = false, typename Row>    // OWN_ROWS: the kernel itself writes some of them
 __device__ __forceinline__ void add_values_fp32(float (&acc)[VB][4][4], Row values, const float (&w)[4], const float (&corr)[2], int keys) {
 #pragma unroll
   for (int vb = 0; vb < VB; ++vb)
@@ -88,7 +88,7 @@ __device__ __forceinline__ void add_values_fp32(float (&acc)[VB][4][4], Row valu
 #pragma unroll
     for (int vb = 0; vb < VB; ++vb) {
       float f[8];
-      unpack<T>(ldg_cached(row + vb * 64), f);
+      unpack<T>(OWN_ROWS ? __ldcg(reinterpret_cast<const uint4*>(row + vb * 64)) : ldg_cached(row + vb * 64), f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float (&o)[4] = acc[vb][i];

@@ -840,14 +840,10 @@ class DecodeState:
         yield
         eng._gemm(self.bqkv, n, w["qkv"])
         yield
-        cabi.check(L.pg_rope_append(ptr(self.q), ptr(self.bqkv), ptr(eng.inv_freq), ptr(self.pos), ptr(kp), ptr(vp),
-                                    ptr(kv.page_table), kv.max_pages, eng.page_size, ptr(kv.kv_len), B, 1, nq, d.nkv,
-                                    d.hd, d.max_pos, dt, st), "rope_append")
-        yield
-        cabi.check(L.pg_decode_attention(ptr(self.att), ptr(self.q), ptr(kp), ptr(vp), ptr(kv.page_table),
-                                         kv.max_pages, eng.page_size, ptr(kv.kv_len), 1, B, nq, d.nkv, d.hd,
-                                         scale_div, ptr(self.ws), ptr(self.counters), eng.max_splits, dt, st),
-                   "decode_attention")
+        cabi.check(L.pg_decode_attention_rope(ptr(self.att), ptr(self.q), ptr(self.bqkv), ptr(eng.inv_freq), ptr(self.pos),
+                                              ptr(kp), ptr(vp), ptr(kv.page_table), kv.max_pages, eng.page_size,
+                                              ptr(kv.kv_len), B, nq, d.nkv, d.hd, d.max_pos, scale_div, dt, st),
+                   "decode_attention_rope")
         yield
         if fab is not None:
             self._partial_push(fab, self.att, w["o"], 2 * li + 1)

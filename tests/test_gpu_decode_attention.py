@@ -104,3 +104,38 @@ def test_infinite_values(dtype, T):
     assert bool((out[:, 3] == math.inf).all()) and bool((out[:, 130] == -math.inf).all()) and bool((out[:, 70] == math.inf).all())
     want = w @ v[:, fine]
     assert float((out[:, fine].to(F64) - want).norm() / want.norm()) < 4e-3      # the bound of bf16 above
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("B,T,G,nkv,page,hd", [(1, 1, 8, 1, 64, 256), (1, 17, 1, 2, 16, 256), (3, 64, 4, 2, 64, 256), (15, 257, 8, 1, 32, 256),
+                                               (40, 49, 2, 1, 64, 256), (80, 130, 8, 1, 64, 256), (150, 33, 8, 1, 64, 256),
+                                               (2, 40, 4, 1, 20, 256), (2, 33, 4, 1, 16, 64)])
+def test_rotary_and_append_inside(dtype, B, T, G, nkv, page, hd):
+    """One call leaves the outputs and the cache that rotary embedding + append and the attention leave as two, bit for bit."""
+    from pg_b200 import _cabi as cabi
+    L, nq, max_pos = cabi.lib(), G * nkv, 512
+    g = torch.Generator(device="cuda").manual_seed(B * 1000 + T)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    kvl = torch.randint(max(0, T - 40), T, (B,), device="cuda", generator=g).to(torch.int32)
+    kvl[0] = T - 1
+    pos = torch.randint(-1, max_pos + 2, (B,), device="cuda", generator=g).to(torch.int32)   # the ends are clamped
+    cols = -(-T // page)
+    pages = B * cols + 2
+    pt = torch.randperm(pages, device="cuda", generator=g)[:B * cols].to(torch.int32).view(B, cols)
+    pools, qkv = [new(pages, page, nkv * hd) for _ in "kv"], new(B, (nq + 2 * nkv) * hd)
+    freq = 1.0 / 10000 ** (torch.arange(0, hd, 2, device="cuda").float() / hd)
+    code, st, scale = cabi.DTYPE_CODE[dtype], cabi.stream(), math.sqrt(hd)
+    results = []
+    for one_call in (False, True):
+        kp, vp = (p.clone() for p in pools)
+        q, out = torch.zeros(B, nq * hd, dtype=dtype, device="cuda"), torch.zeros(B, nq * hd, dtype=dtype, device="cuda")
+        where = (kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page, kvl.data_ptr())
+        if one_call:
+            cabi.check(L.pg_decode_attention_rope(out.data_ptr(), q.data_ptr(), qkv.data_ptr(), freq.data_ptr(), pos.data_ptr(), *where,
+                                                  B, nq, nkv, hd, max_pos, scale, code, st))
+        else:
+            cabi.check(L.pg_rope_append(q.data_ptr(), qkv.data_ptr(), freq.data_ptr(), pos.data_ptr(), *where, B, 1, nq, nkv, hd,
+                                        max_pos, code, st))
+            cabi.check(L.pg_decode_attention(out.data_ptr(), q.data_ptr(), *where, 1, B, nq, nkv, hd, scale, None, None, 0, code, st))
+        results.append((out, kp, vp))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
