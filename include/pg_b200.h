@@ -186,6 +186,12 @@ int pg_decode_attention(void* out, const void* q, const void* k_pool, const void
                         const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, int hd,
                         float scale_div, float* ws, int* counters, int max_splits, int dtype,
                         void* stream);
+/* pg_rope_append of one token per sequence and pg_decode_attention (kv_len_add 1) behind it, in one launch for 16-bit heads of 256 in
+   pages of whole 16-token chunks, as those two launches otherwise.  q: room for the rotated queries [B][nq hd]. */
+int pg_decode_attention_rope(void* out, void* q, const void* qkv, const float* inv_freq, const int32_t* positions,
+                             void* k_pool, void* v_pool, const int32_t* page_table, int pt_stride, int page_size,
+                             const int32_t* kv_len, int B, int nq, int nkv, int hd, int max_pos, float scale_div,
+                             int dtype, void* stream);
 
 /* out[B,N] = (x[B,K] W[N,K]^T) + R  — o_proj / down_proj with the residual add
  * (modeling_gemma.py:291,327 and :134,336).  R may be NULL.  ex != NULL (tensor parallel: W holds this rank's K

@@ -27,7 +27,6 @@ struct SnParams {
   const void* R;
   int M, N, K, ldc, ldr, out_f32;
   int w_param;   // W is no output of a preceding launch: it may be requested before the dependency wait
-  int vec;       // four neighbouring features of C, R and bias are one aligned access
 };
 
 __device__ __forceinline__ void sn_cluster_sync() {
@@ -221,14 +220,9 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     constexpr bool HAS_RES = EPI == PG_EPI_BIAS_RES || EPI == PG_EPI_RES;
     float res[STEPS][4], bn[4] = {0.f, 0.f, 0.f, 0.f};
     auto four = [&](const T* at, float (&v)[4]) {
-      if (p.vec) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2*>(at));
-        unpack_pair<T>(u.x, v);
-        unpack_pair<T>(u.y, v + 2);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = to_f<T>(at[j]);
-      }
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(at));   // gemm_tc takes rows on 16-byte boundaries only
+      unpack_pair<T>(u.x, v);
+      unpack_pair<T>(u.y, v + 2);
     };
     if (warp >= 4) {
       // bias and residual are requested before the accumulator is waited for (N is a multiple of 8)
@@ -280,13 +274,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
           if (HAS_RES) x = rnd<T>(x + res[i][j]);
           v[i][j] = x;
         }
-        if (!p.vec) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (p.out_f32) Cf[(size_t)m * p.ldc + n + j] = v[i][j];
-            else Ct[(size_t)m * p.ldc + n + j] = from_f<T>(v[i][j]);
-          }
-        } else if (p.out_f32) {
+        if (p.out_f32) {
           *reinterpret_cast<float4*>(Cf + (size_t)m * p.ldc + n) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
         } else {
           *reinterpret_cast<uint2*>(Ct + (size_t)m * p.ldc + n) = make_uint2(pack_pair<T>(v[i][0], v[i][1]), pack_pair<T>(v[i][2], v[i][3]));
@@ -369,8 +357,7 @@ int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, cons
   const int w_rows = (epi == PG_EPI_GEGLU) ? 2 * N : N;
   PG_REQUIRE(tc::make_map_2d(&mx, A, M, K, lda, nt, bf) && tc::make_map_2d(&mw, W, w_rows, K, ldw, tc::SN_BM, bf),
              "gemm_tc_skinny: cuTensorMapEncodeTiled failed");
-  const int vec = (uintptr_t)C % (out_f32 ? 16 : 8) == 0 && ((uintptr_t)R | (uintptr_t)bias) % 8 == 0 && (!R || ldr % 4 == 0);
-  tc::SnParams p = {C, bias, R, M, N, K, ldc, ldr, out_f32, w_param, vec};
+  tc::SnParams p = {C, bias, R, M, N, K, ldc, ldr, out_f32, w_param};
 #define PG_SN(E) return bf ? tc::launch_sn_nt<bf16, E>(mx, mw, p, nt, s, st) : tc::launch_sn_nt<f16, E>(mx, mw, p, nt, s, st)
   switch (epi) {
     case PG_EPI_NONE: PG_SN(PG_EPI_NONE);

@@ -82,6 +82,34 @@ def test_few_rows_split_over_clusters(M, N, K, epi, dtype):
     assert bool((out[M] == 0).all())
 
 
+# partial sums of a split over K change hands by whole row pieces: row tiles with missing rows, feature tiles with missing columns,
+# rows past 256 in a second token tile; results have the roundings of the products above, fp32 ones too (the type's values, widened)
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("impl,M,N,K,epi,f32", [
+    (0, 33, 1152, 4304, "res", 0), (0, 129, 1152, 1152, "none", 0), (0, 257, 1160, 4304, "res", 0), (0, 256, 1152, 4304, "res", 0),
+    (0, 260, 2048, 2048, "res", 0), (0, 385, 520, 4096, "none", 1), (0, 161, 2056, 2048, "none", 1),
+    (0, 5, 2048, 2048, "res", 0), (0, 32, 2056, 16384, "res", 0), (0, 17, 2048, 4096, "none", 1),
+    (3, 256, 264, 4096, "res", 0), (3, 257, 2048, 16384, "res", 0), (3, 271, 1000, 2048, "none", 0), (3, 273, 264, 4096, "res", 0),
+    (3, 384, 2056, 2048, "geglu", 0), (3, 511, 136, 8192, "res", 0)])
+def test_partial_sums_change_hands(impl, M, N, K, epi, f32, dtype):
+    cabi, L, st = _cabi()
+    ws = torch.empty(80 << 20, dtype=torch.uint8, device="cuda")
+    cabi.check(L.pg_set_workspace(ws.data_ptr(), ws.numel()))
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rows = 2 * N if epi == "geglu" else N
+    a, w = _randn(g, M, K, dtype=dtype), _randn(g, rows, K, std=K ** -0.5, dtype=dtype)
+    r = _randn(g, M, N, dtype=dtype)
+    out = torch.zeros((M + 1) * N, dtype=torch.float32 if f32 else dtype, device="cuda").view(M + 1, N)
+    code = {"res": cabi.EPI_RES, "none": cabi.EPI_NONE, "geglu": cabi.EPI_GEGLU}[epi]
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr() if epi == "res" else None, M, N, K, K, K, N,
+                         N if epi == "res" else 0, 0, code, f32, impl, cabi.DTYPE_CODE[dtype], st))
+    z = a.to(F64) @ w.to(F64).T
+    want = _gelu(z[:, :N]) * z[:, N:] if epi == "geglu" else z + r.to(F64) if epi == "res" else z
+    assert _rel(out[:M], want) < _tol(dtype, 5e-3 if epi == "geglu" else 4e-3, epi == "geglu")
+    assert bool((out[M] == 0).all())
+    cabi.check(L.pg_set_workspace(None, 0))
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("act,rel", [("none", 4e-3), ("silu", 5e-3), ("clamped", 6e-3), ("relu2", 6e-3)])
 @pytest.mark.parametrize("rows", [[1200, 0, 257, 1], [256, 256, 512, 1024], [3000, 5], [3, 1, 0, 2, 0, 1, 4, 5]])
