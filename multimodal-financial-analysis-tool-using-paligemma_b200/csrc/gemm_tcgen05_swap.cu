@@ -199,10 +199,13 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int j = 0; j < 16; ++j) row[j * SW_WROWS] = v[j];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-        if (store_thread && f0 < p.N && t * p.NT + cc * 16 < p.M) {
-          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"   // clipped at N and at M
-                       ::"l"(reinterpret_cast<uint64_t>(&map_p)), "r"(out_base + (half * 2 + buf) * SW_OUT_BYTES), "r"(f0),
-                       "r"(t * p.NT + cc * 16), "r"(sp) : "memory");
+        if (store_thread) {
+          if (f0 < p.N)
+            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"   // clipped at N and at M
+                         ::"l"(reinterpret_cast<uint64_t>(&map_p)), "r"(out_base + (half * 2 + buf) * SW_OUT_BYTES), "r"(f0),
+                         "r"(t * p.NT + cc * 16), "r"(sp) : "memory");
+          // A group for every chunk, be it empty: the wait above counts groups.  Without one for the chunks of a CTA whose features
+          // lie past N, the group it lets pend is the last store of the item before, out of the buffer that is written next.
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }

@@ -31,3 +31,17 @@ def pytest_collection_modifyitems(config, items):
 @pytest.fixture(scope="session")
 def golden_dir():
     return GOLDEN
+
+
+@pytest.fixture
+def gemm_workspace():
+    """80 MB of scratch for the split products (pg_set_workspace) for one test; then the process's own again: the engines', or none."""
+    import torch
+    from pg_b200 import _cabi as cabi
+    from pg_b200.engine import _WORKSPACES
+    L, ws = cabi.lib(), torch.empty(80 << 20, dtype=torch.uint8, device="cuda")
+    cabi.check(L.pg_set_workspace(ws.data_ptr(), ws.numel()))
+    yield ws
+    torch.cuda.synchronize()
+    own = _WORKSPACES.get((torch.cuda.current_device(),))
+    cabi.check(L.pg_set_workspace(own.data_ptr(), own.numel()) if own is not None else L.pg_set_workspace(None, 0))

@@ -110,6 +110,36 @@ def test_partial_sums_change_hands(impl, M, N, K, epi, f32, dtype):
     cabi.check(L.pg_set_workspace(None, 0))
 
 
+# More weight tiles than CTA pairs (74), the last of them of at most 128 features: a pair's second item, in which one CTA has nothing to
+# store, with so short a K that the first item's last store may still be under way.  Every repetition has to give the same bits.
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("impl,M,N,K,epi", [(0, 100, 19008, 64, "res"), (0, 65, 19072, 256, "res"), (3, 128, 9536, 64, "geglu"),
+                                            (3, 300, 18952, 64, "none"), (3, 33, 37960, 128, "res")])
+def test_a_half_empty_tile_behind_a_whole_one(gemm_workspace, impl, M, N, K, epi, dtype):
+    cabi, L, st = _cabi()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rows = 2 * N if epi == "geglu" else N
+    assert -(-rows // 256) > 74 and 1 <= rows % 256 <= 128
+    a, w = _randn(g, M, K, dtype=dtype), _randn(g, rows, K, std=K ** -0.5, dtype=dtype)
+    r = _randn(g, M, N, dtype=dtype)
+    code = {"res": cabi.EPI_RES, "none": cabi.EPI_NONE, "geglu": cabi.EPI_GEGLU}[epi]
+    z = a.to(F64) @ w.to(F64).T
+    want = _gelu(z[:, :N]) * z[:, N:] if epi == "geglu" else z + r.to(F64) if epi == "res" else z
+    first = None
+    for _ in range(24):
+        gemm_workspace.fill_(0xff)                                             # NaN where nothing is stored
+        out = torch.zeros(M + 1, N, dtype=dtype, device="cuda")
+        before = cabi.launch_count()
+        cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr() if epi == "res" else None, M, N, K, K, K, N,
+                             N if epi == "res" else 0, 0, code, 0, impl, cabi.DTYPE_CODE[dtype], st))
+        assert cabi.launch_count() - before == 2                               # the pair kernel and its reduction
+        if first is None:
+            first = out
+            assert _rel(out[:M], want) < _tol(dtype, 5e-3 if epi == "geglu" else 4e-3, epi == "geglu")
+            assert bool((out[M] == 0).all())
+        assert torch.equal(out, first)
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("act,rel", [("none", 4e-3), ("silu", 5e-3), ("clamped", 6e-3), ("relu2", 6e-3)])
 @pytest.mark.parametrize("rows", [[1200, 0, 257, 1], [256, 256, 512, 1024], [3000, 5], [3, 1, 0, 2, 0, 1, 4, 5]])
