@@ -398,10 +398,10 @@ struct DecodeRope {
   int max_pos;
 };
 
-template <typename T, int NS, bool ROPE>
+template <typename T, int NS, bool ROPE, bool AHEAD>
 __global__ void __launch_bounds__(DM_WARPS * 32, 2)
 decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const T* k_pool, const T* v_pool,
-                            const int32_t* __restrict__ page_table, int pt_stride, int page_size,
+                            const int32_t* __restrict__ page_table, int pt_stride, int page_size, int num_pages,
                             const int32_t* __restrict__ kv_len, int kv_len_add, int nq, int nkv, float scale_div,
                             float scale_mul, DecodeRope rope, Prefetch pf) {
   constexpr int KB = DM_HD / 32, VB = DM_HD / 64;
@@ -420,12 +420,15 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   const int32_t* pt = page_table + (size_t)b * pt_stride;
   const size_t row_elems = (size_t)nkv * DM_HD;
   // While the preceding kernel runs (1.5 to 2.5 us in a captured step): this warp's first four chunks into L2.  A hint only: the length
-  // and the page numbers it goes by are read again behind the wait.
+  // and the page numbers it goes by are read again behind the wait.  The preceding kernel may be about to write them, so a number
+  // names an address only if the pool has that page; where the caller did not say how many it has (!AHEAD), nothing is asked for.
   const int jp = threadIdx.x & 63;
-  int ahead[4];
+  int ahead[4], t_end = 0;
+  if constexpr (AHEAD) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) ahead[i] = __ldcg(pt + min((rank + NS * (wid + DM_WARPS * i)) * 16 / page_size, pt_stride - 1));
-  const int t_end = __ldcg(kv_len + b) + kv_len_add;
+    for (int i = 0; i < 4; ++i) ahead[i] = __ldcg(pt + min((rank + NS * (wid + DM_WARPS * i)) * 16 / page_size, pt_stride - 1));
+    t_end = __ldcg(kv_len + b) + kv_len_add;
+  }
   // ... and the angles of this thread's columns 2 jp, 2 jp + 1, done again if what they come from is another behind the wait
   float angle[2] = {0.f, 0.f}, c[2], s[2];
   auto angles = [&] {
@@ -437,15 +440,17 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
     return other;
   };
   if constexpr (ROPE) angles();
+  if constexpr (AHEAD) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = (rank + NS * (wid + DM_WARPS * i)) * 16 + (lane >> 1);
-    if (t >= t_end || ahead[i] < 0) break;
-    const size_t at = ((size_t)ahead[i] * page_size + t % page_size) * row_elems + (size_t)kvh * DM_HD + (lane & 1) * 128;
-    prefetch_l2(k_pool + at);
-    prefetch_l2(k_pool + at + 64);
-    prefetch_l2(v_pool + at);
-    prefetch_l2(v_pool + at + 64);
+    for (int i = 0; i < 4; ++i) {
+      const int t = (rank + NS * (wid + DM_WARPS * i)) * 16 + (lane >> 1);
+      if (t >= t_end || (unsigned)ahead[i] >= (unsigned)num_pages) break;
+      const size_t at = ((size_t)ahead[i] * page_size + t % page_size) * row_elems + (size_t)kvh * DM_HD + (lane & 1) * 128;
+      prefetch_l2(k_pool + at);
+      prefetch_l2(k_pool + at + 64);
+      prefetch_l2(v_pool + at);
+      prefetch_l2(v_pool + at + 64);
+    }
   }
   if constexpr (ROPE) {
 #pragma unroll
@@ -681,11 +686,11 @@ decode_attention_mma_kernel(T* __restrict__ out, const T* __restrict__ q, const 
   }
 }
 
-template <typename T, int NS, bool ROPE>
+template <typename T, int NS, bool ROPE, bool AHEAD>
 static int launch_dm(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
-                     int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, const DecodeRope& rope,
-                     Prefetch pf, cudaStream_t st) {
-  auto kern = decode_attention_mma_kernel<T, NS, ROPE>;
+                     int page_size, int num_pages, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div,
+                     const DecodeRope& rope, Prefetch pf, cudaStream_t st) {
+  auto kern = decode_attention_mma_kernel<T, NS, ROPE, AHEAD>;
   if (NS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(NS, B, nkv);
@@ -702,7 +707,7 @@ static int launch_dm(void* out, const void* q, const void* k_pool, const void* v
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (T*)out, (const T*)q, (const T*)k_pool, (const T*)v_pool, page_table, pt_stride,
-                                     page_size, kv_len, kv_len_add, nq, nkv, scale_div, exact_reciprocal(scale_div), rope, pf);
+                                     page_size, num_pages, kv_len, kv_len_add, nq, nkv, scale_div, exact_reciprocal(scale_div), rope, pf);
   if (e != cudaSuccess) {
     set_error("decode_attention launch: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -711,16 +716,17 @@ static int launch_dm(void* out, const void* q, const void* k_pool, const void* v
   return check_launch("decode_attention");
 }
 
-template <typename T, bool ROPE = false>
+template <typename T, bool ROPE, bool AHEAD>
 static int launch_dm_ns(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
-                        int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div, Prefetch pf,
-                        cudaStream_t st, const DecodeRope& rope = {}) {
+                        int page_size, int num_pages, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, float scale_div,
+                        Prefetch pf, cudaStream_t st, const DecodeRope& rope) {
   // As many CTAs per (sequence, kv head) as keep the launch within one wave of two per SM (16 is a non-portable size), as far as
   // the GPCs have room for whole clusters: 14 of 16, 33 of 8, 70 of 4.  One cluster more takes a second wave
   // (262 cached tokens: 14 sequences 8.9 us, 15 with clusters of 16 14.3).
   const int seqs = B * nkv;
 #define PG_DM(N_) \
-  return launch_dm<T, N_, ROPE>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, rope, pf, st)
+  return launch_dm<T, N_, ROPE, AHEAD>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, num_pages, kv_len, kv_len_add, B, nq, nkv, \
+                                scale_div, rope, pf, st)
   if (seqs <= 14) PG_DM(16);
   if (seqs <= 33) PG_DM(8);
   if (seqs <= 70) PG_DM(4);
@@ -745,45 +751,32 @@ extern "C" {
 int pg_rope_append(void* q_out, const void* qkv, const float* inv_freq, const int32_t* positions, void* k_pool, void* v_pool,
                    const int32_t* page_table, int pt_stride, int page_size, const int32_t* slot_base, int B, int q_len, int nq,
                    int nkv, int hd, int max_pos, int dtype, void* stream);
-int pg_decode_attention(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
-                        int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, int hd, float scale_div,
-                        float* ws, int* counters, int max_splits, int dtype, void* stream);
-
-// pg_rope_append for one token of each sequence and pg_decode_attention behind it, in one launch where the mma kernel takes them.
-// `q`: room for the rotated queries of the two launches.
-int pg_decode_attention_rope(void* out, void* q, const void* qkv, const float* inv_freq, const int32_t* positions, void* k_pool,
-                             void* v_pool, const int32_t* page_table, int pt_stride, int page_size, const int32_t* kv_len, int B,
-                             int nq, int nkv, int hd, int max_pos, float scale_div, int dtype, void* stream) {
-  PG_REQUIRE(B > 0 && B <= 65535 && nkv > 0 && nq % nkv == 0, "decode_attention_rope: bad shape");
-  const DecodeRope rope{inv_freq, positions, max_pos};
-#define PG_DM_ARGS \
-  out, qkv, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, 1, B, nq, nkv, scale_div, take_prefetch(), (cudaStream_t)stream, rope
-  if (decode_mma_wanted(qkv, k_pool, v_pool, page_size, nq / nkv, hd) && ((uintptr_t)inv_freq & 7) == 0) {
-    if (dtype == PG_BF16) return launch_dm_ns<bf16, true>(PG_DM_ARGS);
-    if (dtype == PG_F16) return launch_dm_ns<f16, true>(PG_DM_ARGS);
-  }
-#undef PG_DM_ARGS
-  const int rc = pg_rope_append(q, qkv, inv_freq, positions, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, B, 1, nq, nkv,
-                                hd, max_pos, dtype, stream);
-  return rc != PG_OK ? rc : pg_decode_attention(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, 1, B, nq, nkv, hd,
-                                                scale_div, nullptr, nullptr, 0, dtype, stream);
-}
-
-long long pg_decode_attention_ws_floats(int, int, int, int) { return 0; }
-
-int pg_decode_attention(void* out, const void* q, const void* k_pool, const void* v_pool,
-                        const int32_t* page_table, int pt_stride, int page_size, const int32_t* kv_len,
-                        int kv_len_add, int B, int nq, int nkv, int hd, float scale_div, float* /*ws*/,
-                        int* /*counters*/, int /*max_splits*/, int dtype, void* stream) {
+// One token of each sequence.  qkv: the q/k/v projections, rotated and appended first, in the same launch where the mma kernel takes
+// them, else by pg_rope_append into `q` (room for the rotated queries); NULL: q is rotated already and the row in the cache.
+int pg_decode_attention_ex(void* out, void* q, void* k_pool, void* v_pool, const int32_t* page_table, int pt_stride, int page_size,
+                           int num_pages, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, int hd, float scale_div,
+                           const void* qkv, const float* inv_freq, const int32_t* positions, int max_pos, int dtype, void* stream) {
   const Prefetch pf = take_prefetch();
-  PG_REQUIRE(B > 0 && B <= 65535 && nq % nkv == 0, "decode_attention: bad shape");
+  PG_REQUIRE(B > 0 && B <= 65535 && nkv > 0 && nq % nkv == 0, "decode_attention: bad shape");
+  PG_REQUIRE(!qkv || kv_len_add == 1, "decode_attention: the appended row is one more than kv_len");
   const int G = nq / nkv;
   cudaStream_t st = (cudaStream_t)stream;
-  if (decode_mma_wanted(q, k_pool, v_pool, page_size, G, hd)) {
-#define PG_DM_ARGS out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st
-    if (dtype == PG_BF16) return launch_dm_ns<bf16>(PG_DM_ARGS);
-    if (dtype == PG_F16) return launch_dm_ns<f16>(PG_DM_ARGS);
-#undef PG_DM_ARGS
+  const void* rows = qkv ? qkv : q;
+  if (decode_mma_wanted(rows, k_pool, v_pool, page_size, G, hd) && (!qkv || ((uintptr_t)inv_freq & 7) == 0) &&
+      (dtype == PG_BF16 || dtype == PG_F16)) {
+    const DecodeRope rope{inv_freq, positions, max_pos};
+#define PG_DM(ROPE, AHEAD)                                                                                                       \
+  return (dtype == PG_BF16 ? launch_dm_ns<bf16, ROPE, AHEAD> : launch_dm_ns<f16, ROPE, AHEAD>)(                                    \
+      out, rows, k_pool, v_pool, page_table, pt_stride, page_size, num_pages, kv_len, kv_len_add, B, nq, nkv, scale_div, pf, st, rope)
+    if (qkv) PG_DM(true, true);       // not counted: its pages are all past the end
+    if (num_pages > 0) PG_DM(false, true);
+    PG_DM(false, false);
+#undef PG_DM
+  }
+  if (qkv) {
+    const int rc = pg_rope_append(q, qkv, inv_freq, positions, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, B, 1, nq, nkv,
+                                  hd, max_pos, dtype, stream);
+    if (rc != PG_OK) return rc;
   }
 #define PG_DA(GG, NCH) \
   return launch_da<T, GG, NCH>(out, q, k_pool, v_pool, page_table, pt_stride, page_size, kv_len, kv_len_add, B, nq, nkv, hd, scale_div, pf, st)
@@ -812,5 +805,22 @@ int pg_decode_attention(void* out, const void* q, const void* k_pool, const void
 #undef PG_DA
   return PG_OK;
 }
+
+int pg_decode_attention(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* page_table, int pt_stride,
+                        int page_size, const int32_t* kv_len, int kv_len_add, int B, int nq, int nkv, int hd, float scale_div,
+                        float* /*ws*/, int* /*counters*/, int /*max_splits*/, int dtype, void* stream) {
+  return pg_decode_attention_ex(out, const_cast<void*>(q), const_cast<void*>(k_pool), const_cast<void*>(v_pool), page_table, pt_stride,
+                                page_size, 0, kv_len, kv_len_add, B, nq, nkv, hd, scale_div, nullptr, nullptr, nullptr, 0, dtype, stream);
+}
+
+int pg_decode_attention_rope(void* out, void* q, const void* qkv, const float* inv_freq, const int32_t* positions, void* k_pool,
+                             void* v_pool, const int32_t* page_table, int pt_stride, int page_size, const int32_t* kv_len, int B,
+                             int nq, int nkv, int hd, int max_pos, float scale_div, int dtype, void* stream) {
+  PG_REQUIRE(qkv, "decode_attention_rope: no projections");
+  return pg_decode_attention_ex(out, q, k_pool, v_pool, page_table, pt_stride, page_size, 0, kv_len, 1, B, nq, nkv, hd, scale_div, qkv,
+                                inv_freq, positions, max_pos, dtype, stream);
+}
+
+long long pg_decode_attention_ws_floats(int, int, int, int) { return 0; }
 
 }  // extern "C"

@@ -51,6 +51,7 @@ SIGNATURES = {
     "pg_set_next_prefetch": [_vp, _ll],
     "pg_decode_qkv": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f,
                       _i, _vp, _vp, _i, _vp],
+    "pg_decode_attention_ex": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp, _i, _i, _vp],
     "pg_decode_attention_rope": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _i, _vp],
     "pg_decode_attention_ws_floats": [_i, _i, _i, _i],
     "pg_decode_attention": [_vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _vp, _vp, _i,

@@ -185,7 +185,6 @@ class PaliGemmaEngine(PagePool):
         self.err_flag = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._err_np = self.err_flag.numpy()
         self.err_info = torch.zeros(3, dtype=torch.int64).pin_memory()   # of the token that set it: id, place, step or -1
-        self.max_splits = 32
         self._decode_states: Dict[tuple, "DecodeState"] = {}
         # scratch for the split-K prompt GEMMs (fp32 partials; 512 tokens x 2F features is the largest user)
         if self.dtype != torch.float32:
@@ -619,8 +618,6 @@ class DecodeState:
         self.q = eng._new(batch, eng.nq_l * d.hd)
         self.att = eng._new(batch, eng.nq_l * d.hd)
         self.g = eng._new(batch, eng.F_l)
-        self.ws = torch.zeros(1, dtype=torch.float32, device=dev)       # (unused by the cluster kernel)
-        self.counters = torch.zeros(batch * d.nkv, dtype=torch.int32, device=dev)
         tp = eng.tp
         self.local_logits = self.logits if not tp.active else torch.zeros((batch, eng.V_l), dtype=torch.float32, device=dev)
         self.gather_logits = torch.zeros((tp.size, batch, eng.V_l), dtype=torch.float32, device=dev) if tp.active else None
@@ -695,10 +692,9 @@ class DecodeState:
                        "decode_qkv")
             yield
         self._pf(w["gu"])                                  # attention pulls the head of gate/up
-        cabi.check(L.pg_decode_attention(ptr(self.att), ptr(self.q), ptr(kp), ptr(vp), ptr(kv.page_table),
-                                         kv.max_pages, eng.page_size, ptr(kv.kv_len), 1, B, nq, d.nkv, d.hd,
-                                         scale_div, ptr(self.ws), ptr(self.counters), eng.max_splits, dt, st),
-                   "decode_attention")
+        cabi.check(L.pg_decode_attention_ex(ptr(self.att), ptr(self.q), ptr(kp), ptr(vp), ptr(kv.page_table),
+                                            kv.max_pages, eng.page_size, eng.num_pages, ptr(kv.kv_len), 1, B, nq, d.nkv, d.hd,
+                                            scale_div, None, None, None, 0, dt, st), "decode_attention")
         yield
         if fab is not None:
             # producer -> consumer pairs: the partial sums travel inside the kernels (csrc/tp_exchange.cuh)
@@ -840,10 +836,10 @@ class DecodeState:
         yield
         eng._gemm(self.bqkv, n, w["qkv"])
         yield
-        cabi.check(L.pg_decode_attention_rope(ptr(self.att), ptr(self.q), ptr(self.bqkv), ptr(eng.inv_freq), ptr(self.pos),
-                                              ptr(kp), ptr(vp), ptr(kv.page_table), kv.max_pages, eng.page_size,
-                                              ptr(kv.kv_len), B, nq, d.nkv, d.hd, d.max_pos, scale_div, dt, st),
-                   "decode_attention_rope")
+        cabi.check(L.pg_decode_attention_ex(ptr(self.att), ptr(self.q), ptr(kp), ptr(vp), ptr(kv.page_table),
+                                            kv.max_pages, eng.page_size, eng.num_pages, ptr(kv.kv_len), 1, B, nq, d.nkv, d.hd,
+                                            scale_div, ptr(self.bqkv), ptr(eng.inv_freq), ptr(self.pos), d.max_pos, dt, st),
+                   "decode_attention")
         yield
         if fab is not None:
             self._partial_push(fab, self.att, w["o"], 2 * li + 1)

@@ -139,3 +139,90 @@ def test_rotary_and_append_inside(dtype, B, T, G, nkv, page, hd):
             cabi.check(L.pg_decode_attention(out.data_ptr(), q.data_ptr(), *where, 1, B, nq, nkv, hd, scale, None, None, 0, code, st))
         results.append((out, kp, vp))
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def _rotated(rows, freq, pos, dtype):
+    """The rotary embedding's products and sums, each rounded to the type.  rows [B, heads, hd]."""
+    ang = pos.clamp(min=0)[:, None, None].float() * freq
+    c, s = ang.cos().to(dtype), ang.sin().to(dtype)
+    x, y = rows.chunk(2, -1)
+    return torch.cat([x * c + -y * s, y * c + x * s], -1)
+
+
+@pytest.mark.parametrize("dtype,rel", [(torch.bfloat16, 4e-3), (torch.float16, 6e-4)])
+@pytest.mark.parametrize("B,T,G,page", [(1, 1, 8, 64), (2, 37, 8, 64), (3, 262, 4, 16), (1, 1345, 2, 64), (80, 100, 8, 64)])
+def test_infinite_values_behind_a_rotation(dtype, rel, B, T, G, page):
+    """The same with the rotation and the new row inside, the last infinity in the new row, against float64."""
+    from pg_b200 import _cabi as cabi
+    hd = 256
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    cols = -(-T // page)
+    pages = B * cols
+    kp, vp, qkv = new(pages, page, hd) * 0.3, new(pages, page, hd), new(B, G + 2, hd) * 0.3
+    pt = torch.randperm(pages, device="cuda", generator=g).to(torch.int32).view(B, cols)
+    kvl, pos = (torch.full((B,), n, dtype=torch.int32, device="cuda") for n in (T - 1, 41))
+    freq = 1.0 / 10000 ** (torch.arange(0, hd, 2, device="cuda").float() / hd)
+    for token, col, value in ((0, 3, math.inf), (T // 2, 130, -math.inf)):
+        if token < T - 1:
+            vp[pt[:, token // page].long(), token % page, col] = value
+        else:
+            qkv[:, G + 1, col] = value
+    qkv[:, G + 1, 70] = math.inf
+    q, out = torch.zeros(B, G * hd, dtype=dtype, device="cuda"), torch.zeros(B, G, hd, dtype=dtype, device="cuda")
+    cabi.check(cabi.lib().pg_decode_attention_ex(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page, pages,
+                                                 kvl.data_ptr(), 1, B, G, 1, hd, 16.0, qkv.data_ptr(), freq.data_ptr(), pos.data_ptr(), 512,
+                                                 cabi.DTYPE_CODE[dtype], cabi.stream()))
+    turned = _rotated(qkv[:, :G + 1], freq, pos, dtype)
+    for b in sorted({0, B // 2, B - 1}):
+        k, v = (torch.cat([p[pt[b].long()].reshape(-1, hd)[:T - 1], row]).to(F64) for p, row in ((kp, turned[b, G:]), (vp, qkv[b, G + 1:])))
+        w = torch.softmax((turned[b, :G].to(F64) @ k.T).to(dtype).to(F64) / 16.0, -1)
+        fine, o = torch.isfinite(v).all(0), out[b]
+        assert bool((o[:, 3] == math.inf).all()) and bool((o[:, 130] == -math.inf).all()) and bool((o[:, 70] == math.inf).all())
+        want = w @ v[:, fine]
+        assert float((o[:, fine].to(F64) - want).norm() / want.norm()) < rel           # the bound of finite values above
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,counted", [(1, 61, "all"), (8, 257, "all"), (8, 257, "one"), (8, 257, "none"), (40, 15, "all")])
+def test_steps_follow_one_another(dtype, B, T, counted):
+    """A captured step whose lengths and positions are moved on in front of it, replayed: what is read ahead of the launch before is
+    read again behind it, whether the table's pages are known to be the pool's or not.  Against the two launches, bit for bit."""
+    from pg_b200 import _cabi as cabi
+    L, hd, G, page, steps = cabi.lib(), 256, 8, 16, 5
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    cols = -(-(T + steps) // page)
+    pages = B * cols
+    pt = torch.randperm(pages, device="cuda", generator=g).to(torch.int32).view(B, cols)
+    pools, qkv, w = [new(pages, page, hd) for _ in "kv"], new(B, (G + 2) * hd), new(1152)
+    freq = 1.0 / 10000 ** (torch.arange(0, hd, 2, device="cuda").float() / hd)
+    kvl, pos = (torch.full((B,), n, dtype=torch.int32, device="cuda") for n in (T - 2, T + 6))
+    ids, keys = torch.zeros(B, dtype=torch.int64, device="cuda"), torch.zeros(B, dtype=torch.int64, device="cuda")
+    x, y = new(B, 1152), new(B, 1152)
+    q, out = torch.zeros(B, G * hd, dtype=dtype, device="cuda"), torch.zeros(B, G * hd, dtype=dtype, device="cuda")
+    (kp, vp), (kr, vr) = pools, [torch.empty_like(p) for p in pools]
+    qr, want = torch.zeros_like(q), torch.zeros_like(out)
+    code, num = cabi.DTYPE_CODE[dtype], {"all": pages, "one": 1, "none": 0}[counted]
+
+    def step():
+        st = cabi.stream()
+        cabi.check(L.pg_step_advance(ids.data_ptr(), None, 0, None, keys.data_ptr(), ids.data_ptr(), kvl.data_ptr(), pos.data_ptr(), B, None, st))
+        cabi.check(L.pg_rmsnorm(y.data_ptr(), x.data_ptr(), w.data_ptr(), B, 1152, 1e-6, code, st))   # lets the next launch start early
+        cabi.check(L.pg_decode_attention_ex(out.data_ptr(), q.data_ptr(), kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), cols, page, num,
+                                            kvl.data_ptr(), 1, B, G, 1, hd, 16.0, qkv.data_ptr(), freq.data_ptr(), pos.data_ptr(), 512, code, st))
+    step()
+    for ref, pool in ((kr, kp), (vr, vp)):
+        ref.copy_(pool)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        step()
+    for _ in range(steps):
+        graph.replay()
+        st, where = cabi.stream(), (kr.data_ptr(), vr.data_ptr(), pt.data_ptr(), cols, page, kvl.data_ptr())
+        cabi.check(L.pg_rope_append(qr.data_ptr(), qkv.data_ptr(), freq.data_ptr(), pos.data_ptr(), *where, B, 1, G, 1, hd, 512, code, st))
+        cabi.check(L.pg_decode_attention(want.data_ptr(), qr.data_ptr(), *where, 1, B, G, 1, hd, 16.0, None, None, 0, code, st))
+        assert torch.equal(out, want) and torch.equal(kp, kr) and torch.equal(vp, vr)
+        qkv.copy_(new(B, (G + 2) * hd))
+    assert int(kvl[0]) == T - 1 + steps

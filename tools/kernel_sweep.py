@@ -85,9 +85,9 @@ def main():
 
     def attn():
         for li, w in enumerate(eng.t_layers):
-            L.pg_decode_attention(ds.att.data_ptr(), ds.q.data_ptr(), eng.k_pool[li].data_ptr(), eng.v_pool[li].data_ptr(),
-                                  kv.page_table.data_ptr(), kv.max_pages, eng.page_size, kv.kv_len.data_ptr(), 1, B, nq, d.nkv,
-                                  d.hd, 16.0, None, None, 32, dt, st)
+            L.pg_decode_attention_ex(ds.att.data_ptr(), ds.q.data_ptr(), eng.k_pool[li].data_ptr(), eng.v_pool[li].data_ptr(),
+                                     kv.page_table.data_ptr(), kv.max_pages, eng.page_size, eng.num_pages, kv.kv_len.data_ptr(), 1,
+                                     B, nq, d.nkv, d.hd, 16.0, None, None, None, 0, dt, st)
     rec("attention", attn, e * B * 2 * (T + 1) * d.nkv * d.hd)
 
     def oproj():
