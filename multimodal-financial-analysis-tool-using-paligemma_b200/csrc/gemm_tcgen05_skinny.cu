@@ -343,16 +343,20 @@ bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
   return M <= 64 ? K >= (epi == PG_EPI_NONE ? 4096 : 8192) : epi == PG_EPI_NONE && n_tiles >= 32 && K >= 4096;
 }
 
-int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
-                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st) {
-  const bool bf = dtype == PG_BF16;
-  const int nt = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
+// Split of K across a cluster until ~148 CTAs stream (each keeps >= 4 K blocks).  A CTA of a cluster of 4 takes an SM's whole shared
+// memory, and no more than 32 such clusters find room at once (N 4304, K 1152, 8 rows: 34 clusters 8.7 us, pairs 5.2)
+int gemm_tc_skinny_split(int N, int K, int epi) {
   const int n_tiles = cdiv(N, tc::SN_BM), kb = cdiv(K, tc::SN_BK);
-  // split K across a cluster until ~148 CTAs stream (each keeps >= 4 K blocks).  A CTA of a cluster of 4 takes an SM's whole
-  // shared memory, and no more than 32 such clusters find room at once (N 4304, K 1152, 8 rows: 34 clusters 11.3 us, pairs 7.7)
   int s = 1;
   if (epi != PG_EPI_GEGLU)
     while (s < 8 && n_tiles * s * 2 <= (s == 2 ? 128 : 160) && kb / (s * 2) >= 4) s *= 2;
+  return s;
+}
+
+int gemm_tc_skinny(void* C, const void* A, const void* W, const void* bias, const void* R, int M, int N, int K, int lda,
+                   int ldw, int ldc, int ldr, int epi, int out_f32, int dtype, bool w_param, cudaStream_t st) {
+  const bool bf = dtype == PG_BF16;
+  const int nt = M <= 32 ? 32 : (M <= 64 ? 64 : 128), s = gemm_tc_skinny_split(N, K, epi);
   CUtensorMap mx, mw;
   const int w_rows = (epi == PG_EPI_GEGLU) ? 2 * N : N;
   PG_REQUIRE(tc::make_map_2d(&mx, A, M, K, lda, nt, bf) && tc::make_map_2d(&mw, W, w_rows, K, ldw, tc::SN_BM, bf),

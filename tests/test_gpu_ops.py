@@ -525,7 +525,7 @@ def test_gemm_tcgen05_skinny_swap_ab(dtype, M, N, K, epi, monkeypatch):
 @pytest.mark.parametrize("M", [8, 32, 100, 129, 144, 260, 272, 300, 512])
 @pytest.mark.parametrize("N,K,epi", [(2560, 2048, "none"), (2048, 2048, "res"), (2048, 16384, "res"), (16384, 2048, "geglu"),
                                      (768, 2048, "none"), (1000, 1088, "res"), (2048, 4096, "geglu")])
-def test_gemm_tcgen05_prompt_rows_swapped_pairs(dtype, M, N, K, epi):
+def test_gemm_tcgen05_prompt_rows_swapped_pairs(gemm_workspace, dtype, M, N, K, epi):
     """Prompt-sized row counts (129..512: the 260-token prefill, the cache-off recompute up to 512 tokens; also the
     batched-decode rows 4..128 for the residual projections) take the
     CTA-pair kernel with the WEIGHTS as the M = 256 operand and all tokens in one or two accumulators, split along K
@@ -533,8 +533,6 @@ def test_gemm_tcgen05_prompt_rows_swapped_pairs(dtype, M, N, K, epi):
     tp 1 / tp 8 (768-row q/k/v shard) and ragged N / K tails.  Against torch in the same dtype."""
     if dtype == torch.float16 and M not in (260, 512):
         pytest.skip("fp16 on two row counts only")
-    ws = torch.empty(80 << 20, dtype=torch.uint8, device="cuda")
-    cabi.check(cabi.lib().pg_set_workspace(ws.data_ptr(), ws.numel()))
     a = gen(M, K, dtype=dtype)
     s = 1.0 / math.sqrt(K)
     w, w2 = gen(N, K, seed=1, scale=s, dtype=dtype), gen(N, K, seed=2, scale=s, dtype=dtype)

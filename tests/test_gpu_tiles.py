@@ -1,5 +1,6 @@
 """The tensor-core kernels at the edges of their tiles, clusters and splits, against float64 products of the same 16-bit
 operands with the rounding points of the epilogues."""
+import ctypes
 import math
 
 import pytest
@@ -82,32 +83,56 @@ def test_few_rows_split_over_clusters(M, N, K, epi, dtype):
     assert bool((out[M] == 0).all())
 
 
+def _route(L, M, N, K, epi, f32):
+    """The kernel that pg_gemm (impl 0) takes, by the library's own rules (C++ functions of namespace pg)."""
+    def rule(name, *args, kind=ctypes.c_bool):
+        f = getattr(L, f"_ZN2pg{len(name)}{name}E" + "i" * len(args))
+        f.argtypes, f.restype = [ctypes.c_int] * len(args), kind
+        return f(*args)
+    if rule("gemm_tc_swap_wanted", M, N, K, epi, f32, 0):
+        return "pairs"
+    if rule("gemm_stream_wanted", M, N, K, epi):
+        return "stream"
+    if rule("gemm_tc_skinny_wanted", M, N, K, epi):
+        return "skinny %d" % rule("gemm_tc_skinny_split", N, K, epi, kind=ctypes.c_int)
+    return "split %d" % rule("gemm_tc_splitk_factor", M, N, K, epi, kind=ctypes.c_int)
+
+
 # partial sums of a split over K change hands by whole row pieces: row tiles with missing rows, feature tiles with missing columns,
-# rows past 256 in a second token tile; results have the roundings of the products above, fp32 ones too (the type's values, widened)
+# every number of CTAs that share a tile, rows past 256 in a second token tile; results have the roundings of the products above, fp32
+# ones too (the type's values, widened)
 @pytest.mark.parametrize("dtype", TYPES)
-@pytest.mark.parametrize("impl,M,N,K,epi,f32", [
-    (0, 33, 1152, 4304, "res", 0), (0, 129, 1152, 1152, "none", 0), (0, 257, 1160, 4304, "res", 0), (0, 256, 1152, 4304, "res", 0),
-    (0, 260, 2048, 2048, "res", 0), (0, 385, 520, 4096, "none", 1), (0, 161, 2056, 2048, "none", 1),
-    (0, 5, 2048, 2048, "res", 0), (0, 32, 2056, 16384, "res", 0), (0, 17, 2048, 4096, "none", 1),
-    (3, 256, 264, 4096, "res", 0), (3, 257, 2048, 16384, "res", 0), (3, 271, 1000, 2048, "none", 0), (3, 273, 264, 4096, "res", 0),
-    (3, 384, 2056, 2048, "geglu", 0), (3, 511, 136, 8192, "res", 0)])
-def test_partial_sums_change_hands(impl, M, N, K, epi, f32, dtype):
+@pytest.mark.parametrize("route,M,N,K,epi,f32", [
+    ("split 4", 33, 1152, 4304, "res", 0), ("split 2", 129, 1152, 1152, "none", 0), ("split 4", 257, 1160, 4304, "bias_res", 0),
+    ("split 4", 256, 1152, 4304, "res", 0), ("split 2", 260, 2048, 2048, "res", 0), ("split 4", 353, 520, 4096, "none", 1),
+    ("split 2", 161, 2056, 2048, "none", 1), ("split 2", 384, 1152, 1152, "bias_gelu", 0), ("split 2", 65, 4304, 1152, "bias", 0),
+    ("skinny 8", 32, 2056, 16384, "res", 0), ("skinny 8", 17, 2048, 4096, "none", 1), ("skinny 8", 64, 2056, 8192, "res", 0),
+    ("skinny 4", 19, 3080, 2048, "none", 0), ("skinny 4", 31, 3080, 2048, "bias_res", 0), ("skinny 4", 50, 3080, 8192, "res", 0),
+    ("skinny 4", 25, 3080, 2048, "bias", 1), ("skinny 4", 20, 2432, 1280, "res", 0), ("skinny 2", 5, 9608, 512, "res", 0),
+    ("skinny 2", 18, 4304, 1152, "bias_gelu", 0), ("skinny 2", 30, 8200, 2048, "none", 1), ("skinny 2", 60, 8200, 4096, "none", 0),
+    ("pairs", 256, 264, 4096, "res", 0), ("pairs", 257, 2048, 16384, "res", 0), ("pairs", 271, 1000, 2048, "none", 0),
+    ("pairs", 273, 264, 4096, "res", 0), ("pairs", 384, 2056, 2048, "geglu", 0), ("pairs", 449, 2048, 8192, "res", 0),
+    ("pairs", 511, 136, 8192, "res", 0)])
+def test_partial_sums_change_hands(gemm_workspace, route, M, N, K, epi, f32, dtype):
     cabi, L, st = _cabi()
-    ws = torch.empty(80 << 20, dtype=torch.uint8, device="cuda")
-    cabi.check(L.pg_set_workspace(ws.data_ptr(), ws.numel()))
+    code, pairs = getattr(cabi, "EPI_" + epi.upper()), route == "pairs"
+    if not pairs:
+        cabi.check(L.pg_set_workspace(None, 0))
+        assert _route(L, M, N, K, code, f32) == route
     g = torch.Generator(device="cuda").manual_seed(M + N)
     rows = 2 * N if epi == "geglu" else N
     a, w = _randn(g, M, K, dtype=dtype), _randn(g, rows, K, std=K ** -0.5, dtype=dtype)
-    r = _randn(g, M, N, dtype=dtype)
+    r, b = _randn(g, M, N, dtype=dtype), _randn(g, N, dtype=dtype)
     out = torch.zeros((M + 1) * N, dtype=torch.float32 if f32 else dtype, device="cuda").view(M + 1, N)
-    code = {"res": cabi.EPI_RES, "none": cabi.EPI_NONE, "geglu": cabi.EPI_GEGLU}[epi]
-    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), None, r.data_ptr() if epi == "res" else None, M, N, K, K, K, N,
-                         N if epi == "res" else 0, 0, code, f32, impl, cabi.DTYPE_CODE[dtype], st))
-    z = a.to(F64) @ w.to(F64).T
-    want = _gelu(z[:, :N]) * z[:, N:] if epi == "geglu" else z + r.to(F64) if epi == "res" else z
-    assert _rel(out[:M], want) < _tol(dtype, 5e-3 if epi == "geglu" else 4e-3, epi == "geglu")
+    before = cabi.launch_count()
+    cabi.check(L.pg_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), b.data_ptr() if "bias" in epi else None,
+                         r.data_ptr() if "res" in epi else None, M, N, K, K, K, N, N if "res" in epi else 0, 0, code, f32,
+                         3 if pairs else 0, cabi.DTYPE_CODE[dtype], st))
+    assert cabi.launch_count() - before == (2 if pairs else 1)                 # the pairs' reduction is a launch of its own
+    z = a.to(F64) @ w.to(F64).T + (b.to(F64) if "bias" in epi else 0.0)
+    want = _gelu(z[:, :N]) * z[:, N:] if epi == "geglu" else _gelu(z) if "gelu" in epi else z + r.to(F64) if "res" in epi else z
+    assert _rel(out[:M], want) < _tol(dtype, 5e-3 if epi == "geglu" else 4e-3, "g" in epi)
     assert bool((out[M] == 0).all())
-    cabi.check(L.pg_set_workspace(None, 0))
 
 
 # More weight tiles than CTA pairs (74), the last of them of at most 128 features: a pair's second item, in which one CTA has nothing to
