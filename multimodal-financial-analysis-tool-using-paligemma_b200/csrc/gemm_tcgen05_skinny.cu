@@ -29,18 +29,6 @@ struct SnParams {
   int w_param;   // W is no output of a preceding launch: it may be requested before the dependency wait
 };
 
-__device__ __forceinline__ void sn_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 sn_ld_dsmem_v4(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-  return v;
-}
-
 template <bool DUAL, int NT, int S>
 constexpr int sn_stages() {
   constexpr int bytes = (DUAL ? 2 : 1) * SN_BM * SN_BK * 2 + (NT * SN_BK * 2 + 1023) / 1024 * 1024;
@@ -79,8 +67,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t crank = 0;
-  if (S > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+  const uint32_t crank = S > 1 ? cluster_rank() : 0;
   const int n_tiles = (p.N + SN_BM - 1) / SN_BM;
   const int k_blocks = (p.K + SN_BK - 1) / SN_BK, per = (k_blocks + S - 1) / S;
   const int kb0 = (int)crank * per, kb1 = min(k_blocks, kb0 + per);
@@ -244,7 +231,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       }
     }
     tc_fence_before();
-    sn_cluster_sync();
+    cluster_sync_all();
     float v[STEPS][4];
     if (warp >= 4) {
 #pragma unroll
@@ -253,7 +240,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
         for (int peer = 0; peer < S; ++peer) {        // all loads in flight before the first add
           const int at = (m0 + 4 * i) * PROW + f;
-          pv[peer] = peer == (int)crank ? *reinterpret_cast<const float4*>(part + at) : sn_ld_dsmem_v4(smem_base + (uint32_t)(at * 4), peer);
+          pv[peer] = peer == (int)crank ? *reinterpret_cast<const float4*>(part + at) : ld_dsmem_v4(smem_base + (uint32_t)(at * 4), peer);
         }
         v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
 #pragma unroll

@@ -60,10 +60,6 @@ __device__ __forceinline__ void sw_commit_cg2(uint32_t bar, uint16_t cta_mask) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(cta_mask) : "memory");
 }
-__device__ __forceinline__ void sw_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <int FMT>  // 1 bf16, 0 f16
 __global__ void __launch_bounds__(SW_THREADS, 1)
@@ -109,7 +105,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  sw_cluster_sync();  // the peer's barriers and TMEM exist before anything lands on them
+  cluster_sync_all();  // the peer's barriers and TMEM exist before anything lands on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
@@ -218,7 +214,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  sw_cluster_sync();  // the leader's MMAs read this CTA's shared memory, its commits arrive on this CTA's barriers
+  cluster_sync_all();  // the leader's MMAs read this CTA's shared memory, its commits arrive on this CTA's barriers
   if (warp == 2) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
