@@ -234,13 +234,15 @@ static int launch_stream_pick(const StreamParams& p, cudaStream_t st) {
 }
 
 // One group a CTA (N up to 2368): up to 16 rows always, up to 32 where the two chunks of K 2048 hold their tokens (us, weights out of
-// HBM, the tiles of 128 rows and this: 8 rows, N 2048 and K 16384 15.6 and 13.2, N 1024 and K 4096 6.2 and 4.2, N 128 and K 128 3.0 and
-// 1.6; 16 rows 16.3 and 15.1; 32 rows, N = K = 2048 7.6 and 4.8; 32 rows of K 16384 17.9 and 25.1).  Several groups, up to 4 (behind
+// HBM, the tiles of 128 rows and this: 8 rows, N 2048 and K 16384 16.5 and 14.0, N 1024 and K 4096 5.6 and 4.2, N 128 and K 128 3.0 and
+// 1.6; 16 rows of K 16384 16.6 and 15.9; 32 rows, N = K = 2048 4.9 and 4.8; 32 rows of K 16384 16.8 and 22).  Several groups, up to 4 (behind
 // them the tiles' own stream is as even: gate/up of 16384 features 22.2 and 22.5), and up to 16 rows whose columns leave the loads in
-// flight their L1: from K 512 on (8 rows, N 8192: K 512 5.3 and 4.9, but K 448 3.8 and 4.9, where the warps of a CTA whose columns lie
+// flight their L1: from K 512 on (8 rows, N 8192: K 512 4.8 and 4.9, but K 448 3.8 and 4.9, where the warps of a CTA whose columns lie
 // behind K only wait), up to K 3072 for 8 rows and K 5120 for more, whose second block of tokens the tiles pay for as well; at 4 groups 1024
-// less (8 rows, N 2560: K 2048 6.2 and 4.5, 3072 6.9 and 6.2, 3584 7.4 and 7.9; N 8192: K 2048 9.8 and 9.3, 2560 10.7 and 12.2; 12 rows,
-// N 2560: K 4096 8.4 and 7.5, 5120 9.5 and 8.8, 8192 12.7 and 12.7).
+// less (8 rows, N 2560: K 2048 5.5 and 4.6, 3584 6.8 and 8.0; N 8192: K 2048 9.7 and 9.8, 2560 10.9 and 12.6).  The upper lines were drawn
+// when the tiles handed their sums round in four times the time; they are ahead of this a little below them now (8 rows, N 2560,
+// K 3072 6.1 and 6.4; 12 rows, N 2560: K 3072 6.1 and 6.6, 5120 8.8 and 9.1; 16 rows, N 8192, K 512 4.9 and 5.6), which the rule does not
+// use yet.
 bool gemm_stream_wanted(int M, int N, int K, int epi) {
   if (M < 4 || M > 32 || epi < PG_EPI_NONE || epi > PG_EPI_RES) return false;
   const int groups = cdiv(cdiv(N, stream_grid(N)), 16);

@@ -3,17 +3,16 @@
 // A operand of tcgen05.mma and the tokens are the N dimension (N_mma = M rounded up to 16).  A pipeline stage is
 // then 16 KB of weights + a few KB of activations, so 8-10 stages (~150 KB of weights) are in flight per SM —
 // what a 6 TB/s stream needs — instead of the 16 KB-activation/8 KB-weight stages of the row-major kernel.
-// The accumulator is D^T: TMEM lane = output feature, column = token, so bias is a per-thread scalar and the
-// stores are coalesced across the warp (consecutive features of one token).
+// The accumulator is D^T: TMEM lane = output feature, column = token.
 //   S == 1 : persistent over the N/128 weight tiles (gate/up with the GeGLU pairing, lm_head), double-buffered
-//            accumulators so the epilogue overlaps the next tile's stream;
+//            accumulators so the epilogue overlaps the next tile's stream; a thread keeps its feature, so bias is one scalar
+//            and the stores are coalesced across the warp (consecutive features of one token);
 //   S  > 1 : a cluster of S CTAs splits K for one weight tile (q/k/v, o_proj, down_proj have 16-20 tiles only).  Every CTA
-//            leaves its partial D^T in its shared memory and finishes the S-th part of the tokens from all of them
-//            (distributed shared memory, summed in rank order).  With S = 8 a CTA keeps to half an SM's shared memory:
-//            clusters of 8 whole SMs do not all fit the GPCs at once.
-// o_proj and down_proj (K 2048 and 16384) together, launches alone with a cold cache: the pair kernel with a workspace and a
-// reduce launch each (gemm_tcgen05_swap.cu) 41.5 us for 8 rows and 42.4 for 32, this 29.0 and 33.3; 10 and 5 us per layer of
-// a captured step.
+//            leaves its partial tile in its shared memory, a row per token, and finishes the S-th part of the tokens from all
+//            of them, four neighbouring features a lane (distributed shared memory, summed in rank order).  With S = 8 a CTA
+//            keeps to half an SM's shared memory: clusters of 8 whole SMs do not all fit the GPCs at once.
+// o_proj and down_proj (K 2048 and 16384) together, weights out of HBM: the pair kernel with a workspace and a reduce launch each
+// (gemm_tcgen05_swap.cu) 25.4 us for 8 rows and 26.3 for 32, this 21.6 and 22.0.
 #include "tc_common.cuh"
 
 namespace pg {
@@ -199,8 +198,8 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int tile = tile_first;
     const bool have_k = kb1 > kb0;
     // This CTA finishes NC of the tokens: a warp one of them at a time, four neighbouring features a lane.  (A feature's row per lane
-    // made every load of a warp 32 lines of the peer's shared memory: 32 rows, N 2048, K 16384 by 8 20.4 us, now 17.3; N 2560, K 2048
-    // 8.7, now 5.4.)
+    // made every load of a warp 32 lines of the peer's shared memory: 32 rows, N 2048, K 16384 by 8 19.6 us, now 16.8; N 2560, K 2048
+    // 8.7, now 5.6.)  All NC tokens go round, whether the matrix has them or not: 17 rows cost what 32 do.
     constexpr int NC = NT / S, STEPS = NC / 4;
     const int m0 = (int)crank * NC + (warp & 3), f = 4 * lane, n = tile * SN_BM + f;
     constexpr bool HAS_BIAS = EPI == PG_EPI_BIAS || EPI == PG_EPI_BIAS_GELU || EPI == PG_EPI_BIAS_RES;
@@ -317,11 +316,13 @@ static int launch_sn_nt(const CUtensorMap& mx, const CUtensorMap& mw, const SnPa
 }  // namespace tc
 
 bool gemm_tc_skinny_wanted(int M, int N, int K, int epi) {
-  // Up to 32 rows the swap-AB stream takes every projection that gemm_stream.cu leaves (gate/up 26.6 vs 29.0 us, lm_head 181 vs 211 us,
-  // q/k/v 9.9 vs 18.3 us on the row-major kernel).  Up to 64 rows it does so for long K; with K 2048 its token-heavy stages and the merge of 64 columns
-  // cost more than the stream gains (64 rows, weights out of HBM: N 2560 13.8 us, the row-major kernel 11.9; N 2048 with a
-  // residual 11.5, the pair kernel 10.2; N 1152, K 4304 13.2, row-major 10.9).  Above, only where CTAs own whole weight tiles or
-  // there are 32 of them (128 rows: N = K = 4096 16.1 us, row-major 17.2; N 2560, K 2048 21.6 and 11.9).
+  // Weights out of HBM, this and the split row-major kernel, us.  Up to 32 rows the swap-AB stream takes every projection that
+  // gemm_stream.cu leaves (32 rows: gate/up 28.0 and 31.1, lm_head 172 and 184, N 2560, K 2048 5.6 and 7.0).  Up to 64 rows it does
+  // so for long K (64 rows, N 2048, K 8192 12.1 and 15.5).  The line at K was drawn when the merge of 64 columns cost four times
+  // what it does now (N 2560, K 2048 13.8 and 11.9 then); today this kernel would be ahead below it too (6.9 and 7.7; N 1152, K 4304
+  // 8.3 and 9.6, the pair kernel that takes it 9.0; N = K = 2048 with a residual 6.4 and 7.2, the pair kernel 8.0), which the rule does not use
+  // yet.  Above, only where CTAs own whole weight tiles or there are 32 of them (128 rows: N = K = 4096 12.6 and 13.3; N 2560, K 2048
+  // 11.4 and 9.2).
   static const int mode = env_int("PG_SKINNY", 1);   // 0 off, 1 where it wins, 2 everywhere it applies
   if (!mode || M < 4 || M > 128 || N < 512 || K < 256 || epi < PG_EPI_NONE || epi > PG_EPI_GEGLU) return false;
   if (mode == 2) return true;

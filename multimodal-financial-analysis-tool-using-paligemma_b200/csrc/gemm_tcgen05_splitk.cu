@@ -218,12 +218,12 @@ static int launch_sk_pick(const CUtensorMap& ma, const CUtensorMap& mw, const Sk
 }  // namespace tc
 
 // Split factor for a problem (0 = do not split): up to three m-tiles whose 64-wide tiles leave room for the split within one
-// wave of two CTAs per SM, and at least 8 K blocks per CTA.  One image's encode (256 rows: every GEMM
-// of its layers; unsplit but for fc2 before) 625 -> 577 us, a 260-token prompt with its image 5021 -> 4915 us.  By 4 with fewer
-// than 16 K blocks a CTA, the second CTA of an SM costs more than the halved chain gains (256 rows, N = K = 2048, weights out of
-// HBM: 12.6 us, by 2 11.4).  By 2 it pays in a chain, for the weights that are on their way early, although a row of equal
-// products is no faster (N 3456, K 1152 by 2 10.0 us, whole 9.6; but one image's encode 544 and 558 us).  Gated pairings stay
-// out: two accumulators a tile already fill the wave.
+// wave of two CTAs per SM, and at least 8 K blocks per CTA.  256 rows, weights out of HBM, whole and split, us: N 3456, K 1152
+// 8.2 and 7.8; N = K = 2048 13.3 and 10.0; N 1152, K 4304 23.3 and 12.9.  By 4 with fewer than 16 K blocks a CTA only while three
+// quarters of a wave are left free: the second CTA of an SM then gave away what the halved chain gains (256 rows, N = K = 2048: by 4
+// 12.6, by 2 11.4 us, when a row of a peer's tile was read by one lane; by whole row pieces 9.7 and 10.0, within what two runs
+// differ, so the line stands).  The limit of three m-tiles is from that time too: beyond it (385 rows: N = K = 2048 13.4 us whole,
+// N 1152, K 4304 23.3) no split has been measured.  Gated pairings stay out: two accumulators a tile already fill the wave.
 int gemm_tc_splitk_factor(int M, int N, int K, int epi) {
   static const int mode = env_int("PG_SPLITK", -1);   // 0 never, 2 / 4: that factor wherever it fits
   if (mode == 0 || epi == PG_EPI_GEGLU || epi == PG_EPI_SWIGLU || M > 3 * tc::SK_BM) return 0;

@@ -15,7 +15,10 @@
 //     gemm_swap_reduce_kernel sums the splits and applies the epilogue (residual / GeGLU / rounding points of
 //     gemm_simt.cu) with fully coalesced rows.
 // Roles per CTA (as gemm_tcgen05_2cta.cu): warp 0 TMA producer, warp 1 (leader CTA) MMA issuer, warp 2 TMEM
-// allocation, warps 4-11 epilogue (TMEM -> fp32 partial rows).
+// allocation, warps 4-11 epilogue (TMEM -> 16 tokens x 128 features in shared memory -> fp32 partial sums by TMA store).
+// The four staging buffers take 32 KB of the ring: 5 stages of 33 KB at 260 rows, 3 of 47 to 48 KB from 481 rows on (6 and 4 without).
+// With them, down_proj (N 2048, K 16384), us: 129 rows 25.0 -> 20.3, 260 33.0 -> 26.4, 384 38.0 -> 31.0, 448 41.0 -> 33.7,
+// 512 44.4 -> 38.9; N 640 at 512 rows 28.9 -> 20.5.
 #include "tc_common.cuh"
 
 namespace pg {
@@ -326,9 +329,11 @@ bool gemm_tc_swap_wanted(int M, int N, int K, int epi, int out_f32, int res_mod)
   if (epi != PG_EPI_NONE && epi != PG_EPI_RES && epi != PG_EPI_GEGLU) return false;
   // which projections take this kernel (measured per projection): bit 0 q/k/v (no epilogue),
   // bit 1 o_proj (residual, K < 8192), bit 2 down_proj (residual, K >= 8192), bit 3 gate/up (GeGLU)
-  // measured: prompt-sized rows (129..512) -- down_proj only (prefill 4.16 -> 3.45 ms; q/k/v, o_proj and gate/up are
-  // faster on the row-major kernels); batched-decode rows (33..128) -- o_proj and down_proj (up to 32 rows, and up to 64 with
-  // a long K, the cluster split of gemm_tcgen05_skinny.cu is faster: it needs no workspace round trip)
+  // measured, us, weights out of HBM: prompt-sized rows (129..512) -- down_proj only (260 rows: 26.2, split over clusters 46.4; but
+  // q/k/v 12.9 and 9.8, o_proj 12.3 and 10.0, gate/up 54 and 38 on the row-major kernels); batched-decode rows (33..128) -- o_proj
+  // and down_proj (128 rows: o_proj 8.7 and 8.8, N 1152, K 4304 9.3 and 10.9, down_proj 20.3 and 28.3; at 64 rows o_proj 8.0, split by 4
+  // 7.2 since its exchange is faster, which the rule does not use yet).  Up to 32 rows, and up to 64 with a long K, the cluster split
+  // of gemm_tcgen05_skinny.cu is faster: it needs no workspace round trip (32 rows: 5.0 and 7.4, K 16384 16.8 and 18.9)
   static const int mask_large = env_int("PG_SWAP_MASK", 4), mask_small = env_int("PG_SWAP_MASK_SMALL", 6);
   if ((M <= 32 || (M <= 64 && K >= 8192)) && !g_force_swap) return false;
   const int mask = M > 128 ? mask_large : mask_small;
