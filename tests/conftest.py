@@ -43,5 +43,5 @@ def gemm_workspace():
     cabi.check(L.pg_set_workspace(ws.data_ptr(), ws.numel()))
     yield ws
     torch.cuda.synchronize()
-    own = _WORKSPACES.get((torch.cuda.current_device(),))
-    cabi.check(L.pg_set_workspace(own.data_ptr(), own.numel()) if own is not None else L.pg_set_workspace(None, 0))
+    own = [w for w in _WORKSPACES.values() if w.device.index == torch.cuda.current_device()]   # the engines' key may name no index
+    cabi.check(L.pg_set_workspace(own[-1].data_ptr(), own[-1].numel()) if own else L.pg_set_workspace(None, 0))
